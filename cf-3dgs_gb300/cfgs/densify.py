@@ -84,18 +84,18 @@ class GaussianOptimizer:
         rows = keep + clone + 2 * child
         xyz, scaling, rotation = self.params["xyz"], self.params["scaling"], self.params["rotation"]
 
-        def write(src: torch.Tensor, role: int) -> torch.Tensor:
-            w = src[0].numel() if src.shape[0] else int(math.prod(src.shape[1:]))
-            out = torch.empty((rows,) + tuple(src.shape[1:]), dtype=torch.float32, device=dev)
-            if n > 0 and rows > 0:
-                native.check(lib.cfgs_densify_write(n, _ptr(ws), counts, int(w), _ptr(src), out.data_ptr(),
-                                                    role, _ptr(xyz), _ptr(scaling), _ptr(rotation), _ptr(z), st),
-                             "cfgs_densify_write")
-            return out
-
-        new_params = {k: write(v, {"xyz": 2, "scaling": 3}.get(k, 0)) for k, v in self.params.items()}
-        self.exp_avg = {k: write(v, 1) for k, v in self.exp_avg.items()}
-        self.exp_avg_sq = {k: write(v, 1) for k, v in self.exp_avg_sq.items()}
+        # every array of the new model in one call: the parameters, then the two Adam moments
+        src = [d[k] for d in (self.params, self.exp_avg, self.exp_avg_sq) for k in GROUPS]
+        roles = [{"xyz": 2, "scaling": 3}.get(k, 0) for k in GROUPS] + [1] * (2 * len(GROUPS))
+        out = [torch.empty((rows,) + tuple(t.shape[1:]), dtype=torch.float32, device=dev) for t in src]
+        if n > 0 and rows > 0:
+            widths = [int(math.prod(t.shape[1:])) for t in src]
+            native.check(lib.cfgs_densify_write_many(n, _ptr(ws), counts, len(src), (C.c_int32 * len(src))(*widths),
+                                                     _vp_array([_ptr(t) for t in src]),
+                                                     _vp_array([t.data_ptr() for t in out]),
+                                                     (C.c_int32 * len(src))(*roles), _ptr(xyz), _ptr(scaling),
+                                                     _ptr(rotation), _ptr(z), st), "cfgs_densify_write_many")
+        new_params, self.exp_avg, self.exp_avg_sq = (dict(zip(GROUPS, out[6 * i:6 * i + 6])) for i in range(3))
         self.params = new_params
         self.grad_accum = torch.zeros(rows, dtype=torch.float32, device=dev)
         self.denom = torch.zeros(rows, dtype=torch.float32, device=dev)

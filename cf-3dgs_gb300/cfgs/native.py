@@ -142,6 +142,8 @@ EXPORTS = {
                                     C.c_int32, _vp, _vp, _vp]),
     "cfgs_densify_write": (C.c_int, [C.c_int64, _vp, _vp, C.c_int32, _vp, _vp, C.c_int32, _vp, _vp, _vp, _vp,
                                      _vp]),
+    "cfgs_densify_write_many": (C.c_int, [C.c_int64, _vp, _vp, C.c_int32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
+                                          _vp]),
     "cfgs_depth_to_points": (C.c_int, [C.c_int32, C.c_int32, _vp, C.c_float, C.c_float, C.c_float, C.c_float, _vp,
                                        _vp]),
     "cfgs_pointcloud_workspace_bytes": (C.c_size_t, [C.c_int64]),

@@ -378,6 +378,12 @@ int cfgs_densify_plan(int64_t num_gaussians, const float* grad_accum, const floa
 int cfgs_densify_write(int64_t num_gaussians, void* workspace, const int64_t counts[4], int32_t width,
                        const float* in, float* out, int32_t role, const float* xyz, const float* scaling,
                        const float* rotation, const float* z, void* stream);
+/* cfgs_densify_write for up to 24 arrays (widths, in, out and roles are host arrays of
+ * num_arrays entries; at most one array each of roles 2 and 3) in one call. */
+int cfgs_densify_write_many(int64_t num_gaussians, void* workspace, const int64_t counts[4], int32_t num_arrays,
+                            const int32_t* widths, const float* const* in, float* const* out, const int32_t* roles,
+                            const float* xyz, const float* scaling, const float* rotation, const float* z,
+                            void* stream);
 
 /* ---- batched pose solves ----------------------------------------------------------
  * Many CF-3DGS pose solves (trainer/cf3dgs_trainer.py:261-285), each with its own
