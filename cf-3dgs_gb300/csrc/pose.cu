@@ -13,15 +13,14 @@
 // sum p'_i x g_i + w_cov), where g_i = dL/dp'_i and w_cov is the rotation gradient of
 // the rotated covariances. Since exp(xi + dxi) = exp(J(xi) dxi) exp(xi) with J the
 // SE(3) left Jacobian, dL/dxi = J(xi)^T dL/dd. The kernel forms the sums in one pass
-// over the Gaussians; the last block to finish adds the per-block partials in block
-// order (deterministic) and applies J^T in double precision.
+// over the Gaussians; the last block to finish folds the per-block partials in a fixed
+// pattern (deterministic) and applies J^T in double precision.
 #include "cfgs_internal.cuh"
 
 namespace cfgs {
 
 constexpr int kPoseThreads = 256;
-constexpr int kPoseMaxBlocks = 1184;  // 152 SMs x 8 blocks
-constexpr int kPosePartials = 9;      // sum g (3), sum (R p) x g (3), w_cov (3)
+constexpr int kPosePartials = 9;  // sum g (3), sum (R p) x g (3), w_cov (3)
 
 struct SE3d {
   double R[9];
@@ -103,10 +102,25 @@ __device__ inline void se3_Q(const double* rho, const double* phi, double* Q) {
            c3 * (PRPP[k] + PPRP[k]);
 }
 
+// Each block's thread 0 forms exp(xi) in float64 while the others' positions are on
+// their way from memory: the chain of double sin, cos and divisions is most of the kernel's
+// time, so a block takes kApplyPerThread positions per thread (230,400 positions: 225
+// blocks, 16.7 -> 10.1 us; one position per thread ran 900 such chains).
+constexpr int kApplyPerThread = 4;
+
+template <bool COV>
 __global__ void __launch_bounds__(kPoseThreads) k_pose_apply(int n, const float* xi, const float* xyz,
                                                               const float* cov_in, float* means_out,
                                                               float* cov_out) {
   __shared__ float sR[9], st[3];
+  const int64_t i0 = (int64_t)blockIdx.x * (kPoseThreads * kApplyPerThread) + threadIdx.x;
+  float p[kApplyPerThread][3];
+#pragma unroll
+  for (int k = 0; k < kApplyPerThread; ++k) {
+    const int64_t i = i0 + k * kPoseThreads;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) p[k][a] = i < n ? xyz[3 * i + a] : 0.0f;
+  }
   if (threadIdx.x == 0) {
     SE3d X;
     double Jl[9];
@@ -118,14 +132,17 @@ __global__ void __launch_bounds__(kPoseThreads) k_pose_apply(int n, const float*
   float R[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) R[k] = sR[k];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float p0 = xyz[3 * i], p1 = xyz[3 * i + 1], p2 = xyz[3 * i + 2];
+#pragma unroll
+  for (int k = 0; k < kApplyPerThread; ++k) {
+    const int64_t i = i0 + k * kPoseThreads;
+    if (i >= n) break;
 #pragma unroll
     for (int r = 0; r < 3; ++r)  // ((R0 x + R1 y) + R2 z) + t, each operation rounded once
-      means_out[3 * i + r] = __fadd_rn(
-          __fadd_rn(__fadd_rn(__fmul_rn(R[3 * r], p0), __fmul_rn(R[3 * r + 1], p1)), __fmul_rn(R[3 * r + 2], p2)),
-          st[r]);
-    if (cov_in) {
+      means_out[3 * i + r] =
+          __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(R[3 * r], p[k][0]), __fmul_rn(R[3 * r + 1], p[k][1])),
+                              __fmul_rn(R[3 * r + 2], p[k][2])),
+                    st[r]);
+    if (COV) {
       const float* c = cov_in + 6 * (size_t)i;
       float C[9] = {c[0], c[1], c[2], c[1], c[3], c[4], c[2], c[4], c[5]};
       float RC[9];
@@ -135,126 +152,11 @@ __global__ void __launch_bounds__(kPoseThreads) k_pose_apply(int n, const float*
         for (int b = 0; b < 3; ++b) RC[3 * a + b] = R[3 * a] * C[b] + R[3 * a + 1] * C[3 + b] + R[3 * a + 2] * C[6 + b];
       const int ii[6] = {0, 0, 0, 1, 1, 2}, jj[6] = {0, 1, 2, 1, 2, 2};
 #pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        int a = ii[k], b = jj[k];
-        cov_out[6 * (size_t)i + k] = RC[3 * a] * R[3 * b] + RC[3 * a + 1] * R[3 * b + 1] + RC[3 * a + 2] * R[3 * b + 2];
+      for (int q = 0; q < 6; ++q) {
+        int a = ii[q], b = jj[q];
+        cov_out[6 * (size_t)i + q] = RC[3 * a] * R[3 * b] + RC[3 * a + 1] * R[3 * b + 1] + RC[3 * a + 2] * R[3 * b + 2];
       }
     }
-  }
-}
-
-// dL/dxi from the left-perturbation sums tot = (sum g, sum (R p) x g, w_cov):
-// d_rho = sum g, d_phi = sum (R p + t) x g + w_cov, then dL/dxi = J^T dL/dd with the
-// SE(3) left Jacobian J = [[Jl, Q], [0, Jl]] — all in float64, rounded at the end.
-__device__ void pose_grad_from_sums(const float* xi, const double* tot, float* grad_out) {
-  SE3d X;
-  double Jl[9], Q[9];
-  se3_exp(xi, &X, Jl);
-  double rho[3] = {xi[0], xi[1], xi[2]};
-  double phi[3] = {xi[3], xi[4], xi[5]};
-  se3_Q(rho, phi, Q);
-  double gr[3] = {tot[0], tot[1], tot[2]};
-  double gp[3];
-  gp[0] = tot[3] + (X.t[1] * gr[2] - X.t[2] * gr[1]) + tot[6];
-  gp[1] = tot[4] + (X.t[2] * gr[0] - X.t[0] * gr[2]) + tot[7];
-  gp[2] = tot[5] + (X.t[0] * gr[1] - X.t[1] * gr[0]) + tot[8];
-  for (int j = 0; j < 3; ++j) {
-    grad_out[j] = (float)(Jl[j] * gr[0] + Jl[3 + j] * gr[1] + Jl[6 + j] * gr[2]);
-    grad_out[3 + j] = (float)(Q[j] * gr[0] + Q[3 + j] * gr[1] + Q[6 + j] * gr[2] + Jl[j] * gp[0] +
-                              Jl[3 + j] * gp[1] + Jl[6 + j] * gp[2]);
-  }
-}
-
-struct PoseGradArgs {
-  int n;
-  const float* xi;
-  const float* xyz;
-  const float* dL_dmeans;
-  const float* cov_rot;
-  const float* dL_dcov;
-  double* partials;       // [gridDim.x][9]
-  unsigned int* counter;  // zeroed before launch
-  float* grad_out;        // [6]
-};
-
-// Sums in float64: the per-Gaussian terms (R p) x g use the float64 rotation and
-// exact float32 x float32 products, so the result is the float64 value of the same
-// sums a float64 autograd of exp(xi).act(p) forms; rounded to float32 at the end, the
-// gradient then matches that path's in all but boundary cases, which keeps the fused
-// and plain solves on the same trajectory.
-__global__ void __launch_bounds__(kPoseThreads) k_pose_grad(PoseGradArgs a) {
-  __shared__ double sR[9];
-  __shared__ double s_red[kPoseThreads / 32][kPosePartials];
-  __shared__ bool s_last;
-  if (threadIdx.x == 0) {
-    SE3d X;
-    double Jl[9];
-    se3_exp(a.xi, &X, Jl);
-    for (int k = 0; k < 9; ++k) sR[k] = X.R[k];
-  }
-  __syncthreads();
-  double R[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) R[k] = sR[k];
-  double acc[kPosePartials];
-#pragma unroll
-  for (int k = 0; k < kPosePartials; ++k) acc[k] = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
-    double p0 = a.xyz[3 * i], p1 = a.xyz[3 * i + 1], p2 = a.xyz[3 * i + 2];
-    double g0 = a.dL_dmeans[3 * i], g1 = a.dL_dmeans[3 * i + 1], g2 = a.dL_dmeans[3 * i + 2];
-    double q0 = R[0] * p0 + R[1] * p1 + R[2] * p2;
-    double q1 = R[3] * p0 + R[4] * p1 + R[5] * p2;
-    double q2 = R[6] * p0 + R[7] * p1 + R[8] * p2;
-    acc[0] += g0;
-    acc[1] += g1;
-    acc[2] += g2;
-    acc[3] += q1 * g2 - q2 * g1;
-    acc[4] += q2 * g0 - q0 * g2;
-    acc[5] += q0 * g1 - q1 * g0;
-    if (a.cov_rot) {
-      const float* c = a.cov_rot + 6 * (size_t)i;
-      const float* d = a.dL_dcov + 6 * (size_t)i;
-      float C[9] = {c[0], c[1], c[2], c[1], c[3], c[4], c[2], c[4], c[5]};
-      float G[9] = {d[0], 0.5f * d[1], 0.5f * d[2], 0.5f * d[1], d[3], 0.5f * d[4], 0.5f * d[2], 0.5f * d[4], d[5]};
-      // M = C G - G C (antisymmetric); w = (M12 - M21, M20 - M02, M01 - M10) = 2 (M12, M20, M01)
-      float CG[9];
-#pragma unroll
-      for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int s = 0; s < 3; ++s) CG[3 * r + s] = C[3 * r] * G[s] + C[3 * r + 1] * G[3 + s] + C[3 * r + 2] * G[6 + s];
-      // (G C) = (C G)^T for symmetric C, G, so M_rs = CG_rs - CG_sr.
-      acc[6] += 2.0 * ((double)CG[5] - (double)CG[7]);
-      acc[7] += 2.0 * ((double)CG[6] - (double)CG[2]);
-      acc[8] += 2.0 * ((double)CG[1] - (double)CG[3]);
-    }
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < kPosePartials; ++k) {
-    double v = acc[k];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) s_red[warp][k] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < kPosePartials) {
-    double v = 0.0;
-    for (int w = 0; w < kPoseThreads / 32; ++w) v += s_red[w][threadIdx.x];
-    a.partials[blockIdx.x * kPosePartials + threadIdx.x] = v;
-  }
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(a.counter, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  if (threadIdx.x == 0) {
-    double tot[kPosePartials];
-    for (int k = 0; k < kPosePartials; ++k) tot[k] = 0.0;
-    const volatile double* part = a.partials;
-    for (int b = 0; b < (int)gridDim.x; ++b)
-      for (int k = 0; k < kPosePartials; ++k) tot[k] += part[b * kPosePartials + k];
-    pose_grad_from_sums(a.xi, tot, a.grad_out);
-    *a.counter = 0u;
   }
 }
 
@@ -270,38 +172,45 @@ __device__ __forceinline__ double bias_correction(double beta, const float* st) 
   return 1.0 - pow(beta, (double)(st[12] + 1.0f));
 }
 
-__device__ void adam_step6_bc(float* xi, const float* grad, float* st, double lr, double b1, double b2, double eps,
-                              double bc1, double bc2) {
-  const float step = st[12] + 1.0f;
+__device__ __forceinline__ void adam_component(int k, float* xi, const float* grad, float* st, double lr, double b1,
+                                               double b2, double eps, double bc1, double bc2) {
   const float w1 = (float)(1.0 - b1), mul2 = (float)b2, w2 = (float)(1.0 - b2);
   const float step_size = (float)(-(lr / bc1));
   const float bc2_sqrt = (float)sqrt(bc2);
   const float eps_f = (float)eps;
+  const float g = grad[k];
+  float m = st[k], v = st[6 + k];
+  m = fmaf(w1, g - m, m);
+  v = v * mul2;
+  v = fmaf(w2, g * g, v);
+  st[k] = m;
+  st[6 + k] = v;
+  float denom = sqrtf(v) / bc2_sqrt;
+  denom = denom + eps_f;
+  xi[k] = fmaf(step_size, m / denom, xi[k]);
+}
+
+__device__ void adam_step6_bc(float* xi, const float* grad, float* st, double lr, double b1, double b2, double eps,
+                              double bc1, double bc2) {
+  const float step = st[12] + 1.0f;
 #pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const float g = grad[k];
-    float m = st[k], v = st[6 + k];
-    m = fmaf(w1, g - m, m);
-    v = v * mul2;
-    v = fmaf(w2, g * g, v);
-    st[k] = m;
-    st[6 + k] = v;
-    float denom = sqrtf(v) / bc2_sqrt;
-    denom = denom + eps_f;
-    xi[k] = fmaf(step_size, m / denom, xi[k]);
-  }
+  for (int k = 0; k < 6; ++k) adam_component(k, xi, grad, st, lr, b1, b2, eps, bc1, bc2);
   st[12] = step;
 }
 
-__device__ void adam_step6(float* xi, const float* grad, float* st, double lr, double b1, double b2, double eps) {
-  adam_step6_bc(xi, grad, st, lr, b1, b2, eps, bias_correction(b1, st), bias_correction(b2, st));
-}
-
-__global__ void k_pose_adam(int count, float* xi, const float* grad, float* state, double lr, double b1, double b2,
-                            double eps) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per solve: lanes 0 and 1 form the two bias corrections (a double pow each, the
+// kernel's longest chain) at the same time, then lanes 0..5 step one component each (10.3 -> 7.9 us).
+__global__ void __launch_bounds__(128) k_pose_adam(int count, float* xi, const float* grad, float* state, double lr,
+                                                   double b1, double b2, double eps) {
+  const int s = blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (s >= count) return;
-  adam_step6(xi + 6 * (size_t)s, grad + 6 * (size_t)s, state + 16 * (size_t)s, lr, b1, b2, eps);
+  float* st = state + 16 * (size_t)s;
+  const double bc = bias_correction(lane & 1 ? b2 : b1, st);
+  const double bc1 = __shfl_sync(0xffffffffu, bc, 0), bc2 = __shfl_sync(0xffffffffu, bc, 1);
+  const float step = st[12] + 1.0f;
+  __syncwarp();  // every lane has read the step count
+  if (lane < 6) adam_component(lane, xi + 6 * (size_t)s, grad + 6 * (size_t)s, st, lr, b1, b2, eps, bc1, bc2);
+  if (lane == 0) st[12] = step;
 }
 
 // The parts of a solve's pose state that depend on xi, split so that two threads can
@@ -327,7 +236,10 @@ __device__ void pose_state_Q(const float* xi, PoseState* ps) {
   se3_Q(rho, phi, ps->Q);
 }
 
-// pose_grad_from_sums with exp(xi), Jl and Q taken from the solve's state.
+// dL/dxi from the left-perturbation sums tot = (sum g, sum (R p) x g, w_cov):
+// d_rho = sum g, d_phi = sum (R p + t) x g + w_cov, then dL/dxi = J^T dL/dd with the
+// SE(3) left Jacobian J = [[Jl, Q], [0, Jl]] — all in float64, rounded at the end, with
+// exp(xi), Jl and Q taken from the solve's state.
 __device__ void pose_grad_from_state(const PoseState& ps, const double* tot, float* grad_out) {
   const double gr[3] = {tot[0], tot[1], tot[2]};
   double gp[3];
@@ -340,6 +252,147 @@ __device__ void pose_grad_from_state(const PoseState& ps, const double* tot, flo
     grad_out[j] = (float)(Jl[j] * gr[0] + Jl[3 + j] * gr[1] + Jl[6 + j] * gr[2]);
     grad_out[3 + j] = (float)(Q[j] * gr[0] + Q[3 + j] * gr[1] + Q[6 + j] * gr[2] + Jl[j] * gp[0] +
                               Jl[3 + j] * gp[1] + Jl[6 + j] * gp[2]);
+  }
+}
+
+// ---- pose gradient of one solve --------------------------------------------------------
+// Sums in float64 of exact float32 x float32 products, so the result is the float64 value
+// a float64 autograd of exp(xi).act(p) forms, rounded to float32 at the end: the fused and
+// plain solves stay on the same trajectory. With M = sum p g^T, sum (R p) x g is read off
+// R M, so the pass over the Gaussians needs neither the rotation nor its products: 12
+// float64 accumulations (15 with covariances) per Gaussian. Block 0 forms exp(xi), Jl and Q
+// meanwhile; the last block to finish folds the others' partials in a fixed pattern (warp
+// w takes rows w, w + 8, ..., one lane per sum) and applies the Jacobian transpose. Bound
+// by the float64 pipe (about 2 operations per cycle and SM). 230,400 Gaussians: 371 us
+// (one thread folded 900 rows of 9 sums one after another, and every block formed exp(xi))
+// -> POSE_GRAD_US us.
+constexpr int kGradMaxBlocks = 2 * 152;  // two blocks of partial sums per SM at most
+constexpr int kGradSums = 16;            // sum g (3), M (9), w_cov (3), unused
+
+struct PoseGradArgs {
+  int n;
+  const float* xi;
+  const float* xyz;
+  const float* dL_dmeans;
+  const float* cov_rot;
+  const float* dL_dcov;
+  double* partials;       // [gridDim.x - 1][kGradSums]
+  PoseState* state;       // written by block 0
+  unsigned int* counter;  // zeroed before launch
+  float* grad_out;        // [6]
+};
+
+// Sums 16 values per lane over the warp by a transposing reduction (8 + 4 + 2 + 1 exchange
+// steps, one plain step): lane 2k ends with the total of value k.
+__device__ __forceinline__ double warp_sum16_f64(double (&v)[16], int lane) {
+#pragma unroll
+  for (int half = 8; half >= 1; half >>= 1) {
+    const bool up = lane & (2 * half);
+#pragma unroll
+    for (int k = 0; k < half; ++k) {
+      const double send = up ? v[k] : v[k + half];
+      const double keep = up ? v[k + half] : v[k];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, 2 * half);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+template <bool COV>
+__global__ void __launch_bounds__(kPoseThreads) k_pose_grad(PoseGradArgs a) {
+  constexpr int kWarpsPerBlock = kPoseThreads / 32;
+  __shared__ double s_red[kWarpsPerBlock][kGradSums];
+  __shared__ bool s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) pose_state_exp(a.xi, a.state);
+    if (threadIdx.x == 32) pose_state_Q(a.xi, a.state);
+  } else {
+    double acc[kGradSums];
+#pragma unroll
+    for (int k = 0; k < kGradSums; ++k) acc[k] = 0.0;
+    const int64_t stride = (int64_t)(gridDim.x - 1) * kPoseThreads;
+    for (int64_t i = (int64_t)(blockIdx.x - 1) * kPoseThreads + threadIdx.x; i < a.n; i += stride) {
+      double g[3], p[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        p[k] = a.xyz[3 * i + k];
+        g[k] = a.dL_dmeans[3 * i + k];
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        acc[k] += g[k];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) acc[3 + 3 * k + j] = fma(p[k], g[j], acc[3 + 3 * k + j]);
+      }
+      if (COV) {
+        const float* c = a.cov_rot + 6 * (size_t)i;
+        const float* d = a.dL_dcov + 6 * (size_t)i;
+        float C[9] = {c[0], c[1], c[2], c[1], c[3], c[4], c[2], c[4], c[5]};
+        float G[9] = {d[0], 0.5f * d[1], 0.5f * d[2], 0.5f * d[1], d[3], 0.5f * d[4], 0.5f * d[2], 0.5f * d[4], d[5]};
+        // w = (M12 - M21, M20 - M02, M01 - M10) of the antisymmetric M = C G - G C, where
+        // G C = (C G)^T for symmetric C, G, so M_rs = CG_rs - CG_sr
+        float CG[9];
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+          for (int q = 0; q < 3; ++q)
+            CG[3 * r + q] = C[3 * r] * G[q] + C[3 * r + 1] * G[3 + q] + C[3 * r + 2] * G[6 + q];
+        acc[12] += 2.0 * ((double)CG[5] - (double)CG[7]);
+        acc[13] += 2.0 * ((double)CG[6] - (double)CG[2]);
+        acc[14] += 2.0 * ((double)CG[1] - (double)CG[3]);
+      }
+    }
+    const double v = warp_sum16_f64(acc, lane);
+    if ((lane & 1) == 0) s_red[warp][lane >> 1] = v;
+    __syncthreads();
+    if (threadIdx.x < kGradSums) {
+      double t = 0.0;
+      for (int w = 0; w < kWarpsPerBlock; ++w) t += s_red[w][threadIdx.x];
+      a.partials[(size_t)(blockIdx.x - 1) * kGradSums + threadIdx.x] = t;
+    }
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(a.counter, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  {
+    double t = 0.0;
+    if (lane < kGradSums) {
+#pragma unroll 4
+      for (int b = warp; b < (int)gridDim.x - 1; b += kWarpsPerBlock) t += __ldcg(a.partials + (size_t)b * kGradSums + lane);
+      s_red[warp][lane] = t;
+    }
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  {
+    double t = 0.0;
+    if (lane < kGradSums)
+#pragma unroll
+      for (int w = 0; w < kWarpsPerBlock; ++w) t += s_red[w][lane];
+    __syncwarp();
+    if (lane < kGradSums) s_red[0][lane] = t;
+    __syncwarp();
+  }
+  if (lane == 0) {
+    const double* s = s_red[0];
+    const volatile PoseState* vs = a.state;  // another block's writes
+    PoseState ps;
+    for (int k = 0; k < 9; ++k) {
+      ps.R64[k] = vs->R64[k];
+      ps.Jl[k] = vs->Jl[k];
+      ps.Q[k] = vs->Q[k];
+    }
+    for (int k = 0; k < 3; ++k) ps.t64[k] = vs->t64[k];
+    double N[9];  // sum (R p) g^T
+    mm3(ps.R64, s + 3, N);
+    const double tot[kPosePartials] = {s[0],        s[1],        s[2],  N[5] - N[7], N[6] - N[2],
+                                       N[1] - N[3], s[12], s[13], s[14]};
+    pose_grad_from_state(ps, tot, a.grad_out);
+    *a.counter = 0u;
   }
 }
 
@@ -422,24 +475,32 @@ void launch_batch_pose_update(int count, const SceneDesc* descs, const double* p
 
 using namespace cfgs;
 
-static int pose_blocks(int n) {
-  int b = div_up(n > 0 ? n : 1, kPoseThreads);
-  return b < kPoseMaxBlocks ? b : kPoseMaxBlocks;
-}
+// Scratch of cfgs_pose_grad: the blocks' partial sums, the pose state, the block counter.
+struct PoseGradLayout {
+  size_t partials = 0, state, counter, total;
+  PoseGradLayout() {
+    state = align256(sizeof(double) * kGradSums * kGradMaxBlocks);
+    counter = state + align256(sizeof(PoseState));
+    total = counter + 256;
+  }
+};
 
 extern "C" int cfgs_pose_apply(int32_t n, const float* xi, const float* xyz, const float* cov_in, float* means_out,
                                float* cov_out, void* stream) {
   if (n < 0 || !xi || (n > 0 && (!xyz || !means_out))) return CFGS_ERR_INVALID_ARGUMENT;
   if ((cov_in == nullptr) != (cov_out == nullptr)) return CFGS_ERR_INVALID_ARGUMENT;
   if (n == 0) return CFGS_OK;
-  k_pose_apply<<<pose_blocks(n), kPoseThreads, 0, (cudaStream_t)stream>>>(n, xi, xyz, cov_in, means_out, cov_out);
+  const int blocks = div_up(n, kPoseThreads * kApplyPerThread);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (cov_in) k_pose_apply<true><<<blocks, kPoseThreads, 0, st>>>(n, xi, xyz, cov_in, means_out, cov_out);
+  else k_pose_apply<false><<<blocks, kPoseThreads, 0, st>>>(n, xi, xyz, cov_in, means_out, cov_out);
   CFGS_CHECK_LAUNCH(0, stream);
   return CFGS_OK;
 }
 
 extern "C" size_t cfgs_pose_scratch_bytes(int32_t n) {
   (void)n;
-  return align256(sizeof(double) * kPosePartials * kPoseMaxBlocks) + 256;
+  return PoseGradLayout().total;
 }
 
 extern "C" int cfgs_pose_grad(int32_t n, const float* xi, const float* xyz, const float* dL_dmeans, const float* cov_rot,
@@ -447,6 +508,8 @@ extern "C" int cfgs_pose_grad(int32_t n, const float* xi, const float* xyz, cons
   if (n < 0 || !xi || !scratch || !grad_out || (n > 0 && (!xyz || !dL_dmeans))) return CFGS_ERR_INVALID_ARGUMENT;
   if ((cov_rot == nullptr) != (dL_dcov == nullptr)) return CFGS_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
+  const PoseGradLayout L;
+  char* base = static_cast<char*>(scratch);
   PoseGradArgs a;
   a.n = n;
   a.xi = xi;
@@ -454,12 +517,15 @@ extern "C" int cfgs_pose_grad(int32_t n, const float* xi, const float* xyz, cons
   a.dL_dmeans = dL_dmeans;
   a.cov_rot = cov_rot;
   a.dL_dcov = dL_dcov;
-  a.partials = static_cast<double*>(scratch);
-  a.counter = reinterpret_cast<unsigned int*>(static_cast<char*>(scratch) +
-                                              align256(sizeof(double) * kPosePartials * kPoseMaxBlocks));
+  a.partials = reinterpret_cast<double*>(base + L.partials);
+  a.state = reinterpret_cast<PoseState*>(base + L.state);
+  a.counter = reinterpret_cast<unsigned int*>(base + L.counter);
   a.grad_out = grad_out;
   if (cudaMemsetAsync(a.counter, 0, sizeof(unsigned int), st) != cudaSuccess) return CFGS_ERR_LAUNCH;
-  k_pose_grad<<<pose_blocks(n), kPoseThreads, 0, st>>>(a);
+  const int sums = div_up(n > 0 ? n : 1, kPoseThreads);
+  const int blocks = 1 + (sums < kGradMaxBlocks ? sums : kGradMaxBlocks);  // block 0 forms the pose state
+  if (cov_rot) k_pose_grad<true><<<blocks, kPoseThreads, 0, st>>>(a);
+  else k_pose_grad<false><<<blocks, kPoseThreads, 0, st>>>(a);
   CFGS_CHECK_LAUNCH(0, st);
   return CFGS_OK;
 }
@@ -468,7 +534,7 @@ extern "C" int cfgs_pose_adam(int32_t count, float* xi, const float* grad, float
                               double beta2, double eps, void* stream) {
   if (count < 0 || (count > 0 && (!xi || !grad || !state))) return CFGS_ERR_INVALID_ARGUMENT;
   if (count == 0) return CFGS_OK;
-  k_pose_adam<<<div_up(count, 128), 128, 0, (cudaStream_t)stream>>>(count, xi, grad, state, lr, beta1, beta2, eps);
+  k_pose_adam<<<div_up(count, 4), 128, 0, (cudaStream_t)stream>>>(count, xi, grad, state, lr, beta1, beta2, eps);
   CFGS_CHECK_LAUNCH(0, stream);
   return CFGS_OK;
 }
