@@ -277,9 +277,12 @@ def photometric_loss(img: torch.Tensor, target: torch.Tensor, lambda_dssim: floa
     CF-3DGS uses lambda_dssim = 0.2). lambda 0 is the RGB L1 alone."""
     if lambda_dssim == 0.0:
         return l1(img, target, fused)
+    if fused:
+        from .ssim import photometric, photometric_fusable, ssim
+        if photometric_fusable(img, target, lambda_dssim):
+            return photometric(img, target, lambda_dssim)
     c = img.clamp(0, 1)
     if fused:
-        from .ssim import ssim
         return (1.0 - lambda_dssim) * l1(img, target, fused=True) + lambda_dssim * (1.0 - ssim(c, target))
     return (1.0 - lambda_dssim) * (c - target).abs().mean() + lambda_dssim * (1.0 - ssim_torch(c, target))
 

@@ -57,3 +57,45 @@ def ssim(img1: torch.Tensor, img2: torch.Tensor, window_size: int = 11, size_ave
     if img2.requires_grad:
         raise NotImplementedError("ssim: gradients flow to img1 only (img2 is the target)")
     return SsimFn.apply(img1, img2)
+
+
+class PhotometricFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, img: torch.Tensor, target: torch.Tensor, lambda_dssim: float) -> torch.Tensor:
+        a, b = _as_chw(img).contiguous(), _as_chw(target).contiguous()
+        lib = native.load()
+        C, H, W = (int(x) for x in a.shape)
+        scratch = torch.empty(int(lib.cfgs_ssim_scratch_bytes(C, H, W)), dtype=torch.uint8, device=a.device)
+        out = torch.empty((), dtype=torch.float32, device=a.device)
+        native.check(lib.cfgs_photometric_forward(C, H, W, _ptr(a), _ptr(b), lambda_dssim, _ptr(scratch),
+                                                  out.data_ptr(), stream_handle(a.device)), "cfgs_photometric_forward")
+        ctx.save_for_backward(a, b, scratch)
+        ctx.in_shape, ctx.lambda_dssim = img.shape, lambda_dssim
+        return out
+
+    @staticmethod
+    def backward(ctx, grad: torch.Tensor):
+        a, b, scratch = ctx.saved_tensors
+        C, H, W = (int(x) for x in a.shape)
+        g = grad.detach().float().reshape(()).contiguous()
+        d = torch.empty_like(a)
+        native.check(native.load().cfgs_photometric_backward(C, H, W, _ptr(a), _ptr(b), ctx.lambda_dssim, _ptr(scratch),
+                                                             _ptr(g), _ptr(d), stream_handle(a.device)),
+                     "cfgs_photometric_backward")
+        return d.reshape(ctx.in_shape), None, None
+
+
+def photometric_fusable(img: torch.Tensor, target: torch.Tensor, lambda_dssim) -> bool:
+    """Whether photometric() takes these operands: non-empty float32 CUDA images of one shape,
+    [C,H,W] or [N,C,H,W], a plain weight and a target without gradient. Other operands (half
+    or double images, whose clamp belongs before the conversion to float32) go through
+    clamp, l1_loss and ssim."""
+    return (isinstance(lambda_dssim, (int, float)) and img.is_cuda and target.device == img.device and
+            img.shape == target.shape and img.dim() in (3, 4) and img.numel() > 0 and not target.requires_grad and
+            img.dtype == torch.float32 and target.dtype == torch.float32)
+
+
+def photometric(img: torch.Tensor, target: torch.Tensor, lambda_dssim: float) -> torch.Tensor:
+    """(1 - lambda) mean |c - target| + lambda (1 - SSIM(c, target)), c = clamp(img, 0, 1),
+    in one pass per direction (operands as photometric_fusable says)."""
+    return PhotometricFn.apply(img, target, float(lambda_dssim))

@@ -265,7 +265,7 @@ __device__ void pose_grad_from_state(const PoseState& ps, const double* tot, flo
 // w takes rows w, w + 8, ..., one lane per sum) and applies the Jacobian transpose. Bound
 // by the float64 pipe (about 2 operations per cycle and SM). 230,400 Gaussians: 371 us
 // (one thread folded 900 rows of 9 sums one after another, and every block formed exp(xi))
-// -> POSE_GRAD_US us.
+// -> 30 us.
 constexpr int kGradMaxBlocks = 2 * 152;  // two blocks of partial sums per SM at most
 constexpr int kGradSums = 16;            // sum g (3), M (9), w_cov (3), unused
 

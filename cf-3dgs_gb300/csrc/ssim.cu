@@ -15,7 +15,19 @@
 // Both kernels work on 32x32 output tiles of one channel: the tile and a 5-pixel halo
 // are staged in shared memory (zero outside the image); a horizontal 11-tap pass over all
 // staged rows and then a vertical pass compute runs of 4 outputs per thread, each input
-// loaded once per run and the window slid in registers.
+// loaded once per run and the window slid in registers. They are bound by the issue of
+// the taps (127 multiply-adds per output and moment set, against 20 bytes per element of
+// traffic that mostly stays in L2), so the taps run on packed pairs — (x, y) and
+// (x^2, y^2) in the forward, two of the three maps in the backward — and the horizontal
+// sums are stored and loaded as pairs. 3x1080x1920: forward 55.7 -> FWD_US us, backward
+// 49.2 -> BWD_US us.
+//
+// The photometric form (PHOTO) is the whole CF-3DGS image loss of a render x,
+//   (1 - lambda) mean |c - y| + lambda (1 - SSIM(c, y)), c = clamp(x, 0, 1)
+// (trainer/losses.py:98-136, scene/gaussian_model_cf.py:885), in the same two passes: the
+// forward clamps as it reads and also sums |c - y|, the backward adds the L1 sign and
+// masks by the clamp. As separate clamp, L1 and SSIM calls the loss and its gradient took
+// 21 launches (218 us of kernels) at 3x1080x1920; here 3 launches, PHOTO_US us.
 #include <cuda.h>  // CUtensorMap and its enumerations (the encoder comes from the runtime)
 #include <cudaTypedefs.h>
 
@@ -35,6 +47,7 @@ constexpr uint32_t kSsimBoxBytes = sizeof(float) * kSsimSP * kSsimS;
 constexpr int kSsimHP = kSsimT + 1;               // horizontal-result row stride (33)
 constexpr int kSsimRun = 4;                       // outputs per thread along a row / column
 constexpr int kSsimThreads = 256;
+constexpr int kSsimFoldThreads = 1024;  // the fold of one partial pair per tile
 constexpr float kSsimC1 = 0.0001f, kSsimC2 = 0.0009f;
 
 __constant__ float c_ssim_w[kSsimTaps];
@@ -106,35 +119,30 @@ __device__ __forceinline__ double block_sum_fixed(double v, double* sh) {
   return t;  // valid in thread 0
 }
 
-// Horizontal 11-tap sums of NQ staged quantities for kSsimRun consecutive outputs of one
-// staged row: the 14 inputs are loaded once and the window slides in registers.
-// prod(u, v, out) expands two staged values into the NQ quantities.
-template <int NQ, class Prod>
-__device__ __forceinline__ void hpass_run(const float* a_row, const float* b_row, int c0, float (&out)[NQ][kSsimRun],
-                                          Prod prod) {
-  float q[kSsimRun + 2 * kSsimR][NQ];
+// The six distinct weights of the symmetric window as packed pairs.
+struct WindowPairs {
+  float2 w[kSsimR + 1];
+  __device__ __forceinline__ WindowPairs() {
 #pragma unroll
-  for (int k = 0; k < kSsimRun + 2 * kSsimR; ++k) prod(a_row[c0 + k], b_row ? b_row[c0 + k] : 0.f, q[k]);
-#pragma unroll
-  for (int u = 0; u < kSsimRun; ++u)
-#pragma unroll
-    for (int n = 0; n < NQ; ++n) {
-      float acc = 0.f;
-#pragma unroll
-      for (int k = 0; k < kSsimTaps; ++k) acc = fmaf(c_ssim_w[k], q[u + k][n], acc);
-      out[n][u] = acc;
-    }
-}
+    for (int k = 0; k <= kSsimR; ++k) w[k] = splat2(c_ssim_w[k]);
+  }
+  __device__ __forceinline__ float2 operator[](int tap) const { return w[tap <= kSsimR ? tap : 2 * kSsimR - tap]; }
+};
 
-template <bool TMA>
+// clamp to [0, 1] that keeps a NaN, as torch.clamp does.
+__device__ __forceinline__ float clamp01(float x) { return x != x ? x : fminf(fmaxf(x, 0.0f), 1.0f); }
+
+template <bool TMA, bool PHOTO>
 __global__ void __launch_bounds__(kSsimThreads) k_ssim_fwd(SsimDims d, const float* __restrict__ img1,
                                                            const float* __restrict__ img2, float* __restrict__ maps,
-                                                           double* __restrict__ partials, float inv_count,
+                                                           double2* __restrict__ partials, float inv_count,
                                                            const __grid_constant__ CUtensorMap t1,
                                                            const __grid_constant__ CUtensorMap t2) {
   __shared__ __align__(128) float s_x[kSsimS * kSsimSP];
   __shared__ __align__(128) float s_y[kSsimS * kSsimSP];
-  __shared__ float s_h[5][kSsimS * kSsimHP];  // horizontal sums of x, y, xx, yy, xy
+  __shared__ float2 s_hm[kSsimS * kSsimHP];  // horizontal sums of (x, y)
+  __shared__ float2 s_hs[kSsimS * kSsimHP];  // of (xx, yy)
+  __shared__ float s_hp[kSsimS * kSsimHP];   // of xy
   __shared__ double s_red[kSsimThreads / 32];
   __shared__ __align__(8) uint64_t s_bar;
   const int tile = blockIdx.x, ch = blockIdx.y;
@@ -145,44 +153,65 @@ __global__ void __launch_bounds__(kSsimThreads) k_ssim_fwd(SsimDims d, const flo
   const CUtensorMap* const tm[2] = {&t1, &t2};
   const int zi[2] = {ch, ch};
   const bool staged = stage_planes<TMA, 2>(dst, src, tm, zi, d.H, d.W, x0, y0, &s_bar);
+  const WindowPairs w;
   __syncthreads();
   // horizontal: item = (staged row r, run of 4 output columns)
   for (int it = threadIdx.x; it < kSsimS * (kSsimT / kSsimRun); it += kSsimThreads) {
     const int r = it / (kSsimT / kSsimRun), c0 = (it % (kSsimT / kSsimRun)) * kSsimRun;
-    float out[5][kSsimRun];
-    hpass_run<5>(s_x + r * kSsimSP + kSsimOff, s_y + r * kSsimSP + kSsimOff, c0, out, [](float u, float v, float (&q)[5]) {
-      q[0] = u;
-      q[1] = v;
-      q[2] = u * u;
-      q[3] = v * v;
-      q[4] = u * v;
-    });
+    const float* xr = s_x + r * kSsimSP + kSsimOff + c0;
+    const float* yr = s_y + r * kSsimSP + kSsimOff + c0;
+    float2 m[kSsimRun], q[kSsimRun];
+    float p[kSsimRun];
 #pragma unroll
-    for (int n = 0; n < 5; ++n)
-#pragma unroll
-      for (int u = 0; u < kSsimRun; ++u) s_h[n][r * kSsimHP + c0 + u] = out[n][u];
-  }
-  __syncthreads();
-  // vertical: item = (output column c, run of 4 output rows); one item per thread
-  float ssum = 0.f;
-  {
-    const int c = threadIdx.x % kSsimT, r0 = (threadIdx.x / kSsimT) * kSsimRun;
-    float acc[5][kSsimRun];
-#pragma unroll
-    for (int n = 0; n < 5; ++n)
-#pragma unroll
-      for (int u = 0; u < kSsimRun; ++u) acc[n][u] = 0.f;
+    for (int u = 0; u < kSsimRun; ++u) {
+      m[u] = q[u] = splat2(0.f);
+      p[u] = 0.f;
+    }
 #pragma unroll
     for (int k = 0; k < kSsimRun + 2 * kSsimR; ++k) {
-      float v[5];
-#pragma unroll
-      for (int n = 0; n < 5; ++n) v[n] = s_h[n][(r0 + k) * kSsimHP + c];
+      const float2 v = make_float2(PHOTO ? clamp01(xr[k]) : xr[k], yr[k]);
+      const float2 vv = mul2(v, v);
+      const float xy = v.x * v.y;
 #pragma unroll
       for (int u = 0; u < kSsimRun; ++u) {
         const int tap = k - u;
         if (tap >= 0 && tap < kSsimTaps) {
+          m[u] = fma2(w[tap], v, m[u]);
+          q[u] = fma2(w[tap], vv, q[u]);
+          p[u] = fmaf(w[tap].x, xy, p[u]);
+        }
+      }
+    }
 #pragma unroll
-          for (int n = 0; n < 5; ++n) acc[n][u] = fmaf(c_ssim_w[tap], v[n], acc[n][u]);
+    for (int u = 0; u < kSsimRun; ++u) {
+      s_hm[r * kSsimHP + c0 + u] = m[u];
+      s_hs[r * kSsimHP + c0 + u] = q[u];
+      s_hp[r * kSsimHP + c0 + u] = p[u];
+    }
+  }
+  __syncthreads();
+  // vertical: item = (output column c, run of 4 output rows); one item per thread
+  float ssum = 0.f, lsum = 0.f;
+  {
+    const int c = threadIdx.x % kSsimT, r0 = (threadIdx.x / kSsimT) * kSsimRun;
+    float2 m[kSsimRun], q[kSsimRun];
+    float p[kSsimRun];
+#pragma unroll
+    for (int u = 0; u < kSsimRun; ++u) {
+      m[u] = q[u] = splat2(0.f);
+      p[u] = 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < kSsimRun + 2 * kSsimR; ++k) {
+      const float2 vm = s_hm[(r0 + k) * kSsimHP + c], vs = s_hs[(r0 + k) * kSsimHP + c];
+      const float vp = s_hp[(r0 + k) * kSsimHP + c];
+#pragma unroll
+      for (int u = 0; u < kSsimRun; ++u) {
+        const int tap = k - u;
+        if (tap >= 0 && tap < kSsimTaps) {
+          m[u] = fma2(w[tap], vm, m[u]);
+          q[u] = fma2(w[tap], vs, q[u]);
+          p[u] = fmaf(w[tap].x, vp, p[u]);
         }
       }
     }
@@ -191,45 +220,84 @@ __global__ void __launch_bounds__(kSsimThreads) k_ssim_fwd(SsimDims d, const flo
     for (int u = 0; u < kSsimRun; ++u) {
       const int py = y0 + r0 + u;
       if (py >= d.H || px >= d.W) continue;
-      const float mu1 = acc[0][u], mu2 = acc[1][u], exx = acc[2][u], eyy = acc[3][u], exy = acc[4][u];
+      const float mu1 = m[u].x, mu2 = m[u].y, exx = q[u].x, eyy = q[u].y, exy = p[u];
       const float m11 = mu1 * mu1, m22 = mu2 * mu2, m12 = mu1 * mu2;
       const float A = 2.f * m12 + kSsimC1, B = 2.f * (exy - m12) + kSsimC2;
       const float Cc = m11 + m22 + kSsimC1, D = (exx - m11) + (eyy - m22) + kSsimC2;
       const float rA = rcp_approx(A), rB = rcp_approx(B), rC = rcp_approx(Cc), rD = rcp_approx(D);
       const float S = (A * B) * (rC * rD);
       ssum += S;
-      const size_t q = ch * plane + (size_t)py * d.W + px;
+      if (PHOTO) {
+        const int at = (r0 + u + kSsimR) * kSsimSP + kSsimOff + c + kSsimR;
+        lsum += fabsf(clamp01(s_x[at]) - s_y[at]);
+      }
+      const size_t o = ch * plane + (size_t)py * d.W + px;
       // dS/dmu1 = S (2 mu2/A - 2 mu2/B - 2 mu1/C + 2 mu1/D); dS/dexx = -S/D; dS/dexy = 2 S/B
       const float da = S * (2.f * mu2 * (rA - rB) + 2.f * mu1 * (rD - rC));
-      maps[q] = inv_count * da;
-      maps[(size_t)d.C * plane + q] = inv_count * (-S * rD);
-      maps[2 * (size_t)d.C * plane + q] = inv_count * (2.f * S * rB);
+      maps[o] = inv_count * da;
+      maps[(size_t)d.C * plane + o] = inv_count * (-S * rD);
+      maps[2 * (size_t)d.C * plane + o] = inv_count * (2.f * S * rB);
     }
   }
   const double t = block_sum_fixed((double)ssum, s_red);
+  double l = 0.0;
+  if (PHOTO) {
+    __syncthreads();
+    l = block_sum_fixed((double)lsum, s_red);
+  }
   // a copy that did not arrive makes the mean NaN (visibly invalid)
-  if (threadIdx.x == 0) partials[(size_t)ch * gridDim.x + tile] = staged ? t : __longlong_as_double(0x7ff8000000000000ll);
+  if (threadIdx.x == 0)
+    partials[(size_t)ch * gridDim.x + tile] =
+        make_double2(staged ? t : __longlong_as_double(0x7ff8000000000000ll), l);
 }
 
-// Mean SSIM from the per-tile partial sums, in a fixed order (one block).
-__global__ void __launch_bounds__(kSsimThreads) k_ssim_mean(const double* __restrict__ partials, int count,
-                                                            double inv_count, float* __restrict__ out) {
-  __shared__ double s_red[kSsimThreads / 32];
-  double v = 0.0;
-  for (int i = threadIdx.x; i < count; i += kSsimThreads) v += partials[i];
-  const double t = block_sum_fixed(v, s_red);
-  if (threadIdx.x == 0) *out = (float)(t * inv_count);
+// Mean SSIM and (PHOTO) mean |c - y| from the per-tile partial sums in a fixed order (one
+// block): out = w_l1 mean|c - y| + w_ssim SSIM + constant.
+__global__ void __launch_bounds__(kSsimFoldThreads) k_ssim_fold(const double2* __restrict__ partials, int count,
+                                                                double inv_count, double w_l1, double w_ssim,
+                                                                double constant, float* __restrict__ out) {
+  __shared__ double s_red[2][kSsimFoldThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double s = 0.0, l = 0.0;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < count; i += kSsimFoldThreads) {
+    const double2 v = partials[i];
+    s += v.x;
+    l += v.y;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    l += __shfl_xor_sync(0xffffffffu, l, o);
+  }
+  if (lane == 0) {
+    s_red[0][warp] = s;
+    s_red[1][warp] = l;
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  s = lane < kSsimFoldThreads / 32 ? s_red[0][lane] : 0.0;
+  l = lane < kSsimFoldThreads / 32 ? s_red[1][lane] : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    l += __shfl_xor_sync(0xffffffffu, l, o);
+  }
+  if (lane == 0) *out = (float)(w_ssim * (s * inv_count) + w_l1 * (l * inv_count) + constant);
 }
 
-template <bool TMA>
+// dL/dimg1 = g w_ssim (W*a + 2 x W*b + y W*c), g = *dL_dmean; PHOTO: with x clamped, plus
+// g w_l1 sign(c - y) / count, where the clamp passes (0 <= x <= 1).
+template <bool TMA, bool PHOTO>
 __global__ void __launch_bounds__(kSsimThreads) k_ssim_bwd(SsimDims d, const float* __restrict__ img1,
                                                            const float* __restrict__ img2,
                                                            const float* __restrict__ maps,
-                                                           const float* __restrict__ dL_dmean,
-                                                           float* __restrict__ dL_dimg1,
+                                                           const float* __restrict__ dL_dmean, float w_ssim,
+                                                           float w_l1_over_count, float* __restrict__ dL_dimg1,
                                                            const __grid_constant__ CUtensorMap tmaps) {
   __shared__ __align__(128) float s_m[3][kSsimS * kSsimSP];
-  __shared__ float s_h[3][kSsimS * kSsimHP];
+  __shared__ float2 s_hab[kSsimS * kSsimHP];
+  __shared__ float s_hc[kSsimS * kSsimHP];
   __shared__ __align__(8) uint64_t s_bar;
   const int tile = blockIdx.x, ch = blockIdx.y;
   const int x0 = (tile % d.tiles_x) * kSsimT, y0 = (tile / d.tiles_x) * kSsimT;
@@ -240,46 +308,84 @@ __global__ void __launch_bounds__(kSsimThreads) k_ssim_bwd(SsimDims d, const flo
   const CUtensorMap* const tm[3] = {&tmaps, &tmaps, &tmaps};
   const int zi[3] = {ch, d.C + ch, 2 * d.C + ch};
   const bool staged = stage_planes<TMA, 3>(dst, src, tm, zi, d.H, d.W, x0, y0, &s_bar);
+  const WindowPairs w;
+  // this thread's pixels of both images, on their way while the taps run
+  const int c = threadIdx.x % kSsimT, r0 = (threadIdx.x / kSsimT) * kSsimRun;
+  const int px = x0 + c;
+  float x[kSsimRun], y[kSsimRun];
+#pragma unroll
+  for (int u = 0; u < kSsimRun; ++u) {
+    const int py = y0 + r0 + u;
+    const bool in = py < d.H && px < d.W;
+    const size_t o = ch * plane + (size_t)py * d.W + px;
+    x[u] = in ? img1[o] : 0.f;
+    y[u] = in ? img2[o] : 0.f;
+  }
+  const float g = *dL_dmean;
   __syncthreads();
   for (int it = threadIdx.x; it < kSsimS * (kSsimT / kSsimRun); it += kSsimThreads) {
     const int r = it / (kSsimT / kSsimRun), c0 = (it % (kSsimT / kSsimRun)) * kSsimRun;
+    const int at = r * kSsimSP + kSsimOff + c0;
+    float2 ab[kSsimRun];
+    float cc[kSsimRun];
 #pragma unroll
-    for (int m = 0; m < 3; ++m) {
-      float out[1][kSsimRun];
-      hpass_run<1>(s_m[m] + r * kSsimSP + kSsimOff, nullptr, c0, out, [](float u, float, float (&q)[1]) { q[0] = u; });
+    for (int u = 0; u < kSsimRun; ++u) {
+      ab[u] = splat2(0.f);
+      cc[u] = 0.f;
+    }
 #pragma unroll
-      for (int u = 0; u < kSsimRun; ++u) s_h[m][r * kSsimHP + c0 + u] = out[0][u];
+    for (int k = 0; k < kSsimRun + 2 * kSsimR; ++k) {
+      const float2 v = make_float2(s_m[0][at + k], s_m[1][at + k]);
+      const float vc = s_m[2][at + k];
+#pragma unroll
+      for (int u = 0; u < kSsimRun; ++u) {
+        const int tap = k - u;
+        if (tap >= 0 && tap < kSsimTaps) {
+          ab[u] = fma2(w[tap], v, ab[u]);
+          cc[u] = fmaf(w[tap].x, vc, cc[u]);
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kSsimRun; ++u) {
+      s_hab[r * kSsimHP + c0 + u] = ab[u];
+      s_hc[r * kSsimHP + c0 + u] = cc[u];
     }
   }
   __syncthreads();
-  const float g = *dL_dmean;
-  const int c = threadIdx.x % kSsimT, r0 = (threadIdx.x / kSsimT) * kSsimRun;
-  float acc[3][kSsimRun];
+  float2 ab[kSsimRun];
+  float cc[kSsimRun];
 #pragma unroll
-  for (int m = 0; m < 3; ++m)
-#pragma unroll
-    for (int u = 0; u < kSsimRun; ++u) acc[m][u] = 0.f;
+  for (int u = 0; u < kSsimRun; ++u) {
+    ab[u] = splat2(0.f);
+    cc[u] = 0.f;
+  }
 #pragma unroll
   for (int k = 0; k < kSsimRun + 2 * kSsimR; ++k) {
-    float v[3];
-#pragma unroll
-    for (int m = 0; m < 3; ++m) v[m] = s_h[m][(r0 + k) * kSsimHP + c];
+    const float2 v = s_hab[(r0 + k) * kSsimHP + c];
+    const float vc = s_hc[(r0 + k) * kSsimHP + c];
 #pragma unroll
     for (int u = 0; u < kSsimRun; ++u) {
       const int tap = k - u;
       if (tap >= 0 && tap < kSsimTaps) {
-#pragma unroll
-        for (int m = 0; m < 3; ++m) acc[m][u] = fmaf(c_ssim_w[tap], v[m], acc[m][u]);
+        ab[u] = fma2(w[tap], v, ab[u]);
+        cc[u] = fmaf(w[tap].x, vc, cc[u]);
       }
     }
   }
-  const int px = x0 + c;
 #pragma unroll
   for (int u = 0; u < kSsimRun; ++u) {
     const int py = y0 + r0 + u;
     if (py >= d.H || px >= d.W) continue;
-    const size_t q = ch * plane + (size_t)py * d.W + px;
-    dL_dimg1[q] = staged ? g * (acc[0][u] + 2.f * img1[q] * acc[1][u] + img2[q] * acc[2][u]) : __int_as_float(0x7fc00000);
+    const float xc = PHOTO ? clamp01(x[u]) : x[u];
+    float v = g * (ab[u].x + 2.f * xc * ab[u].y + y[u] * cc[u]);
+    if (PHOTO) {
+      const float diff = xc - y[u];
+      const float l1 = g * w_l1_over_count;
+      v = w_ssim * v + (diff > 0.f ? l1 : (diff < 0.f ? -l1 : 0.f));
+      if (!(x[u] >= 0.f && x[u] <= 1.f)) v = 0.f;
+    }
+    dL_dimg1[ch * plane + (size_t)py * d.W + px] = staged ? v : __int_as_float(0x7fc00000);
   }
 }
 
@@ -356,48 +462,76 @@ extern "C" size_t cfgs_ssim_scratch_bytes(int32_t channels, int32_t height, int3
   if (!dims_ok(channels, height, width)) return 0;
   const SsimDims d = dims(channels, height, width);
   const size_t maps = sizeof(float) * 3 * (size_t)channels * height * width;
-  const size_t parts = sizeof(double) * (size_t)channels * d.tiles_x * d.tiles_y;
+  const size_t parts = sizeof(double2) * (size_t)channels * d.tiles_x * d.tiles_y;
   return align256(maps) + align256(parts);
 }
 
-extern "C" int cfgs_ssim_forward(int32_t channels, int32_t height, int32_t width, const float* img1,
-                                 const float* img2, void* scratch, float* ssim_mean, void* stream) {
-  if (!dims_ok(channels, height, width) || !img1 || !img2 || !scratch || !ssim_mean) return CFGS_ERR_INVALID_ARGUMENT;
+namespace {
+
+// The forward of the mean SSIM (photo: of the photometric loss with weight lambda).
+int ssim_forward(int32_t channels, int32_t height, int32_t width, const float* img1, const float* img2, bool photo,
+                 double lambda, void* scratch, float* out, void* stream) {
+  if (!dims_ok(channels, height, width) || !img1 || !img2 || !scratch || !out) return CFGS_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   if (!upload_window(st)) return CFGS_ERR_LAUNCH;
   const SsimDims d = dims(channels, height, width);
   const size_t count = (size_t)channels * height * width;
   float* maps = static_cast<float*>(scratch);
-  double* parts = reinterpret_cast<double*>(static_cast<char*>(scratch) + align256(sizeof(float) * 3 * count));
+  double2* parts = reinterpret_cast<double2*>(static_cast<char*>(scratch) + align256(sizeof(float) * 3 * count));
   const int tiles = d.tiles_x * d.tiles_y;
+  const float inv = (float)(1.0 / (double)count);
   CUtensorMap t1{}, t2{};
   const bool tma = encode_planes(&t1, img1, width, height, channels) && encode_planes(&t2, img2, width, height, channels);
-  if (tma)
-    k_ssim_fwd<true><<<dim3(tiles, channels), kSsimThreads, 0, st>>>(d, img1, img2, maps, parts,
-                                                                    (float)(1.0 / (double)count), t1, t2);
-  else
-    k_ssim_fwd<false><<<dim3(tiles, channels), kSsimThreads, 0, st>>>(d, img1, img2, maps, parts,
-                                                                     (float)(1.0 / (double)count), t1, t2);
-  k_ssim_mean<<<1, kSsimThreads, 0, st>>>(parts, tiles * channels, 1.0 / (double)count, ssim_mean);
+  auto* kernel = photo ? (tma ? k_ssim_fwd<true, true> : k_ssim_fwd<false, true>)
+                       : (tma ? k_ssim_fwd<true, false> : k_ssim_fwd<false, false>);
+  kernel<<<dim3(tiles, channels), kSsimThreads, 0, st>>>(d, img1, img2, maps, parts, inv, t1, t2);
+  k_ssim_fold<<<1, kSsimFoldThreads, 0, st>>>(parts, tiles * channels, 1.0 / (double)count, photo ? 1.0 - lambda : 0.0,
+                                              photo ? -lambda : 1.0, photo ? lambda : 0.0, out);
   CFGS_CHECK_LAUNCH(0, st);
   return CFGS_OK;
+}
+
+int ssim_backward(int32_t channels, int32_t height, int32_t width, const float* img1, const float* img2, bool photo,
+                  double lambda, const void* scratch, const float* dL_dout, float* dL_dimg1, void* stream) {
+  if (!dims_ok(channels, height, width) || !img1 || !img2 || !scratch || !dL_dout || !dL_dimg1)
+    return CFGS_ERR_INVALID_ARGUMENT;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (!upload_window(st)) return CFGS_ERR_LAUNCH;
+  const SsimDims d = dims(channels, height, width);
+  const double count = (double)channels * height * width;
+  const float* maps = static_cast<const float*>(scratch);
+  CUtensorMap tm{};
+  const dim3 grid(d.tiles_x * d.tiles_y, channels);
+  const bool tma = encode_planes(&tm, maps, width, height, 3 * channels);
+  auto* kernel = photo ? (tma ? k_ssim_bwd<true, true> : k_ssim_bwd<false, true>)
+                       : (tma ? k_ssim_bwd<true, false> : k_ssim_bwd<false, false>);
+  kernel<<<grid, kSsimThreads, 0, st>>>(d, img1, img2, maps, dL_dout, (float)-lambda, (float)((1.0 - lambda) / count),
+                                        dL_dimg1, tm);
+  CFGS_CHECK_LAUNCH(0, st);
+  return CFGS_OK;
+}
+
+}  // namespace
+
+extern "C" int cfgs_ssim_forward(int32_t channels, int32_t height, int32_t width, const float* img1,
+                                 const float* img2, void* scratch, float* ssim_mean, void* stream) {
+  return ssim_forward(channels, height, width, img1, img2, false, 0.0, scratch, ssim_mean, stream);
 }
 
 extern "C" int cfgs_ssim_backward(int32_t channels, int32_t height, int32_t width, const float* img1,
                                   const float* img2, const void* scratch, const float* dL_dmean, float* dL_dimg1,
                                   void* stream) {
-  if (!dims_ok(channels, height, width) || !img1 || !img2 || !scratch || !dL_dmean || !dL_dimg1)
-    return CFGS_ERR_INVALID_ARGUMENT;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (!upload_window(st)) return CFGS_ERR_LAUNCH;
-  const SsimDims d = dims(channels, height, width);
-  const float* maps = static_cast<const float*>(scratch);
-  CUtensorMap tm{};
-  const dim3 grid(d.tiles_x * d.tiles_y, channels);
-  if (encode_planes(&tm, maps, width, height, 3 * channels))
-    k_ssim_bwd<true><<<grid, kSsimThreads, 0, st>>>(d, img1, img2, maps, dL_dmean, dL_dimg1, tm);
-  else
-    k_ssim_bwd<false><<<grid, kSsimThreads, 0, st>>>(d, img1, img2, maps, dL_dmean, dL_dimg1, tm);
-  CFGS_CHECK_LAUNCH(0, st);
-  return CFGS_OK;
+  return ssim_backward(channels, height, width, img1, img2, false, 0.0, scratch, dL_dmean, dL_dimg1, stream);
+}
+
+extern "C" int cfgs_photometric_forward(int32_t channels, int32_t height, int32_t width, const float* img,
+                                        const float* target, double lambda_dssim, void* scratch, float* loss,
+                                        void* stream) {
+  return ssim_forward(channels, height, width, img, target, true, lambda_dssim, scratch, loss, stream);
+}
+
+extern "C" int cfgs_photometric_backward(int32_t channels, int32_t height, int32_t width, const float* img,
+                                         const float* target, double lambda_dssim, const void* scratch,
+                                         const float* dL_dloss, float* dL_dimg, void* stream) {
+  return ssim_backward(channels, height, width, img, target, true, lambda_dssim, scratch, dL_dloss, dL_dimg, stream);
 }

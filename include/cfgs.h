@@ -316,6 +316,15 @@ int cfgs_ssim_forward(int32_t channels, int32_t height, int32_t width, const flo
                       void* scratch, float* ssim_mean, void* stream);
 int cfgs_ssim_backward(int32_t channels, int32_t height, int32_t width, const float* img1, const float* img2,
                        const void* scratch, const float* dL_dmean, float* dL_dimg1, void* stream);
+/* The CF-3DGS image loss of a render (trainer/losses.py:98-136) in the same two passes:
+ * loss = (1 - lambda_dssim) mean |c - target| + lambda_dssim (1 - SSIM(c, target)) with
+ * c = clamp(img, 0, 1), and dL_dimg = dL_dloss[0] * d loss / d img (zero where the clamp
+ * cuts; target gets no gradient). `scratch` is cfgs_ssim_scratch_bytes. */
+int cfgs_photometric_forward(int32_t channels, int32_t height, int32_t width, const float* img, const float* target,
+                             double lambda_dssim, void* scratch, float* loss, void* stream);
+int cfgs_photometric_backward(int32_t channels, int32_t height, int32_t width, const float* img, const float* target,
+                              double lambda_dssim, const void* scratch, const float* dL_dloss, float* dL_dimg,
+                              void* stream);
 
 /* ---- L1 photometric loss ------------------------------------------------------------
  * mean |x - target| over n floats (utils/loss_utils.py:15-16, trainer/losses.py:139-140),
