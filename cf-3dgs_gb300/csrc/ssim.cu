@@ -19,15 +19,16 @@
 // the taps (127 multiply-adds per output and moment set, against 20 bytes per element of
 // traffic that mostly stays in L2), so the taps run on packed pairs — (x, y) and
 // (x^2, y^2) in the forward, two of the three maps in the backward — and the horizontal
-// sums are stored and loaded as pairs. 3x1080x1920: forward 55.7 -> FWD_US us, backward
-// 49.2 -> BWD_US us.
+// sums are stored and loaded as pairs. 3x1080x1920: photometric forward 61 us (issue 67%
+// busy, shared-memory pipe 52%), backward 42 us; SSIM alone took 55.7 and 49.2 us with
+// scalar taps.
 //
 // The photometric form (PHOTO) is the whole CF-3DGS image loss of a render x,
 //   (1 - lambda) mean |c - y| + lambda (1 - SSIM(c, y)), c = clamp(x, 0, 1)
 // (trainer/losses.py:98-136, scene/gaussian_model_cf.py:885), in the same two passes: the
 // forward clamps as it reads and also sums |c - y|, the backward adds the L1 sign and
 // masks by the clamp. As separate clamp, L1 and SSIM calls the loss and its gradient took
-// 21 launches (218 us of kernels) at 3x1080x1920; here 3 launches, PHOTO_US us.
+// 21 launches (218 us of kernels) at 3x1080x1920; here 3 launches, 111 us.
 #include <cuda.h>  // CUtensorMap and its enumerations (the encoder comes from the runtime)
 #include <cudaTypedefs.h>
 
@@ -47,7 +48,7 @@ constexpr uint32_t kSsimBoxBytes = sizeof(float) * kSsimSP * kSsimS;
 constexpr int kSsimHP = kSsimT + 1;               // horizontal-result row stride (33)
 constexpr int kSsimRun = 4;                       // outputs per thread along a row / column
 constexpr int kSsimThreads = 256;
-constexpr int kSsimFoldThreads = 1024;  // the fold of one partial pair per tile
+constexpr int kSsimFoldBlocks = 16;  // blocks of the fold of one partial pair per tile at most
 constexpr float kSsimC1 = 0.0001f, kSsimC2 = 0.0009f;
 
 __constant__ float c_ssim_w[kSsimTaps];
@@ -106,17 +107,34 @@ __device__ __forceinline__ bool stage_planes(float* (&dst)[NP], const float* con
   }
 }
 
-// Block-wide sum of one double per thread (kSsimThreads threads), fixed order.
-__device__ __forceinline__ double block_sum_fixed(double v, double* sh) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (lane == 0) sh[warp] = v;
+// Block-wide float64 sum of one float per thread (kSsimThreads threads), fixed order,
+// valid in thread 0. One warp adds the floats from shared memory: the float64 pipe issues
+// about two operations per cycle and SM, and a shuffle reduction by every warp kept it
+// busy for half of the forward.
+__device__ __forceinline__ double block_sum_fixed(float v, float* sh) {
+  sh[threadIdx.x] = v;
   __syncthreads();
   double t = 0.0;
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int w = 0; w < kSsimThreads / 32; ++w) t += (double)sh[threadIdx.x + 32 * w];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  }
+  return t;
+}
+
+// Block-wide float sum (the precision of the L1 loss's own block sums), fixed order, valid
+// in thread 0.
+__device__ __forceinline__ float block_sum_float(float v, float* sh) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  float t = 0.0f;
   if (threadIdx.x == 0)
     for (int w = 0; w < kSsimThreads / 32; ++w) t += sh[w];
-  return t;  // valid in thread 0
+  return t;
 }
 
 // The six distinct weights of the symmetric window as packed pairs.
@@ -135,7 +153,8 @@ __device__ __forceinline__ float clamp01(float x) { return x != x ? x : fminf(fm
 template <bool TMA, bool PHOTO>
 __global__ void __launch_bounds__(kSsimThreads) k_ssim_fwd(SsimDims d, const float* __restrict__ img1,
                                                            const float* __restrict__ img2, float* __restrict__ maps,
-                                                           double2* __restrict__ partials, float inv_count,
+                                                           double2* __restrict__ partials,
+                                                           unsigned int* __restrict__ fold_counter, float inv_count,
                                                            const __grid_constant__ CUtensorMap t1,
                                                            const __grid_constant__ CUtensorMap t2) {
   __shared__ __align__(128) float s_x[kSsimS * kSsimSP];
@@ -143,7 +162,7 @@ __global__ void __launch_bounds__(kSsimThreads) k_ssim_fwd(SsimDims d, const flo
   __shared__ float2 s_hm[kSsimS * kSsimHP];  // horizontal sums of (x, y)
   __shared__ float2 s_hs[kSsimS * kSsimHP];  // of (xx, yy)
   __shared__ float s_hp[kSsimS * kSsimHP];   // of xy
-  __shared__ double s_red[kSsimThreads / 32];
+  __shared__ float s_red[kSsimThreads], s_red_l1[kSsimThreads / 32];
   __shared__ __align__(8) uint64_t s_bar;
   const int tile = blockIdx.x, ch = blockIdx.y;
   const int x0 = (tile % d.tiles_x) * kSsimT, y0 = (tile / d.tiles_x) * kSsimT;
@@ -239,51 +258,64 @@ __global__ void __launch_bounds__(kSsimThreads) k_ssim_fwd(SsimDims d, const flo
       maps[2 * (size_t)d.C * plane + o] = inv_count * (2.f * S * rB);
     }
   }
-  const double t = block_sum_fixed((double)ssum, s_red);
-  double l = 0.0;
-  if (PHOTO) {
-    __syncthreads();
-    l = block_sum_fixed((double)lsum, s_red);
-  }
-  // a copy that did not arrive makes the mean NaN (visibly invalid)
-  if (threadIdx.x == 0)
+  const double t = block_sum_fixed(ssum, s_red);
+  const float l = PHOTO ? block_sum_float(lsum, s_red_l1) : 0.0f;
+  if (threadIdx.x == 0) {
+    // a copy that did not arrive makes the mean NaN (visibly invalid)
     partials[(size_t)ch * gridDim.x + tile] =
-        make_double2(staged ? t : __longlong_as_double(0x7ff8000000000000ll), l);
+        make_double2(staged ? t : __longlong_as_double(0x7ff8000000000000ll), (double)l);
+    if (blockIdx.x == 0 && blockIdx.y == 0) *fold_counter = 0u;  // for the fold, the next launch
+  }
 }
 
-// Mean SSIM and (PHOTO) mean |c - y| from the per-tile partial sums in a fixed order (one
-// block): out = w_l1 mean|c - y| + w_ssim SSIM + constant.
-__global__ void __launch_bounds__(kSsimFoldThreads) k_ssim_fold(const double2* __restrict__ partials, int count,
-                                                                double inv_count, double w_l1, double w_ssim,
-                                                                double constant, float* __restrict__ out) {
-  __shared__ double s_red[2][kSsimFoldThreads / 32];
+// Mean SSIM and (PHOTO) mean |c - y| from the per-tile partial sums, in a fixed order: out =
+// w_l1 mean|c - y| + w_ssim SSIM + constant. Block b sums its share of the partials into
+// block_sums[b], the last block to finish adds those in block order. Several blocks,
+// because one SM's float64 pipe took 9.4 us for the 6120 pairs of 3x1080x1920; 7.5 us with
+// up to 16.
+__device__ __forceinline__ double2 block_sum_pair(double2 v, double2* sh) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  double s = 0.0, l = 0.0;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < count; i += kSsimFoldThreads) {
-    const double2 v = partials[i];
-    s += v.x;
-    l += v.y;
-  }
+  // after the first exchange lanes below 16 sum v.x, the others v.y
+  const bool up = lane & 16;
+  double t = (up ? v.y : v.x) + __shfl_xor_sync(0xffffffffu, up ? v.x : v.y, 16);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    s += __shfl_xor_sync(0xffffffffu, s, o);
-    l += __shfl_xor_sync(0xffffffffu, l, o);
-  }
-  if (lane == 0) {
-    s_red[0][warp] = s;
-    s_red[1][warp] = l;
-  }
+  for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) sh[warp].x = t;
+  if (lane == 16) sh[warp].y = t;
   __syncthreads();
-  if (warp != 0) return;
-  s = lane < kSsimFoldThreads / 32 ? s_red[0][lane] : 0.0;
-  l = lane < kSsimFoldThreads / 32 ? s_red[1][lane] : 0.0;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    s += __shfl_xor_sync(0xffffffffu, s, o);
-    l += __shfl_xor_sync(0xffffffffu, l, o);
+  double2 r = make_double2(0.0, 0.0);
+  if (threadIdx.x == 0)
+    for (int w = 0; w < kSsimThreads / 32; ++w) {
+      r.x += sh[w].x;
+      r.y += sh[w].y;
+    }
+  return r;  // valid in thread 0
+}
+
+__global__ void __launch_bounds__(kSsimThreads) k_ssim_fold(const double2* __restrict__ partials, int count,
+                                                            double2* block_sums, unsigned int* counter,
+                                                            double inv_count, double w_l1, double w_ssim,
+                                                            double constant, float* __restrict__ out) {
+  __shared__ double2 s_red[kSsimThreads / 32];
+  double2 v = make_double2(0.0, 0.0);
+#pragma unroll 2
+  for (int i = blockIdx.x * kSsimThreads + threadIdx.x; i < count; i += gridDim.x * kSsimThreads) {
+    const double2 p = partials[i];
+    v.x += p.x;
+    v.y += p.y;
   }
-  if (lane == 0) *out = (float)(w_ssim * (s * inv_count) + w_l1 * (l * inv_count) + constant);
+  v = block_sum_pair(v, s_red);
+  if (threadIdx.x != 0) return;
+  block_sums[blockIdx.x] = v;
+  __threadfence();
+  if (atomicAdd(counter, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  double2 t = make_double2(0.0, 0.0);
+  for (unsigned b = 0; b < gridDim.x; ++b) {
+    t.x += __ldcg(&block_sums[b].x);
+    t.y += __ldcg(&block_sums[b].y);
+  }
+  *out = (float)(w_ssim * (t.x * inv_count) + w_l1 * (t.y * inv_count) + constant);
 }
 
 // dL/dimg1 = g w_ssim (W*a + 2 x W*b + y W*c), g = *dL_dmean; PHOTO: with x clamped, plus
@@ -463,7 +495,7 @@ extern "C" size_t cfgs_ssim_scratch_bytes(int32_t channels, int32_t height, int3
   const SsimDims d = dims(channels, height, width);
   const size_t maps = sizeof(float) * 3 * (size_t)channels * height * width;
   const size_t parts = sizeof(double2) * (size_t)channels * d.tiles_x * d.tiles_y;
-  return align256(maps) + align256(parts);
+  return align256(maps) + align256(parts) + align256(sizeof(double2) * (kSsimFoldBlocks + 1));
 }
 
 namespace {
@@ -478,15 +510,19 @@ int ssim_forward(int32_t channels, int32_t height, int32_t width, const float* i
   const size_t count = (size_t)channels * height * width;
   float* maps = static_cast<float*>(scratch);
   double2* parts = reinterpret_cast<double2*>(static_cast<char*>(scratch) + align256(sizeof(float) * 3 * count));
-  const int tiles = d.tiles_x * d.tiles_y;
+  const int tiles = d.tiles_x * d.tiles_y, pairs = tiles * channels;
+  double2* sums = reinterpret_cast<double2*>(reinterpret_cast<char*>(parts) + align256(sizeof(double2) * (size_t)pairs));
+  unsigned int* counter = reinterpret_cast<unsigned int*>(sums + kSsimFoldBlocks);
   const float inv = (float)(1.0 / (double)count);
   CUtensorMap t1{}, t2{};
   const bool tma = encode_planes(&t1, img1, width, height, channels) && encode_planes(&t2, img2, width, height, channels);
   auto* kernel = photo ? (tma ? k_ssim_fwd<true, true> : k_ssim_fwd<false, true>)
                        : (tma ? k_ssim_fwd<true, false> : k_ssim_fwd<false, false>);
-  kernel<<<dim3(tiles, channels), kSsimThreads, 0, st>>>(d, img1, img2, maps, parts, inv, t1, t2);
-  k_ssim_fold<<<1, kSsimFoldThreads, 0, st>>>(parts, tiles * channels, 1.0 / (double)count, photo ? 1.0 - lambda : 0.0,
-                                              photo ? -lambda : 1.0, photo ? lambda : 0.0, out);
+  kernel<<<dim3(tiles, channels), kSsimThreads, 0, st>>>(d, img1, img2, maps, parts, counter, inv, t1, t2);
+  const int fold_blocks = min(kSsimFoldBlocks, div_up(pairs, kSsimThreads));
+  k_ssim_fold<<<fold_blocks, kSsimThreads, 0, st>>>(parts, pairs, sums, counter, 1.0 / (double)count,
+                                                    photo ? 1.0 - lambda : 0.0, photo ? -lambda : 1.0,
+                                                    photo ? lambda : 0.0, out);
   CFGS_CHECK_LAUNCH(0, st);
   return CFGS_OK;
 }
