@@ -148,6 +148,8 @@ EXPORTS = {
                                        _vp]),
     "cfgs_pointcloud_workspace_bytes": (C.c_size_t, [C.c_int64]),
     "cfgs_knn3_mean_dist2": (C.c_int, [C.c_int64, _vp, _vp, _vp, _vp]),
+    "cfgs_init_gaussians": (C.c_int, [C.c_int64, C.c_int32, _vp, _vp, _vp, C.c_float, _vp, _vp, _vp, _vp, _vp, _vp,
+                                      _vp]),
     "cfgs_voxel_down_sample": (C.c_int, [C.c_int64, _vp, _vp, C.c_double, _vp, _vp, _vp, C.POINTER(C.c_int64),
                                          _vp]),
     "cfgs_ssim_scratch_bytes": (C.c_size_t, [C.c_int32, C.c_int32, C.c_int32]),

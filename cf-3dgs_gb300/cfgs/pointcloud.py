@@ -76,14 +76,18 @@ def gaussians_from_points(points: torch.Tensor, colors: torch.Tensor, sh_degree:
     p = _cuda_f32(points, "gaussians_from_points").reshape(-1, 3)
     col = _cuda_f32(colors, "gaussians_from_points").reshape(-1, 3)
     n = p.shape[0]
-    dc = (col - 0.5) / C0 if view_dependent else col
-    features = torch.zeros((n, 3, (sh_degree + 1) ** 2), dtype=torch.float32, device=p.device)
-    features[:, :3, 0] = dc
-    dist2 = torch.clamp_min(dist_cuda2(p), 0.0000001)
-    scales = torch.log(torch.sqrt(dist2))[..., None].repeat(1, 3)
-    rots = torch.zeros((n, 4), dtype=torch.float32, device=p.device)
-    rots[:, 0] = 1
-    opacities = torch.full((n, 1), math.log(0.1 / 0.9), dtype=torch.float32, device=p.device)
-    return {"xyz": p.clone(), "features_dc": features[:, :, 0:1].transpose(1, 2).contiguous(),
-            "features_rest": features[:, :, 1:].transpose(1, 2).contiguous(), "scaling": scales,
-            "rotation": rots, "opacity": opacities}
+    dc = ((col - 0.5) / C0 if view_dependent else col).to(p.device).expand(n, 3).contiguous()
+    rest = (sh_degree + 1) ** 2 - 1
+    f = dict(dtype=torch.float32, device=p.device)
+    out = {"xyz": torch.empty_like(p), "features_dc": torch.empty((n, 1, 3), **f),
+           "features_rest": torch.empty((n, rest, 3), **f), "scaling": torch.empty((n, 3), **f),
+           "rotation": torch.empty((n, 4), **f), "opacity": torch.empty((n, 1), **f)}
+    if n > 0:
+        dist2 = dist_cuda2(p)
+        native.check(native.load().cfgs_init_gaussians(
+            n, 3 * rest, _ptr(p), _ptr(dc), _ptr(dist2), math.log(0.1 / 0.9), _ptr(out["xyz"]),
+            _ptr(out["features_dc"]), _ptr(out["features_rest"]), _ptr(out["scaling"]), _ptr(out["rotation"]),
+            _ptr(out["opacity"]), stream_handle(p.device)), "cfgs_init_gaussians")
+    if torch.is_grad_enabled() and (p.requires_grad or dc.requires_grad):
+        out["xyz"], out["features_dc"] = p.clone(), dc.reshape(n, 1, 3).clone()  # copies that gradients pass
+    return out

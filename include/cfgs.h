@@ -352,6 +352,13 @@ size_t cfgs_pointcloud_workspace_bytes(int64_t num_points);
  * distances from point i to its three nearest other points (FLT_MAX for missing ones).
  * Exact (Morton-ordered boxes with bounded pruning). */
 int cfgs_knn3_mean_dist2(int64_t num_points, const float* xyz, void* workspace, float* dist2, void* stream);
+/* The initial parameters of create_from_pcd (scene/gaussian_model_cf.py:175-210): positions
+ * and DC colours (dc [N,3], in SH units) copied, `rest_floats` zeros per point (the higher
+ * bands), scaling log(sqrt(max(dist2, 1e-7))) on all three axes, identity rotations and one
+ * opacity logit. out_rotation [N,4] is 16-byte aligned. */
+int cfgs_init_gaussians(int64_t num_points, int32_t rest_floats, const float* xyz, const float* dc,
+                        const float* dist2, float opacity, float* out_xyz, float* out_dc, float* out_rest,
+                        float* out_scaling, float* out_rotation, float* out_opacity, void* stream);
 /* Open3D voxel_down_sample (trainer/trainer.py:507): points (and colours, may be NULL)
  * of each occupied voxel floor((p - (min - s/2)) / s) averaged in float64 in input
  * order; out_xyz/out_rgb need room for num_points rows; *num_voxels receives the count
