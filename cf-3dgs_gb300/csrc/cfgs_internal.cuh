@@ -490,19 +490,21 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) {
 }
 __device__ __forceinline__ float2 splat2(float a) { return make_float2(a, a); }
 
-// gauss_power for the pixels (dx, dy.x) and (dx, dy.y): the same rounding sequence.
-__device__ __forceinline__ float2 gauss_power2(float ca, float cb, float cc, float dx, float2 dy) {
-  float2 e = mul2(splat2(cb), mul2(splat2(dx), dy));
-  e = fma2(mul2(splat2(cc), dy), dy, e);
-  const float cadx = ca * dx;
-  return fma2(splat2(cadx), splat2(dx), e);
+// gauss_power of a pixel pair, the Gaussian's factors given as pairs of equal halves: the
+// same rounding sequence.
+__device__ __forceinline__ float2 gauss_power2(float2 ca, float2 cb, float2 cc, float2 dx, float2 dy) {
+  float2 e = mul2(cb, mul2(dx, dy));
+  e = fma2(mul2(cc, dy), dy, e);
+  return fma2(mul2(ca, dx), dx, e);
 }
 
-// exp_ref_inrange of both halves: the same rounding sequence (fmaf(-k, c, x) is
-// fmaf(k, -c, x) exactly).
+// exp_ref_inrange of both halves: the same results (fmaf(-k, c, x) is fmaf(k, -c, x)
+// exactly). rintf(t) is formed as (t + 1.5 * 2^23) - 1.5 * 2^23, which rounds to the nearest
+// even integer exactly for |t| < 2^22 and leaves the integer in the sum's low bits, so that
+// 2^k is one shift and add: no conversion instruction (a quarter-rate pipe) remains.
 __device__ __forceinline__ float2 exp_ref_inrange2(float2 x) {
-  const float2 t = mul2(x, splat2(1.4426950216293335f));
-  const float2 kf = make_float2(rintf(t.x), rintf(t.y));
+  const float2 t = add2(mul2(x, splat2(1.4426950216293335f)), splat2(12582912.0f));
+  const float2 kf = add2(t, splat2(-12582912.0f));
   float2 r = fma2(kf, splat2(-0.693145751953125f), x);
   r = fma2(kf, splat2(-1.428606765330187e-06f), r);
   float2 p = fma2(splat2(0.00019841270113829523f), r, splat2(0.0013888889225199819f));
@@ -512,7 +514,9 @@ __device__ __forceinline__ float2 exp_ref_inrange2(float2 x) {
   p = fma2(p, r, splat2(0.5f));
   p = fma2(p, r, splat2(1.0f));
   p = fma2(p, r, splat2(1.0f));
-  const float2 sc = make_float2(__int_as_float(((int)kf.x + 127) << 23), __int_as_float(((int)kf.y + 127) << 23));
+  // (k + 127) << 23: the constant's own bits leave the word
+  const float2 sc = make_float2(__uint_as_float((__float_as_uint(t.x) << 23) + 0x3f800000u),
+                                __uint_as_float((__float_as_uint(t.y) << 23) + 0x3f800000u));
   return mul2(p, sc);
 }
 

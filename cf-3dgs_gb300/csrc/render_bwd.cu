@@ -3,7 +3,7 @@
 //
 // Upstream accumulates every (pixel, Gaussian) gradient with a global atomicAdd.
 // Here each tile reduces the gradients of its 256 pixels per instance inside the
-// block (a transposing warp reduction, then a fixed-order sum over the 4 warps) and
+// block (eight instances at a time per warp, then a fixed-order sum over the 4 warps) and
 // writes one 48-byte record per (Gaussian, tile) instance, at the instance's
 // pre-sort index. A Gaussian's instances are contiguous in pre-sort order, so the
 // preprocess backward sums its records in a fixed order: no atomics, bit-identical
@@ -17,46 +17,7 @@ namespace cfgs {
 
 constexpr int kBwdThreads = 128;  // 2 pixels per thread, 4 warps per 16x16 tile
 constexpr int kWarps = kBwdThreads / 32;
-
-// Sums an instance's per-lane terms over the warp. v[0..7] go through a transposing
-// reduction (each step halves the values a lane carries: 4 + 2 + 1 shuffles, then two
-// plain steps), after which lane L holds the total of v[L >> 2]; v[8] (and v[9] with
-// depth gradients) take plain butterflies, every lane ending with the total. With GEOM
-// (only v[0..4] formed, v[5..9] zero) the v[8] butterfly is skipped; the tree that sums
-// v[0..4] is the same either way, so their totals are the same bits.
-template <bool DEPTH, bool GEOM = false>
-__device__ __forceinline__ void warp_reduce_terms(float (&v)[10], int lane) {
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const bool up = lane & 16;
-    const float send = up ? v[k] : v[k + 4];
-    const float keep = up ? v[k + 4] : v[k];
-    v[k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-  }
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const bool up = lane & 8;
-    const float send = up ? v[k] : v[k + 2];
-    const float keep = up ? v[k + 2] : v[k];
-    v[k] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-  }
-  {
-    const bool up = lane & 4;
-    const float send = up ? v[0] : v[1];
-    const float keep = up ? v[1] : v[0];
-    v[0] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-  }
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-  if (!GEOM) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[8] += __shfl_xor_sync(0xffffffffu, v[8], o);
-  }
-  if (DEPTH) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[9] += __shfl_xor_sync(0xffffffffu, v[9], o);
-  }
-}
+constexpr int kSlots = 8;  // instances a warp reduces at a time, four lanes each
 
 // d/dc of mean |clamp(c, 0, 1) - t| as autograd forms it.
 __device__ __forceinline__ float l1_grad(float c, float t, float inv_numel) {
@@ -100,7 +61,7 @@ __device__ __forceinline__ void load_pixel(PixelBwd& p, const RenderBwdArgs<Scen
   p.dA_bg = dA - (__ldg(sd.bg + 0) * p.dC0 + __ldg(sd.bg + 1) * p.dC1 + __ldg(sd.bg + 2) * p.dC2);
 }
 
-// Back-to-front state of a lane's two pixels (.x: row r, .y: row r + 4): upstream
+// Back-to-front state of a lane's two pixels (.x: column c, .y: column c + 4): upstream
 // gradients, the transmittance being unwound, and the colour/depth accumulated behind the
 // current instance (updated right after each contributing instance, which gives the
 // value upstream forms from the previous instance's alpha and colour).
@@ -125,47 +86,47 @@ __device__ __forceinline__ PairBwd make_pair(const PixelBwd& p, const PixelBwd& 
   return P;
 }
 
-// Unwinds one instance at list position c for both pixels and adds their terms to v:
-// with g = G dL/dalpha (G the Gaussian's value at the pixel, d = mean - pixel),
-// v0..v4 += g (dx, dy, dx^2, dx dy, dy^2), v5 += g, v6..v8 += w dL/drgb, v9 += w
-// dL/ddepth (w = alpha T). The per-instance factors (opacity, conic) are applied after
-// the reduction (finish_record). A pixel the instance did not reach in the forward pass
-// keeps its state: its factors are 1 (transmittance) and 0 (alpha, G). Returns whether
-// the instance contributed to either pixel. With GEOM only v0..v4 are formed (the terms
-// of dL/dmean2D and dL/dconic; v5..v8 stay zero), with the same operations.
-template <bool DEPTH, bool GEOM = false>
-__device__ __forceinline__ bool unwind_pair(PairBwd& P, int c, float pxf, float2 pyf, const float4& m, const float4& co,
-                                            const float4* s_rgbd, int j, float (&v)[10]) {
+// A staged instance as the unwinding reads it: every factor twice, so that the packed
+// operations take their operands as loaded, without a move per factor.
+struct StagedInstance {
+  float4 xy;   // (x, x, y, y)
+  float4 ab;   // (ca, ca, cb, cb)
+  float4 co;   // (cc, cc, opacity, opacity)
+  float4 rg;   // (r, r, g, g)
+  float4 bd;   // (b, b, depth, depth)
+};
+__device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
+
+// Unwinds one instance at list position c for both pixels: g = G dL/dalpha (G the
+// Gaussian's value at the pixel) and w = alpha T, zero where the instance did not
+// contribute. A pixel the instance did not reach in the forward pass keeps its state: its
+// alpha and G count as 0. Returns whether the instance contributed to either pixel.
+template <bool DEPTH>
+__device__ __forceinline__ bool unwind_pair(PairBwd& P, int c, float2 px, float2 py, const StagedInstance& s, float thr,
+                                            float2& g, float2& w) {
   const bool in0 = c < (int)P.last0, in1 = c < (int)P.last1;
-  if (!(in0 || in1)) return false;
-  const float dx = m.x - pxf;
-  const float2 dy = sub2(splat2(m.y), pyf);
-  const float2 power = gauss_power2(co.x, co.y, co.z, dx, dy);
-  bool a0 = in0 && !(power.x > 0.0f || power.x < m.z);
-  bool a1 = in1 && !(power.y > 0.0f || power.y < m.z);
+  const float2 dx = sub2(lo2(s.xy), px), dy = sub2(hi2(s.xy), py);
+  const float2 power = gauss_power2(lo2(s.ab), hi2(s.ab), lo2(s.co), dx, dy);
+  bool a0 = in0 && !(power.x > 0.0f || power.x < thr);
+  bool a1 = in1 && !(power.y > 0.0f || power.y < thr);
+  g = w = make_float2(0.f, 0.f);
   if (!(a0 || a1)) return false;
   const float2 G = exp_ref_inrange2(power);
-  float2 alpha = mul2(splat2(co.w), G);
+  float2 alpha = mul2(hi2(s.co), G);
   alpha.x = fminf(CFGS_ALPHA_MAX, alpha.x);
   alpha.y = fminf(CFGS_ALPHA_MAX, alpha.y);
   a0 = a0 && !(alpha.x < CFGS_ALPHA_MIN);
   a1 = a1 && !(alpha.y < CFGS_ALPHA_MIN);
   if (!(a0 || a1)) return false;
-  const float4 col = s_rgbd[j];
-  const float2 om = sub2(splat2(1.0f), alpha);
-  float r0, r1;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(om.x));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(om.y));
-  const float2 inv = make_float2(a0 ? r0 : 1.0f, a1 ? r1 : 1.0f);
   const float2 am = make_float2(a0 ? alpha.x : 0.0f, a1 ? alpha.y : 0.0f);
+  const float2 om = sub2(splat2(1.0f), am);
+  float2 inv;  // 1 where the instance did not contribute (the approximation is exact at 1)
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv.x) : "f"(om.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv.y) : "f"(om.y));
   P.T = mul2(P.T, inv);
-  const float2 w = mul2(am, P.T);
-  if (!GEOM) {
-    v[6] = fmaf(P.dC0.y, w.y, fmaf(P.dC0.x, w.x, v[6]));
-    v[7] = fmaf(P.dC1.y, w.y, fmaf(P.dC1.x, w.x, v[7]));
-    v[8] = fmaf(P.dC2.y, w.y, fmaf(P.dC2.x, w.x, v[8]));
-  }
-  const float2 e0 = sub2(splat2(col.x), P.acc0), e1 = sub2(splat2(col.y), P.acc1), e2 = sub2(splat2(col.z), P.acc2);
+  w = mul2(am, P.T);
+  const float2 e0 = sub2(lo2(s.rg), P.acc0), e1 = sub2(hi2(s.rg), P.acc1), e2 = sub2(lo2(s.bd), P.acc2);
   float2 dLda = mul2(e0, P.dC0);
   dLda = fma2(e1, P.dC1, dLda);
   dLda = fma2(e2, P.dC2, dLda);
@@ -173,23 +134,13 @@ __device__ __forceinline__ bool unwind_pair(PairBwd& P, int c, float pxf, float2
   P.acc1 = fma2(am, e1, P.acc1);
   P.acc2 = fma2(am, e2, P.acc2);
   if (DEPTH) {
-    v[9] = fmaf(P.dD.y, w.y, fmaf(P.dD.x, w.x, v[9]));
-    const float2 ed = sub2(splat2(col.w), P.accd);
+    const float2 ed = sub2(hi2(s.bd), P.accd);
     dLda = fma2(ed, P.dD, dLda);
     P.accd = fma2(am, ed, P.accd);
   }
   dLda = mul2(dLda, P.T);
   dLda = fma2(mul2(P.T_final, inv), P.dA_bg, dLda);
-  const float2 g = mul2(make_float2(a0 ? G.x : 0.0f, a1 ? G.y : 0.0f), dLda);  // d/d opacity
-  const float sg = g.x + g.y;
-  if (!GEOM) v[5] += sg;
-  const float sx = sg * dx;  // both pixels share dx
-  const float2 gy = mul2(g, dy);
-  v[0] += sx;
-  v[1] += gy.x + gy.y;
-  v[2] = fmaf(sx, dx, v[2]);
-  v[3] = fmaf(g.y * dx, dy.y, fmaf(g.x * dx, dy.x, v[3]));
-  v[4] = fmaf(gy.y, dy.y, fmaf(gy.x, dy.x, v[4]));
+  g = mul2(make_float2(a0 ? G.x : 0.0f, a1 ? G.y : 0.0f), dLda);  // d/d opacity
   return true;
 }
 
@@ -207,27 +158,155 @@ __device__ __forceinline__ void finish_record(float4* rec, const float (&s)[10],
   rec[2] = make_float4(s[8], s[9], 0.f, 0.f);
 }
 
-// One block of 128 threads per tile with the forward's pixel boxes (warp w: 8x8 box,
-// lane: rows r and r + 4) and exact shortcuts (box_may_contribute per warp and
-// instance, alpha_threshold per pixel). A lane adds its two pixels' terms before the
-// warp reduction; the cross-warp sum of an instance adds only the warps that kept it
-// (the others' terms are exact zeros). BATCH instances are staged per round; the
-// records do not depend on it (each instance's sums are formed the same way whatever
-// batch it is staged in), so the batch is a schedule choice.
-template <class Scenes, bool DEPTH, int BATCH, bool GEOM = false>
-__global__ void __launch_bounds__(kBwdThreads, 7) k_render_bwd(RenderBwdArgs<Scenes> a) {
+// Shared memory of a block. The gradient terms an instance sums: moments g (dx, dy, dx^2,
+// dx dy, dy^2), and unless GEOM g, w dL/drgb, with DEPTH w dL/ddepth.
+template <bool DEPTH, int BATCH, bool GEOM>
+struct BwdShared {
+  static constexpr int kTerms = GEOM ? 5 : (DEPTH ? 10 : 9);
+  static constexpr int kPlanes = GEOM ? 0 : (DEPTH ? 4 : 3);
+  float4 raw_co[BATCH], raw_rgbd[BATCH];  // the next batch, on its way (cp.async)
+  float2 raw_xy[BATCH];
+  uint32_t raw_pidx[BATCH];
+  StagedInstance inst[BATCH];  // the current batch
+  float thr[BATCH];
+  uint32_t pidx[BATCH];
+  float g[kWarps][kSlots][64];                 // a warp's slots: g per pixel of its 8x8 box (pair_offset)
+  float w[kWarps][GEOM ? 1 : kSlots][GEOM ? 4 : 64];
+  float image_grad[kWarps][GEOM ? 1 : kPlanes][GEOM ? 4 : 64];  // dL/dcolour (and depth) per pixel
+  float part[kWarps][BATCH][kTerms];           // a warp's sums per instance
+  uint8_t reached[BATCH][kWarps];              // 1: the instance reached some pixel of the warp
+  uint32_t max_last;
+};
+
+// Where a warp's 8x8 box keeps a pixel pair (columns q and q + 4 of row y = 4 h + 2 m + l):
+// the eight floats of a lane's rows l, l + 2, l + 4, l + 6 in two 16-byte words per l, the
+// halves of a word swapped for m = 1. Both the pairs' stores (a half-warp at a time) and
+// the 16-byte loads of sum_slots (eight lanes at a time) then meet 32 different banks.
+__device__ __forceinline__ int pair_offset(int q, int y) {
+  const int h = y >> 2, m = (y >> 1) & 1, l = y & 1;
+  return 32 * m + 8 * q + 4 * l + 2 * (h ^ m);
+}
+
+// One warp's sums of its n <= 8 pending instances over the 64 pixels of its box. Four lanes
+// take an instance: lane 4 s + q sums slot s over columns q and q + 4 (one packed pair per
+// row), then the four lanes combine by a transposing exchange. An instance costs about 24
+// warp instructions here; forming every pixel's moments in its own lane and reducing each
+// instance over all 32 lanes by shuffles took about 70. The order of every sum is the one
+// of that reduction — rows y and y + 4, then y and y + 2, y and y + 1, then columns 4, 2
+// and 1 apart — so the records keep its bits. Odd slots take the odd rows first (an
+// exchange of the operands of one addition), so that loads meet no common bank.
+template <bool DEPTH, int BATCH, bool GEOM>
+__device__ __forceinline__ void sum_slots(BwdShared<DEPTH, BATCH, GEOM>& sh, int warp, int lane, int n, int j, int bx0,
+                                          int by0) {
+  using Sh = BwdShared<DEPTH, BATCH, GEOM>;
+  constexpr int kTerms = Sh::kTerms, kPlanes = Sh::kPlanes;
+  const int slot = lane >> 2, q = lane & 3, odd_first = slot & 1;
+  __syncwarp();
+  float v[10];
+#pragma unroll
+  for (int k = 0; k < 10; ++k) v[k] = 0.0f;
+  if constexpr (!GEOM) {  // w dL/dcolour (and depth), apart from the moments: fewer live registers
+    float2 c[kPlanes];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int o = 8 * q + 4 * (i ^ odd_first);
+      const float4 wa = *reinterpret_cast<const float4*>(sh.w[warp][slot] + o);
+      const float4 wb = *reinterpret_cast<const float4*>(sh.w[warp][slot] + o + 32);
+#pragma unroll
+      for (int k = 0; k < kPlanes; ++k) {
+        const float4 da = *reinterpret_cast<const float4*>(sh.image_grad[warp][k] + o);
+        const float4 db = *reinterpret_cast<const float4*>(sh.image_grad[warp][k] + o + 32);
+        const float2 u = add2(fma2(hi2(da), hi2(wa), mul2(lo2(da), lo2(wa))),
+                              fma2(lo2(db), lo2(wb), mul2(hi2(db), hi2(wb))));
+        c[k] = i ? add2(c[k], u) : u;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kPlanes; ++k) v[6 + k] = c[k].x + c[k].y;
+  }
+  __syncwarp();
+  {
+    const float4 xy = sh.inst[j].xy;
+    const float2 dx = sub2(lo2(xy), make_float2((float)(bx0 + q), (float)(bx0 + q + 4)));
+    float2 v2[6];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int l = i ^ odd_first;
+      const float2 y0 = splat2((float)(by0 + l));
+      float2 u[6];
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {  // rows l + 2 m (x) and l + 2 m + 4 (y) of both columns
+        const float4 gv = *reinterpret_cast<const float4*>(sh.g[warp][slot] + 32 * m + 8 * q + 4 * l);
+        const float2 gx = m ? hi2(gv) : lo2(gv), gy = m ? lo2(gv) : hi2(gv);
+        const float2 dyx = sub2(hi2(xy), m ? add2(y0, splat2(2.0f)) : y0);
+        const float2 dyy = sub2(hi2(xy), add2(y0, splat2(m ? 6.0f : 4.0f)));
+        const float2 hx = mul2(gx, dyx), hy = mul2(gy, dyy), sg = add2(gx, gy), sx = mul2(sg, dx);
+        const float2 t1 = add2(hx, hy);
+        const float2 t3 = fma2(mul2(gy, dx), dyy, mul2(mul2(gx, dx), dyx));
+        const float2 t4 = fma2(hy, dyy, mul2(hx, dyx));
+        // scalar products: a packed one would be fused with the addition
+        const float2 t2 = make_float2(__fmul_rn(sx.x, dx.x), __fmul_rn(sx.y, dx.y));
+        u[2] = m ? add2(u[2], t2) : t2;
+        u[0] = m ? add2(u[0], sx) : sx;
+        u[1] = m ? add2(u[1], t1) : t1;
+        u[3] = m ? add2(u[3], t3) : t3;
+        u[4] = m ? add2(u[4], t4) : t4;
+        if (!GEOM) u[5] = m ? add2(u[5], sg) : sg;
+      }
+#pragma unroll
+      for (int k = 0; k < (GEOM ? 5 : 6); ++k) v2[k] = i ? add2(v2[k], u[k]) : u[k];
+    }
+#pragma unroll
+    for (int k = 0; k < (GEOM ? 5 : 6); ++k) v[k] = v2[k].x + v2[k].y;
+  }
+  // over the four lanes: lane q ends with terms 0-2, 3-4, 5-7, 8-9 of the instance (GEOM:
+  // 0-1, 2, 3, 4)
+  const bool up = q & 2, odd = q & 1;
+  constexpr int kHalf = GEOM ? 3 : 5, kQuarter = GEOM ? 2 : 3;
+#pragma unroll
+  for (int k = 0; k < kHalf; ++k) {
+    const float other = k + kHalf < 10 ? v[k + kHalf] : 0.0f;
+    const float send = up ? v[k] : other, keep = up ? other : v[k];
+    v[k] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+  }
+#pragma unroll
+  for (int k = 0; k < kQuarter; ++k) {
+    const float other = k + kQuarter < kHalf ? v[k + kQuarter] : 0.0f;
+    const float send = odd ? v[k] : other, keep = odd ? other : v[k];
+    v[k] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+  }
+  if (slot < n) {
+    if (q == 0) sh.reached[j][warp] = 1;
+    float* part = sh.part[warp][j];
+    const int first = (up ? kHalf : 0) + (odd ? kQuarter : 0), end = min(up ? kTerms : kHalf, first + kQuarter);
+#pragma unroll
+    for (int k = 0; k < kQuarter; ++k)
+      if (first + k < end) part[first + k] = v[k];
+  }
+  __syncwarp();  // the slots are free again
+}
+
+// One block of 128 threads per tile with the forward's pixel boxes (warp w: an 8x8 box,
+// lane: columns q and q + 4 of a row) and exact shortcuts (box_may_contribute per
+// warp and instance, alpha_threshold per pixel). A lane leaves its two pixels' g and w of a
+// contributing instance in the warp's next slot; every eight instances the warp sums its
+// slots (sum_slots). The cross-warp sum of an instance adds only the warps it contributed
+// in (the others' terms are exact zeros). BATCH instances are staged per round; the
+// records do not depend on it (each instance's sums are formed the same way whatever batch
+// it is staged in), so the batch is a schedule choice. GEOM forms only the moments (the
+// terms of dL/dmean2D and dL/dconic), the same bits. Bound by instruction issue, and where
+// fewer tiles than resident blocks run, by a warp's own chain. BLOCKS is the number of
+// resident blocks per SM the registers are cut for (launch_render_bwd_batch). Against the
+// per-instance shuffle reduction: 1,000,000 Gaussians at 1920x1080 984 -> 907 us (912 ->
+// 711 million warp instructions), 16,384 at 256x256 134 -> 94 us, with depth gradients
+// (250,007 at 977x545) 406 -> 313 us, one 640x360 pose solve (GEOM) 218 -> 175 us, 16
+// solves 2989 -> 2429 us.
+template <class Scenes, bool DEPTH, int BATCH, bool GEOM, int BLOCKS>
+__global__ void __launch_bounds__(kBwdThreads, BLOCKS) k_render_bwd(RenderBwdArgs<Scenes> a) {
   static_assert(BATCH % 32 == 0 && BATCH <= kBwdThreads, "whole ballot words, one staged instance per thread");
-  constexpr int kBwdBatch = BATCH;
-  // Staging buffers come in pairs: batch b - 1 is copied asynchronously (cp.async; its
-  // Gaussian ids were loaded a batch earlier) while batch b is unwound; two block
-  // barriers per batch (staged, then partial sums complete).
-  __shared__ float4 s_xyt[2][kBwdBatch];
-  __shared__ float4 s_co[2][kBwdBatch];
-  __shared__ float4 s_rgbd[2][kBwdBatch];
-  __shared__ uint32_t s_pidx[2][kBwdBatch];
-  __shared__ float s_part[kWarps][kBwdBatch][10];
-  __shared__ uint32_t s_keep[kWarps][kBwdBatch / 32];
-  __shared__ uint32_t s_max;
+  using Sh = BwdShared<DEPTH, BATCH, GEOM>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Sh& sh = *reinterpret_cast<Sh*>(smem_raw);
   if ((int64_t)a.counts->num_rendered > a.cap) return;
   const int tile = blockIdx.x;
   const SceneDesc& sd = a.scenes.for_tile(tile);
@@ -235,122 +314,139 @@ __global__ void __launch_bounds__(kBwdThreads, 7) k_render_bwd(RenderBwdArgs<Sce
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int bx0 = (lt % sd.grid_x) * kTileX + (warp & 1) * 8;
   const int by0 = (lt / sd.grid_x) * kTileY + (warp >> 1) * 8;
-  const int px = bx0 + (lane & 7), py0 = by0 + (lane >> 3), py1 = py0 + 4;
+  const int px0 = bx0 + (lane & 3), px1 = px0 + 4, py = by0 + (lane >> 2);
+  const int slot_at = pair_offset(lane & 3, lane >> 2);
   const float bxf0 = (float)bx0, bxf1 = (float)(bx0 + 7), byf0 = (float)by0, byf1 = (float)(by0 + 7);
-  const bool in0 = px < sd.W && py0 < sd.H, in1 = px < sd.W && py1 < sd.H;
-  const float pxf = (float)px, pyf0 = (float)py0, pyf1 = (float)py1;
+  const bool in0 = px0 < sd.W && py < sd.H, in1 = px1 < sd.W && py < sd.H;
+  const float2 px = make_float2((float)px0, (float)px1), pyf = splat2((float)py);
   const uint32_t lo = a.tile_range[tile];
-  const int n = (int)(a.tile_range[tile + 1] - lo);
 
   PixelBwd p0, p1;
-  load_pixel(p0, a, sd, in0, in0 ? (size_t)py0 * sd.W + px : 0);
-  load_pixel(p1, a, sd, in1, in1 ? (size_t)py1 * sd.W + px : 0);
+  load_pixel(p0, a, sd, in0, in0 ? (size_t)py * sd.W + px0 : 0);
+  load_pixel(p1, a, sd, in1, in1 ? (size_t)py * sd.W + px1 : 0);
   PairBwd pp = make_pair(p0, p1);
-  const float2 pyf = make_float2(pyf0, pyf1);
-  if (threadIdx.x == 0) s_max = 0;
+  if constexpr (!GEOM) {
+    *reinterpret_cast<float2*>(sh.image_grad[warp][0] + slot_at) = pp.dC0;
+    *reinterpret_cast<float2*>(sh.image_grad[warp][1] + slot_at) = pp.dC1;
+    *reinterpret_cast<float2*>(sh.image_grad[warp][2] + slot_at) = pp.dC2;
+    if (DEPTH) *reinterpret_cast<float2*>(sh.image_grad[warp][3] + slot_at) = pp.dD;
+  }
+  if (threadIdx.x == 0) sh.max_last = 0;
   __syncthreads();
   const uint32_t my_last = max(p0.last, p1.last);
-  if (my_last) atomicMax(&s_max, my_last);
+  if (my_last) atomicMax(&sh.max_last, my_last);
   // instances at or past the warp's largest contributor count reach none of its pixels
   const int warp_last = (int)__reduce_max_sync(0xffffffffu, my_last);
   __syncthreads();
-  const int max_last = (int)s_max;
+  const int max_last = (int)sh.max_last;
 
   const int t = threadIdx.x;
-  auto count_of = [&](int b) { return min(kBwdBatch, max_last - b * kBwdBatch); };
+  auto count_of = [&](int b) { return min(BATCH, max_last - b * BATCH); };
   uint32_t gnext = 0;
-  auto load_id = [&](int b) { gnext = t < count_of(b) ? a.sorted_gid[lo + b * kBwdBatch + t] : 0u; };
-  auto issue = [&](int b, int buf) {
+  auto load_id = [&](int b) { gnext = t < count_of(b) ? a.sorted_gid[lo + b * BATCH + t] : 0u; };
+  auto issue = [&](int b) {
     if (t < count_of(b)) {
-      const uint32_t i = lo + (uint32_t)(b * kBwdBatch + t);
-      cp_async4(&s_pidx[buf][t], a.sorted_pidx + i);
-      cp_async8(&s_xyt[buf][t], a.xy + gnext);
-      cp_async16(&s_co[buf][t], a.conic_op + gnext);
-      cp_async16(&s_rgbd[buf][t], a.rgbd + gnext);
+      cp_async4(&sh.raw_pidx[t], a.sorted_pidx + lo + (uint32_t)(b * BATCH + t));
+      cp_async8(&sh.raw_xy[t], a.xy + gnext);
+      cp_async16(&sh.raw_co[t], a.conic_op + gnext);
+      cp_async16(&sh.raw_rgbd[t], a.rgbd + gnext);
     }
     cp_async_commit();
   };
-  const int nb = (max_last + kBwdBatch - 1) / kBwdBatch;
+  const int nb = (max_last + BATCH - 1) / BATCH;
   if (nb > 0) {
     load_id(nb - 1);
-    issue(nb - 1, 0);
+    issue(nb - 1);
     if (nb > 1) load_id(nb - 2);
   }
-  for (int k = 0; k < nb; ++k) {
-    const int b = nb - 1 - k, cur = k & 1;
-    const int base = b * kBwdBatch;
+  // Batch b - 1 is copied asynchronously (its Gaussian ids were loaded a batch earlier)
+  // while batch b is unwound; two block barriers per batch (staged, then partial sums
+  // complete).
+  for (int b = nb - 1; b >= 0; --b) {
+    const int base = b * BATCH;
     const int cnt = count_of(b);
     cp_async_wait_all();
-    if (t < cnt) {  // raw (x, y) and conic -> render form, own slot
-      const float4 co = s_co[cur][t];
-      s_xyt[cur][t].z = alpha_threshold(co.w);
-      s_co[cur][t] = make_float4(-0.5f * co.x, -co.y, -0.5f * co.z, co.w);
+    if (t < cnt) {  // raw values -> render form, own slot
+      const float2 m = sh.raw_xy[t];
+      const float4 co = sh.raw_co[t], c = sh.raw_rgbd[t];
+      StagedInstance& s = sh.inst[t];
+      const float ca = -0.5f * co.x, cb = -co.y, cc = -0.5f * co.z;
+      s.xy = make_float4(m.x, m.x, m.y, m.y);
+      s.ab = make_float4(ca, ca, cb, cb);
+      s.co = make_float4(cc, cc, co.w, co.w);
+      s.rg = make_float4(c.x, c.x, c.y, c.y);
+      s.bd = make_float4(c.z, c.z, c.w, c.w);
+      sh.thr[t] = alpha_threshold(co.w);
+      sh.pidx[t] = sh.raw_pidx[t];
+      *reinterpret_cast<uint32_t*>(sh.reached[t]) = 0u;
     }
-    __syncthreads();  // batch b staged; batch b + 1 finished, so its buffers are free
+    __syncthreads();  // batch b staged; batch b + 1 finished
     if (b > 0) {
-      issue(b - 1, cur ^ 1);
+      issue(b - 1);  // into this thread's own raw slot, read above
       if (b > 1) load_id(b - 2);
     }
-    const float4* s_xyt_b = s_xyt[cur];
-    const float4* s_co_b = s_co[cur];
-    const float4* s_rgbd_b = s_rgbd[cur];
-    uint32_t keep[kBwdBatch / 32];
+    uint32_t keep[BATCH / 32];
 #pragma unroll
-    for (int r = 0; r < kBwdBatch / 32; ++r) {
+    for (int r = 0; r < BATCH / 32; ++r) {
       const int j = r * 32 + lane;
       bool kp = false;
       if (j < cnt && base + j < warp_last) {
-        const float4 xyt = s_xyt_b[j];
-        const float4 co = s_co_b[j];
-        kp = box_may_contribute(make_float2(xyt.x, xyt.y), co.x, co.y, co.z, xyt.z, bxf0, bxf1, byf0, byf1);
+        const StagedInstance& s = sh.inst[j];
+        const float4 xy = s.xy, ab = s.ab;
+        kp = box_may_contribute(make_float2(xy.x, xy.z), ab.x, ab.z, s.co.x, sh.thr[j], bxf0, bxf1, byf0, byf1);
       }
       keep[r] = __ballot_sync(0xffffffffu, kp);
-      if (lane == 0) s_keep[warp][r] = keep[r];
     }
+    // Back to front over the kept instances; the warp sums its slots whenever eight are
+    // pending and after the last instance.
+    int r = BATCH / 32 - 1;
+    uint32_t mk = keep[r];
+    for (bool more = true; more;) {
+      int used = 0;    // slots pending
+      int j_slot = 0;  // the instance in this lane's slot
+      while (used < kSlots) {
+        if (mk == 0) {
+          if (r == 0) {
+            more = false;
+            break;
+          }
+          --r;
+          mk = keep[0];
 #pragma unroll
-    for (int r = kBwdBatch / 32 - 1; r >= 0; --r) {
-      uint32_t mk = keep[r];
-      while (mk) {
+          for (int k = 1; k < BATCH / 32; ++k)
+            if (k == r) mk = keep[k];
+          continue;
+        }
         const int bit = 31 - __clz(mk);
         mk &= ~(1u << bit);
         const int j = r * 32 + bit;
-        const int c = base + j;
-        float v[10];
-#pragma unroll
-        for (int q = 0; q < 10; ++q) v[q] = 0.f;
-        const float4 m = s_xyt_b[j];
-        const float4 co = s_co_b[j];
-        const bool contrib = unwind_pair<DEPTH, GEOM>(pp, c, pxf, pyf, m, co, s_rgbd_b, j, v);
-        if (__ballot_sync(0xffffffffu, contrib)) {
-          warp_reduce_terms<DEPTH, GEOM>(v, lane);
-          if ((lane & 3) == 0) s_part[warp][j][lane >> 2] = v[0];
-          if (lane == 0) {
-            s_part[warp][j][8] = v[8];
-            s_part[warp][j][9] = v[9];
-          }
-        } else if (lane < 10) {
-          s_part[warp][j][lane] = 0.f;
-        }
+        float2 g, w;
+        const bool contrib = unwind_pair<DEPTH>(pp, base + j, px, pyf, sh.inst[j], sh.thr[j], g, w);
+        if (!__any_sync(0xffffffffu, contrib)) continue;
+        *reinterpret_cast<float2*>(sh.g[warp][used] + slot_at) = g;
+        if constexpr (!GEOM) *reinterpret_cast<float2*>(sh.w[warp][used] + slot_at) = w;
+        if ((lane >> 2) == used) j_slot = j;
+        ++used;
       }
+      if (used) sum_slots(sh, warp, lane, used, j_slot, bx0, by0);
     }
     __syncthreads();  // every warp's partial sums of batch b are in
     if (t < cnt) {
-      const int j = t;
       float sum[10];
 #pragma unroll
       for (int q = 0; q < 10; ++q) sum[q] = 0.f;
-      bool kept = false;
+      const uint32_t reached = *reinterpret_cast<const uint32_t*>(sh.reached[t]);
 #pragma unroll
       for (int w = 0; w < kWarps; ++w)
-        if ((s_keep[w][j >> 5] >> (j & 31)) & 1u) {
-          kept = true;
+        if ((reached >> (8 * w)) & 0xffu) {
 #pragma unroll
-          for (int q = 0; q < 10; ++q) sum[q] += s_part[w][j][q];
+          for (int q = 0; q < Sh::kTerms; ++q) sum[q] += sh.part[w][t][q];
         }
-      // An instance no warp kept has exact-zero gradients: no record, its byte stays 0.
-      if (kept) {
-        const uint32_t pidx = s_pidx[cur][j];
-        finish_record(a.records + (size_t)kRecordFloat4 * pidx, sum, s_co_b[j]);
+      // An instance that reached no pixel has exact-zero gradients: no record, its byte stays 0.
+      if (reached) {
+        const uint32_t pidx = sh.pidx[t];
+        const float4 ab = sh.inst[t].ab, co = sh.inst[t].co;
+        finish_record(a.records + (size_t)kRecordFloat4 * pidx, sum, make_float4(ab.x, ab.z, co.x, co.z));
         a.written[pidx] = 1;
       }
     }
@@ -358,11 +454,38 @@ __global__ void __launch_bounds__(kBwdThreads, 7) k_render_bwd(RenderBwdArgs<Sce
   // Instances at or past the tile's last contributor reach no pixel: nothing to write.
 }
 
+constexpr int kBwdSms = 152;
+
+template <class Scenes, bool DEPTH, int BATCH, bool GEOM, int BLOCKS>
+void launch_render_bwd_blocks(const RenderBwdArgs<Scenes>& a, int tiles, cudaStream_t st) {
+  static std::atomic<uint64_t> smem_set{0};
+  constexpr int bytes = (int)sizeof(BwdShared<DEPTH, BATCH, GEOM>);
+  // a failure of the attribute call surfaces as a launch error
+  ensure_dynamic_smem(k_render_bwd<Scenes, DEPTH, BATCH, GEOM, BLOCKS>, bytes, smem_set);
+  k_render_bwd<Scenes, DEPTH, BATCH, GEOM, BLOCKS><<<tiles, kBwdThreads, bytes, st>>>(a);
+}
+
+// Registers against resident blocks. With fewer tiles than the blocks would fill, the
+// registers win (fewer instructions per warp): 256 tiles 94 us at four blocks per SM, 99
+// at five; 920 pose tiles 175 us at six, 187 at seven. With many tiles the extra block
+// does: 8160 tiles 907 us at five, 987 at four; 20,960 pose tiles 2429 us at seven, 2551 at
+// six. The depth form, with more live sums, keeps four (2170 tiles: 313 us, 342 at five).
+template <class Scenes, bool DEPTH, int BATCH, bool GEOM>
+void launch_render_bwd_batch(const RenderBwdArgs<Scenes>& a, int tiles, cudaStream_t st) {
+  if constexpr (GEOM) {
+    if (tiles <= 8 * kBwdSms) launch_render_bwd_blocks<Scenes, DEPTH, BATCH, GEOM, 6>(a, tiles, st);
+    else launch_render_bwd_blocks<Scenes, DEPTH, BATCH, GEOM, 7>(a, tiles, st);
+  } else {
+    if (DEPTH || tiles <= 4 * kBwdSms) launch_render_bwd_blocks<Scenes, DEPTH, BATCH, GEOM, 4>(a, tiles, st);
+    else launch_render_bwd_blocks<Scenes, DEPTH, BATCH, GEOM, 5>(a, tiles, st);
+  }
+}
+
 template <class Scenes, bool DEPTH, bool GEOM = false>
 void launch_render_bwd_depth(const RenderBwdArgs<Scenes>& a, int tiles, int batch, cudaStream_t st) {
-  if (batch == 32) k_render_bwd<Scenes, DEPTH, 32, GEOM><<<tiles, kBwdThreads, 0, st>>>(a);
-  else if (batch == 128) k_render_bwd<Scenes, DEPTH, 128, GEOM><<<tiles, kBwdThreads, 0, st>>>(a);
-  else k_render_bwd<Scenes, DEPTH, 64, GEOM><<<tiles, kBwdThreads, 0, st>>>(a);
+  if (batch == 32) launch_render_bwd_batch<Scenes, DEPTH, 32, GEOM>(a, tiles, st);
+  else if (batch == 128) launch_render_bwd_batch<Scenes, DEPTH, 128, GEOM>(a, tiles, st);
+  else launch_render_bwd_batch<Scenes, DEPTH, 64, GEOM>(a, tiles, st);
 }
 
 template <class Scenes>

@@ -29,7 +29,7 @@ struct PairFwd {
 template <bool DEPTH>
 __device__ __forceinline__ void composite_pair(PairFwd& p, float pxf, float2 pyf, const float4& xyt, const float4& co,
                                                const float4* s_rgbd, int j, uint32_t pos1) {
-  const float2 power = gauss_power2(co.x, co.y, co.z, xyt.x - pxf, sub2(splat2(xyt.y), pyf));
+  const float2 power = gauss_power2(splat2(co.x), splat2(co.y), splat2(co.z), splat2(xyt.x - pxf), sub2(splat2(xyt.y), pyf));
   bool a0 = !p.done0 && !(power.x > 0.0f || power.x < xyt.z);
   bool a1 = !p.done1 && !(power.y > 0.0f || power.y < xyt.z);
   if (!(a0 || a1)) return;
