@@ -38,7 +38,7 @@ class L1LossFn(torch.autograd.Function):
     def backward(ctx, grad: torch.Tensor):
         a, b = ctx.saved_tensors
         lib = native.load()
-        g = grad.detach().float().reshape(()).contiguous()
+        g = grad if grad.dtype == torch.float32 else grad.float()  # one element
         dx = torch.empty_like(a)
         native.check(lib.cfgs_l1_loss_backward(a.numel(), _ptr(a), _ptr(b), int(ctx.clamp), g.data_ptr(), _ptr(dx),
                                                stream_handle(a.device)), "cfgs_l1_loss_backward")

@@ -114,6 +114,9 @@ EXPORTS = {
     "cfgs_geom_layout": (None, [C.c_int32, C.POINTER(C.c_size_t)]),
     "cfgs_image_layout": (None, [C.c_int32, C.c_int32, C.POINTER(C.c_size_t)]),
     "cfgs_binning_layout": (None, [C.c_int64, C.POINTER(C.c_size_t)]),
+    "cfgs_preprocess_counted": (C.c_int, [C.POINTER(Settings), C.POINTER(Gaussians), _vp, _vp, _vp, _vp,
+                                          C.POINTER(C.c_uint32), _vp]),
+    "cfgs_wait_counts": (C.c_int, [_vp, C.c_uint32, C.POINTER(Counts), _vp]),
     "cfgs_preprocess_forward": (C.c_int, [C.POINTER(Settings), C.POINTER(Gaussians), _vp, _vp, _vp, _vp]),
     "cfgs_read_counts": (C.c_int, [_vp, C.POINTER(Counts), _vp]),
     "cfgs_render_forward": (C.c_int, [C.POINTER(Settings), C.POINTER(Gaussians), _vp, _vp, _vp, C.c_int64,

@@ -144,7 +144,7 @@ class PoseApply(torch.autograd.Function):
         if cov6 is not None:
             cov_in = cov6.detach().float().contiguous()
             cov_out = torch.empty_like(cov_in)
-        st = torch.cuda.current_stream(xyz_c.device).cuda_stream
+        st = raster.stream_handle(xyz_c.device)
         native.check(lib.cfgs_pose_apply(n, xi_c.data_ptr(), xyz_c.data_ptr(),
                                          cov_in.data_ptr() if cov_in is not None else None, means.data_ptr(),
                                          cov_out.data_ptr() if cov_out is not None else None, st), "cfgs_pose_apply")
@@ -165,7 +165,7 @@ class PoseApply(torch.autograd.Function):
         g_cov_c = g_cov.float().contiguous() if use_cov else None
         scratch = torch.empty(lib.cfgs_pose_scratch_bytes(n), dtype=torch.uint8, device=dev)
         out = torch.empty(6, dtype=torch.float32, device=dev)
-        st = torch.cuda.current_stream(dev).cuda_stream
+        st = raster.stream_handle(dev)
         native.check(lib.cfgs_pose_grad(n, xi_c.data_ptr(), xyz_c.data_ptr(), g_means.data_ptr(),
                                         cov_rot.data_ptr() if use_cov else None,
                                         g_cov_c.data_ptr() if use_cov else None, scratch.data_ptr(),
@@ -193,7 +193,7 @@ class FusedAdam:
 
     def step(self, grad: torch.Tensor):
         lib = native.load()
-        st = torch.cuda.current_stream(self.xi.device).cuda_stream
+        st = raster.stream_handle(self.xi.device)
         native.check(lib.cfgs_pose_adam(self.count, self.xi.data_ptr(), grad.contiguous().data_ptr(),
                                         self.state.data_ptr(), self.lr, self.b1, self.b2, self.eps, st),
                      "cfgs_pose_adam")

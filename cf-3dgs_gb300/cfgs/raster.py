@@ -6,6 +6,7 @@ Everything here calls libcfgs.so through its C ABI; there is no other execution 
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from dataclasses import dataclass
 
 import torch
@@ -36,7 +37,10 @@ def _req(t: torch.Tensor) -> torch.Tensor:
 
 
 def stream_handle(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    """The device's current stream as a raw handle (torch.cuda.current_stream builds a Stream
+    object around it, about 11 us per call against 0.4)."""
+    i = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if i is None else i)
 
 
 def make_settings(rs, keep: list, schedule=None) -> native.Settings:
@@ -87,6 +91,7 @@ class ForwardState:
     binning: torch.Tensor
     num_rendered: int
     radii: torch.Tensor
+    inputs_only: bool = False  # the backward forms the inputs' gradients only
 
 
 class _Timed:
@@ -107,25 +112,17 @@ class _Timed:
             self.timers.setdefault(self.name, []).append(self.ev)
 
 
-_SIDE_STREAMS: dict = {}
+_thread = threading.local()
+_ABANDONED: list = []  # slots of forwards that were interrupted before their count arrived
 
 
-def _read_counts_after(image: torch.Tensor, ready: torch.cuda.Event, dev) -> native.Counts:
-    """The CfgsCounts at the head of an image workspace, copied to pinned host memory
-    on a side stream once `ready` has completed (work enqueued after it on the current
-    stream keeps running). Waits for that copy only."""
-    side = _SIDE_STREAMS.get(dev)
-    if side is None:
-        side = _SIDE_STREAMS[dev] = torch.cuda.Stream(dev)
-    host = torch.empty(C.sizeof(native.Counts), dtype=torch.uint8, pin_memory=True)
-    with torch.cuda.stream(side):
-        side.wait_event(ready)
-        host.copy_(image[: host.numel()], non_blocking=True)
-        done = torch.cuda.Event()
-        done.record(side)
-    image.record_stream(side)
-    done.synchronize()
-    return native.Counts.from_buffer_copy(host.numpy().tobytes())
+def _count_slot() -> torch.Tensor:
+    """The calling thread's page-locked words for the instance count: a thread has one forward
+    waiting for its count at a time."""
+    slot = getattr(_thread, "slot", None)
+    if slot is None:
+        slot = _thread.slot = torch.zeros(4, dtype=torch.int32, pin_memory=True)
+    return slot
 
 
 def forward(rs, means3D, opacities, shs, colors_precomp, scales, rotations, cov3D_precomp, timers=None):
@@ -143,25 +140,30 @@ def forward(rs, means3D, opacities, shs, colors_precomp, scales, rotations, cov3
     geom = torch.empty(lib.cfgs_geom_bytes(N), dtype=torch.uint8, device=dev)
     image = torch.empty(lib.cfgs_image_bytes(W, H), dtype=torch.uint8, device=dev)
     radii = torch.empty(N, dtype=torch.int32, device=dev)
-    with _Timed(timers, "preprocess"):
-        native.check(lib.cfgs_preprocess_forward(C.byref(s), C.byref(g), geom.data_ptr(), image.data_ptr(),
-                                                 radii.data_ptr() if N else None, st), "cfgs_preprocess_forward")
-    # K is final here; the depth sort does not need it, so it is enqueued before the host
-    # waits for K (read on a side stream), and keeps the GPU busy meanwhile.
-    k_ready = torch.cuda.Event()
-    k_ready.record(torch.cuda.current_stream(dev))
-    with _Timed(timers, "depth_sort"):
-        native.check(lib.cfgs_depth_order(N, geom.data_ptr(), st), "cfgs_depth_order")
-    counts = _read_counts_after(image, k_ready, dev)
+    color = torch.empty((3, H, W), dtype=torch.float32, device=dev)
+    depth = torch.empty((1, H, W), dtype=torch.float32, device=dev)
+    alpha = torch.empty((1, H, W), dtype=torch.float32, device=dev)
+    slot, ticket, counts = _count_slot(), C.c_uint32(), native.Counts()
+    try:
+        with _Timed(timers, "preprocess"):
+            native.check(lib.cfgs_preprocess_counted(C.byref(s), C.byref(g), geom.data_ptr(), image.data_ptr(),
+                                                     radii.data_ptr() if N else None, slot.data_ptr(), C.byref(ticket),
+                                                     st), "cfgs_preprocess_counted")
+        # The depth sort does not need K, so it is enqueued before the host waits for K, and
+        # keeps the GPU busy meanwhile.
+        with _Timed(timers, "depth_sort"):
+            native.check(lib.cfgs_depth_order(N, geom.data_ptr(), st), "cfgs_depth_order")
+        native.check(lib.cfgs_wait_counts(slot.data_ptr(), ticket, C.byref(counts), st), "cfgs_wait_counts")
+    except BaseException:
+        _ABANDONED.append(slot)  # the kernel may still write to it
+        _thread.slot = None
+        raise
     if counts.flags & native.FLAG_FRUSTUM_VIOLATION:
         raise RuntimeError("prefiltered=True but a Gaussian lies at view z <= 0.2 (outside the frustum)")
     if counts.flags & native.FLAG_CAPACITY_OVERFLOW:
         raise RuntimeError("more than 2^31 tile instances")
     K = int(counts.num_rendered)
     binning = torch.empty(lib.cfgs_binning_bytes(K), dtype=torch.uint8, device=dev)
-    color = torch.empty((3, H, W), dtype=torch.float32, device=dev)
-    depth = torch.empty((1, H, W), dtype=torch.float32, device=dev)
-    alpha = torch.empty((1, H, W), dtype=torch.float32, device=dev)
     with _Timed(timers, "bin"):
         native.check(lib.cfgs_bin_instances(C.byref(s), C.byref(g), geom.data_ptr(), image.data_ptr(),
                                             binning.data_ptr(), K, st), "cfgs_bin_instances")
@@ -174,7 +176,8 @@ def forward(rs, means3D, opacities, shs, colors_precomp, scales, rotations, cov3
 
 def backward(rs, state: ForwardState, means3D, opacities, shs, colors_precomp, scales, rotations,
              cov3D_precomp, grad_color, grad_depth, grad_alpha, timers=None):
-    """Returns (dmeans2D, dcolors, dopacity, dmeans3D, dcov3D, dsh, dscales, drotations)."""
+    """Returns (dmeans2D, dcolors, dopacity, dmeans3D, dcov3D, dsh, dscales, drotations); with
+    state.inputs_only, None for dcolors of SH colours and dcov3D of scales and rotations."""
     lib = native.load()
     dev = means3D.device
     keep: list = []
@@ -189,10 +192,10 @@ def backward(rs, state: ForwardState, means3D, opacities, shs, colors_precomp, s
     scratch = torch.empty(lib.cfgs_backward_scratch_bytes(K), dtype=torch.uint8, device=dev)
     f = dict(device=dev, dtype=torch.float32)
     d_m2 = torch.empty((N, 3), **f)
-    d_col = torch.empty((N, 3), **f)
+    d_col = torch.empty((N, 3), **f) if shs is None or not state.inputs_only else None
     d_op = torch.empty((N, 1), **f)
     d_m3 = torch.empty((N, 3), **f)
-    d_cov = torch.empty((N, 6), **f)
+    d_cov = torch.empty((N, 6), **f) if cov3D_precomp is not None or not state.inputs_only else None
     d_sh = torch.empty_like(shs) if shs is not None else None
     d_sc = torch.empty((N, 3), **f) if cov3D_precomp is None else None
     d_rot = torch.empty((N, 4), **f) if cov3D_precomp is None else None
@@ -247,9 +250,10 @@ class RasterizeGaussiansFn(torch.autograd.Function):
                 print("\nAn error occurred in the rasteriser forward; inputs saved to snapshot_fw.dump.")
             raise
         ctx.raster_settings = raster_settings
+        state.inputs_only = True
         ctx.state = state
         ctx.has = (sh is not None, colors_precomp is not None, cov3Ds_precomp is not None)
-        ctx.save_for_backward(*[a if a is not None else torch.empty(0) for a in args])
+        ctx.save_for_backward(*args)
         ctx.mark_non_differentiable(radii)
         # Outputs the loss does not use (often depth and alpha) arrive as None rather than
         # as zero tensors, so the backward skips their terms (the gradients are the same).
@@ -260,12 +264,7 @@ class RasterizeGaussiansFn(torch.autograd.Function):
     def backward(ctx, grad_color, grad_radii, grad_depth, grad_alpha):
         means3D, opac, sh, colors_precomp, scales, rotations, cov3Ds = ctx.saved_tensors
         has_sh, has_col, has_cov = ctx.has
-        sh = sh if has_sh else None
-        colors_precomp = colors_precomp if has_col else None
-        cov3Ds = cov3Ds if has_cov else None
-        if not has_cov:
-            pass
-        else:
+        if has_cov:
             scales = rotations = None
         rs = ctx.raster_settings
         if grad_color is None:

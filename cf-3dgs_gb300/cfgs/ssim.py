@@ -42,7 +42,7 @@ class SsimFn(torch.autograd.Function):
         a, b, scratch = ctx.saved_tensors
         lib = native.load()
         C, H, W = (int(x) for x in a.shape)
-        g = grad.detach().float().reshape(()).contiguous()
+        g = grad if grad.dtype == torch.float32 else grad.float()  # one element
         d1 = torch.empty_like(a)
         native.check(lib.cfgs_ssim_backward(C, H, W, _ptr(a), _ptr(b), _ptr(scratch), g.data_ptr(), _ptr(d1),
                                             stream_handle(a.device)), "cfgs_ssim_backward")
@@ -77,7 +77,7 @@ class PhotometricFn(torch.autograd.Function):
     def backward(ctx, grad: torch.Tensor):
         a, b, scratch = ctx.saved_tensors
         C, H, W = (int(x) for x in a.shape)
-        g = grad.detach().float().reshape(()).contiguous()
+        g = grad if grad.dtype == torch.float32 else grad.float()  # one element
         d = torch.empty_like(a)
         native.check(native.load().cfgs_photometric_backward(C, H, W, _ptr(a), _ptr(b), ctx.lambda_dssim, _ptr(scratch),
                                                              _ptr(g), _ptr(d), stream_handle(a.device)),

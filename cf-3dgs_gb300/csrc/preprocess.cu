@@ -302,8 +302,11 @@ void launch_preprocess(const PreArgs<Scenes>& a, int blocks, cudaStream_t st) {
 template void launch_preprocess<SingleScene>(const PreArgs<SingleScene>&, int, cudaStream_t);
 template void launch_preprocess<SceneTable>(const PreArgs<SceneTable>&, int, cudaStream_t);
 
-// Instance count K = sum of the per-block touched sums (one block of 1024 threads).
-__global__ void __launch_bounds__(1024) k_scan(const uint32_t* block_sums, int num_blocks, CfgsCounts* counts) {
+// Instance count K = sum of the per-block touched sums (one block of 1024 threads). With
+// `host` (page-locked host memory) the counts also go there, followed by the ticket the
+// host waits for.
+__global__ void __launch_bounds__(1024) k_scan(const uint32_t* block_sums, int num_blocks, CfgsCounts* counts,
+                                               volatile uint32_t* host, uint32_t ticket) {
   __shared__ unsigned long long sh[32];
   unsigned long long v = 0;
   for (int i = threadIdx.x; i < num_blocks; i += blockDim.x) v += block_sums[i];
@@ -313,8 +316,16 @@ __global__ void __launch_bounds__(1024) k_scan(const uint32_t* block_sums, int n
   if (threadIdx.x == 0) {
     unsigned long long K = 0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) K += sh[w];
-    counts->num_rendered = K > 0xffffffffull ? 0xffffffffu : (uint32_t)K;
-    if (K > 0x7fffffffull) atomicOr(&counts->flags, CFGS_FLAG_CAPACITY_OVERFLOW);
+    const uint32_t rendered = K > 0xffffffffull ? 0xffffffffu : (uint32_t)K;
+    counts->num_rendered = rendered;
+    const uint32_t flags = counts->flags | (K > 0x7fffffffull ? CFGS_FLAG_CAPACITY_OVERFLOW : 0u);
+    counts->flags = flags;  // the preprocess, which raises the other flag, is over
+    if (host) {
+      host[0] = rendered;
+      host[1] = flags;
+      __threadfence_system();
+      host[2] = ticket;
+    }
   }
 }
 
@@ -331,7 +342,7 @@ __global__ void __launch_bounds__(256) k_mark_visible(int n, const float* means,
 }
 
 void launch_scan(uint32_t* block_sums, int num_blocks, CfgsCounts* counts, cudaStream_t st) {
-  k_scan<<<1, 1024, 0, st>>>(block_sums, num_blocks, counts);
+  k_scan<<<1, 1024, 0, st>>>(block_sums, num_blocks, counts, nullptr, 0u);
 }
 
 }  // namespace cfgs
@@ -366,8 +377,8 @@ static bool settings_ok(const CfgsSettings* s) {
          s->image_height <= 65535 * kTileY;
 }
 
-extern "C" int cfgs_preprocess_forward(const CfgsSettings* s, const CfgsGaussians* g, void* geom,
-                                       void* image, int32_t* radii, void* stream) {
+static int preprocess_forward(const CfgsSettings* s, const CfgsGaussians* g, void* geom, void* image, int32_t* radii,
+                              uint32_t* host_slot, uint32_t ticket, void* stream) {
   if (!settings_ok(s) || !g || !geom || !image) return CFGS_ERR_INVALID_ARGUMENT;
   if (g->num_gaussians < 0) return CFGS_ERR_INVALID_ARGUMENT;
   if (g->num_gaussians > 0) {
@@ -397,9 +408,46 @@ extern "C" int cfgs_preprocess_forward(const CfgsSettings* s, const CfgsGaussian
     k_preprocess<SingleScene><<<GL.num_blocks, kPreprocessBlock, 0, st>>>(a);
     CFGS_CHECK_LAUNCH(s->debug, st);
   }
-  launch_scan(gv.block_sums, GL.num_blocks, iv.counts, st);
+  k_scan<<<1, 1024, 0, st>>>(gv.block_sums, GL.num_blocks, iv.counts, host_slot, ticket);
   CFGS_CHECK_LAUNCH(s->debug, st);
   return CFGS_OK;
+}
+
+extern "C" int cfgs_preprocess_forward(const CfgsSettings* s, const CfgsGaussians* g, void* geom, void* image,
+                                       int32_t* radii, void* stream) {
+  return preprocess_forward(s, g, geom, image, radii, nullptr, 0u, stream);
+}
+
+extern "C" int cfgs_preprocess_counted(const CfgsSettings* s, const CfgsGaussians* g, void* geom, void* image,
+                                       int32_t* radii, uint32_t* host_slot, uint32_t* ticket, void* stream) {
+  if (!host_slot || !ticket) return CFGS_ERR_INVALID_ARGUMENT;
+  void* dev = nullptr;
+  if (cudaHostGetDevicePointer(&dev, host_slot, 0) != cudaSuccess) {
+    cudaGetLastError();  // not page-locked memory: an argument error, not a launch failure
+    return CFGS_ERR_INVALID_ARGUMENT;
+  }
+  static std::atomic<uint32_t> next_ticket{0};
+  do *ticket = next_ticket.fetch_add(1, std::memory_order_relaxed) + 1u;
+  while (*ticket == 0);  // a fresh slot holds zero
+  return preprocess_forward(s, g, geom, image, radii, static_cast<uint32_t*>(dev), *ticket, stream);
+}
+
+// The wait reads the slot's ticket word until the kernel's write arrives; every thousand
+// reads it asks the stream for an error or for having finished without the write.
+extern "C" int cfgs_wait_counts(const uint32_t* host_slot, uint32_t ticket, CfgsCounts* out, void* stream) {
+  if (!host_slot || !out) return CFGS_ERR_INVALID_ARGUMENT;
+  for (bool finished = false;; ) {
+    for (int i = 0; i < 1000; ++i)
+      if (__atomic_load_n(&host_slot[2], __ATOMIC_ACQUIRE) == ticket) {
+        out->num_rendered = host_slot[0];
+        out->flags = host_slot[1];
+        return CFGS_OK;
+      }
+    if (finished) return CFGS_ERR_LAUNCH;
+    const cudaError_t e = cudaStreamQuery((cudaStream_t)stream);
+    if (e == cudaSuccess) finished = true;  // one more look, then give up
+    else if (e != cudaErrorNotReady) return CFGS_ERR_LAUNCH;
+  }
 }
 
 extern "C" int cfgs_read_counts(const void* image, CfgsCounts* out, void* stream) {

@@ -155,9 +155,11 @@ __device__ __forceinline__ void gaussian_backward(const PreBwdArgs<Scenes>& a, c
       a.out.dL_dmeans2D[3 * idx + 1] = dndc_y;
       a.out.dL_dmeans2D[3 * idx + 2] = 0.f;
       a.out.dL_dopacity[idx] = acc[5];
-      a.out.dL_dcolors[3 * idx + 0] = dcol[0];
-      a.out.dL_dcolors[3 * idx + 1] = dcol[1];
-      a.out.dL_dcolors[3 * idx + 2] = dcol[2];
+      if (a.out.dL_dcolors) {
+        a.out.dL_dcolors[3 * idx + 0] = dcol[0];
+        a.out.dL_dcolors[3 * idx + 1] = dcol[1];
+        a.out.dL_dcolors[3 * idx + 2] = dcol[2];
+      }
     }
 
     float V[16], P[16];
@@ -251,7 +253,7 @@ __device__ __forceinline__ void gaussian_backward(const PreBwdArgs<Scenes>& a, c
     dcov[1] = 2.f * da * T0[0] * T0[1] + db * (T0[0] * T1[1] + T0[1] * T1[0]) + 2.f * dc * T1[0] * T1[1];
     dcov[2] = 2.f * da * T0[0] * T0[2] + db * (T0[0] * T1[2] + T0[2] * T1[0]) + 2.f * dc * T1[0] * T1[2];
     dcov[4] = 2.f * da * T0[1] * T0[2] + db * (T0[1] * T1[2] + T0[2] * T1[1]) + 2.f * dc * T1[1] * T1[2];
-    if (!pose_only)
+    if (!pose_only && a.out.dL_dcov3D)
       for (int k = 0; k < 6; ++k) a.out.dL_dcov3D[6 * idx + k] = dcov[k];
     float dT0[3], dT1[3];
     for (int i = 0; i < 3; ++i) {
@@ -353,12 +355,13 @@ template <class Scenes>
 __device__ __forceinline__ void zero_gradients(const PreBwdArgs<Scenes>& a, int64_t idx, int M, float* dsh_dst) {
   for (int k = 0; k < 3; ++k) {
     a.out.dL_dmeans2D[3 * idx + k] = 0.f;
-    a.out.dL_dcolors[3 * idx + k] = 0.f;
+    if (a.out.dL_dcolors) a.out.dL_dcolors[3 * idx + k] = 0.f;
     a.out.dL_dmeans3D[3 * idx + k] = 0.f;
     if (a.out.dL_dscales) a.out.dL_dscales[3 * idx + k] = 0.f;
   }
   a.out.dL_dopacity[idx] = 0.f;
-  for (int k = 0; k < 6; ++k) a.out.dL_dcov3D[6 * idx + k] = 0.f;
+  if (a.out.dL_dcov3D)
+    for (int k = 0; k < 6; ++k) a.out.dL_dcov3D[6 * idx + k] = 0.f;
   if (a.out.dL_drotations)
     for (int k = 0; k < 4; ++k) a.out.dL_drotations[4 * idx + k] = 0.f;
   if (dsh_dst)

@@ -553,7 +553,8 @@ extern "C" int cfgs_preprocess_backward(const CfgsSettings* s, const CfgsGaussia
     return CFGS_ERR_INVALID_ARGUMENT;
   if (g->num_gaussians == 0) return CFGS_OK;
   if (g->num_gaussians < 0 || !radii || !g->means3D || !g->opacities) return CFGS_ERR_INVALID_ARGUMENT;
-  if (!out->dL_dmeans2D || !out->dL_dcolors || !out->dL_dopacity || !out->dL_dmeans3D || !out->dL_dcov3D)
+  if (!out->dL_dmeans2D || !out->dL_dopacity || !out->dL_dmeans3D || (!out->dL_dcolors && !g->shs) ||
+      (!out->dL_dcov3D && g->cov3D_precomp))
     return CFGS_ERR_INVALID_ARGUMENT;
   if (!g->cov3D_precomp && (!out->dL_dscales || !out->dL_drotations || !g->scales || !g->rotations))
     return CFGS_ERR_INVALID_ARGUMENT;

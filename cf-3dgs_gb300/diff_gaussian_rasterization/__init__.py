@@ -74,17 +74,6 @@ class GaussianRasterizer(nn.Module):
         if ((scales is None or rotations is None) and cov3D_precomp is None) or (
                 (scales is not None or rotations is not None) and cov3D_precomp is not None):
             raise Exception("Please provide exactly one of either scale/rotation pair or precomputed 3D covariance!")
-        empty = torch.Tensor([])
-        if shs is None:
-            shs = empty
-        if colors_precomp is None:
-            colors_precomp = empty
-        if scales is None:
-            scales = empty
-        if rotations is None:
-            rotations = empty
-        if cov3D_precomp is None:
-            cov3D_precomp = empty
         return rasterize_gaussians(means3D, means2D, shs, colors_precomp, opacities, scales, rotations,
                                    cov3D_precomp, rs)
 

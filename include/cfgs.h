@@ -114,7 +114,9 @@ typedef struct CfgsGaussians {
 } CfgsGaussians;
 
 /* Gradient outputs of the backward pass (the 8 tensors upstream returns, in its
- * order). Every non-null array is fully overwritten (zeros for culled Gaussians). */
+ * order). Every non-null array is fully overwritten (zeros for culled Gaussians).
+ * dL_dcolors may be NULL with SH colours and dL_dcov3D with scales and rotations (neither
+ * is then an input's gradient). */
 typedef struct CfgsGradients {
   float* dL_dmeans2D;   /* [N,3] d/d(NDC x, NDC y), third column 0             */
   float* dL_dcolors;    /* [N,3] d/d(per-Gaussian RGB)                        */
@@ -173,6 +175,17 @@ int cfgs_preprocess_forward(const CfgsSettings* settings, const CfgsGaussians* g
 /* Copies the CfgsCounts of an image workspace to host memory and synchronises
  * `stream`. (Upstream reads num_rendered back the same way.) */
 int cfgs_read_counts(const void* image, CfgsCounts* counts_host, void* stream);
+
+/* cfgs_preprocess_forward whose counts also reach the host on their own, without a copy or
+ * an event: the count kernel writes them to `host_slot` (four page-locked uint32, zero at
+ * first; one call at a time per slot, until cfgs_wait_counts has returned) and then the
+ * ticket returned in *ticket (never zero, no two calls' the same for 2^32 calls).
+ * cfgs_wait_counts returns them once they are there (it reads the slot; it does not
+ * synchronise `stream`, so work enqueued in between keeps running), or CFGS_ERR_LAUNCH when
+ * the stream has failed or finished without them. */
+int cfgs_preprocess_counted(const CfgsSettings* settings, const CfgsGaussians* gaussians, void* geom, void* image,
+                            int32_t* radii, uint32_t* host_slot, uint32_t* ticket, void* stream);
+int cfgs_wait_counts(const uint32_t* host_slot, uint32_t ticket, CfgsCounts* counts_host, void* stream);
 
 /* ---- rasteriser forward, phase 2 ---------------------------------------------
  * Replaces duplicateWithKeys / SortPairs / identifyTileRanges / render: sorts the
