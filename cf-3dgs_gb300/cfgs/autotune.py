@@ -49,8 +49,11 @@ _thread = threading.local()
 
 
 def c_schedule(s: Schedule | None = None) -> "native.RenderSchedule":
-    """The C struct of schedule s (default: the calling thread's current schedule)."""
-    s = get_schedule() if s is None else s
+    """The C struct of schedule s (default: the calling thread's current schedule, or zeros,
+    the library's own choice for the call's size, when it has set none)."""
+    s = getattr(_thread, "schedule", None) if s is None else s
+    if s is None:
+        return native.RenderSchedule()
     return native.RenderSchedule(s.fwd_batch, s.fwd_warps, s.bwd_batch, s.bin_launch)
 
 
@@ -64,18 +67,18 @@ def set_schedule(s: Schedule) -> None:
 
 def get_schedule() -> Schedule:
     """The calling thread's current schedule (DEFAULT until set)."""
-    return getattr(_thread, "schedule", DEFAULT)
+    return getattr(_thread, "schedule", None) or DEFAULT
 
 
 @contextmanager
 def using(s: Schedule):
     """Runs the body under schedule s (in this thread) and restores the previous one."""
-    old = get_schedule()
+    old = getattr(_thread, "schedule", None)
     set_schedule(s)
     try:
         yield s
     finally:
-        set_schedule(old)
+        _thread.schedule = old
 
 
 def bucket(n: int) -> int:

@@ -431,17 +431,18 @@ __device__ __forceinline__ float gauss_power(float ca, float cb, float cc, float
   return fmaf(ca * dx, dx, e);
 }
 
-// exp_ref for x in [-103, 0] (and NaN): the same operation sequence without the range
-// guards, and the scaling by 2^k as one multiply — exact, and equal to exp_ref's
-// two-step scaling, whenever the result is a normal float (k >= -125), which holds
-// for every x the render kernels pass (see alpha_threshold).
+// exp_ref for x in [-103, 0] (and NaN): the same results without the range guards. The
+// scaling by 2^k is one multiply — exact, and equal to exp_ref's two-step scaling, whenever
+// the result is a normal float (k >= -125), which holds for every x the render kernels pass
+// (see alpha_threshold). rintf(t) is formed as (t + 1.5 * 2^23) - 1.5 * 2^23, which rounds
+// to the nearest even integer exactly for |t| < 2^22 and leaves the integer in the sum's low
+// bits, so that 2^k is one shift and add: no conversion instruction (a quarter-rate pipe)
+// remains.
 __device__ __forceinline__ float exp_ref_inrange(float x) {
-  const float kLog2e = 1.4426950216293335f;
-  const float kLn2Hi = 0.693145751953125f;
-  const float kLn2Lo = 1.428606765330187e-06f;
-  float kf = rintf(x * kLog2e);
-  float r = fmaf(-kf, kLn2Hi, x);
-  r = fmaf(-kf, kLn2Lo, r);
+  const float t = __fadd_rn(__fmul_rn(x, 1.4426950216293335f), 12582912.0f);
+  const float kf = __fadd_rn(t, -12582912.0f);
+  float r = fmaf(kf, -0.693145751953125f, x);
+  r = fmaf(kf, -1.428606765330187e-06f, r);
   float p = 0.00019841270113829523f;
   p = fmaf(p, r, 0.0013888889225199819f);
   p = fmaf(p, r, 0.008333333767950535f);
@@ -450,7 +451,8 @@ __device__ __forceinline__ float exp_ref_inrange(float x) {
   p = fmaf(p, r, 0.5f);
   p = fmaf(p, r, 1.0f);
   p = fmaf(p, r, 1.0f);
-  return p * __int_as_float(((int)kf + 127) << 23);
+  // (k + 127) << 23: the constant's own bits leave the word
+  return p * __uint_as_float((__float_as_uint(t) << 23) + 0x3f800000u);
 }
 
 // ---------------------------------------------------------------------------
@@ -499,9 +501,7 @@ __device__ __forceinline__ float2 gauss_power2(float2 ca, float2 cb, float2 cc, 
 }
 
 // exp_ref_inrange of both halves: the same results (fmaf(-k, c, x) is fmaf(k, -c, x)
-// exactly). rintf(t) is formed as (t + 1.5 * 2^23) - 1.5 * 2^23, which rounds to the nearest
-// even integer exactly for |t| < 2^22 and leaves the integer in the sum's low bits, so that
-// 2^k is one shift and add: no conversion instruction (a quarter-rate pipe) remains.
+// exactly).
 __device__ __forceinline__ float2 exp_ref_inrange2(float2 x) {
   const float2 t = add2(mul2(x, splat2(1.4426950216293335f)), splat2(12582912.0f));
   const float2 kf = add2(t, splat2(-12582912.0f));

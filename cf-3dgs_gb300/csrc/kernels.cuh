@@ -122,9 +122,11 @@ template <class Scenes>
 void launch_render_bwd(const RenderBwdArgs<Scenes>& a, int tiles, cudaStream_t st);
 template <class Scenes>
 void launch_preprocess_bwd(const PreBwdArgs<Scenes>& a, int blocks, cudaStream_t st);
-// The schedule a call uses: zeros become the default {128, 4, 64}; false when the
+// The schedule a call over `tiles` tiles (0: unknown), with room for `capacity` instances of
+// `gaussians` Gaussians, uses: zeros become the default for those sizes; false when the
 // combination is not one the render kernels are instantiated for.
-bool resolve_schedule(const CfgsRenderSchedule& in, CfgsRenderSchedule* out);
+bool resolve_schedule(const CfgsRenderSchedule& in, int64_t tiles, int64_t gaussians, int64_t capacity,
+                      CfgsRenderSchedule* out);
 
 void launch_batch_pose_init(int count, const float* xi, const float* adam_state, PoseState* states, double b1,
                             double b2, cudaStream_t st);

@@ -274,6 +274,8 @@ __global__ void __launch_bounds__(kPreprocessBlock) k_preprocess(PreArgs<Scenes>
             rgb = sh_to_rgb(sd.sh_degree, shp, p, campos, &cl,
                             sd.sh_coeffs == kMaxShCoeffs && (((uintptr_t)shp) & 15) == 0);
           }
+          if (!(isfinite(rgb.x) && isfinite(rgb.y) && isfinite(rgb.z) && isfinite(t.z)))
+            atomicOr(&a.counts->flags, CFGS_FLAG_NONFINITE_COLOUR);
           a.geom.xy[idx] = pimg;
           a.geom.conic_op[idx] = make_float4(conic.x, conic.y, conic.z, a.g.opacities[idx]);
           a.geom.rgbd[idx] = make_float4(rgb.x, rgb.y, rgb.z, t.z);

@@ -5,35 +5,49 @@
 // descriptor table for batched solves); the arithmetic is the same for both.
 // Compiled with -fmad=false; the fmaf() calls are the only fused operations, and the
 // CPU oracle performs the same sequence.
+#include <type_traits>
+
 #include "cfgs_internal.cuh"
 #include "kernels.cuh"
 
 namespace cfgs {
 
-// Launch schedules (cfgs_set_render_schedule): kRenderBatch instances staged per round
-// and 4 or 8 warps per tile. Every schedule gives bit-identical outputs: each pixel sees
-// the same instances in the same order with the same arithmetic.
+// Launch schedules: kRenderBatch instances staged per round and 4 or 8 warps per tile. Every
+// schedule gives bit-identical outputs: each pixel sees the same instances in the same
+// order with the same arithmetic.
 constexpr int kRenderBatch = 128;
 
-// Front-to-back state of a lane's two pixels (.x: row r, .y: row r + 4) and one
+// A staged instance as the compositing reads it: every factor twice, so that the packed
+// operations take their operands as loaded, without a move per factor.
+struct StagedInstance {
+  float4 xy;   // (x, x, y, y)
+  float4 ab;   // (ca, ca, cb, cb)
+  float4 co;   // (cc, cc, opacity, opacity)
+};
+
+// Front-to-back state of a lane's two pixels (.x: column c, .y: column c + 4) and one
 // compositing step of both: the published loop body per pixel, with the exponential
 // skipped below the alpha threshold (exact, see alpha_threshold). The arithmetic runs on
 // packed pairs (bit-identical to the scalar operations); each pixel's decisions are its
-// own, and a pixel that does not take the step keeps its state.
+// own, and a pixel that does not take the step keeps its state: its weight is 0, which adds
+// nothing times a finite colour. ODD (a view with a colour or depth that is not finite)
+// selects instead.
 struct PairFwd {
   float2 T, C0, C1, C2, D;
   uint32_t last0, last1;
   bool done0, done1;
 };
 
-template <bool DEPTH>
-__device__ __forceinline__ void composite_pair(PairFwd& p, float pxf, float2 pyf, const float4& xyt, const float4& co,
+template <bool DEPTH, bool ODD>
+__device__ __forceinline__ void composite_pair(PairFwd& p, float2 px, float2 py, const StagedInstance& s, float thr,
                                                const float4* s_rgbd, int j, uint32_t pos1) {
-  const float2 power = gauss_power2(splat2(co.x), splat2(co.y), splat2(co.z), splat2(xyt.x - pxf), sub2(splat2(xyt.y), pyf));
-  bool a0 = !p.done0 && !(power.x > 0.0f || power.x < xyt.z);
-  bool a1 = !p.done1 && !(power.y > 0.0f || power.y < xyt.z);
+  const float2 dx = sub2(make_float2(s.xy.x, s.xy.y), px), dy = sub2(make_float2(s.xy.z, s.xy.w), py);
+  const float2 power = gauss_power2(make_float2(s.ab.x, s.ab.y), make_float2(s.ab.z, s.ab.w),
+                                    make_float2(s.co.x, s.co.y), dx, dy);
+  bool a0 = !p.done0 && !(power.x > 0.0f || power.x < thr);
+  bool a1 = !p.done1 && !(power.y > 0.0f || power.y < thr);
   if (!(a0 || a1)) return;
-  float2 alpha = mul2(splat2(co.w), exp_ref_inrange2(power));
+  float2 alpha = mul2(make_float2(s.co.z, s.co.w), exp_ref_inrange2(power));
   alpha.x = fminf(CFGS_ALPHA_MAX, alpha.x);
   alpha.y = fminf(CFGS_ALPHA_MAX, alpha.y);
   a0 = a0 && !(alpha.x < CFGS_ALPHA_MIN);
@@ -43,69 +57,114 @@ __device__ __forceinline__ void composite_pair(PairFwd& p, float pxf, float2 pyf
   const bool end0 = a0 && test_T.x < CFGS_T_MIN, end1 = a1 && test_T.y < CFGS_T_MIN;
   p.done0 = p.done0 || end0;
   p.done1 = p.done1 || end1;
-  const bool u0 = a0 && !end0, u1 = a1 && !end1;
-  if (!(u0 || u1)) return;
   const float4 c = s_rgbd[j];
   const float2 w = mul2(alpha, p.T);
-  const float2 C0 = fma2(splat2(c.x), w, p.C0);
-  const float2 C1 = fma2(splat2(c.y), w, p.C1);
-  const float2 C2 = fma2(splat2(c.z), w, p.C2);
-  const float2 D = DEPTH ? fma2(splat2(c.w), w, p.D) : p.D;
-  if (u0) {
-    p.C0.x = C0.x;
-    p.C1.x = C1.x;
-    p.C2.x = C2.x;
-    p.D.x = D.x;
-    p.T.x = test_T.x;
-    p.last0 = pos1;
-  }
-  if (u1) {
-    p.C0.y = C0.y;
-    p.C1.y = C1.y;
-    p.C2.y = C2.y;
-    p.D.y = D.y;
-    p.T.y = test_T.y;
-    p.last1 = pos1;
-  }
+  const bool u0 = a0 && !end0, u1 = a1 && !end1;
+  const float2 wm = ODD ? w : make_float2(u0 ? w.x : 0.0f, u1 ? w.y : 0.0f);
+  auto add = [&](float2& C, float v) {
+    const float2 sum = fma2(splat2(v), wm, C);
+    C = ODD ? make_float2(u0 ? sum.x : C.x, u1 ? sum.y : C.y) : sum;
+  };
+  add(p.C0, c.x);
+  add(p.C1, c.y);
+  add(p.C2, c.z);
+  if (DEPTH) add(p.D, c.w);
+  p.T = make_float2(u0 ? test_T.x : p.T.x, u1 ? test_T.y : p.T.y);
+  p.last0 = u0 ? pos1 : p.last0;
+  p.last1 = u1 ? pos1 : p.last1;
 }
 
-// One block of 32 WARPS threads per 16x16 tile. With 4 warps, warp w covers the 8x8
-// pixel box (8 (w & 1), 8 (w >> 1)) and each lane two pixels of it, rows r and r + 4;
-// with 8 warps, warp w covers the 8x4 box (8 (w & 1), 4 (w >> 1)) and each lane one
-// pixel (the pair's second pixel is never inside). Batches of BATCH instances are
-// gathered into shared memory (per-Gaussian data stays L2-resident).
-// Two exact shortcuts skip work whose outcome is known: each warp keeps only the
-// instances whose alpha >= 1/255 ellipse can reach its box (box_may_contribute, one test
-// per instance and warp), and a pixel skips the exponential when the exponent lies
-// below the instance's alpha_threshold. Neither changes a decision of the published
-// algorithm, so every output — contributor counts included, which count positions in
-// the tile's list — is what the plain per-pixel loop gives. Compositing runs front to
-// back; a warp stops when its pixels are saturated and the block when all are.
-template <class Scenes, int BATCH, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS) k_render_fwd(RenderArgs<Scenes> a) {
-  static_assert(BATCH % 32 == 0 && (WARPS == 4 || WARPS == 8), "whole ballot words; 8x8 or 8x4 warp boxes");
+// The same step of one pixel (the 8-warp form's lanes have one each).
+struct OneFwd {
+  float T, C0, C1, C2, D;
+  uint32_t last;
+  bool done;
+};
+
+template <bool DEPTH, bool ODD>
+__device__ __forceinline__ void composite_one(OneFwd& p, float px, float py, const StagedInstance& s, float thr,
+                                              const float4* s_rgbd, int j, uint32_t pos1) {
+  const float power = gauss_power(s.ab.x, s.ab.z, s.co.x, s.xy.x - px, s.xy.z - py);
+  bool a = !p.done && !(power > 0.0f || power < thr);
+  if (!a) return;
+  const float alpha = fminf(CFGS_ALPHA_MAX, s.co.z * exp_ref_inrange(power));
+  if (alpha < CFGS_ALPHA_MIN) return;
+  const float test_T = p.T * (1.0f - alpha);
+  if (test_T < CFGS_T_MIN) {
+    p.done = true;
+    return;
+  }
+  const float4 c = s_rgbd[j];
+  const float w = alpha * p.T;
+  p.C0 = fmaf(c.x, w, p.C0);
+  p.C1 = fmaf(c.y, w, p.C1);
+  p.C2 = fmaf(c.z, w, p.C2);
+  if (DEPTH) p.D = fmaf(c.w, w, p.D);
+  p.T = test_T;
+  p.last = pos1;
+}
+
+// Warp boxes and pixels of a lane: with 4 warps, warp w covers the 8x8 pixel box
+// (8 (w & 1), 8 (w >> 1)) and each lane two pixels of a row, columns c and c + 4; with 8
+// warps, warp w covers the 8x4 box (8 (w & 1), 4 (w >> 1)) and each lane one pixel.
+template <bool DEPTH, bool ODD>
+struct PairPixels {
+  PairFwd p;
+  float2 px, py;
+  __device__ __forceinline__ PairPixels(int x, int y, bool in0, bool in1)
+      : p{splat2(1.0f), splat2(0.0f), splat2(0.0f), splat2(0.0f), splat2(0.0f), 0u, 0u, !in0, !in1},
+        px(make_float2((float)x, (float)(x + 4))),
+        py(splat2((float)y)) {}
+  __device__ __forceinline__ bool done() const { return p.done0 && p.done1; }
+  __device__ __forceinline__ void step(const StagedInstance& s, float thr, const float4* rgbd, int j, uint32_t pos1) {
+    composite_pair<DEPTH, ODD>(p, px, py, s, thr, rgbd, j, pos1);
+  }
+  __device__ __forceinline__ OneFwd pixel(int q) const {
+    return q ? OneFwd{p.T.y, p.C0.y, p.C1.y, p.C2.y, p.D.y, p.last1, p.done1}
+             : OneFwd{p.T.x, p.C0.x, p.C1.x, p.C2.x, p.D.x, p.last0, p.done0};
+  }
+};
+template <bool DEPTH, bool ODD>
+struct OnePixel {
+  OneFwd p;
+  float px, py;
+  __device__ __forceinline__ OnePixel(int x, int y, bool in0, bool)
+      : p{1.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0u, !in0}, px((float)x), py((float)y) {}
+  __device__ __forceinline__ bool done() const { return p.done; }
+  __device__ __forceinline__ void step(const StagedInstance& s, float thr, const float4* rgbd, int j, uint32_t pos1) {
+    composite_one<DEPTH, ODD>(p, px, py, s, thr, rgbd, j, pos1);
+  }
+  __device__ __forceinline__ OneFwd pixel(int) const { return p; }
+};
+
+template <int BATCH>
+struct FwdShared {
+  StagedInstance inst[BATCH];
+  float4 rgbd[BATCH];
+  float thr[BATCH];
+};
+
+template <class Scenes, int BATCH, int WARPS, bool ODD>
+__device__ __forceinline__ void composite_tile(const RenderArgs<Scenes>& a, FwdShared<BATCH>& sh) {
+  constexpr bool kDepth = !Scenes::kBatched;  // batches ask for no depth
   constexpr int kThreads = 32 * WARPS;
   constexpr int kBoxRows = WARPS == 4 ? 8 : 4;
-  __shared__ float4 s_xyt[BATCH];   // (x, y, alpha threshold, -)
-  __shared__ float4 s_co[BATCH];    // (ca, cb, cc, opacity)
-  __shared__ float4 s_rgbd[BATCH];
-  if ((int64_t)a.counts->num_rendered > a.cap) return;
+  constexpr int kPixels = WARPS == 4 ? 2 : 1;
+  using Pixels = std::conditional_t<WARPS == 4, PairPixels<kDepth, ODD>, OnePixel<kDepth, ODD>>;
   const int tile = blockIdx.x;
   const SceneDesc& sd = a.scenes.for_tile(tile);
   const int lt = tile - sd.tile_base;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int bx0 = (lt % sd.grid_x) * kTileX + (warp & 1) * 8;
   const int by0 = (lt / sd.grid_x) * kTileY + (warp >> 1) * kBoxRows;
-  const int px = bx0 + (lane & 7), py0 = by0 + (lane >> 3), py1 = py0 + 4;
+  const int px0 = bx0 + (WARPS == 4 ? lane & 3 : lane & 7);
+  const int py = by0 + (WARPS == 4 ? lane >> 2 : lane >> 3);
   const float bxf0 = (float)bx0, bxf1 = (float)(bx0 + 7), byf0 = (float)by0, byf1 = (float)(by0 + kBoxRows - 1);
-  const bool in0 = px < sd.W && py0 < sd.H, in1 = WARPS == 4 && px < sd.W && py1 < sd.H;
-  const float pxf = (float)px, pyf0 = (float)py0, pyf1 = (float)py1;
   const uint32_t lo = a.tile_range[tile];
   const int n = (int)(a.tile_range[tile + 1] - lo);
-  PairFwd pp{splat2(1.0f), splat2(0.0f), splat2(0.0f), splat2(0.0f), splat2(0.0f), 0u, 0u, !in0, !in1};
-  const float2 pyf = make_float2(pyf0, pyf1);
+  Pixels pixels(px0, py, px0 < sd.W && py < sd.H, px0 + 4 < sd.W && py < sd.H);
   for (int base = 0; base < n; base += BATCH) {
-    if (__syncthreads_count(pp.done0 && pp.done1) == kThreads) break;
+    if (__syncthreads_count(pixels.done()) == kThreads) break;
 #pragma unroll
     for (int j = threadIdx.x; j < BATCH; j += kThreads) {
       const int i = base + j;
@@ -113,9 +172,12 @@ __global__ void __launch_bounds__(32 * WARPS) k_render_fwd(RenderArgs<Scenes> a)
         uint32_t g = a.sorted_gid[lo + i];
         float2 m = a.xy[g];
         float4 co = a.conic_op[g];
-        s_xyt[j] = make_float4(m.x, m.y, alpha_threshold(co.w), 0.0f);
-        s_co[j] = make_float4(-0.5f * co.x, -co.y, -0.5f * co.z, co.w);
-        s_rgbd[j] = a.rgbd[g];
+        const float ca = -0.5f * co.x, cb = -co.y, cc = -0.5f * co.z;
+        sh.inst[j].xy = make_float4(m.x, m.x, m.y, m.y);
+        sh.inst[j].ab = make_float4(ca, ca, cb, cb);
+        sh.inst[j].co = make_float4(cc, cc, co.w, co.w);
+        sh.thr[j] = alpha_threshold(co.w);
+        sh.rgbd[j] = a.rgbd[g];
       }
     }
     __syncthreads();
@@ -126,43 +188,62 @@ __global__ void __launch_bounds__(32 * WARPS) k_render_fwd(RenderArgs<Scenes> a)
       const int j = r * 32 + lane;
       bool k = false;
       if (j < cnt) {
-        const float4 xyt = s_xyt[j];
-        const float4 co = s_co[j];
-        k = box_may_contribute(make_float2(xyt.x, xyt.y), co.x, co.y, co.z, xyt.z, bxf0, bxf1, byf0, byf1);
+        const float4 xy = sh.inst[j].xy, ab = sh.inst[j].ab;
+        k = box_may_contribute(make_float2(xy.x, xy.z), ab.x, ab.z, sh.inst[j].co.x, sh.thr[j], bxf0, bxf1, byf0, byf1);
       }
       keep[r] = __ballot_sync(0xffffffffu, k);
     }
 #pragma unroll
     for (int r = 0; r < BATCH / 32; ++r) {
-      if (__all_sync(0xffffffffu, pp.done0 && pp.done1)) break;
+      if (__all_sync(0xffffffffu, pixels.done())) break;
       uint32_t mk = keep[r];
       while (mk) {
         const int j = r * 32 + __ffs(mk) - 1;
         mk &= mk - 1;
-        const float4 xyt = s_xyt[j];
-        const float4 co = s_co[j];
-        const uint32_t pos1 = (uint32_t)(base + j + 1);
-        composite_pair<!Scenes::kBatched>(pp, pxf, pyf, xyt, co, s_rgbd, j, pos1);  // batches ask for no depth
+        pixels.step(sh.inst[j], sh.thr[j], sh.rgbd, j, (uint32_t)(base + j + 1));
       }
     }
   }
   const size_t HW = (size_t)sd.W * sd.H;
   float* col = a.out_color + 3 * (size_t)sd.pix_base;
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const int py = q ? py1 : py0;
-    if (!(q ? in1 : in0)) continue;
-    const float T = q ? pp.T.y : pp.T.x;
+  for (int q = 0; q < kPixels; ++q) {
+    const int px = px0 + 4 * q;
+    if (px >= sd.W || py >= sd.H) continue;
+    const OneFwd p = pixels.pixel(q);
     const size_t pix = (size_t)py * sd.W + px;
     const size_t gp = (size_t)sd.pix_base + pix;
-    a.final_T[gp] = T;
-    a.n_contrib[gp] = q ? pp.last1 : pp.last0;
-    col[pix] = fmaf(T, __ldg(sd.bg + 0), q ? pp.C0.y : pp.C0.x);
-    col[HW + pix] = fmaf(T, __ldg(sd.bg + 1), q ? pp.C1.y : pp.C1.x);
-    col[2 * HW + pix] = fmaf(T, __ldg(sd.bg + 2), q ? pp.C2.y : pp.C2.x);
-    if (a.out_depth) a.out_depth[gp] = q ? pp.D.y : pp.D.x;
-    if (a.out_alpha) a.out_alpha[gp] = 1.0f - T;
+    a.final_T[gp] = p.T;
+    a.n_contrib[gp] = p.last;
+    col[pix] = fmaf(p.T, __ldg(sd.bg + 0), p.C0);
+    col[HW + pix] = fmaf(p.T, __ldg(sd.bg + 1), p.C1);
+    col[2 * HW + pix] = fmaf(p.T, __ldg(sd.bg + 2), p.C2);
+    if (a.out_depth) a.out_depth[gp] = p.D;
+    if (a.out_alpha) a.out_alpha[gp] = 1.0f - p.T;
   }
+}
+
+// One block of 32 WARPS threads per 16x16 tile. Batches of BATCH instances are gathered
+// into shared memory (per-Gaussian data stays L2-resident).
+// Two exact shortcuts skip work whose outcome is known: each warp keeps only the
+// instances whose alpha >= 1/255 ellipse can reach its box (box_may_contribute, one test
+// per instance and warp), and a pixel skips the exponential when the exponent lies
+// below the instance's alpha_threshold. Neither changes a decision of the published
+// algorithm, so every output — contributor counts included, which count positions in
+// the tile's list — is what the plain per-pixel loop gives. Compositing runs front to
+// back; a warp stops when its pixels are saturated and the block when all are.
+// Bound by instruction issue (75% busy at 1M Gaussians 1080p), and with few tiles by a
+// warp's own chain. Every factor is staged twice and masked weights are added instead of
+// results moved under predicates: 489 -> 457 million warp instructions at 1080p (517 us both
+// ways, fewer warps ready), 127 -> 121 us for one 640x360 pose solve, 80 -> 74 us for 256
+// tiles; the default shapes (resolve_schedule) then take the latter two to 108 and 58 us.
+template <class Scenes, int BATCH, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, WARPS == 4 ? 9 : 6) k_render_fwd(RenderArgs<Scenes> a) {
+  static_assert(BATCH % 32 == 0 && (WARPS == 4 || WARPS == 8), "whole ballot words; 8x8 or 8x4 warp boxes");
+  __shared__ FwdShared<BATCH> sh;
+  if ((int64_t)a.counts->num_rendered > a.cap) return;
+  if (WARPS == 4 && (a.counts->flags & CFGS_FLAG_NONFINITE_COLOUR)) composite_tile<Scenes, BATCH, WARPS, true>(a, sh);
+  else composite_tile<Scenes, BATCH, WARPS, false>(a, sh);
 }
 
 template <class Scenes>
@@ -180,9 +261,24 @@ void launch_render_fwd(const RenderArgs<Scenes>& a, int tiles, cudaStream_t st) 
 template void launch_render_fwd<SingleScene>(const RenderArgs<SingleScene>&, int, cudaStream_t);
 template void launch_render_fwd<SceneTable>(const RenderArgs<SceneTable>&, int, cudaStream_t);
 
-bool resolve_schedule(const CfgsRenderSchedule& in, CfgsRenderSchedule* out) {
+// The default shape. Eight warps of one pixel per lane issue more instructions per pixel
+// than four of two, but their 8x4 boxes keep fewer instances, and a warp's chain is
+// shorter. They win with at most two tiles per SM, where a tile's longest warp sets the
+// time (256 tiles: 58 against 74 us), and with small Gaussians, which reach fewer than four
+// tiles each (one 640x360 pose solve, 2.1 tiles each: 108 against 121 us; 16 solves: 1455
+// against 1535 us). With larger ones four win (1M at 1920x1080, 12.4 tiles each: 517 against
+// 649 us; 250,007 at 977x545, 4.5 each: 204 against 216 us).
+constexpr int64_t kFewTiles = 2 * 152;
+constexpr int64_t kSmallTouch = 4;
+
+bool resolve_schedule(const CfgsRenderSchedule& in, int64_t tiles, int64_t gaussians, int64_t capacity,
+                      CfgsRenderSchedule* out) {
   if (in.bin_launch != 0 && in.bin_launch != 1) return false;
   if (in.fwd_batch == 0 && in.fwd_warps == 0 && in.bwd_batch == 0) {
+    if (tiles > 0 && (tiles <= kFewTiles || capacity < kSmallTouch * gaussians)) {
+      *out = CfgsRenderSchedule{256, 8, 64, in.bin_launch};
+      return true;
+    }
     *out = CfgsRenderSchedule{kRenderBatch, 4, 64, in.bin_launch};
     return true;
   }
@@ -201,7 +297,7 @@ using namespace cfgs;
 extern "C" int cfgs_render_schedule_check(const CfgsRenderSchedule* s, CfgsRenderSchedule* resolved) {
   if (!s) return CFGS_ERR_INVALID_ARGUMENT;
   CfgsRenderSchedule r;
-  if (!resolve_schedule(*s, &r)) return CFGS_ERR_INVALID_ARGUMENT;
+  if (!resolve_schedule(*s, 0, 0, 0, &r)) return CFGS_ERR_INVALID_ARGUMENT;
   if (resolved) *resolved = r;
   return CFGS_OK;
 }
@@ -232,7 +328,7 @@ extern "C" int cfgs_composite_forward(const CfgsSettings* s, int32_t num_gaussia
   ra.out_alpha = out_alpha;
   ra.cap = capacity;
   ra.counts = iv.counts;
-  if (!resolve_schedule(s->schedule, &ra.sched)) return CFGS_ERR_INVALID_ARGUMENT;
+  if (!resolve_schedule(s->schedule, IL.num_tiles, num_gaussians, capacity, &ra.sched)) return CFGS_ERR_INVALID_ARGUMENT;
   launch_render_fwd(ra, IL.num_tiles, st);
   CFGS_CHECK_LAUNCH(s->debug, st);
   return CFGS_OK;

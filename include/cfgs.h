@@ -50,6 +50,8 @@ typedef enum CfgsStatus {
                                          /* that call's outputs are invalid               */
 #define CFGS_FLAG_BARRIER_TIMEOUT 0x8u   /* a bounded grid-wide wait of the one-launch    */
                                          /* binning ran out; outputs are invalid          */
+#define CFGS_FLAG_NONFINITE_COLOUR 0x10u /* a visible Gaussian's colour or depth is not   */
+                                         /* finite (information, not an error)            */
 
 /* Tile size of the screen-space binning (pixels). */
 #define CFGS_TILE_X 16
@@ -69,8 +71,9 @@ typedef enum CfgsStatus {
  *              sort, emission, tile sort, tile ranges) as one launch per stage, 1 as one
  *              persistent cooperative launch with a bounded grid-wide wait between
  *              stages (same outputs)
- * All-zero fields mean the default {128, 4, 64, 0}; an unsupported combination makes the
- * call return CFGS_ERR_INVALID_ARGUMENT. */
+ * All-zero fields mean the default: {128, 4, 64, 0}, or {256, 8, 64, 0} for a call over at
+ * most 304 tiles or with room for fewer than four instances per Gaussian (the resolved
+ * schedule reported below is the former); an unsupported combination makes the call return CFGS_ERR_INVALID_ARGUMENT. */
 typedef struct CfgsRenderSchedule {
   int32_t fwd_batch, fwd_warps, bwd_batch, bin_launch;
 } CfgsRenderSchedule;
