@@ -5,23 +5,32 @@
 // one global stable radix sort over 32 + log2(tiles) bits. Here the depth part is
 // sorted once per Gaussian instead of once per instance:
 //   1. depth sort: stable LSD radix sort of the N depth keys (4 passes of 8 bits), so
-//      the Gaussians come out by (depth, id);
-//   2. emission: the instances are written in that order (a Gaussian's tiles in
-//      row-major order of its tile rectangle), with coalesced stores; an instance's
-//      index is its position in this list;
+//      the Gaussians come out by (depth, id), and the prefix of their tile counts in that
+//      order: an instance's index is its position in the list of all Gaussians' tiles
+//      (row-major in the tile rectangle) in depth order;
+//   2. tile keys: that list's tile indices, written in order (the list's other columns
+//      are not: its Gaussian is found again from the prefix, its index is its position);
 //   3. tile sort: stable LSD radix sort of the instances by tile index alone
-//      (ceil(log2 tiles) bits, at most 8 per pass: 2 passes at 1080p).
+//      (ceil(log2 tiles) bits, at most 8 per pass: 2 passes at 1080p). The first pass's
+//      scatter reads the keys and finds the Gaussians.
 // A stable sort by tile of a list ordered by (depth, id) is ordered by (tile, depth,
 // id): exactly the stable sort of upstream's keys over instances emitted by id. The
 // last tile pass also counts the instances of every tile (runs of equal tiles), and a
 // scan turns the counts into tile ranges.
 //
-// Every radix pass is three launches over chunks of kSortChunk elements: count (digit
-// histogram per chunk), scan (per digit, over chunks: the chunk's first global slot),
-// scatter (rank inside the chunk, stage in shared memory by digit, then write each
-// digit's run to its global slots). Ranking inside a chunk is stable: warp w owns the
-// contiguous slice [w C/8, (w+1) C/8) and walks it 32 elements per round; lanes with
-// equal digits find each other with one ballot per digit bit.
+// Every radix pass is three launches over chunks of elements: count (digit histogram per
+// chunk), scan (per digit, over chunks: the chunk's first global slot), scatter (rank
+// inside the chunk, exchange through shared memory by digit, then write each digit's run
+// to its global slots). Ranking inside a chunk is stable: a warp owns a contiguous slice
+// and walks it 64 elements per round; lanes with equal digits meet in a mask in shared
+// memory.
+//
+// The scatters are bound by shared memory (84 to 87 % of its wavefronts), the rest by latency
+// per block, so a thread holds its keys in registers, all loads in flight at once, an element
+// goes through shared memory once, as one 8-byte value beside or with its key, and the first
+// tile pass carries positions only. 1,000,000 Gaussians, 12.4 million instances, 8160 tiles:
+// the depth order 114 us, tile keys 48, tile sort 172, ranges 5; with the list written out
+// first, chunks staged through shared memory and a ballot per digit bit, 130, 84, 250 and 10.
 #include "cfgs_internal.cuh"
 #include "kernels.cuh"
 
@@ -29,23 +38,36 @@ namespace cfgs {
 
 constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kMaxDigitBits = 8;
 
-// One radix pass over elements [0, n) split into chunks of `chunk` elements. Keys come
-// from key_in, or (depth mode) from the geometry: the depth bits of Gaussians that
-// touch a tile, ~0 for the others, so they sort last. Payloads come from val_in /
-// aux_in, or are the element's own index when those are NULL.
+// Elements per thread of a radix chunk: 8 for long lists, whose digit runs get longer (12.4
+// million instances, two passes: keys 41, counts 14, scatters 72 and 72 us; with 4 elements
+// 42, 20, 83 and 86), 4 where the wide chunks would fill the GPU only a few times (1,000,000
+// depths: scatters 12.4 us each, with 8 elements 13.3): from 16 of those blocks per SM.
+constexpr int64_t kWideListMin = 16 * 152 * 4 * kSortThreads;
+inline int radix_items(int64_t n) { return n >= kWideListMin ? 8 : 4; }
+
+// What a radix pass carries beside the key.
+enum Payload {
+  kValue,      // one value: val_in, or the element's own index when that is NULL
+  kFirstPair,  // Gaussian and position of an instance, found from the list (InstanceList)
+  kPair,       // the same, from pair_in
+};
+
+// One radix pass over elements [0, n).
 struct SortPass {
+  const uint32_t* depth_touched;  // first depth pass: the count forms the keys from these (key_form)
+  const float4* depth_rgbd;
+  uint32_t* key_form;
   const uint32_t* key_in;
   const uint32_t* val_in;
-  const uint32_t* aux_in;
-  const float4* depth_rgbd;    // depth mode
-  const uint32_t* depth_touched;
+  const uint2* pair_in;
   uint32_t* key_out;           // NULL: keys are not written (last pass)
   uint32_t* val_out;
-  uint32_t* aux_out;           // NULL: one payload
+  uint32_t* aux_out;           // last tile pass: the pairs' positions (val_out: the Gaussians)
+  uint2* pair_out;             // tile passes before the last
   uint32_t* tile_count;        // last tile pass: instances per tile
   int shift, bits;
+  int items;                   // elements per thread (radix_items): chunks of kSortThreads * items
   int64_t n;                   // element count, when counts is NULL
   const CfgsCounts* counts;    // element count = num_rendered (nothing to do above cap)
   int64_t cap;
@@ -54,93 +76,29 @@ struct SortPass {
   uint32_t* digit_totals;      // [1 << bits], written by the scan
 };
 
+// Shared memory of a block of any stage.
+constexpr int kScanItems = 8;
+template <int ITEMS>
+struct CountShared {
+  uint32_t whist[kSortWarps][kSortDigits];  // per-warp digit counters, then first positions
+  uint32_t mark[kSortWarps * ITEMS];        // bit i set where a Gaussian's instances begin
+  uint32_t mark_before[kSortWarps * ITEMS]; // marks in earlier words
+  uint32_t scan[kScanItems * 32 + 4];
+};
+template <int ITEMS>
+struct BinShared : CountShared<ITEMS> {
+  union {
+    uint32_t same[2][kSortWarps][kSortDigits];  // ranking: the lanes that hold a digit, for two elements per lane
+    uint2 buf[kSortThreads * ITEMS];            // a chunk in digit order
+  };
+  uint32_t keys[kSortThreads * ITEMS];      // its keys, where buf holds pairs
+  uint32_t slot[kSortDigits];               // global slot minus position of a digit's first element
+};
+
 __device__ __forceinline__ uint32_t pass_elements(const SortPass& p) {
   if (!p.counts) return (uint32_t)p.n;
   const int64_t k = (int64_t)p.counts->num_rendered;
   return k > p.cap ? 0u : (uint32_t)k;
-}
-
-// Loads the keys of elements [c0 + 4 j, c0 + 4 j + 4) (those below n) with one vector
-// load where the four are in range.
-template <bool DEPTH>
-__device__ __forceinline__ uint4 load_keys4(const SortPass& p, uint32_t i, uint32_t n) {
-  uint4 k = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
-  if (DEPTH) {
-    uint32_t* kk = &k.x;
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (i + e < n) kk[e] = p.depth_touched[i + e] ? __float_as_uint(p.depth_rgbd[i + e].w) : 0xffffffffu;
-  } else if (i + 3 < n) {
-    k = *reinterpret_cast<const uint4*>(p.key_in + i);
-  } else {
-    uint32_t* kk = &k.x;
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (i + e < n) kk[e] = p.key_in[i + e];
-  }
-  return k;
-}
-
-__device__ __forceinline__ uint4 load_u32x4(const uint32_t* a, uint32_t i, uint32_t n) {
-  if (i + 3 < n) return *reinterpret_cast<const uint4*>(a + i);
-  uint4 v = make_uint4(0u, 0u, 0u, 0u);
-  uint32_t* vv = &v.x;
-#pragma unroll
-  for (int e = 0; e < 4; ++e)
-    if (i + e < n) vv[e] = a[i + e];
-  return v;
-}
-
-// Lanes of `active` whose digit equals this lane's: one ballot per digit bit. Every
-// lane of the warp must call it.
-__device__ __forceinline__ unsigned digit_peers(uint32_t d, int bits, unsigned active) {
-  unsigned peers = active;
-#pragma unroll
-  for (int b = 0; b < kMaxDigitBits; ++b) {
-    if (b < bits) {
-      const bool set = (d >> b) & 1u;
-      const unsigned bal = __ballot_sync(0xffffffffu, set);
-      peers &= set ? bal : ~bal;
-    }
-  }
-  return peers;
-}
-
-// Digit histogram of one chunk (per-warp shared-memory counters), written to
-// chunk_counts[d][chunk].
-template <int CHUNK, bool DEPTH>
-__device__ __forceinline__ void sort_count_block(const SortPass& p, uint32_t bid) {
-  __shared__ uint32_t hist[kSortWarps][kSortDigits];
-  const uint32_t n = pass_elements(p);
-  const uint32_t c0 = bid * (uint32_t)CHUNK;
-  if (c0 >= n) return;
-  const int ndig = 1 << p.bits;
-  const uint32_t mask = (uint32_t)ndig - 1u;
-  const int warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < kSortWarps * kSortDigits; i += kSortThreads) (&hist[0][0])[i] = 0u;
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < CHUNK / (4 * kSortThreads); ++k) {
-    const uint32_t i = c0 + 4u * (k * kSortThreads + threadIdx.x);
-    if (i < n) {
-      const uint4 kk = load_keys4<DEPTH>(p, i, n);
-      atomicAdd(&hist[warp][(kk.x >> p.shift) & mask], 1u);
-      if (i + 1 < n) atomicAdd(&hist[warp][(kk.y >> p.shift) & mask], 1u);
-      if (i + 2 < n) atomicAdd(&hist[warp][(kk.z >> p.shift) & mask], 1u);
-      if (i + 3 < n) atomicAdd(&hist[warp][(kk.w >> p.shift) & mask], 1u);
-    }
-  }
-  __syncthreads();
-  for (int d = threadIdx.x; d < ndig; d += kSortThreads) {
-    uint32_t s = 0;
-#pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) s += hist[w][d];
-    p.chunk_counts[(size_t)d * p.num_chunks + bid] = s;
-  }
-}
-template <int CHUNK, bool DEPTH>
-__global__ void __launch_bounds__(kSortThreads) k_sort_count(SortPass p) {
-  sort_count_block<CHUNK, DEPTH>(p, blockIdx.x);
 }
 
 // Block-wide inclusive scan of one value per thread (blockDim.x <= 1024); returns the
@@ -171,322 +129,564 @@ __device__ __forceinline__ uint32_t block_inclusive_scan(uint32_t v, uint32_t* s
   return r;
 }
 
+// Exclusive scan of load(0 .. n) by one block into store(i, prefix); returns the total.
+// IT values per thread and round, so that a few thousand take one round; blockDim.x is a
+// multiple of 128. sh holds IT * 32 + 1 values.
+template <int IT, class Load, class Store>
+__device__ __forceinline__ uint32_t block_exclusive_scan(int64_t n, uint32_t* sh, Load load, Store store) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
+  uint32_t carry = 0;
+  for (int64_t base = 0; base < n; base += IT * (int64_t)blockDim.x) {
+    uint32_t v[IT], x[IT];
+#pragma unroll
+    for (int k = 0; k < IT; ++k) {
+      const int64_t i = base + k * (int64_t)blockDim.x + threadIdx.x;
+      v[k] = i < n ? load(i) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < IT; ++k) {
+      x[k] = v[k];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x[k], o);
+        if (lane >= o) x[k] += y;
+      }
+      if (lane == 31) sh[k * nw + warp] = x[k];
+    }
+    __syncthreads();
+    if (warp == 0) {  // the IT * nw warp totals, a multiple of 32: consecutive ones per lane
+      const int per = IT * nw / 32;
+      uint32_t sum = 0;
+      for (int k = 0; k < per; ++k) sum += sh[lane * per + k];
+      uint32_t incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      uint32_t before = incl - sum;
+      for (int k = 0; k < per; ++k) {
+        const uint32_t t = sh[lane * per + k];
+        sh[lane * per + k] = before;
+        before += t;
+      }
+      if (lane == 31) sh[IT * nw] = incl;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < IT; ++k) {
+      const int64_t i = base + k * (int64_t)blockDim.x + threadIdx.x;
+      if (i < n) store(i, carry + sh[k * nw + warp] + x[k] - v[k]);
+    }
+    carry += sh[IT * nw];
+    __syncthreads();
+  }
+  return carry;
+}
+
+// Adds up a block's per-warp digit counters and writes them to chunk_counts[d][chunk].
+template <int ITEMS>
+__device__ __forceinline__ void write_chunk_counts(const SortPass& p, CountShared<ITEMS>& sh, uint32_t bid) {
+  __syncthreads();
+  for (int d = threadIdx.x; d < (1 << p.bits); d += kSortThreads) {
+    uint32_t s = 0;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) s += sh.whist[w][d];
+    p.chunk_counts[(size_t)d * p.num_chunks + bid] = s;
+  }
+}
+
+// Clears n tables of per-warp digit counters.
+__device__ __forceinline__ void clear_digits(uint32_t* tables, int n) {
+  uint4* w = reinterpret_cast<uint4*>(tables);
+#pragma unroll
+  for (int i = 0; i < n * (kSortWarps * kSortDigits / 4 / kSortThreads); ++i)
+    w[i * kSortThreads + threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Digit histogram of one chunk. FORM: the first depth pass, whose keys (depth bits; Gaussians
+// that touch no tile sort last) are written here as well.
+template <int ITEMS, bool FORM>
+__device__ __forceinline__ void sort_count_block(const SortPass& p, CountShared<ITEMS>& sh, uint32_t bid) {
+  constexpr uint32_t kChunk = kSortThreads * ITEMS;
+  const uint32_t n = pass_elements(p);
+  const uint32_t c0 = bid * kChunk;
+  if (c0 >= n) return;
+  const uint32_t mask = (1u << p.bits) - 1u;
+  const int warp = threadIdx.x >> 5;
+  clear_digits(&sh.whist[0][0], 1);
+  uint4 k[ITEMS / 4];
+#pragma unroll
+  for (int q = 0; q < ITEMS / 4; ++q) {
+    const uint32_t i = c0 + 4u * (q * kSortThreads + threadIdx.x);
+    if (FORM) {
+      uint32_t e[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        e[c] = i + c < n && p.depth_touched[i + c] ? __float_as_uint(p.depth_rgbd[i + c].w) : 0xffffffffu;
+      k[q] = make_uint4(e[0], e[1], e[2], e[3]);
+      if (i < n) *reinterpret_cast<uint4*>(p.key_form + i) = k[q];  // the buffer's stride is a multiple of 4
+    } else if (i + 3 < n) {
+      k[q] = *reinterpret_cast<const uint4*>(p.key_in + i);
+    } else {
+      k[q].x = i < n ? p.key_in[i] : 0u;
+      k[q].y = i + 1 < n ? p.key_in[i + 1] : 0u;
+      k[q].z = i + 2 < n ? p.key_in[i + 2] : 0u;
+      k[q].w = 0u;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < ITEMS / 4; ++q) {
+    const uint32_t i = c0 + 4u * (q * kSortThreads + threadIdx.x);
+    if (i < n) atomicAdd(&sh.whist[warp][(k[q].x >> p.shift) & mask], 1u);
+    if (i + 1 < n) atomicAdd(&sh.whist[warp][(k[q].y >> p.shift) & mask], 1u);
+    if (i + 2 < n) atomicAdd(&sh.whist[warp][(k[q].z >> p.shift) & mask], 1u);
+    if (i + 3 < n) atomicAdd(&sh.whist[warp][(k[q].w >> p.shift) & mask], 1u);
+  }
+  write_chunk_counts(p, sh, bid);
+}
+template <int ITEMS, bool FORM>
+__global__ void __launch_bounds__(kSortThreads) k_sort_count(SortPass p) {
+  __shared__ __align__(16) CountShared<ITEMS> sh;
+  sort_count_block<ITEMS, FORM>(p, sh, blockIdx.x);
+}
+
 // One block per digit d: chunk_counts[d][c] becomes the number of digit-d elements in
 // earlier chunks, and digit_totals[d] the digit's count. The scatter adds the counts of
 // the smaller digits.
-template <int CHUNK>
-__device__ __forceinline__ void sort_scan_block(const SortPass& p, int d) {
-  __shared__ uint32_t sh[64];
+__device__ __forceinline__ void sort_scan_block(const SortPass& p, uint32_t* sh, int d) {
   const uint32_t n = pass_elements(p);
-  const int64_t nc = ((int64_t)n + CHUNK - 1) / CHUNK;
-  uint32_t tot, carry = 0;
+  const int64_t chunk = (int64_t)kSortThreads * p.items, nc = ((int64_t)n + chunk - 1) / chunk;
   uint32_t* col = p.chunk_counts + (size_t)d * p.num_chunks;
-  for (int64_t c0 = 0; c0 < nc; c0 += blockDim.x) {
-    const int64_t c = c0 + threadIdx.x;
-    const uint32_t v = c < nc ? col[c] : 0u;
-    const uint32_t incl = block_inclusive_scan(v, sh, &tot);
-    if (c < nc) col[c] = carry + incl - v;
-    carry += tot;
-  }
-  if (threadIdx.x == 0) p.digit_totals[d] = carry;
+  const uint32_t total = block_exclusive_scan<kScanItems>(
+      nc, sh, [&](int64_t c) { return col[c]; }, [&](int64_t c, uint32_t v) { col[c] = v; });
+  if (threadIdx.x == 0) p.digit_totals[d] = total;
 }
-template <int CHUNK>
 __global__ void __launch_bounds__(1024) k_sort_scan(SortPass p) {
-  sort_scan_block<CHUNK>(p, blockIdx.x);
+  __shared__ uint32_t sh[kScanItems * 32 + 1];
+  sort_scan_block(p, sh, blockIdx.x);
 }
 
-// Shared memory of the scatter: keys and payloads in input order, the permutation
-// (sorted position -> input position), per-warp digit counters, per-digit block-local
-// starts and global slots.
-template <int CHUNK>
-struct ScatterSmem {
-  static constexpr size_t kKey = 0;
-  static constexpr size_t kVal = kKey + 4 * CHUNK;
-  static constexpr size_t kAux = kVal + 4 * CHUNK;
-  __host__ __device__ static size_t perm(bool aux) { return kAux + (aux ? 4 * CHUNK : 0); }
-  __host__ __device__ static size_t whist(bool aux) { return perm(aux) + 2 * CHUNK; }
-  __host__ __device__ static size_t start(bool aux) { return whist(aux) + 4 * kSortWarps * kSortDigits; }
-  __host__ __device__ static size_t slot(bool aux) { return start(aux) + 4 * kSortDigits; }
-  __host__ __device__ static size_t bytes(bool aux) { return slot(aux) + 4 * kSortDigits; }
-};
+// ---- the instance list -------------------------------------------------------------------
+// A chunk [c0, c0 + cnt) of the list of instances in depth order: starts[bid] is the depth
+// rank whose instances cover position c0, starts[bid + 1] the one that covers the next
+// chunk's first position (or the last instance). A mark at every position where a
+// Gaussian's instances begin gives an instance's rank as starts[bid] plus the marks up to
+// it: one shared word, one population count.
+template <int ITEMS>
+__device__ __forceinline__ void mark_chunk(const InstanceList& a, CountShared<ITEMS>& sh, uint32_t bid, uint32_t c0,
+                                           uint32_t cnt) {
+  constexpr int kWords = kSortWarps * ITEMS;
+  if (threadIdx.x < kWords) sh.mark[threadIdx.x] = 0u;
+  __syncthreads();
+  const uint32_t r0 = a.starts[bid], r1 = a.starts[bid + 1];
+  for (uint32_t r = r0 + 1 + threadIdx.x; r <= r1; r += kSortThreads) {
+    const uint32_t at = a.prefix[r] - c0;
+    if (at < cnt) atomicOr(&sh.mark[at >> 5], 1u << (at & 31));
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    constexpr int kPer = kWords / 32;
+    uint32_t own[kPer], sum = 0;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      own[k] = (uint32_t)__popc(sh.mark[threadIdx.x * kPer + k]);
+      sum += own[k];
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if ((int)threadIdx.x >= o) incl += y;
+    }
+    uint32_t before = incl - sum;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      sh.mark_before[threadIdx.x * kPer + k] = before;
+      before += own[k];
+    }
+  }
+  __syncthreads();
+}
 
-template <int CHUNK, bool DEPTH>
-__device__ __forceinline__ void sort_scatter_block(const SortPass& p, uint32_t bid) {
-  using L = ScatterSmem<CHUNK>;
-  constexpr int kSlice = CHUNK / kSortWarps;  // elements per warp
-  constexpr int kRounds = kSlice / 32;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const bool has_val = p.val_in != nullptr, has_aux = p.aux_in != nullptr;
-  uint32_t* s_key = reinterpret_cast<uint32_t*>(smem_raw + L::kKey);
-  uint32_t* s_val = reinterpret_cast<uint32_t*>(smem_raw + L::kVal);
-  uint32_t* s_aux = reinterpret_cast<uint32_t*>(smem_raw + L::kAux);
-  uint16_t* s_perm = reinterpret_cast<uint16_t*>(smem_raw + L::perm(has_aux));
-  uint32_t* s_whist = reinterpret_cast<uint32_t*>(smem_raw + L::whist(has_aux));  // [warp][digit]
-  uint32_t* s_start = reinterpret_cast<uint32_t*>(smem_raw + L::start(has_aux));
-  uint32_t* s_slot = reinterpret_cast<uint32_t*>(smem_raw + L::slot(has_aux));
-  __shared__ uint32_t sh[64];
+// Depth rank of the instance at chunk position i.
+template <int ITEMS>
+__device__ __forceinline__ uint32_t instance_rank(const CountShared<ITEMS>& sh, uint32_t r0, uint32_t i) {
+  const uint32_t w = i >> 5;
+  return r0 + sh.mark_before[w] + (uint32_t)__popc(sh.mark[w] & (0xffffffffu >> (31 - (i & 31))));
+}
 
+// Tile of instance j of a rectangle: row j / w, column j % w of the rectangle's w columns.
+// The quotient is estimated with a reciprocal of 1 ulp (off by at most one for j < 2^22) and
+// corrected exactly.
+__device__ __forceinline__ uint32_t instance_tile(uint2 rc, uint32_t j, uint32_t tile_base, uint32_t grid_x) {
+  const uint32_t x0 = rc.x & 0xffffu, y0 = rc.x >> 16, w = (rc.y & 0xffffu) - x0;
+  uint32_t ty, tx;
+  if (j < (1u << 22)) {
+    float inv;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"((float)w));
+    ty = (uint32_t)((float)j * inv);
+    tx = j - ty * w;
+    if ((int32_t)tx < 0) {
+      --ty;
+      tx += w;
+    } else if (tx >= w) {
+      ++ty;
+      tx -= w;
+    }
+  } else {
+    ty = j / w;
+    tx = j - ty * w;
+  }
+  return tile_base + (y0 + ty) * grid_x + x0 + tx;
+}
+
+// One chunk's tile keys, and its digit histogram for the first tile pass p.
+template <class Scenes, int ITEMS>
+__device__ __forceinline__ void emit_keys_block(const EmitArgs<Scenes>& a, const SortPass& p, CountShared<ITEMS>& sh,
+                                                uint32_t bid) {
+  constexpr uint32_t kChunk = kSortThreads * ITEMS;
   const uint32_t n = pass_elements(p);
-  const uint32_t c0 = bid * (uint32_t)CHUNK;
+  const uint32_t c0 = bid * kChunk;
   if (c0 >= n) return;
-  const int cnt = (int)min((uint32_t)CHUNK, n - c0);
+  const uint32_t cnt = min(kChunk, n - c0);
+  const uint32_t mask = (1u << p.bits) - 1u;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  clear_digits(&sh.whist[0][0], 1);
+  mark_chunk(a.list, sh, bid, c0, cnt);
+  const uint32_t r0 = a.list.starts[bid];
+  uint32_t g[ITEMS], j[ITEMS];
+  uint2 rc[ITEMS];
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const uint32_t i = (uint32_t)(warp * 32 * ITEMS + k * 32 + lane);
+    if (i < cnt) {
+      const uint32_t r = instance_rank(sh, r0, i);
+      g[k] = a.list.order[r];
+      j[k] = c0 + i - a.list.prefix[r];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const uint32_t i = (uint32_t)(warp * 32 * ITEMS + k * 32 + lane);
+    if (i < cnt) rc[k] = a.geom.rect[g[k]];
+  }
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const uint32_t i = (uint32_t)(warp * 32 * ITEMS + k * 32 + lane);
+    if (i < cnt) {
+      const SceneDesc& sd = a.scenes.for_gaussian(g[k]);
+      const uint32_t key = instance_tile(rc[k], j[k], (uint32_t)sd.tile_base, (uint32_t)sd.grid_x);
+      a.keys[c0 + i] = key;
+      atomicAdd(&sh.whist[warp][(key >> p.shift) & mask], 1u);
+    }
+  }
+  write_chunk_counts(p, sh, bid);
+}
+template <class Scenes, int ITEMS>
+__global__ void __launch_bounds__(kSortThreads) k_emit_keys(EmitArgs<Scenes> a, SortPass p) {
+  __shared__ __align__(16) CountShared<ITEMS> sh;
+  emit_keys_block<Scenes, ITEMS>(a, p, sh, blockIdx.x);
+}
+
+// ---- scatter -----------------------------------------------------------------------------
+template <int ITEMS, Payload P, bool FULL>
+__device__ __forceinline__ void scatter_chunk(const SortPass& p, const InstanceList& a, BinShared<ITEMS>& sh,
+                                              uint32_t bid, int cnt) {
+  constexpr uint32_t kChunk = kSortThreads * ITEMS;
+  static_assert(ITEMS % 2 == 0, "elements are ranked two at a time");
+  const uint32_t c0 = bid * kChunk;
   const int ndig = 1 << p.bits;
   const uint32_t mask = (uint32_t)ndig - 1u;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int i0 = warp * 32 * ITEMS + lane;  // this thread's elements: i0 + 32 k
 
-  // input chunk -> shared memory (vector loads, all in flight together)
+  uint32_t key[ITEMS];
 #pragma unroll
-  for (int k = 0; k < CHUNK / (4 * kSortThreads); ++k) {
-    const int j = 4 * (k * kSortThreads + t);
-    const uint32_t i = c0 + (uint32_t)j;
-    if (i < n) {
-      *reinterpret_cast<uint4*>(s_key + j) = load_keys4<DEPTH>(p, i, n);
-      if (has_val) *reinterpret_cast<uint4*>(s_val + j) = load_u32x4(p.val_in, i, n);
-      if (has_aux) *reinterpret_cast<uint4*>(s_aux + j) = load_u32x4(p.aux_in, i, n);
-    }
-  }
-  for (int i = t; i < kSortWarps * kSortDigits; i += kSortThreads) s_whist[i] = 0u;
+  for (int k = 0; k < ITEMS; ++k) key[k] = FULL || i0 + 32 * k < cnt ? p.key_in[c0 + i0 + 32 * k] : 0u;
+  const uint32_t dtot = t < ndig ? p.digit_totals[t] : 0u;
+  const uint32_t earlier = t < ndig ? p.chunk_counts[(size_t)t * p.num_chunks + bid] : 0u;
+  clear_digits(&sh.whist[0][0], 1);
+  clear_digits(&sh.same[0][0][0], 2);
+  if (P == kFirstPair) mark_chunk(a, sh, bid, c0, (uint32_t)cnt);
   __syncthreads();
 
-  // rank of every element among the equal digits of its warp's slice
-  uint32_t rank[kRounds];
+  // Rank of every element among the equal digits of its warp's slice, two elements per lane
+  // at a time: the lanes of a digit meet in a mask in shared memory. (First tile pass of the
+  // size above, before the pairs: 85 us and 53 million instructions; with a ballot per digit
+  // bit 116 and 90 million, with match.any 139 us.)
+  uint32_t pos[ITEMS];
   const unsigned lt = (1u << lane) - 1u;
+  uint32_t* hist = sh.whist[warp];
+  uint32_t* m0 = sh.same[0][warp];
+  uint32_t* m1 = sh.same[1][warp];
 #pragma unroll
-  for (int k = 0; k < kRounds; ++k) {
-    const int i = warp * kSlice + k * 32 + lane;
-    const bool act = i < cnt;
-    const unsigned am = __ballot_sync(0xffffffffu, act);
-    const uint32_t d = act ? (s_key[i] >> p.shift) & mask : 0u;
-    const unsigned peers = digit_peers(d, p.bits, am);
-    const uint32_t before = act ? s_whist[warp * kSortDigits + d] : 0u;
-    rank[k] = before + (uint32_t)__popc(peers & lt);
+  for (int k = 0; k < ITEMS; k += 2) {
+    const bool act0 = FULL || i0 + 32 * k < cnt, act1 = FULL || i0 + 32 * (k + 1) < cnt;
+    const uint32_t d0 = (key[k] >> p.shift) & mask, d1 = (key[k + 1] >> p.shift) & mask;
+    if (act0) atomicOr(&m0[d0], 1u << lane);
+    if (act1) atomicOr(&m1[d1], 1u << lane);
     __syncwarp();
-    if (act && (peers & lt) == 0) s_whist[warp * kSortDigits + d] = before + (uint32_t)__popc(peers);
+    const uint32_t peers0 = m0[d0], peers1 = m1[d1];
+    const uint32_t before0 = hist[d0];
+    const uint32_t before1 = hist[d1] + (uint32_t)__popc(m0[d1]);
+    pos[k] = before0 + (uint32_t)__popc(peers0 & lt);
+    pos[k + 1] = before1 + (uint32_t)__popc(peers1 & lt);
+    __syncwarp();
+    if (act0 && (peers0 & lt) == 0) {
+      hist[d0] = before0 + (uint32_t)__popc(peers0);
+      m0[d0] = 0u;
+    }
+    __syncwarp();
+    if (act1 && (peers1 & lt) == 0) {
+      hist[d1] = before1 + (uint32_t)__popc(peers1);
+      m1[d1] = 0u;
+    }
     __syncwarp();
   }
   __syncthreads();
 
-  // digit t: warp offsets inside the digit, block-local start, global slot
-  uint32_t dsum = 0;
+  // digit t: the warps' first positions, the digit's global slot
+  uint32_t dsum = 0, first[kSortWarps];
   if (t < ndig) {
 #pragma unroll
     for (int w = 0; w < kSortWarps; ++w) {
-      const uint32_t c = s_whist[w * kSortDigits + t];
-      s_whist[w * kSortDigits + t] = dsum;
-      dsum += c;
+      first[w] = dsum;
+      dsum += sh.whist[w][t];
     }
   }
-  uint32_t tot;
-  const uint32_t incl = block_inclusive_scan(dsum, sh, &tot);
-  const uint32_t dtot = t < ndig ? p.digit_totals[t] : 0u;
-  const uint32_t below = block_inclusive_scan(dtot, sh, &tot) - dtot;  // elements of smaller digits
-  if (t < ndig) {
-    s_start[t] = incl - dsum;
-    s_slot[t] = dsum ? below + p.chunk_counts[(size_t)t * p.num_chunks + bid] : 0u;
-  }
-  __syncthreads();
-
-  // permutation: block-local sorted position -> input position
+  uint32_t start = dsum, below = dtot;  // elements of smaller digits, in the chunk and in all
 #pragma unroll
-  for (int k = 0; k < kRounds; ++k) {
-    const int i = warp * kSlice + k * 32 + lane;
-    if (i < cnt) {
-      const uint32_t d = (s_key[i] >> p.shift) & mask;
-      s_perm[s_start[d] + s_whist[warp * kSortDigits + d] + rank[k]] = (uint16_t)i;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t x = __shfl_up_sync(0xffffffffu, start, o), y = __shfl_up_sync(0xffffffffu, below, o);
+    if (lane >= o) {
+      start += x;
+      below += y;
     }
+  }
+  if (lane == 31) {
+    sh.scan[warp] = start;
+    sh.scan[32 + warp] = below;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kSortWarps - 1; ++w)
+    if (w < warp) {
+      start += sh.scan[w];
+      below += sh.scan[32 + w];
+    }
+  start -= dsum;
+  below -= dtot;
+  if (t < ndig) {
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) sh.whist[w][t] = start + first[w];
+    sh.slot[t] = below + earlier - start;
   }
   __syncthreads();
 
-  // each digit's run goes to consecutive global slots
-  for (int q = t; q < cnt; q += kSortThreads) {
-    const int o = s_perm[q];
-    const uint32_t kk = s_key[o];
-    const uint32_t d = (kk >> p.shift) & mask;
-    const uint32_t g = s_slot[d] + (uint32_t)q - s_start[d];
-    if (p.key_out) p.key_out[g] = kk;
-    p.val_out[g] = has_val ? s_val[o] : c0 + (uint32_t)o;
-    if (p.aux_out) p.aux_out[g] = has_aux ? s_aux[o] : c0 + (uint32_t)o;
-    if (p.tile_count) {
-      // The chunk is fully sorted now (its input was sorted by the lower digits), so
-      // equal tiles form runs: a run [b, e) adds e - b.
-      if (q == 0 || s_key[s_perm[q - 1]] != kk) atomicSub(&p.tile_count[kk], (uint32_t)q);
-      if (q == cnt - 1 || s_key[s_perm[q + 1]] != kk) atomicAdd(&p.tile_count[kk], (uint32_t)(q + 1));
+  // into digit order
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const int i = i0 + 32 * k;
+    if (FULL || i < cnt) {
+      const uint32_t q = pos[k] + hist[(key[k] >> p.shift) & mask];
+      if (P == kPair) {
+        sh.keys[q] = key[k];
+        sh.buf[q] = p.pair_in[c0 + i];
+      } else {
+        sh.buf[q] = make_uint2(key[k], P == kFirstPair ? (uint32_t)i : p.val_in ? p.val_in[c0 + i] : c0 + i);
+      }
+    }
+  }
+  __syncthreads();
+  const uint32_t r0 = P == kFirstPair ? a.starts[bid] : 0u;
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const int q = t + kSortThreads * k;
+    if (FULL || q < cnt) {
+      uint2 e = sh.buf[q];
+      const uint32_t kk = P == kPair ? sh.keys[q] : e.x;
+      const uint32_t out = sh.slot[(kk >> p.shift) & mask] + (uint32_t)q;
+      if (P == kFirstPair) e = make_uint2(a.order[instance_rank(sh, r0, e.y)], c0 + e.y);
+      if (p.key_out) p.key_out[out] = kk;
+      if (P == kValue) {
+        p.val_out[out] = e.y;
+      } else if (p.pair_out) {
+        p.pair_out[out] = e;
+      } else {
+        p.val_out[out] = e.x;
+        p.aux_out[out] = e.y;
+        // The chunk is fully sorted now (its input was sorted by the lower digits), so
+        // equal tiles form runs: a run [b, e) adds e - b.
+        const uint32_t before = q == 0 ? kk : P == kPair ? sh.keys[q - 1] : sh.buf[q - 1].x;
+        if (before != kk) {
+          atomicSub(&p.tile_count[kk], (uint32_t)q);
+          atomicAdd(&p.tile_count[before], (uint32_t)q);
+        }
+        if (q == cnt - 1) atomicAdd(&p.tile_count[kk], (uint32_t)cnt);
+      }
     }
   }
 }
-template <int CHUNK, bool DEPTH>
-__global__ void __launch_bounds__(kSortThreads) k_sort_scatter(SortPass p) {
-  sort_scatter_block<CHUNK, DEPTH>(p, blockIdx.x);
+
+template <int ITEMS, Payload P>
+__device__ __forceinline__ void sort_scatter_block(const SortPass& p, const InstanceList& a, BinShared<ITEMS>& sh,
+                                                   uint32_t bid) {
+  constexpr uint32_t kChunk = kSortThreads * ITEMS;
+  const uint32_t n = pass_elements(p);
+  const uint32_t c0 = bid * kChunk;
+  if (c0 >= n) return;
+  if (n - c0 >= kChunk) scatter_chunk<ITEMS, P, true>(p, a, sh, bid, (int)kChunk);
+  else scatter_chunk<ITEMS, P, false>(p, a, sh, bid, (int)(n - c0));
+}
+// Resident blocks: pairs read from memory want the registers of 4 (72 us; with 5: 77), the
+// others 5 (first tile pass 72 us; with 4: 74).
+template <int ITEMS, Payload P>
+__global__ void __launch_bounds__(kSortThreads, P == kPair ? 4 : 5) k_sort_scatter(SortPass p, InstanceList a) {
+  __shared__ __align__(16) BinShared<ITEMS> sh;
+  sort_scatter_block<ITEMS, P>(p, a, sh, blockIdx.x);
 }
 
-// Instances of every 256 depth-ordered Gaussians (the emission's block prefix).
-__device__ __forceinline__ void rank_sums_block(const uint32_t* order, const uint32_t* touched, int64_t total_slots,
-                                                uint32_t* rank_sums, int bid) {
-  __shared__ uint32_t sh[64];
-  const int64_t r = (int64_t)bid * blockDim.x + threadIdx.x;
-  const uint32_t v = r < total_slots ? touched[order[r]] : 0u;
+// ---- the depth order's prefix ------------------------------------------------------------
+constexpr int kRankItems = 4;  // depth ranks per thread
+constexpr int kRankBlock = kPreprocessBlock * kRankItems;
+
+// Instances of every kRankBlock depth-ordered Gaussians; the instances of each go to the
+// first depth-key buffer (free by now).
+__device__ __forceinline__ void rank_sums_block(const GeomView& gv, int64_t slots, uint32_t* sh, int bid) {
+  const int64_t r = (int64_t)bid * kRankBlock + kRankItems * threadIdx.x;
+  uint4 n = make_uint4(0u, 0u, 0u, 0u);
+  if (r < slots) {
+    const uint4 g = *reinterpret_cast<const uint4*>(gv.depth_val[1] + r);
+    n.x = gv.touched[g.x];
+    if (r + 1 < slots) n.y = gv.touched[g.y];
+    if (r + 2 < slots) n.z = gv.touched[g.z];
+    if (r + 3 < slots) n.w = gv.touched[g.w];
+    *reinterpret_cast<uint4*>(gv.depth_key[0] + r) = n;
+  }
   uint32_t tot;
-  block_inclusive_scan(v, sh, &tot);
-  if (threadIdx.x == 0) rank_sums[bid] = tot;
+  block_inclusive_scan(n.x + n.y + n.z + n.w, sh, &tot);
+  if (threadIdx.x == 0) gv.rank_sums[bid] = tot;
 }
-__global__ void __launch_bounds__(kPreprocessBlock) k_rank_sums(const uint32_t* order, const uint32_t* touched,
-                                                                int64_t total_slots, uint32_t* rank_sums) {
-  rank_sums_block(order, touched, total_slots, rank_sums, blockIdx.x);
+__global__ void __launch_bounds__(kPreprocessBlock) k_rank_sums(GeomView gv, int64_t slots) {
+  __shared__ uint32_t sh[64];
+  rank_sums_block(gv, slots, sh, blockIdx.x);
 }
 
-// The per-block instance counts become their exclusive prefix, in place (one block): the
-// emission's first instance index of each block of 256 depth-ordered Gaussians. Run for
-// large batches only: below kRankScanMinBlocks blocks each emission block sums its
-// predecessors itself (cheaper than a launch; quadratic in the block count above it).
-constexpr int kRankScanMinBlocks = 8192;
+// The per-block instance counts become their exclusive prefix, in place (one block). Run for
+// large batches only: below kRankScanMinBlocks blocks each block sums its predecessors
+// itself (cheaper than a launch; quadratic in the block count above it).
+constexpr int kRankScanMinBlocks = 2048;
 inline bool rank_scan_needed(int rank_blocks) { return rank_blocks > kRankScanMinBlocks; }
-__device__ __forceinline__ void rank_scan_block(uint32_t* rank_sums, int n) {
-  __shared__ uint32_t sh[64];
-  uint32_t carry = 0, tot;
-  for (int c0 = 0; c0 < n; c0 += blockDim.x) {
-    const int c = c0 + threadIdx.x;
-    const uint32_t v = c < n ? rank_sums[c] : 0u;
-    const uint32_t incl = block_inclusive_scan(v, sh, &tot);
-    if (c < n) rank_sums[c] = carry + incl - v;
-    carry += tot;
-  }
+__device__ __forceinline__ void rank_scan_block(uint32_t* rank_sums, int n, uint32_t* sh) {
+  block_exclusive_scan<kScanItems>(
+      n, sh, [&](int64_t c) { return rank_sums[c]; }, [&](int64_t c, uint32_t v) { rank_sums[c] = v; });
 }
-__global__ void __launch_bounds__(1024) k_rank_scan(uint32_t* rank_sums, int n) { rank_scan_block(rank_sums, n); }
+__global__ void __launch_bounds__(1024) k_rank_scan(uint32_t* rank_sums, int n) {
+  __shared__ uint32_t sh[kScanItems * 32 + 1];
+  rank_scan_block(rank_sums, n, sh);
+}
 
-// One thread per depth-ordered Gaussian; the block's first instance index is the sum of
-// the earlier blocks' rank_sums (formed by k_rank_scan for large batches, else by the
-// block itself), the thread's is that plus a block scan. The
-// instances are then written warp-cooperatively: the warp's instances are dealt out
-// 32 per round, one per lane, so the stores of a round are consecutive. In a round, the
-// lanes whose instance ranges meet it mark where their range begins (an OR reduction),
-// and a lane's owner is the last mark at or before it; the owner's rectangle comes over
-// by shuffle. Instance j of a rectangle of width w is tile row j / w, column j % w; the
-// quotient is estimated with a float reciprocal (off by at most one for j < 2^22) and
-// corrected exactly.
-template <class Scenes>
-__device__ __forceinline__ void emit_block(const EmitArgs<Scenes>& a, int bid) {
-  __shared__ uint32_t sh[64];
-  __shared__ uint8_t s_owner[kPreprocessBlock / 32][32];
-  if ((int64_t)a.counts->num_rendered > a.cap) {
-    if (bid == 0 && threadIdx.x == 0) atomicOr(&a.counts->flags, CFGS_FLAG_CAPACITY_OVERFLOW);
-    return;
-  }
+// First instance index of every depth rank (the prefix, over its instance counts) and of
+// every Gaussian (offset).
+__device__ __forceinline__ void rank_place_block(const GeomView& gv, int64_t slots, bool scanned, uint32_t* sh, int bid) {
   uint32_t tot, block_first;
-  if (a.rank_scanned) {
-    block_first = a.rank_sums[bid];  // exclusive prefix (k_rank_scan)
+  if (scanned) {
+    block_first = gv.rank_sums[bid];
   } else {
     uint32_t pre = 0;
-#pragma unroll 4
-    for (int b = threadIdx.x; b < bid; b += blockDim.x) pre += a.rank_sums[b];
+    for (int b = threadIdx.x; b < bid; b += blockDim.x) pre += gv.rank_sums[b];
     block_inclusive_scan(pre, sh, &tot);
     block_first = tot;
   }
+  const int64_t r = (int64_t)bid * kRankBlock + kRankItems * threadIdx.x;
+  uint4 g = make_uint4(0u, 0u, 0u, 0u), n = g;
+  if (r < slots) {
+    g = *reinterpret_cast<const uint4*>(gv.depth_val[1] + r);
+    n = *reinterpret_cast<const uint4*>(gv.depth_key[0] + r);
+  }
+  const uint32_t own = n.x + n.y + n.z + n.w;
+  uint4 at;
+  at.x = block_first + block_inclusive_scan(own, sh, &tot) - own;
+  at.y = at.x + n.x;
+  at.z = at.y + n.y;
+  at.w = at.z + n.z;
+  if (r < slots) *reinterpret_cast<uint4*>(gv.depth_key[0] + r) = at;
+  if (n.x) gv.offset[g.x] = at.x;
+  if (n.y) gv.offset[g.y] = at.y;
+  if (n.z) gv.offset[g.z] = at.z;
+  if (n.w) gv.offset[g.w] = at.w;
+}
+__global__ void __launch_bounds__(kPreprocessBlock) k_rank_place(GeomView gv, int64_t slots, bool scanned) {
+  __shared__ uint32_t sh[64];
+  rank_place_block(gv, slots, scanned, sh, blockIdx.x);
+}
+
+// starts[c] = the depth rank whose instances cover position c * chunk, starts[last + 1] the
+// rank of the last instance. Raises the overflow flag when the instances exceed the
+// capacity.
+template <class Scenes>
+__device__ __forceinline__ void emit_starts_block(const EmitArgs<Scenes>& a, uint32_t chunk, int bid) {
+  const int64_t K = (int64_t)a.counts->num_rendered;
+  if (K > a.cap) {
+    if (bid == 0 && threadIdx.x == 0) atomicOr(&a.counts->flags, CFGS_FLAG_CAPACITY_OVERFLOW);
+    return;
+  }
   const int64_t r = (int64_t)bid * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t g = 0, nt = 0;
-  if (r < a.total_slots) {
-    g = a.order[r];
-    nt = a.geom.touched[g];
-  }
-  const uint32_t first = block_first + block_inclusive_scan(nt, sh, &tot) - nt;
-  uint2 rc = make_uint2(0u, 0u);
-  uint32_t tile_base = 0, grid_x = 0;
-  float rinv = 0.0f;
-  if (nt) {
-    a.geom.offset[g] = first;
-    const SceneDesc& sd = a.scenes.for_gaussian(g);
-    rc = a.geom.rect[g];
-    tile_base = (uint32_t)sd.tile_base;
-    grid_x = (uint32_t)sd.grid_x;
-    rinv = 1.0f / (float)((rc.y & 0xffffu) - (rc.x & 0xffffu));
-  }
-  // warp-exclusive start of this lane's instances
-  uint32_t x = nt;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  const uint32_t warp_total = __shfl_sync(0xffffffffu, x, 31);
-  const uint32_t start = x - nt;
-  const unsigned upto = 0xffffffffu >> (31 - lane);  // bits 0..lane
-  for (uint32_t base = 0; base < warp_total; base += 32) {
-    const bool meets = nt != 0 && start < base + 32u && start + nt > base;
-    const uint32_t pos = start > base ? start - base : 0u;
-    const unsigned marks = __reduce_or_sync(0xffffffffu, meets ? (1u << pos) : 0u);
-    if (meets) s_owner[warp][pos] = (uint8_t)lane;
-    __syncwarp();
-    const int o = s_owner[warp][31 - __clz(marks & upto)];
-    __syncwarp();
-    const uint32_t o_start = __shfl_sync(0xffffffffu, start, o);
-    const uint32_t o_rx = __shfl_sync(0xffffffffu, rc.x, o);
-    const uint32_t o_ry = __shfl_sync(0xffffffffu, rc.y, o);
-    const uint32_t o_first = __shfl_sync(0xffffffffu, first, o);
-    const uint32_t o_gid = __shfl_sync(0xffffffffu, g, o);
-    const float o_rinv = __shfl_sync(0xffffffffu, rinv, o);
-    const uint32_t o_tb = __shfl_sync(0xffffffffu, tile_base, o);
-    const uint32_t o_gx = __shfl_sync(0xffffffffu, grid_x, o);
-    const uint32_t w = base + (uint32_t)lane;
-    if (w < warp_total) {
-      const uint32_t j = w - o_start;
-      const uint32_t x0 = o_rx & 0xffffu, y0 = o_rx >> 16;
-      const uint32_t rw = (o_ry & 0xffffu) - x0;
-      uint32_t ty, tx;
-      if (j < (1u << 22)) {
-        ty = (uint32_t)((float)j * o_rinv);
-        tx = j - ty * rw;
-        if ((int32_t)tx < 0) {
-          --ty;
-          tx += rw;
-        } else if (tx >= rw) {
-          ++ty;
-          tx -= rw;
-        }
-      } else {
-        ty = j / rw;
-        tx = j - ty * rw;
-      }
-      const uint32_t q = o_first + j;
-      a.bin.key[0][q] = o_tb + (y0 + ty) * o_gx + x0 + tx;
-      a.bin.gid[0][q] = o_gid;
-    }
-  }
+  if (r >= a.total_slots) return;
+  const uint32_t b = a.list.prefix[r], e = r + 1 < a.total_slots ? a.list.prefix[r + 1] : (uint32_t)K;
+  if (b == e) return;
+  for (uint32_t c = (b + chunk - 1) / chunk; (int64_t)c * chunk < e; ++c) a.list.starts[c] = (uint32_t)r;
+  if (e == (uint32_t)K) a.list.starts[(uint32_t)((K + chunk - 1) / chunk)] = (uint32_t)r;
 }
 template <class Scenes>
-__global__ void __launch_bounds__(kPreprocessBlock) k_emit(EmitArgs<Scenes> a) {
-  emit_block<Scenes>(a, blockIdx.x);
+__global__ void __launch_bounds__(kPreprocessBlock) k_emit_starts(EmitArgs<Scenes> a, uint32_t chunk) {
+  emit_starts_block<Scenes>(a, chunk, blockIdx.x);
 }
 
 // Tile ranges from the per-tile instance counts (one block).
-__device__ __forceinline__ void tile_ranges_block(const uint32_t* tile_count, uint32_t* tile_range, int num_tiles) {
-  __shared__ uint32_t sh[64];
-  uint32_t carry = 0, tot;
-  for (int base = 0; base < num_tiles; base += blockDim.x) {
-    const int i = base + threadIdx.x;
-    const uint32_t v = i < num_tiles ? tile_count[i] : 0u;
-    const uint32_t incl = block_inclusive_scan(v, sh, &tot);
-    if (i < num_tiles) tile_range[i] = carry + incl - v;
-    carry += tot;
-  }
-  if (threadIdx.x == 0) tile_range[num_tiles] = carry;
+template <int IT>
+__device__ __forceinline__ void tile_ranges_block(const uint32_t* tile_count, uint32_t* tile_range, int num_tiles,
+                                                  uint32_t* sh) {
+  const uint32_t total = block_exclusive_scan<IT>(
+      num_tiles, sh, [&](int64_t i) { return tile_count[i]; }, [&](int64_t i, uint32_t v) { tile_range[i] = v; });
+  if (threadIdx.x == 0) tile_range[num_tiles] = total;
 }
 __global__ void __launch_bounds__(1024) k_tile_ranges(const uint32_t* tile_count, uint32_t* tile_range, int num_tiles) {
-  tile_ranges_block(tile_count, tile_range, num_tiles);
+  __shared__ uint32_t sh[kScanItems * 32 + 1];
+  tile_ranges_block<kScanItems>(tile_count, tile_range, num_tiles, sh);
 }
 
 namespace {
 
-template <int CHUNK, bool DEPTH>
-int launch_pass(const SortPass& p, cudaStream_t st) {
-  static std::atomic<uint64_t> smem_set{0};
-  if (!ensure_dynamic_smem(k_sort_scatter<CHUNK, DEPTH>, (int)ScatterSmem<CHUNK>::bytes(true), smem_set))
-    return CFGS_ERR_LAUNCH;
+// The scan's block: a digit's chunks in one round where they are few.
+void launch_scan(const SortPass& p, cudaStream_t st) {
+  k_sort_scan<<<1 << p.bits, p.num_chunks <= 256 * kScanItems ? 256 : 1024, 0, st>>>(p);
+}
+
+template <int ITEMS>
+void launch_pass_items(const SortPass& p, cudaStream_t st) {
   const int grid = (int)p.num_chunks;
-  k_sort_count<CHUNK, DEPTH><<<grid, kSortThreads, 0, st>>>(p);
-  k_sort_scan<CHUNK><<<1 << p.bits, 1024, 0, st>>>(p);
-  k_sort_scatter<CHUNK, DEPTH>
-      <<<grid, kSortThreads, ScatterSmem<CHUNK>::bytes(p.aux_in != nullptr), st>>>(p);
-  return CFGS_OK;
+  if (p.key_form) k_sort_count<ITEMS, true><<<grid, kSortThreads, 0, st>>>(p);
+  else k_sort_count<ITEMS, false><<<grid, kSortThreads, 0, st>>>(p);
+  launch_scan(p, st);
+  if (p.pair_in) k_sort_scatter<ITEMS, kPair><<<grid, kSortThreads, 0, st>>>(p, InstanceList{});
+  else k_sort_scatter<ITEMS, kValue><<<grid, kSortThreads, 0, st>>>(p, InstanceList{});
+}
+
+void launch_pass(const SortPass& p, cudaStream_t st) {
+  if (p.items == 8) launch_pass_items<8>(p, st);
+  else launch_pass_items<4>(p, st);
+}
+
+// The first tile pass, keys included.
+template <class Scenes, int ITEMS>
+void launch_emit_items(const EmitArgs<Scenes>& a, const SortPass& p, cudaStream_t st) {
+  const int grid = (int)p.num_chunks;
+  k_emit_keys<Scenes, ITEMS><<<grid, kSortThreads, 0, st>>>(a, p);
+  launch_scan(p, st);
+  k_sort_scatter<ITEMS, kFirstPair><<<grid, kSortThreads, 0, st>>>(p, a.list);
 }
 
 }  // namespace
@@ -500,90 +700,114 @@ void tile_sort_plan(int64_t num_tiles, int* passes, int* width) {
   *width = (bits + *passes - 1) / *passes;
 }
 
-// Step 1 of the binning, which needs no instance capacity: the depth order of the
-// Gaussians and their instance counts per 256 in that order.
-int launch_depth_order(const GeomView& gv, int64_t slots, cudaStream_t st) {
-  if (slots > 0) {
-    // 1. depth sort of the Gaussians: geometry -> 0 -> 1 -> 0 -> depth_val[1]
-    int src = -1;
-    for (int pass = 0; pass < kDepthPasses; ++pass) {
-      SortPass p{};
-      const bool last = pass == kDepthPasses - 1;
-      const int dst = src == 0 ? 1 : 0;
-      p.key_in = src < 0 ? nullptr : gv.depth_key[src];
-      p.val_in = src < 0 ? nullptr : gv.depth_val[src];
-      p.depth_rgbd = gv.rgbd;
-      p.depth_touched = gv.touched;
-      p.key_out = last ? nullptr : gv.depth_key[dst];
-      p.val_out = last ? gv.depth_val[1] : gv.depth_val[dst];
-      p.shift = 8 * pass;
-      p.bits = 8;
-      p.n = slots;
-      p.cap = slots;
-      p.num_chunks = sort_chunks(slots, kDepthChunk);
-      p.chunk_counts = gv.depth_counts;
-      p.digit_totals = gv.depth_totals + kSortDigits * pass;
-      int s = src < 0 ? launch_pass<kDepthChunk, true>(p, st) : launch_pass<kDepthChunk, false>(p, st);
-      if (s != CFGS_OK) return s;
-      src = dst;
-    }
-    const int rank_blocks = (int)((slots + kPreprocessBlock - 1) / kPreprocessBlock);
-    k_rank_sums<<<rank_blocks, kPreprocessBlock, 0, st>>>(gv.depth_val[1], gv.touched, slots, gv.rank_sums);
-    if (rank_scan_needed(rank_blocks)) k_rank_scan<<<1, 1024, 0, st>>>(gv.rank_sums, rank_blocks);
+namespace {
+
+void set_chunks(SortPass& p, int64_t n) {
+  p.items = radix_items(n);
+  p.num_chunks = sort_chunks(n, kSortThreads * p.items);
+}
+
+// Pass `pass` of the depth sort: the depths (keys formed in depth_key[1]) -> 0 -> 1 -> 0 ->
+// depth_val[1].
+SortPass depth_pass(const GeomView& gv, int64_t slots, int pass) {
+  SortPass p{};
+  const bool last = pass == kDepthPasses - 1;
+  const int src = pass & 1 ? 0 : 1, dst = src ^ 1;
+  if (pass == 0) {
+    p.depth_touched = gv.touched;
+    p.depth_rgbd = gv.rgbd;
+    p.key_form = gv.depth_key[src];
   }
+  p.key_in = gv.depth_key[src];
+  p.val_in = pass == 0 ? nullptr : gv.depth_val[src];
+  p.key_out = last ? nullptr : gv.depth_key[dst];
+  p.val_out = gv.depth_val[dst];
+  p.shift = 8 * pass;
+  p.bits = 8;
+  p.n = slots;
+  p.cap = slots;
+  set_chunks(p, slots);
+  p.chunk_counts = gv.depth_counts;
+  p.digit_totals = gv.depth_totals + kSortDigits * pass;
+  return p;
+}
+
+// Pass `pass` of the tile sort: keys 0 (and the list itself) -> keys and pairs 1 -> 0 ... ->
+// sorted.
+template <class Scenes>
+SortPass tile_pass(const BinArgs<Scenes>& a, int pass, int passes, int width) {
+  const BinningView& bv = a.bin;
+  SortPass p{};
+  const bool last = pass == passes - 1;
+  const int src = pass & 1, dst = src ^ 1;
+  p.key_in = bv.key[src];
+  p.pair_in = pass == 0 ? nullptr : bv.pair[src];
+  if (last) {
+    p.val_out = bv.sorted_gid;
+    p.aux_out = bv.sorted_pidx;
+    p.tile_count = a.tile_count;
+  } else {
+    p.key_out = bv.key[dst];
+    p.pair_out = bv.pair[dst];
+  }
+  p.shift = width * pass;
+  p.bits = width;
+  p.counts = a.counts;
+  p.cap = a.cap;
+  set_chunks(p, a.cap);
+  p.chunk_counts = bv.chunk_counts;
+  p.digit_totals = bv.totals + kSortDigits * pass;
+  return p;
+}
+
+template <class Scenes>
+EmitArgs<Scenes> emit_args(const BinArgs<Scenes>& a) {
+  EmitArgs<Scenes> e;
+  e.scenes = a.scenes;
+  e.total_slots = a.total_slots;
+  e.list.order = a.geom.depth_val[1];
+  e.list.prefix = a.geom.depth_key[0];
+  e.list.starts = a.bin.starts;
+  e.keys = a.bin.key[0];
+  e.geom = a.geom;
+  e.cap = a.cap;
+  e.counts = a.counts;
+  return e;
+}
+
+int slot_blocks(int64_t slots) { return (int)((slots + kPreprocessBlock - 1) / kPreprocessBlock); }
+int rank_blocks_of(int64_t slots) { return (int)((slots + kRankBlock - 1) / kRankBlock); }
+
+}  // namespace
+
+// Step 1 of the binning, which needs no instance capacity: the depth order of the
+// Gaussians and the prefix of their instance counts in that order.
+int launch_depth_order(const GeomView& gv, int64_t slots, cudaStream_t st) {
+  if (slots <= 0) return CFGS_OK;
+  for (int pass = 0; pass < kDepthPasses; ++pass) launch_pass(depth_pass(gv, slots, pass), st);
+  const int blocks = rank_blocks_of(slots);
+  k_rank_sums<<<blocks, kPreprocessBlock, 0, st>>>(gv, slots);
+  const bool scan = rank_scan_needed(blocks);
+  if (scan) k_rank_scan<<<1, 1024, 0, st>>>(gv.rank_sums, blocks);
+  k_rank_place<<<blocks, kPreprocessBlock, 0, st>>>(gv, slots, scan);
   return CFGS_OK;
 }
 
-// Steps 2-3, after launch_depth_order: emission in depth order, tile sort, tile ranges.
+// Steps 2-3, after launch_depth_order: tile keys, tile sort, tile ranges.
 template <class Scenes>
 int launch_instances(const BinArgs<Scenes>& a, cudaStream_t st) {
-  const GeomView& gv = a.geom;
-  const BinningView& bv = a.bin;
-  const int64_t slots = a.total_slots;
-  if (slots > 0) {
-    // 2. emission in depth order
-    const int rank_blocks = (int)((slots + kPreprocessBlock - 1) / kPreprocessBlock);
-    EmitArgs<Scenes> e;
-    e.scenes = a.scenes;
-    e.total_slots = slots;
-    e.order = gv.depth_val[1];
-    e.rank_sums = gv.rank_sums;
-    e.rank_scanned = rank_scan_needed(rank_blocks);
-    e.geom = gv;
-    e.bin = bv;
-    e.cap = a.cap;
-    e.counts = a.counts;
-    k_emit<Scenes><<<rank_blocks, kPreprocessBlock, 0, st>>>(e);
+  if (a.total_slots > 0) {
+    const EmitArgs<Scenes> e = emit_args(a);
+    int passes, width;
+    tile_sort_plan(a.num_tiles, &passes, &width);
+    const SortPass first = tile_pass(a, 0, passes, width);
+    k_emit_starts<Scenes><<<slot_blocks(a.total_slots), kPreprocessBlock, 0, st>>>(
+        e, (uint32_t)(kSortThreads * first.items));
+    if (first.items == 8) launch_emit_items<Scenes, 8>(e, first, st);
+    else launch_emit_items<Scenes, 4>(e, first, st);
+    for (int pass = 1; pass < passes; ++pass) launch_pass(tile_pass(a, pass, passes, width), st);
   }
-  // 3. tile sort of the instances: 0 -> 1 -> 0 ... -> sorted
-  int passes, width;
-  tile_sort_plan(a.num_tiles, &passes, &width);
-  const int total_bits = passes * width;
-  (void)total_bits;
-  int src = 0;
-  for (int pass = 0; pass < passes; ++pass) {
-    SortPass p{};
-    const bool last = pass == passes - 1;
-    const int dst = src ^ 1;
-    p.key_in = bv.key[src];
-    p.val_in = bv.gid[src];
-    p.aux_in = pass == 0 ? nullptr : bv.pidx[src];
-    p.key_out = last ? nullptr : bv.key[dst];
-    p.val_out = last ? bv.sorted_gid : bv.gid[dst];
-    p.aux_out = last ? bv.sorted_pidx : bv.pidx[dst];
-    p.tile_count = last ? a.tile_count : nullptr;
-    p.shift = width * pass;
-    p.bits = width;
-    p.counts = a.counts;
-    p.cap = a.cap;
-    p.num_chunks = sort_chunks(a.cap, kTileChunk);
-    p.chunk_counts = bv.chunk_counts;
-    p.digit_totals = bv.totals + kSortDigits * pass;
-    int s = launch_pass<kTileChunk, false>(p, st);
-    if (s != CFGS_OK) return s;
-    src = dst;
-  }
-  k_tile_ranges<<<1, 1024, 0, st>>>(a.tile_count, a.tile_range, a.num_tiles);
+  k_tile_ranges<<<1, 1024, 0, st>>>(a.tile_count, a.tile_range, (int)a.num_tiles);
   return CFGS_OK;
 }
 
@@ -595,11 +819,10 @@ int launch_instances(const BinArgs<Scenes>& a, cudaStream_t st) {
 template <class Scenes>
 struct PersistentBinArgs {
   SortPass depth[kDepthPasses];
-  const uint32_t* order;
-  const uint32_t* touched;
+  GeomView geom;
   int64_t slots;
-  uint32_t* rank_sums;
-  int rank_blocks;
+  int rank_blocks, start_blocks;
+  bool rank_scanned;
   EmitArgs<Scenes> emit;
   SortPass tile[kMaxTilePasses];
   int tile_passes;
@@ -611,8 +834,10 @@ struct PersistentBinArgs {
 };
 
 template <class Scenes>
-__global__ void __launch_bounds__(kSortThreads) k_binning_persistent(PersistentBinArgs<Scenes> a) {
-  static_assert(kSortThreads == kPreprocessBlock && kDepthChunk == kTileChunk, "one block shape for every stage");
+__global__ void __launch_bounds__(kSortThreads, 3) k_binning_persistent(PersistentBinArgs<Scenes> a) {
+  static_assert(kSortThreads == kPreprocessBlock, "one block shape for every stage");
+  constexpr int kItems = 4;  // every pass's chunks (launch_binning_persistent)
+  __shared__ __align__(16) BinShared<kItems> sh;
   auto each = [&](int64_t blocks, auto&& block_fn) {
     for (int64_t b = blockIdx.x; b < blocks; b += gridDim.x) {
       block_fn((uint32_t)b);
@@ -621,104 +846,61 @@ __global__ void __launch_bounds__(kSortThreads) k_binning_persistent(PersistentB
   };
   for (int pass = 0; pass < kDepthPasses; ++pass) {
     const SortPass& p = a.depth[pass];
-    if (pass == 0) each(p.num_chunks, [&](uint32_t b) { sort_count_block<kDepthChunk, true>(p, b); });
-    else each(p.num_chunks, [&](uint32_t b) { sort_count_block<kDepthChunk, false>(p, b); });
+    if (pass == 0) each(p.num_chunks, [&](uint32_t b) { sort_count_block<kItems, true>(p, sh, b); });
+    else each(p.num_chunks, [&](uint32_t b) { sort_count_block<kItems, false>(p, sh, b); });
     if (!grid_barrier(a.barrier, a.flags)) return;
-    each(1 << p.bits, [&](uint32_t b) { sort_scan_block<kDepthChunk>(p, (int)b); });
+    each(1 << p.bits, [&](uint32_t b) { sort_scan_block(p, sh.scan, (int)b); });
     if (!grid_barrier(a.barrier, a.flags)) return;
-    if (pass == 0) each(p.num_chunks, [&](uint32_t b) { sort_scatter_block<kDepthChunk, true>(p, b); });
-    else each(p.num_chunks, [&](uint32_t b) { sort_scatter_block<kDepthChunk, false>(p, b); });
+    each(p.num_chunks, [&](uint32_t b) { sort_scatter_block<kItems, kValue>(p, a.emit.list, sh, b); });
     if (!grid_barrier(a.barrier, a.flags)) return;
   }
-  each(a.rank_blocks, [&](uint32_t b) { rank_sums_block(a.order, a.touched, a.slots, a.rank_sums, (int)b); });
+  each(a.rank_blocks, [&](uint32_t b) { rank_sums_block(a.geom, a.slots, sh.scan, (int)b); });
   if (!grid_barrier(a.barrier, a.flags)) return;
-  if (a.emit.rank_scanned) {
-    if (blockIdx.x == 0) rank_scan_block(a.rank_sums, a.rank_blocks);
+  if (a.rank_scanned) {
+    if (blockIdx.x == 0) rank_scan_block(a.geom.rank_sums, a.rank_blocks, sh.scan);
     if (!grid_barrier(a.barrier, a.flags)) return;
   }
-  each(a.rank_blocks, [&](uint32_t b) { emit_block<Scenes>(a.emit, (int)b); });
+  each(a.rank_blocks, [&](uint32_t b) { rank_place_block(a.geom, a.slots, a.rank_scanned, sh.scan, (int)b); });
+  if (!grid_barrier(a.barrier, a.flags)) return;
+  each(a.start_blocks, [&](uint32_t b) { emit_starts_block<Scenes>(a.emit, kSortThreads * kItems, (int)b); });
   if (!grid_barrier(a.barrier, a.flags)) return;
   for (int pass = 0; pass < a.tile_passes; ++pass) {
     const SortPass& p = a.tile[pass];
-    each(p.num_chunks, [&](uint32_t b) { sort_count_block<kTileChunk, false>(p, b); });
+    if (pass == 0) each(p.num_chunks, [&](uint32_t b) { emit_keys_block<Scenes, kItems>(a.emit, p, sh, b); });
+    else each(p.num_chunks, [&](uint32_t b) { sort_count_block<kItems, false>(p, sh, b); });
     if (!grid_barrier(a.barrier, a.flags)) return;
-    each(1 << p.bits, [&](uint32_t b) { sort_scan_block<kTileChunk>(p, (int)b); });
+    each(1 << p.bits, [&](uint32_t b) { sort_scan_block(p, sh.scan, (int)b); });
     if (!grid_barrier(a.barrier, a.flags)) return;
-    each(p.num_chunks, [&](uint32_t b) { sort_scatter_block<kTileChunk, false>(p, b); });
+    if (pass == 0) each(p.num_chunks, [&](uint32_t b) { sort_scatter_block<kItems, kFirstPair>(p, a.emit.list, sh, b); });
+    else each(p.num_chunks, [&](uint32_t b) { sort_scatter_block<kItems, kPair>(p, a.emit.list, sh, b); });
     if (!grid_barrier(a.barrier, a.flags)) return;
   }
-  if (blockIdx.x == 0) tile_ranges_block(a.tile_count, a.tile_range, a.num_tiles);
+  if (blockIdx.x == 0) tile_ranges_block<kScanItems>(a.tile_count, a.tile_range, a.num_tiles, sh.scan);
 }
 
 // The pass descriptions of launch_depth_order and launch_instances, for one launch.
 template <class Scenes>
 int launch_binning_persistent(const BinArgs<Scenes>& a, GridBarrier* barrier, cudaStream_t st) {
-  const GeomView& gv = a.geom;
-  const BinningView& bv = a.bin;
-  const int64_t slots = a.total_slots;
-  if (slots <= 0) return launch_instances(a, st);
+  if (a.total_slots <= 0) return launch_instances(a, st);
   PersistentBinArgs<Scenes> pa{};
-  int src = -1;
-  for (int pass = 0; pass < kDepthPasses; ++pass) {
-    SortPass& p = pa.depth[pass];
-    const bool last = pass == kDepthPasses - 1;
-    const int dst = src == 0 ? 1 : 0;
-    p.key_in = src < 0 ? nullptr : gv.depth_key[src];
-    p.val_in = src < 0 ? nullptr : gv.depth_val[src];
-    p.depth_rgbd = gv.rgbd;
-    p.depth_touched = gv.touched;
-    p.key_out = last ? nullptr : gv.depth_key[dst];
-    p.val_out = last ? gv.depth_val[1] : gv.depth_val[dst];
-    p.shift = 8 * pass;
-    p.bits = 8;
-    p.n = slots;
-    p.cap = slots;
-    p.num_chunks = sort_chunks(slots, kDepthChunk);
-    p.chunk_counts = gv.depth_counts;
-    p.digit_totals = gv.depth_totals + kSortDigits * pass;
-    src = dst;
-  }
-  const int rank_blocks = (int)((slots + kPreprocessBlock - 1) / kPreprocessBlock);
-  pa.order = gv.depth_val[1];
-  pa.touched = gv.touched;
-  pa.slots = slots;
-  pa.rank_sums = gv.rank_sums;
-  pa.rank_blocks = rank_blocks;
-  EmitArgs<Scenes>& e = pa.emit;
-  e.scenes = a.scenes;
-  e.total_slots = slots;
-  e.order = gv.depth_val[1];
-  e.rank_sums = gv.rank_sums;
-  e.rank_scanned = rank_scan_needed(rank_blocks);
-  e.geom = gv;
-  e.bin = bv;
-  e.cap = a.cap;
-  e.counts = a.counts;
+  auto narrow = [](SortPass p, int64_t n) {
+    p.items = 4;
+    p.num_chunks = sort_chunks(n, kSortThreads * 4);
+    return p;
+  };
+  for (int pass = 0; pass < kDepthPasses; ++pass)
+    pa.depth[pass] = narrow(depth_pass(a.geom, a.total_slots, pass), a.total_slots);
+  pa.geom = a.geom;
+  pa.slots = a.total_slots;
+  pa.rank_blocks = rank_blocks_of(a.total_slots);
+  pa.start_blocks = slot_blocks(a.total_slots);
+  pa.rank_scanned = rank_scan_needed(pa.rank_blocks);
+  pa.emit = emit_args(a);
   int passes, width;
   tile_sort_plan(a.num_tiles, &passes, &width);
   if (passes > kMaxTilePasses) return CFGS_ERR_TOO_LARGE;
   pa.tile_passes = passes;
-  src = 0;
-  for (int pass = 0; pass < passes; ++pass) {
-    SortPass& p = pa.tile[pass];
-    const bool last = pass == passes - 1;
-    const int dst = src ^ 1;
-    p.key_in = bv.key[src];
-    p.val_in = bv.gid[src];
-    p.aux_in = pass == 0 ? nullptr : bv.pidx[src];
-    p.key_out = last ? nullptr : bv.key[dst];
-    p.val_out = last ? bv.sorted_gid : bv.gid[dst];
-    p.aux_out = last ? bv.sorted_pidx : bv.pidx[dst];
-    p.tile_count = last ? a.tile_count : nullptr;
-    p.shift = width * pass;
-    p.bits = width;
-    p.counts = a.counts;
-    p.cap = a.cap;
-    p.num_chunks = sort_chunks(a.cap, kTileChunk);
-    p.chunk_counts = bv.chunk_counts;
-    p.digit_totals = bv.totals + kSortDigits * pass;
-    src = dst;
-  }
+  for (int pass = 0; pass < passes; ++pass) pa.tile[pass] = narrow(tile_pass(a, pass, passes, width), a.cap);
   pa.tile_count = a.tile_count;
   pa.tile_range = a.tile_range;
   pa.num_tiles = (int)a.num_tiles;
@@ -726,9 +908,6 @@ int launch_binning_persistent(const BinArgs<Scenes>& a, GridBarrier* barrier, cu
   pa.flags = &a.counts->flags;
 
   // every block resident: the grid is the kernel's occupancy times the SM count (per device)
-  const int smem = (int)ScatterSmem<kTileChunk>::bytes(true);
-  static std::atomic<uint64_t> smem_set{0};
-  if (!ensure_dynamic_smem(k_binning_persistent<Scenes>, smem, smem_set)) return CFGS_ERR_LAUNCH;
   static std::atomic<int> grid_of_device[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return CFGS_ERR_LAUNCH;
@@ -736,7 +915,7 @@ int launch_binning_persistent(const BinArgs<Scenes>& a, GridBarrier* barrier, cu
   if (grid <= 0) {
     int sms = 0, per_sm = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_binning_persistent<Scenes>, kSortThreads, smem) !=
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_binning_persistent<Scenes>, kSortThreads, 0) !=
             cudaSuccess ||
         sms <= 0 || per_sm <= 0)
       return CFGS_ERR_LAUNCH;
@@ -746,7 +925,6 @@ int launch_binning_persistent(const BinArgs<Scenes>& a, GridBarrier* barrier, cu
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(kSortThreads);
-  cfg.dynamicSmemBytes = (size_t)smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -786,11 +964,10 @@ int sort_pairs(uint32_t* keys[2], uint32_t* vals[2], int64_t n, int bits, uint32
     p.bits = min(width, bits - width * pass);
     p.n = n;
     p.cap = n;
-    p.num_chunks = sort_chunks(n, kTileChunk);
+    set_chunks(p, n);
     p.chunk_counts = chunk_counts;
     p.digit_totals = totals + kSortDigits * pass;
-    int s = launch_pass<kTileChunk, false>(p, st);
-    if (s != CFGS_OK) return s;
+    if (n > 0) launch_pass(p, st);
     src = dst;
   }
   *result = src;

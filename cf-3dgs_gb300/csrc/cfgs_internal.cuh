@@ -38,9 +38,9 @@ inline bool ensure_dynamic_smem(Kernel* kernel, int bytes, std::atomic<uint64_t>
   return true;
 }
 
-// Binning sorts (stable LSD radix, at most 8 bits per pass) work on chunks of
-// elements: kDepthChunk for the depth sort of the Gaussians (4 passes), kTileChunk for
-// the tile sort of the instances.
+// Binning sorts (stable LSD radix, at most 8 bits per pass) work on chunks of at least
+// kDepthChunk elements for the depth sort of the Gaussians (4 passes) and kTileChunk for
+// the tile sort of the instances (the workspaces are sized for these).
 constexpr int kDepthChunk = 1024;
 constexpr int kTileChunk = 1024;
 constexpr int kSortDigits = 256;  // digits per pass at most (8 bits)
@@ -86,9 +86,9 @@ struct GeomView {
   uint32_t* offset;    // first instance index of the Gaussian (instances are numbered in depth order)
   uint8_t* clamped;    // bit c set: SH colour channel c was clamped at 0
   uint32_t* block_sums;
-  uint32_t* depth_key[2];  // depth sort ping-pong keys
+  uint32_t* depth_key[2];  // depth sort ping-pong keys; depth_key[0] ends as the instance prefix by depth rank
   uint32_t* depth_val[2];  // depth sort ping-pong Gaussian ids; depth_val[1] = Gaussians in depth order
-  uint32_t* rank_sums;     // instances per 256 depth-ordered Gaussians
+  uint32_t* rank_sums;     // instances per 1024 depth-ordered Gaussians
   uint32_t* depth_counts;  // [256][chunks] per-pass digit counts, then first slots
   uint32_t* depth_totals;  // [passes][256] digit totals
   __host__ __device__ GeomView() {}
@@ -150,12 +150,13 @@ struct ImageView {
   }
 };
 
-// Instances (one per Gaussian and touched tile). The emission writes them in depth
-// order (tile key, Gaussian id; the instance index is the position); the tile sort
-// passes ping-pong between the two buffers and the last one writes sorted_gid and
+// Instances (one per Gaussian and touched tile). Their tile keys are written in depth
+// order (the instance index is the position in that order); the tile sort passes
+// ping-pong between two key buffers and two buffers of (Gaussian id, instance index)
+// pairs, in the room of `gid` and of `pidx`, and the last one writes sorted_gid and
 // sorted_pidx.
 struct BinningLayout {
-  size_t key, gid, pidx, sorted_gid, sorted_pidx, chunk_counts, totals, total;
+  size_t key, gid, pidx, sorted_gid, sorted_pidx, chunk_counts, totals, starts, total;
   __host__ __device__ explicit BinningLayout(int64_t cap) {
     const size_t c = pingpong_stride(cap);
     size_t o = 0;
@@ -166,18 +167,19 @@ struct BinningLayout {
     sorted_pidx = o;  o = align256(o + sizeof(uint32_t) * c);
     chunk_counts = o; o = align256(o + sizeof(uint32_t) * kSortDigits * (size_t)sort_chunks(cap, kTileChunk));
     totals = o;       o = align256(o + sizeof(uint32_t) * kSortDigits * kMaxTilePasses);
+    starts = o;       o = align256(o + sizeof(uint32_t) * ((size_t)sort_chunks(cap, kTileChunk) + 1));
     total = o;
   }
 };
 
 struct BinningView {
   uint32_t* key[2];       // global tile index of the instance
-  uint32_t* gid[2];       // Gaussian id
-  uint32_t* pidx[2];      // instance index (position in depth order)
+  uint2* pair[2];         // Gaussian id, instance index (position in depth order)
   uint32_t* sorted_gid;   // sorted position -> Gaussian id
   uint32_t* sorted_pidx;  // sorted position -> instance index
   uint32_t* chunk_counts; // [256][chunks] per-pass digit counts, then first slots
   uint32_t* totals;       // [passes][256] digit totals
+  uint32_t* starts;       // [chunks + 1] depth rank whose instances cover a chunk's first position
   __host__ __device__ BinningView() {}
   __host__ __device__ BinningView(void* base, int64_t cap) {
     BinningLayout L(cap);
@@ -185,14 +187,13 @@ struct BinningView {
     char* b = static_cast<char*>(base);
     key[0] = reinterpret_cast<uint32_t*>(b + L.key);
     key[1] = key[0] + c;
-    gid[0] = reinterpret_cast<uint32_t*>(b + L.gid);
-    gid[1] = gid[0] + c;
-    pidx[0] = reinterpret_cast<uint32_t*>(b + L.pidx);
-    pidx[1] = pidx[0] + c;
+    pair[0] = reinterpret_cast<uint2*>(b + L.gid);
+    pair[1] = reinterpret_cast<uint2*>(b + L.pidx);
     sorted_gid = reinterpret_cast<uint32_t*>(b + L.sorted_gid);
     sorted_pidx = reinterpret_cast<uint32_t*>(b + L.sorted_pidx);
     chunk_counts = reinterpret_cast<uint32_t*>(b + L.chunk_counts);
     totals = reinterpret_cast<uint32_t*>(b + L.totals);
+    starts = reinterpret_cast<uint32_t*>(b + L.starts);
   }
 };
 

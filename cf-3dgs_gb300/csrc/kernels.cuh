@@ -17,7 +17,7 @@ struct PreArgs {
   int64_t total_slots;  // Gaussian slots covered by the launch (padded in batches)
 };
 
-// Binning: depth sort, emission in depth order, tile sort, tile ranges.
+// Binning: depth sort, tile keys in depth order, tile sort, tile ranges.
 template <class Scenes>
 struct BinArgs {
   Scenes scenes;
@@ -31,15 +31,20 @@ struct BinArgs {
   uint32_t* tile_range;
 };
 
+// The list of instances in depth order, which is not stored: these give the Gaussian of any
+// position, its rectangle the tile.
+struct InstanceList {
+  const uint32_t* order;   // Gaussians in (depth, id) order
+  const uint32_t* prefix;  // first instance of each depth rank
+  uint32_t* starts;        // depth rank at each chunk's first position
+};
 template <class Scenes>
 struct EmitArgs {
   Scenes scenes;
   int64_t total_slots;
-  const uint32_t* order;      // Gaussians in (depth, id) order
-  const uint32_t* rank_sums;  // instances per 256 of them (exclusive prefix when rank_scanned)
-  bool rank_scanned;          // k_rank_scan ran (rank_scan_needed)
+  InstanceList list;
+  uint32_t* keys;  // tile of every instance
   GeomView geom;
-  BinningView bin;
   int64_t cap;
   CfgsCounts* counts;
 };
