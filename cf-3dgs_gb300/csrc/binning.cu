@@ -18,12 +18,12 @@
 // last tile pass also counts the instances of every tile (runs of equal tiles), and a
 // scan turns the counts into tile ranges.
 //
-// Every radix pass is three launches over chunks of elements: count (digit histogram per
-// chunk), scan (per digit, over chunks: the chunk's first global slot), scatter (rank
-// inside the chunk, exchange through shared memory by digit, then write each digit's run
-// to its global slots). Ranking inside a chunk is stable: a warp owns a contiguous slice
-// and walks it 64 elements per round; lanes with equal digits meet in a mask in shared
-// memory.
+// Every radix pass is three launches over chunks of elements (two where the chunks are
+// few): count (digit histogram per chunk), scan (per digit, over chunks: the chunk's first
+// global slot), scatter (rank inside the chunk, exchange through shared memory by digit,
+// then write each digit's run to its global slots). Ranking inside a chunk is stable: a warp
+// owns a contiguous slice and walks it 64 elements per round; lanes with equal digits meet
+// in a mask in shared memory.
 //
 // The scatters are bound by shared memory (84 to 87 % of its wavefronts), the rest by latency
 // per block, so a thread holds its keys in registers, all loads in flight at once, an element
@@ -31,6 +31,8 @@
 // tile pass carries positions only. 1,000,000 Gaussians, 12.4 million instances, 8160 tiles:
 // the depth order 114 us, tile keys 48, tile sort 172, ranges 5; with the list written out
 // first, chunks staged through shared memory and a ballot per digit bit, 130, 84, 250 and 10.
+
+
 #include "cfgs_internal.cuh"
 #include "kernels.cuh"
 
@@ -45,6 +47,14 @@ constexpr int kSortWarps = kSortThreads / 32;
 // depths: scatters 12.4 us each, with 8 elements 13.3): from 16 of those blocks per SM.
 constexpr int64_t kWideListMin = 16 * 152 * 4 * kSortThreads;
 inline int radix_items(int64_t n) { return n >= kWideListMin ? 8 : 4; }
+
+// Few chunks are added up by every scatter block itself, from counts stored chunk by chunk;
+// more by the scan kernel, from counts stored digit by digit. (Forward of 16,384 Gaussians at
+// 256x256, chunks 16 and below 128: 154 -> 141 us, with the line at 64 chunks 145. At 225
+// chunks the sums cost what the launch did: 12.64 against 12.58 ms for 25 pose iterations.)
+constexpr int64_t kFoldMaxChunks = 128;
+constexpr int kFoldUnroll = 6;  // loads in flight per thread
+inline bool fold_counts(int64_t num_chunks) { return num_chunks <= kFoldMaxChunks; }
 
 // What a radix pass carries beside the key.
 enum Payload {
@@ -72,7 +82,8 @@ struct SortPass {
   const CfgsCounts* counts;    // element count = num_rendered (nothing to do above cap)
   int64_t cap;
   int64_t num_chunks;          // chunks covered by the grid
-  uint32_t* chunk_counts;      // [1 << bits][num_chunks]
+  bool fold;                   // no scan launch: the scatter adds up the counts (fold_counts)
+  uint32_t* chunk_counts;      // [1 << bits][num_chunks]; with fold [num_chunks][kSortDigits]
   uint32_t* digit_totals;      // [1 << bits], written by the scan
 };
 
@@ -192,7 +203,7 @@ __device__ __forceinline__ void write_chunk_counts(const SortPass& p, CountShare
     uint32_t s = 0;
 #pragma unroll
     for (int w = 0; w < kSortWarps; ++w) s += sh.whist[w][d];
-    p.chunk_counts[(size_t)d * p.num_chunks + bid] = s;
+    p.chunk_counts[p.fold ? (size_t)bid * kSortDigits + d : (size_t)d * p.num_chunks + bid] = s;
   }
 }
 
@@ -405,8 +416,38 @@ __device__ __forceinline__ void scatter_chunk(const SortPass& p, const InstanceL
   uint32_t key[ITEMS];
 #pragma unroll
   for (int k = 0; k < ITEMS; ++k) key[k] = FULL || i0 + 32 * k < cnt ? p.key_in[c0 + i0 + 32 * k] : 0u;
-  const uint32_t dtot = t < ndig ? p.digit_totals[t] : 0u;
-  const uint32_t earlier = t < ndig ? p.chunk_counts[(size_t)t * p.num_chunks + bid] : 0u;
+  // digit t: elements in all chunks and in earlier chunks; folded, digits 4 (t % 64) ... + 3
+  // over every fourth chunk first
+  uint32_t dtot = 0, earlier = 0;
+  uint4 tot4 = make_uint4(0u, 0u, 0u, 0u), earlier4 = tot4;
+  const bool fold = ITEMS == 4 && p.fold;
+  if (fold) {
+    const uint32_t nc = (pass_elements(p) + kChunk - 1) / kChunk;
+    const uint4* counts = reinterpret_cast<const uint4*>(p.chunk_counts) + (t & 63);
+    if (4 * (t & 63) < ndig) {
+      for (uint32_t c = t >> 6; c < nc; c += 4 * kFoldUnroll) {
+        uint4 v[kFoldUnroll];
+#pragma unroll
+        for (int k = 0; k < kFoldUnroll; ++k)
+          v[k] = c + 4 * k < nc ? counts[(c + 4 * k) * (kSortDigits / 4)] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int k = 0; k < kFoldUnroll; ++k) {
+          const uint32_t use = c + 4 * k < bid ? 0xffffffffu : 0u;
+          tot4.x += v[k].x;
+          tot4.y += v[k].y;
+          tot4.z += v[k].z;
+          tot4.w += v[k].w;
+          earlier4.x += v[k].x & use;
+          earlier4.y += v[k].y & use;
+          earlier4.z += v[k].z & use;
+          earlier4.w += v[k].w & use;
+        }
+      }
+    }
+  } else if (t < ndig) {
+    dtot = p.digit_totals[t];
+    earlier = p.chunk_counts[(size_t)t * p.num_chunks + bid];
+  }
   clear_digits(&sh.whist[0][0], 1);
   clear_digits(&sh.same[0][0][0], 2);
   if (P == kFirstPair) mark_chunk(a, sh, bid, c0, (uint32_t)cnt);
@@ -446,6 +487,18 @@ __device__ __forceinline__ void scatter_chunk(const SortPass& p, const InstanceL
     __syncwarp();
   }
   __syncthreads();
+  if (fold) {
+    uint4* parts = reinterpret_cast<uint4*>(&sh.same[0][0][0]);  // [2][4][kSortDigits]
+    parts[t] = tot4;
+    parts[kSortThreads + t] = earlier4;
+    __syncthreads();
+    const uint32_t* part = &sh.same[0][0][0];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      dtot += part[g * kSortDigits + t];
+      earlier += part[(4 + g) * kSortDigits + t];
+    }
+  }
 
   // digit t: the warps' first positions, the digit's global slot
   uint32_t dsum = 0, first[kSortWarps];
@@ -662,6 +715,7 @@ namespace {
 
 // The scan's block: a digit's chunks in one round where they are few.
 void launch_scan(const SortPass& p, cudaStream_t st) {
+  if (p.fold) return;
   k_sort_scan<<<1 << p.bits, p.num_chunks <= 256 * kScanItems ? 256 : 1024, 0, st>>>(p);
 }
 
@@ -705,6 +759,7 @@ namespace {
 void set_chunks(SortPass& p, int64_t n) {
   p.items = radix_items(n);
   p.num_chunks = sort_chunks(n, kSortThreads * p.items);
+  p.fold = p.items == 4 && fold_counts(p.num_chunks);
 }
 
 // Pass `pass` of the depth sort: the depths (keys formed in depth_key[1]) -> 0 -> 1 -> 0 ->
@@ -849,8 +904,10 @@ __global__ void __launch_bounds__(kSortThreads, 3) k_binning_persistent(Persiste
     if (pass == 0) each(p.num_chunks, [&](uint32_t b) { sort_count_block<kItems, true>(p, sh, b); });
     else each(p.num_chunks, [&](uint32_t b) { sort_count_block<kItems, false>(p, sh, b); });
     if (!grid_barrier(a.barrier, a.flags)) return;
-    each(1 << p.bits, [&](uint32_t b) { sort_scan_block(p, sh.scan, (int)b); });
-    if (!grid_barrier(a.barrier, a.flags)) return;
+    if (!p.fold) {
+      each(1 << p.bits, [&](uint32_t b) { sort_scan_block(p, sh.scan, (int)b); });
+      if (!grid_barrier(a.barrier, a.flags)) return;
+    }
     each(p.num_chunks, [&](uint32_t b) { sort_scatter_block<kItems, kValue>(p, a.emit.list, sh, b); });
     if (!grid_barrier(a.barrier, a.flags)) return;
   }
@@ -869,8 +926,10 @@ __global__ void __launch_bounds__(kSortThreads, 3) k_binning_persistent(Persiste
     if (pass == 0) each(p.num_chunks, [&](uint32_t b) { emit_keys_block<Scenes, kItems>(a.emit, p, sh, b); });
     else each(p.num_chunks, [&](uint32_t b) { sort_count_block<kItems, false>(p, sh, b); });
     if (!grid_barrier(a.barrier, a.flags)) return;
-    each(1 << p.bits, [&](uint32_t b) { sort_scan_block(p, sh.scan, (int)b); });
-    if (!grid_barrier(a.barrier, a.flags)) return;
+    if (!p.fold) {
+      each(1 << p.bits, [&](uint32_t b) { sort_scan_block(p, sh.scan, (int)b); });
+      if (!grid_barrier(a.barrier, a.flags)) return;
+    }
     if (pass == 0) each(p.num_chunks, [&](uint32_t b) { sort_scatter_block<kItems, kFirstPair>(p, a.emit.list, sh, b); });
     else each(p.num_chunks, [&](uint32_t b) { sort_scatter_block<kItems, kPair>(p, a.emit.list, sh, b); });
     if (!grid_barrier(a.barrier, a.flags)) return;
@@ -886,6 +945,7 @@ int launch_binning_persistent(const BinArgs<Scenes>& a, GridBarrier* barrier, cu
   auto narrow = [](SortPass p, int64_t n) {
     p.items = 4;
     p.num_chunks = sort_chunks(n, kSortThreads * 4);
+    p.fold = fold_counts(p.num_chunks);
     return p;
   };
   for (int pass = 0; pass < kDepthPasses; ++pass)

@@ -26,6 +26,8 @@ CASES = {
     "three_pass": (4112, 4112, 3_000, 3.0),                  # 257 * 257 tiles
     "three_pass_giant": (4112, 4112, 12, 1000.0),
     "equal_depths": (320, 240, 5_000, 2.0),
+    "depth_chunks_added_up": (100, 80, 128 * 1024, 0.3),     # last count without a scan launch
+    "depth_chunks_scanned": (100, 80, 128 * 1024 + 1, 0.3),
 }
 
 
