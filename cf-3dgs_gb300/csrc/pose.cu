@@ -22,90 +22,116 @@ namespace cfgs {
 constexpr int kPoseThreads = 256;
 constexpr int kPosePartials = 9;  // sum g (3), sum (R p) x g (3), w_cov (3)
 
-struct SE3d {
-  double R[9];
-  double t[3];
-};
-
-__host__ __device__ inline void hat(const double* w, double* M) {
-  M[0] = 0;     M[1] = -w[2]; M[2] = w[1];
-  M[3] = w[2];  M[4] = 0;     M[5] = -w[0];
-  M[6] = -w[1]; M[7] = w[0];  M[8] = 0;
-}
 __host__ __device__ inline void mm3(const double* A, const double* B, double* C) {
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j) C[3 * i + j] = A[3 * i] * B[j] + A[3 * i + 1] * B[3 + j] + A[3 * i + 2] * B[6 + j];
 }
 
-// Coefficients of exp / left Jacobian as functions of theta, with series near 0.
-__device__ inline void so3_coeffs(double th2, double* a, double* b, double* c) {
-  // a = sin(th)/th, b = (1-cos th)/th^2, c = (th - sin th)/th^3
-  if (th2 < 1e-8) {
-    *a = 1.0 - th2 / 6.0;
-    *b = 0.5 - th2 / 24.0;
-    *c = 1.0 / 6.0 - th2 / 120.0;
+// ---- exp(xi) and its Jacobian blocks by one warp ------------------------------------------
+// Lane 3 i + j (mod 9) holds element (i, j) of every 3x3 matrix.
+struct LanePose {
+  double R, t;   // exp(xi): element of the rotation; lane i mod 3: component i of the translation
+  double Jl, Q;  // SO(3) left Jacobian of phi, upper-right block of the SE(3) one
+};
+
+__device__ __forceinline__ double lane_mm3(double A, double B, int i, int j) {
+  const double a0 = __shfl_sync(0xffffffffu, A, 3 * i), a1 = __shfl_sync(0xffffffffu, A, 3 * i + 1),
+               a2 = __shfl_sync(0xffffffffu, A, 3 * i + 2);
+  const double b0 = __shfl_sync(0xffffffffu, B, j), b1 = __shfl_sync(0xffffffffu, B, 3 + j),
+               b2 = __shfl_sync(0xffffffffu, B, 6 + j);
+  return a0 * b0 + a1 * b1 + a2 * b2;
+}
+
+// Element (i, j) of the cross-product matrix of w.
+__device__ __forceinline__ double lane_hat(const double (&w)[3], int i, int j) {
+  if (i == j) return 0.0;
+  const double v = w[3 - i - j];
+  return (j - i + 3) % 3 == 1 ? -v : v;
+}
+
+// With theta = |phi|: R = I + a P + b P^2, Jl = I + b P + c P^2 (P the matrix of phi), t = Jl
+// rho, and Q(rho, phi) after Barfoot, "State Estimation for Robotics", eq. 7.86. Every lane of
+// a warp calls it with the same xi. Bound by latency (a float64 operation takes the pipe 16
+// cycles, its result longer): the sine and cosine share their reduction, the five divisions
+// run on five lanes at once, the matrices element by element. By single threads, one for exp
+// and one for Q, the two took 14,000 and 26,000 cycles, each with its own sines.
+__device__ __forceinline__ LanePose lane_pose(const double (&rho)[3], const double (&phi)[3], int lane) {
+  const int e = lane % 9, i = e / 3, j = e % 3;
+  const double th2 = phi[0] * phi[0] + phi[1] * phi[1] + phi[2] * phi[2];
+  double a, b, c, c1, c2, c3;
+  // a = sin(th)/th, b = (1-cos th)/th^2, c = c1 = (th - sin th)/th^3, c2 = (th^2 + 2 cos th -
+  // 2)/(2 th^4), c3 = (2 th - 3 sin th + th cos th)/(2 th^5), with series near 0
+  if (!(th2 < 1e-8)) {
+    const double th = sqrt(th2);
+    double s, co;
+    sincos(th, &s, &co);
+    const double th3 = th2 * th, th4 = th2 * th2, th5 = th4 * th;
+    double num = s, den = th;
+    if (lane == 1) {
+      num = 1.0 - co;
+      den = th2;
+    } else if (lane == 2) {
+      num = th - s;
+      den = th3;
+    } else if (lane == 3) {
+      num = th2 + 2.0 * co - 2.0;
+      den = 2.0 * th4;
+    } else if (lane == 4) {
+      num = 2.0 * th - 3.0 * s + th * co;
+      den = 2.0 * th5;
+    }
+    const double q = num / den;
+    a = __shfl_sync(0xffffffffu, q, 0);
+    b = __shfl_sync(0xffffffffu, q, 1);
+    c = c1 = __shfl_sync(0xffffffffu, q, 2);
+    c2 = __shfl_sync(0xffffffffu, q, 3);
+    c3 = __shfl_sync(0xffffffffu, q, 4);
   } else {
-    double th = sqrt(th2);
-    double s = sin(th), co = cos(th);
-    *a = s / th;
-    *b = (1.0 - co) / th2;
-    *c = (th - s) / (th2 * th);
+    a = 1.0 - th2 / 6.0;
+    b = 0.5 - th2 / 24.0;
+    c = 1.0 / 6.0 - th2 / 120.0;
   }
-}
-
-__device__ inline void se3_exp(const float* xi, SE3d* X, double* Jl) {
-  double rho[3] = {xi[0], xi[1], xi[2]};
-  double phi[3] = {xi[3], xi[4], xi[5]};
-  double th2 = phi[0] * phi[0] + phi[1] * phi[1] + phi[2] * phi[2];
-  double a, b, c;
-  so3_coeffs(th2, &a, &b, &c);
-  double P[9], P2[9];
-  hat(phi, P);
-  mm3(P, P, P2);
-  for (int k = 0; k < 9; ++k) {
-    double I = (k % 4 == 0) ? 1.0 : 0.0;
-    X->R[k] = I + a * P[k] + b * P2[k];
-    Jl[k] = I + b * P[k] + c * P2[k];
-  }
-  for (int i = 0; i < 3; ++i) X->t[i] = Jl[3 * i] * rho[0] + Jl[3 * i + 1] * rho[1] + Jl[3 * i + 2] * rho[2];
-}
-
-// Q(rho, phi): the upper-right block of the SE(3) left Jacobian (Barfoot, "State
-// Estimation for Robotics", eq. 7.86).
-__device__ inline void se3_Q(const double* rho, const double* phi, double* Q) {
-  double th2 = phi[0] * phi[0] + phi[1] * phi[1] + phi[2] * phi[2];
-  double c1, c2, c3;
   if (th2 < 1e-6) {
     c1 = 1.0 / 6.0 - th2 / 120.0;
     c2 = 1.0 / 24.0 - th2 / 720.0;
     c3 = 1.0 / 120.0 - th2 / 2520.0;
-  } else {
-    double th = sqrt(th2), s = sin(th), co = cos(th);
-    double th3 = th2 * th, th4 = th2 * th2, th5 = th4 * th;
-    c1 = (th - s) / th3;
-    c2 = (th2 + 2.0 * co - 2.0) / (2.0 * th4);
-    c3 = (2.0 * th - 3.0 * s + th * co) / (2.0 * th5);
   }
-  double Rh[9], Ph[9], PR[9], RP[9], PRP[9], PP[9], PPR[9], RPP[9], PRPP[9], PPRP[9];
-  hat(rho, Rh);
-  hat(phi, Ph);
-  mm3(Ph, Rh, PR);
-  mm3(Rh, Ph, RP);
-  mm3(PR, Ph, PRP);
-  mm3(Ph, Ph, PP);
-  mm3(PP, Rh, PPR);
-  mm3(Rh, PP, RPP);
-  mm3(PRP, Ph, PRPP);
-  mm3(Ph, PRP, PPRP);
-  for (int k = 0; k < 9; ++k)
-    Q[k] = 0.5 * Rh[k] + c1 * (PR[k] + RP[k] + PRP[k]) + c2 * (PPR[k] + RPP[k] - 3.0 * PRP[k]) +
-           c3 * (PRPP[k] + PPRP[k]);
+  const double I = i == j ? 1.0 : 0.0, P = lane_hat(phi, i, j), Rh = lane_hat(rho, i, j);
+  const double PP = lane_mm3(P, P, i, j);
+  LanePose o;
+  o.R = I + a * P + b * PP;
+  o.Jl = I + b * P + c * PP;
+  const int r = lane % 3;
+  const double j0 = __shfl_sync(0xffffffffu, o.Jl, 3 * r), j1 = __shfl_sync(0xffffffffu, o.Jl, 3 * r + 1),
+               j2 = __shfl_sync(0xffffffffu, o.Jl, 3 * r + 2);
+  o.t = j0 * rho[0] + j1 * rho[1] + j2 * rho[2];
+  const double PR = lane_mm3(P, Rh, i, j), RP = lane_mm3(Rh, P, i, j);
+  const double PRP = lane_mm3(PR, P, i, j), PPR = lane_mm3(PP, Rh, i, j), RPP = lane_mm3(Rh, PP, i, j);
+  const double PRPP = lane_mm3(PRP, P, i, j), PPRP = lane_mm3(P, PRP, i, j);
+  o.Q = 0.5 * Rh + c1 * (PR + RP + PRP) + c2 * (PPR + RPP - 3.0 * PRP) + c3 * (PRPP + PPRP);
+  return o;
 }
 
-// Each block's thread 0 forms exp(xi) in float64 while the others' positions are on
+// The same into a solve's state.
+__device__ __forceinline__ void store_pose_state(const float (&xi)[6], PoseState* ps, int lane) {
+  const double rho[3] = {xi[0], xi[1], xi[2]}, phi[3] = {xi[3], xi[4], xi[5]};
+  const LanePose o = lane_pose(rho, phi, lane);
+  if (lane < 9) {
+    ps->R64[lane] = o.R;
+    ps->R[lane] = (float)o.R;
+    ps->Jl[lane] = o.Jl;
+    ps->Q[lane] = o.Q;
+  }
+  if (lane < 3) {
+    ps->t64[lane] = o.t;
+    ps->t[lane] = (float)o.t;
+  }
+}
+
+// Each block's first warp forms exp(xi) in float64 while the others' positions are on
 // their way from memory: the chain of double sin, cos and divisions is most of the kernel's
 // time, so a block takes kApplyPerThread positions per thread (230,400 positions: 225
-// blocks, 16.7 -> 10.1 us; one position per thread ran 900 such chains).
+// blocks, 16.7 -> 7.6 us; one position per thread ran 900 such chains).
 constexpr int kApplyPerThread = 4;
 
 template <bool COV>
@@ -121,12 +147,11 @@ __global__ void __launch_bounds__(kPoseThreads) k_pose_apply(int n, const float*
 #pragma unroll
     for (int a = 0; a < 3; ++a) p[k][a] = i < n ? xyz[3 * i + a] : 0.0f;
   }
-  if (threadIdx.x == 0) {
-    SE3d X;
-    double Jl[9];
-    se3_exp(xi, &X, Jl);
-    for (int k = 0; k < 9; ++k) sR[k] = (float)X.R[k];
-    for (int k = 0; k < 3; ++k) st[k] = (float)X.t[k];
+  if (threadIdx.x < 32) {
+    const double rho[3] = {xi[0], xi[1], xi[2]}, phi[3] = {xi[3], xi[4], xi[5]};
+    const LanePose o = lane_pose(rho, phi, threadIdx.x);  // (its Q is not used)
+    if (threadIdx.x < 9) sR[threadIdx.x] = (float)o.R;
+    if (threadIdx.x < 3) st[threadIdx.x] = (float)o.t;
   }
   __syncthreads();
   float R[9];
@@ -168,34 +193,31 @@ __global__ void __launch_bounds__(kPoseThreads) k_pose_apply(int n, const float*
 // passes them, so both optimisers take the same steps. bc1 = 1 - b1^t and
 // bc2 = 1 - b2^t are float64, as torch forms them on the host.
 // state per solve: m[6], v[6], step, 3 unused floats.
-__device__ __forceinline__ double bias_correction(double beta, const float* st) {
-  return 1.0 - pow(beta, (double)(st[12] + 1.0f));
+__device__ __forceinline__ double bias_correction(double beta, float step) {
+  return 1.0 - pow(beta, (double)step);
 }
 
-__device__ __forceinline__ void adam_component(int k, float* xi, const float* grad, float* st, double lr, double b1,
-                                               double b2, double eps, double bc1, double bc2) {
+// The step size and the root of the second correction.
+struct AdamScale {
+  float step_size, bc2_sqrt;
+};
+__device__ __forceinline__ AdamScale adam_scale(double lr, double bc1, double bc2) {
+  return {(float)(-(lr / bc1)), (float)sqrt(bc2)};
+}
+
+__device__ __forceinline__ void adam_component(int k, float* xi, float g, float* st, AdamScale c, double b1, double b2,
+                                               double eps) {
   const float w1 = (float)(1.0 - b1), mul2 = (float)b2, w2 = (float)(1.0 - b2);
-  const float step_size = (float)(-(lr / bc1));
-  const float bc2_sqrt = (float)sqrt(bc2);
   const float eps_f = (float)eps;
-  const float g = grad[k];
   float m = st[k], v = st[6 + k];
   m = fmaf(w1, g - m, m);
   v = v * mul2;
   v = fmaf(w2, g * g, v);
   st[k] = m;
   st[6 + k] = v;
-  float denom = sqrtf(v) / bc2_sqrt;
+  float denom = sqrtf(v) / c.bc2_sqrt;
   denom = denom + eps_f;
-  xi[k] = fmaf(step_size, m / denom, xi[k]);
-}
-
-__device__ void adam_step6_bc(float* xi, const float* grad, float* st, double lr, double b1, double b2, double eps,
-                              double bc1, double bc2) {
-  const float step = st[12] + 1.0f;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) adam_component(k, xi, grad, st, lr, b1, b2, eps, bc1, bc2);
-  st[12] = step;
+  xi[k] = fmaf(c.step_size, m / denom, xi[k]);
 }
 
 // One warp per solve: lanes 0 and 1 form the two bias corrections (a double pow each, the
@@ -205,35 +227,13 @@ __global__ void __launch_bounds__(128) k_pose_adam(int count, float* xi, const f
   const int s = blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (s >= count) return;
   float* st = state + 16 * (size_t)s;
-  const double bc = bias_correction(lane & 1 ? b2 : b1, st);
-  const double bc1 = __shfl_sync(0xffffffffu, bc, 0), bc2 = __shfl_sync(0xffffffffu, bc, 1);
   const float step = st[12] + 1.0f;
+  const double bc = bias_correction(lane & 1 ? b2 : b1, step);
+  const double bc1 = __shfl_sync(0xffffffffu, bc, 0), bc2 = __shfl_sync(0xffffffffu, bc, 1);
   __syncwarp();  // every lane has read the step count
-  if (lane < 6) adam_component(lane, xi + 6 * (size_t)s, grad + 6 * (size_t)s, st, lr, b1, b2, eps, bc1, bc2);
+  if (lane < 6)
+    adam_component(lane, xi + 6 * (size_t)s, grad[6 * (size_t)s + lane], st, adam_scale(lr, bc1, bc2), b1, b2, eps);
   if (lane == 0) st[12] = step;
-}
-
-// The parts of a solve's pose state that depend on xi, split so that two threads can
-// form them at once: exp(xi) with the left Jacobian, and the Q block.
-__device__ void pose_state_exp(const float* xi, PoseState* ps) {
-  SE3d X;
-  double Jl[9];
-  se3_exp(xi, &X, Jl);
-  for (int k = 0; k < 9; ++k) {
-    ps->R64[k] = X.R[k];
-    ps->R[k] = (float)X.R[k];
-    ps->Jl[k] = Jl[k];
-  }
-  for (int k = 0; k < 3; ++k) {
-    ps->t64[k] = X.t[k];
-    ps->t[k] = (float)X.t[k];
-  }
-}
-
-__device__ void pose_state_Q(const float* xi, PoseState* ps) {
-  const double rho[3] = {xi[0], xi[1], xi[2]};
-  const double phi[3] = {xi[3], xi[4], xi[5]};
-  se3_Q(rho, phi, ps->Q);
 }
 
 // dL/dxi from the left-perturbation sums tot = (sum g, sum (R p) x g, w_cov):
@@ -265,7 +265,7 @@ __device__ void pose_grad_from_state(const PoseState& ps, const double* tot, flo
 // w takes rows w, w + 8, ..., one lane per sum) and applies the Jacobian transpose. Bound
 // by the float64 pipe (about 2 operations per cycle and SM). 230,400 Gaussians: 371 us
 // (one thread folded 900 rows of 9 sums one after another, and every block formed exp(xi))
-// -> 30 us.
+// -> 22 us.
 constexpr int kGradMaxBlocks = 2 * 152;  // two blocks of partial sums per SM at most
 constexpr int kGradSums = 16;            // sum g (3), M (9), w_cov (3), unused
 
@@ -305,8 +305,10 @@ __global__ void __launch_bounds__(kPoseThreads) k_pose_grad(PoseGradArgs a) {
   __shared__ bool s_last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (blockIdx.x == 0) {
-    if (threadIdx.x == 0) pose_state_exp(a.xi, a.state);
-    if (threadIdx.x == 32) pose_state_Q(a.xi, a.state);
+    if (warp == 0) {
+      const float x[6] = {a.xi[0], a.xi[1], a.xi[2], a.xi[3], a.xi[4], a.xi[5]};
+      store_pose_state(x, a.state, lane);
+    }
   } else {
     double acc[kGradSums];
 #pragma unroll
@@ -396,69 +398,104 @@ __global__ void __launch_bounds__(kPoseThreads) k_pose_grad(PoseGradArgs a) {
   }
 }
 
-// One block per solve: the state of xi (exp, Q, the next step's bias corrections) by
-// four threads at once.
+// One block per solve: the state of xi by one warp, the next step's bias corrections by two
+// others.
 __global__ void k_batch_pose_init(const float* xi, const float* adam_state, PoseState* states, double b1,
                                   double b2) {
   const int s = blockIdx.x;
   const float* x = xi + 6 * (size_t)s;
-  const float* st = adam_state + 16 * (size_t)s;
-  switch (threadIdx.x) {
-    case 0: pose_state_exp(x, states + s); break;
-    case 32: pose_state_Q(x, states + s); break;
-    case 64: states[s].bc1 = bias_correction(b1, st); break;
-    case 96: states[s].bc2 = bias_correction(b2, st); break;
-    default: break;
+  const float step = adam_state[16 * (size_t)s + 12] + 1.0f;
+  if (threadIdx.x < 32) {
+    const float xs[6] = {x[0], x[1], x[2], x[3], x[4], x[5]};
+    store_pose_state(xs, states + s, threadIdx.x);
   }
+  if (threadIdx.x == 64) states[s].bc1 = bias_correction(b1, step);
+  if (threadIdx.x == 96) states[s].bc2 = bias_correction(b2, step);
 }
 
 // One block per solve: the solve's per-block pose partials summed in a fixed pattern
-// (thread i takes blocks i, i+256, ...; then a fixed tree), the SE(3) Jacobian
-// transpose and the Adam step with the state's cached Jacobian blocks and bias
-// corrections, then the state of the new xi by four threads at once. A solve's result
-// depends only on its own blocks, so it is the same whatever else is in the batch.
-__global__ void __launch_bounds__(256) k_batch_pose_update(const SceneDesc* descs, const double* partials,
-                                                           float* xi, float* adam_state, PoseState* states,
-                                                           const CfgsCounts* counts, int64_t cap, double lr,
-                                                           double b1, double b2, double eps) {
+// (thread i takes blocks i, i+256, ...; then a fixed tree), then by one warp the SE(3)
+// Jacobian transpose and the Adam step (a lane per component) with the state's cached
+// Jacobian blocks and bias corrections, and the state of the new xi, while two other warps
+// form the following step's corrections. A solve's result depends only on its own blocks, so
+// it is the same whatever else is in the batch. Bound by the latency of one chain of float64
+// operations per solve: 27 -> 13 us (900 partials; 24 us of it one thread's sums, gradient, step
+// and then one thread's Q).
+constexpr int kUpdateThreads = 256, kUpdateBatch = 4;
+__global__ void __launch_bounds__(kUpdateThreads) k_batch_pose_update(const SceneDesc* descs, const double* partials,
+                                                                      float* xi, float* adam_state, PoseState* states,
+                                                                      const CfgsCounts* counts, int64_t cap, double lr,
+                                                                      double b1, double b2, double eps) {
   __shared__ double s_red[8][6];
-  __shared__ float s_x[6];
   if ((int64_t)counts->num_rendered > cap) return;  // overflowed iteration: no update
   const int s = blockIdx.x;
   const SceneDesc& sd = descs[s];
   const int b0 = sd.gauss_base / kPreprocessBlock;
   const int nb = (sd.num_gaussians + kPreprocessBlock - 1) / kPreprocessBlock;
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < nb; b += blockDim.x)
-#pragma unroll
-    for (int k = 0; k < 6; ++k) acc[k] += partials[(size_t)(b0 + b) * 9 + k];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float* x = xi + 6 * (size_t)s;
+  float* st = adam_state + 16 * (size_t)s;
+  PoseState* ps = states + s;
+  const float step = st[12];
+  double acc[6] = {0, 0, 0, 0, 0, 0};
+  for (int b = threadIdx.x; b < nb; b += kUpdateThreads * kUpdateBatch) {
+    double v[kUpdateBatch][6];
+#pragma unroll
+    for (int q = 0; q < kUpdateBatch; ++q)
+#pragma unroll
+      for (int k = 0; k < 6; ++k)
+        v[q][k] = b + q * kUpdateThreads < nb ? partials[(size_t)(b0 + b + q * kUpdateThreads) * 9 + k] : 0.0;
+#pragma unroll
+    for (int q = 0; q < kUpdateBatch; ++q)
+#pragma unroll
+      for (int k = 0; k < 6; ++k) acc[k] += v[q][k];
+  }
+  // warp 0, before it waits for the sums: what the step needs of the state
+  const int j = lane % 3;
+  double Jl[3], Q[3], t64[3];
+  AdamScale scale{};
+  if (warp == 0) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      Jl[k] = ps->Jl[3 * k + j];
+      Q[k] = ps->Q[3 * k + j];
+      t64[k] = ps->t64[k];
+    }
+    scale = adam_scale(lr, ps->bc1, ps->bc2);
+  }
   {
     const double tot = warp_sum6_f64(acc, lane);  // lane 4k: partial k of the warp
     if ((lane & 3) == 0 && (lane >> 2) < 6) s_red[warp][lane >> 2] = tot;
   }
   __syncthreads();
-  float* x = xi + 6 * (size_t)s;
-  float* st = adam_state + 16 * (size_t)s;
-  PoseState* ps = states + s;
-  if (threadIdx.x == 0) {
-    double tot[kPosePartials];
-    for (int k = 0; k < kPosePartials; ++k) tot[k] = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w)
-      for (int k = 0; k < 6; ++k) tot[k] += s_red[w][k];
-    float grad[6];
-    pose_grad_from_state(*ps, tot, grad);
-    adam_step6_bc(x, grad, st, lr, b1, b2, eps, ps->bc1, ps->bc2);
-    for (int k = 0; k < 6; ++k) s_x[k] = x[k];
+  if (threadIdx.x == 64) ps->bc1 = bias_correction(b1, (step + 1.0f) + 1.0f);
+  if (threadIdx.x == 96) ps->bc2 = bias_correction(b2, (step + 1.0f) + 1.0f);
+  if (warp != 0) return;
+  double sum = 0.0;
+#pragma unroll
+  for (int w = 0; w < kUpdateThreads / 32; ++w) sum += s_red[w][lane < 6 ? lane : 0];
+  // as pose_grad_from_state: lane j component j, lane 3 + j component 3 + j
+  double gr[3], gp[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) gr[k] = __shfl_sync(0xffffffffu, sum, k);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) gp[k] = __shfl_sync(0xffffffffu, sum, 3 + k);
+  gp[0] = gp[0] + (t64[1] * gr[2] - t64[2] * gr[1]);
+  gp[1] = gp[1] + (t64[2] * gr[0] - t64[0] * gr[2]);
+  gp[2] = gp[2] + (t64[0] * gr[1] - t64[1] * gr[0]);
+  const float g_rho = (float)(Jl[0] * gr[0] + Jl[1] * gr[1] + Jl[2] * gr[2]);
+  const float g_phi =
+      (float)(Q[0] * gr[0] + Q[1] * gr[1] + Q[2] * gr[2] + Jl[0] * gp[0] + Jl[1] * gp[1] + Jl[2] * gp[2]);
+  float moved = 0.f;
+  if (lane < 6) {
+    adam_component(lane, x, lane < 3 ? g_rho : g_phi, st, scale, b1, b2, eps);
+    moved = x[lane];
   }
-  __syncthreads();
-  switch (threadIdx.x) {
-    case 0: pose_state_exp(s_x, ps); break;
-    case 32: pose_state_Q(s_x, ps); break;
-    case 64: ps->bc1 = bias_correction(b1, st); break;
-    case 96: ps->bc2 = bias_correction(b2, st); break;
-    default: break;
-  }
+  if (lane == 0) st[12] = step + 1.0f;
+  float xs[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) xs[k] = __shfl_sync(0xffffffffu, moved, k);
+  store_pose_state(xs, ps, lane);
 }
 
 void launch_batch_pose_init(int count, const float* xi, const float* adam_state, PoseState* states, double b1,
@@ -468,7 +505,7 @@ void launch_batch_pose_init(int count, const float* xi, const float* adam_state,
 void launch_batch_pose_update(int count, const SceneDesc* descs, const double* partials, float* xi,
                               float* adam_state, PoseState* states, const CfgsCounts* counts, int64_t cap, double lr,
                               double b1, double b2, double eps, cudaStream_t st) {
-  k_batch_pose_update<<<count, 256, 0, st>>>(descs, partials, xi, adam_state, states, counts, cap, lr, b1, b2, eps);
+  k_batch_pose_update<<<count, kUpdateThreads, 0, st>>>(descs, partials, xi, adam_state, states, counts, cap, lr, b1, b2, eps);
 }
 
 }  // namespace cfgs
