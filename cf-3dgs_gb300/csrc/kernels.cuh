@@ -92,7 +92,7 @@ struct RenderBwdArgs {
   int64_t cap;
   const CfgsCounts* counts;
   CfgsRenderSchedule sched;  // resolved launch shape (resolve_schedule)
-  bool geom_only;            // form only the 2D-mean and conic sums (batched SH-degree-0 pose solves)
+  bool geom_only;            // form only the 2D-mean and conic sums (pose solves, means-only backward)
 };
 
 template <class Scenes>
@@ -110,6 +110,7 @@ struct PreBwdArgs {
   double* pose_partials;  // pose-only form: [block][9] float64 sums; NULL for the full backward
   bool sh_bulk;           // degree-3 SH moved by bulk copies (16-byte aligned arrays)
   uint32_t* flags;        // CFGS_FLAG_COPY_TIMEOUT
+  bool means_only = false;  // full backward of one image: only dL_dmeans2D and dL_dmeans3D
 };
 
 template <class Scenes>

@@ -49,6 +49,8 @@ __device__ __forceinline__ void group8_sum16(float (&v)[16], int lane) {
   }
 }
 
+enum BwdForm { kFullForm, kMeansForm, kPoseForm };
+
 // SH backward at unit direction (x,y,z): dL/dsh[k][c] = b_k g_c (g already masked by
 // the forward's clamp) and the gradient of sum_k (sh_k . g) b_k with respect to the
 // direction. The basis follows utils/sh_utils.py:57-112.
@@ -149,19 +151,21 @@ __device__ __forceinline__ void sh_backward(int deg, int M, const float* sh, flo
 // 2D grads, conic -> 2D covariance -> 3D covariance -> scale/rotation, projection ->
 // mean, SH -> coefficients and view direction. SH coefficients are read from sh_src and
 // their gradients written to dsh_dst (NULL: not wanted). Returns dL/dmean in dmean.
-template <class Scenes>
+template <BwdForm FORM, class Scenes>
 __device__ __forceinline__ void gaussian_backward(const PreBwdArgs<Scenes>& a, const SceneDesc& sd, int64_t idx,
                                                   uint32_t nt, const float (&acc)[10], const float* sh_src,
-                                                  float* dsh_dst, bool pose_only, float (&dmean)[3]) {
+                                                  float* dsh_dst, float (&dmean)[3]) {
   const int M = sd.sh_coeffs;
   {
     const float W = (float)sd.W, H = (float)sd.H;
     const float dndc_x = acc[0] * (0.5f * W), dndc_y = acc[1] * (0.5f * H);
     const float dcol[3] = {acc[6], acc[7], acc[8]};
-    if (!pose_only) {
+    if (FORM != kPoseForm) {
       a.out.dL_dmeans2D[3 * idx + 0] = dndc_x;
       a.out.dL_dmeans2D[3 * idx + 1] = dndc_y;
       a.out.dL_dmeans2D[3 * idx + 2] = 0.f;
+    }
+    if (FORM == kFullForm) {
       a.out.dL_dopacity[idx] = acc[5];
       if (a.out.dL_dcolors) {
         a.out.dL_dcolors[3 * idx + 0] = dcol[0];
@@ -261,7 +265,7 @@ __device__ __forceinline__ void gaussian_backward(const PreBwdArgs<Scenes>& a, c
     dcov[1] = 2.f * da * T0[0] * T0[1] + db * (T0[0] * T1[1] + T0[1] * T1[0]) + 2.f * dc * T1[0] * T1[1];
     dcov[2] = 2.f * da * T0[0] * T0[2] + db * (T0[0] * T1[2] + T0[2] * T1[0]) + 2.f * dc * T1[0] * T1[2];
     dcov[4] = 2.f * da * T0[1] * T0[2] + db * (T0[1] * T1[2] + T0[2] * T1[1]) + 2.f * dc * T1[1] * T1[2];
-    if (!pose_only && a.out.dL_dcov3D)
+    if (FORM == kFullForm && a.out.dL_dcov3D)
       for (int k = 0; k < 6; ++k) a.out.dL_dcov3D[6 * idx + k] = dcov[k];
     float dT0[3], dT1[3];
     for (int i = 0; i < 3; ++i) {
@@ -296,7 +300,7 @@ __device__ __forceinline__ void gaussian_backward(const PreBwdArgs<Scenes>& a, c
     }
 
     // ---- SH colour ----------------------------------------------------------------
-    if (a.g.shs) {
+    if (FORM != kMeansForm && a.g.shs) {  // (the means form's colours do not depend on the direction)
       const uint8_t cl = a.geom.clamped[idx];
       const float g0 = (cl & 1) ? 0.f : dcol[0];
       const float g1 = (cl & 2) ? 0.f : dcol[1];
@@ -313,9 +317,9 @@ __device__ __forceinline__ void gaussian_backward(const PreBwdArgs<Scenes>& a, c
       dmean[1] += (gdy - y * dotv) / len;
       dmean[2] += (gdz - z * dotv) / len;
     }
-    if (!pose_only) {
+    if (FORM != kPoseForm)
       for (int j = 0; j < 3; ++j) a.out.dL_dmeans3D[3 * idx + j] = dmean[j];
-
+    if (FORM == kFullForm) {
       // ---- 3D covariance -> scale and rotation ----------------------------------
       if (!a.g.cov3D_precomp) {
         const float s3[3] = {sx, sy, sz};
@@ -358,13 +362,16 @@ __device__ __forceinline__ void gaussian_backward(const PreBwdArgs<Scenes>& a, c
   }
 }
 
-// Zero gradients of a Gaussian that touched no tile (full form).
-template <class Scenes>
+// Zero gradients of a Gaussian that touched no tile (full and means forms).
+template <BwdForm FORM, class Scenes>
 __device__ __forceinline__ void zero_gradients(const PreBwdArgs<Scenes>& a, int64_t idx, int M, float* dsh_dst) {
   for (int k = 0; k < 3; ++k) {
     a.out.dL_dmeans2D[3 * idx + k] = 0.f;
-    if (a.out.dL_dcolors) a.out.dL_dcolors[3 * idx + k] = 0.f;
     a.out.dL_dmeans3D[3 * idx + k] = 0.f;
+  }
+  if (FORM == kMeansForm) return;
+  for (int k = 0; k < 3; ++k) {
+    if (a.out.dL_dcolors) a.out.dL_dcolors[3 * idx + k] = 0.f;
     if (a.out.dL_dscales) a.out.dL_dscales[3 * idx + k] = 0.f;
   }
   a.out.dL_dopacity[idx] = 0.f;
@@ -401,15 +408,20 @@ __device__ __forceinline__ void add_record(float (&v)[16], const Record& r) {
   v[8] += r.r2.x; v[9] += r.r2.y;
 }
 
-// Full form: all eight gradient arrays. Pose-only form (pose_partials set): only
+// Full form: all eight gradient arrays. Means form (means_only): the 2D and 3D means alone,
+// for colours that do not depend on the viewing direction. Pose-only form (pose_partials
+// set): only
 // dL/dmean (through projection, covariance and SH view direction) is formed and the
 // block's SE(3) gradient terms — sum g and sum (R p) x g in float64 with the scene's
 // float64 rotation and the un-posed positions p — go to pose_partials[block].
 // With sh_bulk (degree-3 SH, 16-byte aligned), each warp's 32 x 192 bytes of SH
 // coefficients arrive in shared memory by one bulk copy issued before phase 1, and
 // their gradients leave by one bulk store.
-template <class Scenes, bool POSE>
-__global__ void __launch_bounds__(POSE ? 256 : kBwdThreads, POSE ? 4 : 6) k_preprocess_bwd(PreBwdArgs<Scenes> a) {
+template <class Scenes, BwdForm FORM>
+__global__ void __launch_bounds__(FORM == kPoseForm ? 256 : kBwdThreads, FORM == kPoseForm ? 4 : FORM == kMeansForm ? 8 : 6)
+    k_preprocess_bwd(PreBwdArgs<Scenes> a) {
+  constexpr bool POSE = FORM == kPoseForm;  // a.pose_partials is set exactly for this form
+  constexpr bool kPrefetch = FORM == kFullForm;
   constexpr int kThreads = POSE ? 256 : kBwdThreads, kWarps = kThreads / 32;
   extern __shared__ __align__(128) float4 s_sh[];  // [kThreads][12] with sh_bulk
   __shared__ float s_acc[kThreads][11];
@@ -418,11 +430,10 @@ __global__ void __launch_bounds__(POSE ? 256 : kBwdThreads, POSE ? 4 : 6) k_prep
   if ((int64_t)a.counts->num_rendered > a.cap) return;  // forward overflowed: outputs untouched
   const int64_t blk0 = (int64_t)blockIdx.x * kThreads;
   const SceneDesc& sd = POSE ? a.scenes.for_block(blockIdx.x) : a.scenes.for_gaussian(blk0);
-  constexpr bool pose_only = POSE;  // a.pose_partials is set exactly for this form
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t idx = blk0 + threadIdx.x, warp0 = idx - lane;
   const int M = sd.sh_coeffs;
-  const bool bulk = a.sh_bulk && a.g.shs != nullptr && M == kMaxShCoeffs && warp0 < a.total_slots;
+  const bool bulk = FORM != kMeansForm && a.sh_bulk && a.g.shs != nullptr && M == kMaxShCoeffs && warp0 < a.total_slots;
   const uint32_t sh_bytes =
       (uint32_t)max((int64_t)0, min((int64_t)32, a.total_slots - warp0)) * 3u * kMaxShCoeffs * (uint32_t)sizeof(float);
   const uint32_t bar = smem_addr(&s_bar[warp]);
@@ -462,28 +473,28 @@ __global__ void __launch_bounds__(POSE ? 256 : kBwdThreads, POSE ? 4 : 6) k_prep
       if ((uint32_t)sub < nt && __ldg(a.written + off + sub)) marks |= 1u << (2 * q);
       if ((uint32_t)sub + 8 < nt && __ldg(a.written + off + sub + 8)) marks |= 2u << (2 * q);
     }
-    // Each round's first records are loaded while the round before is reduced (the pose form,
-    // whose fourth block leaves 64 registers, loads them as it needs them).
+    // Each round's first records are loaded while the round before is reduced (the other forms,
+    // in 64 registers, load them as they need them).
     Record n0, n1;
     auto load_round = [&](int q) {
       const uint32_t off = __shfl_sync(0xffffffffu, off_l, 4 * q + grp);
       n0 = load_record(a.records, off + sub, marks & (1u << (2 * q)));
       n1 = load_record(a.records, off + sub + 8, marks & (2u << (2 * q)));
     };
-    if (!POSE) load_round(0);
+    if (kPrefetch) load_round(0);
 #pragma unroll 2
     for (int q = 0; q < 8; ++q) {
       const int src = 4 * q + grp;
       const uint32_t nt = __shfl_sync(0xffffffffu, nt_l, src);
       const uint32_t off = __shfl_sync(0xffffffffu, off_l, src);
-      if (POSE) load_round(q);
+      if (!kPrefetch) load_round(q);
       float v[16];
 #pragma unroll
       for (int k = 0; k < 16; ++k) v[k] = 0.f;
       // slots r = sub, sub + 8, sub + 16, ... in order; unwritten slots are exact zeros
       add_record(v, n0);
       add_record(v, n1);
-      if (!POSE && q < 7) load_round(q + 1);
+      if (kPrefetch && q < 7) load_round(q + 1);
       // The rest 64 slots at a time: eight marks per lane in flight together, then the written
       // records two at a time.
       for (uint32_t first = sub + 16; first < nt; first += 64) {
@@ -518,7 +529,7 @@ __global__ void __launch_bounds__(POSE ? 256 : kBwdThreads, POSE ? 4 : 6) k_prep
     if (!sh_ready) atomicOr(a.flags, CFGS_FLAG_COPY_TIMEOUT);
   }
   const uint32_t nt = nt_l;
-  const bool want_dsh = !pose_only && a.out.dL_dsh != nullptr;
+  const bool want_dsh = FORM == kFullForm && a.out.dL_dsh != nullptr;
   float* own_sh = reinterpret_cast<float*>(s_sh + 12 * threadIdx.x);
   const float* sh_src = nullptr;
   float* dsh_dst = nullptr;
@@ -532,9 +543,9 @@ __global__ void __launch_bounds__(POSE ? 256 : kBwdThreads, POSE ? 4 : 6) k_prep
       float acc[10];
 #pragma unroll
       for (int k = 0; k < 10; ++k) acc[k] = s_acc[threadIdx.x][k];
-      gaussian_backward(a, sd, idx, nt, acc, sh_src, dsh_dst, pose_only, dmean);
-    } else if (!pose_only) {
-      zero_gradients(a, idx, M, dsh_dst);
+      gaussian_backward<FORM>(a, sd, idx, nt, acc, sh_src, dsh_dst, dmean);
+    } else if (!POSE) {
+      zero_gradients<FORM>(a, idx, M, dsh_dst);
     }
   }
   if (bulk && want_dsh) {
@@ -549,7 +560,7 @@ __global__ void __launch_bounds__(POSE ? 256 : kBwdThreads, POSE ? 4 : 6) k_prep
       asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
   }
-  if (!pose_only) return;
+  if (!POSE) return;
   // ---- pose-only form: the block's SE(3) gradient terms in float64 -----------------
   double term[6] = {0, 0, 0, 0, 0, 0};
   if (nt > 0 && sd.pose) {
@@ -586,13 +597,19 @@ void launch_preprocess_bwd(const PreBwdArgs<Scenes>& a, int blocks, cudaStream_t
   static std::atomic<uint64_t> smem_set{0}, smem_set_pose{0};
   // a failure of the attribute call surfaces as a launch error
   if (a.pose_partials) {  // pose-only form: fewer live values, a fourth resident block per SM
-    ensure_dynamic_smem(k_preprocess_bwd<Scenes, true>, 2 * kShBulkBytes, smem_set_pose);
-    k_preprocess_bwd<Scenes, true><<<blocks, 256, a.sh_bulk ? 2 * kShBulkBytes : 0, st>>>(a);
-  } else {
-    ensure_dynamic_smem(k_preprocess_bwd<Scenes, false>, kShBulkBytes, smem_set);
-    k_preprocess_bwd<Scenes, false>
-        <<<blocks * (256 / kBwdThreads), kBwdThreads, a.sh_bulk ? kShBulkBytes : 0, st>>>(a);
+    ensure_dynamic_smem(k_preprocess_bwd<Scenes, kPoseForm>, 2 * kShBulkBytes, smem_set_pose);
+    k_preprocess_bwd<Scenes, kPoseForm><<<blocks, 256, a.sh_bulk ? 2 * kShBulkBytes : 0, st>>>(a);
+    return;
   }
+  blocks *= 256 / kBwdThreads;
+  if constexpr (!Scenes::kBatched) {
+    if (a.means_only) {
+      k_preprocess_bwd<Scenes, kMeansForm><<<blocks, kBwdThreads, 0, st>>>(a);
+      return;
+    }
+  }
+  ensure_dynamic_smem(k_preprocess_bwd<Scenes, kFullForm>, kShBulkBytes, smem_set);
+  k_preprocess_bwd<Scenes, kFullForm><<<blocks, kBwdThreads, a.sh_bulk ? kShBulkBytes : 0, st>>>(a);
 }
 template void launch_preprocess_bwd<SingleScene>(const PreBwdArgs<SingleScene>&, int, cudaStream_t);
 template void launch_preprocess_bwd<SceneTable>(const PreBwdArgs<SceneTable>&, int, cudaStream_t);

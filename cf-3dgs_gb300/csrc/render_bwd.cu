@@ -495,7 +495,8 @@ void launch_render_bwd(const RenderBwdArgs<Scenes>& a, int tiles, cudaStream_t s
     if (a.geom_only) launch_render_bwd_depth<Scenes, false, true>(a, tiles, batch, st);
     else launch_render_bwd_depth<Scenes, false>(a, tiles, batch, st);
   } else {
-    if (a.dL_ddepth) launch_render_bwd_depth<Scenes, true>(a, tiles, batch, st);
+    if (a.geom_only) launch_render_bwd_depth<Scenes, false, true>(a, tiles, batch, st);
+    else if (a.dL_ddepth) launch_render_bwd_depth<Scenes, true>(a, tiles, batch, st);
     else launch_render_bwd_depth<Scenes, false>(a, tiles, batch, st);
   }
 }
@@ -506,9 +507,9 @@ template void launch_render_bwd<SceneTable>(const RenderBwdArgs<SceneTable>&, in
 
 using namespace cfgs;
 
-extern "C" int cfgs_render_backward(const CfgsSettings* s, int32_t num_gaussians, const void* geom, const void* image,
-                                    const void* binning, int64_t capacity, void* scratch, const float* dL_dcolor,
-                                    const float* dL_ddepth, const float* dL_dalpha, void* stream) {
+static int render_backward(const CfgsSettings* s, int32_t num_gaussians, const void* geom, const void* image,
+                           const void* binning, int64_t capacity, void* scratch, const float* dL_dcolor,
+                           const float* dL_ddepth, const float* dL_dalpha, bool means_only, void* stream) {
   if (!s || !geom || !image || !binning || !scratch || !dL_dcolor || !s->bg || num_gaussians < 0)
     return CFGS_ERR_INVALID_ARGUMENT;
   if (s->image_width <= 0 || s->image_height <= 0) return CFGS_ERR_INVALID_ARGUMENT;
@@ -539,25 +540,40 @@ extern "C" int cfgs_render_backward(const CfgsSettings* s, int32_t num_gaussians
   ra.cap = capacity;
   ra.counts = iv.counts;
   if (!resolve_schedule(s->schedule, IL.num_tiles, num_gaussians, capacity, &ra.sched)) return CFGS_ERR_INVALID_ARGUMENT;
-  ra.geom_only = false;
+  ra.geom_only = means_only;
   if (capacity > 0 && cudaMemsetAsync(ra.written, 0, (size_t)capacity, st) != cudaSuccess) return CFGS_ERR_LAUNCH;
   launch_render_bwd(ra, IL.num_tiles, st);
   CFGS_CHECK_LAUNCH(s->debug, st);
   return CFGS_OK;
 }
 
-extern "C" int cfgs_preprocess_backward(const CfgsSettings* s, const CfgsGaussians* g, const int32_t* radii,
-                                        const void* geom, const void* image, int64_t capacity, const void* scratch,
-                                        const CfgsGradients* out, void* stream) {
+extern "C" int cfgs_render_backward(const CfgsSettings* s, int32_t num_gaussians, const void* geom, const void* image,
+                                    const void* binning, int64_t capacity, void* scratch, const float* dL_dcolor,
+                                    const float* dL_ddepth, const float* dL_dalpha, void* stream) {
+  return render_backward(s, num_gaussians, geom, image, binning, capacity, scratch, dL_dcolor, dL_ddepth, dL_dalpha,
+                         false, stream);
+}
+
+extern "C" int cfgs_render_backward_means(const CfgsSettings* s, int32_t num_gaussians, const void* geom,
+                                          const void* image, const void* binning, int64_t capacity, void* scratch,
+                                          const float* dL_dcolor, const float* dL_dalpha, void* stream) {
+  return render_backward(s, num_gaussians, geom, image, binning, capacity, scratch, dL_dcolor, nullptr, dL_dalpha, true,
+                         stream);
+}
+
+static int preprocess_backward(const CfgsSettings* s, const CfgsGaussians* g, const int32_t* radii, const void* geom,
+                               const void* image, int64_t capacity, const void* scratch, const CfgsGradients* out,
+                               bool means_only, void* stream) {
   if (!s || !g || !geom || !image || !scratch || !out || !s->viewmatrix || !s->projmatrix)
     return CFGS_ERR_INVALID_ARGUMENT;
   if (g->num_gaussians == 0) return CFGS_OK;
   if (g->num_gaussians < 0 || !radii || !g->means3D || !g->opacities) return CFGS_ERR_INVALID_ARGUMENT;
-  if (!out->dL_dmeans2D || !out->dL_dopacity || !out->dL_dmeans3D || (!out->dL_dcolors && !g->shs) ||
-      (!out->dL_dcov3D && g->cov3D_precomp))
+  if (!out->dL_dmeans2D || !out->dL_dmeans3D) return CFGS_ERR_INVALID_ARGUMENT;
+  if (!means_only && (!out->dL_dopacity || (!out->dL_dcolors && !g->shs) || (!out->dL_dcov3D && g->cov3D_precomp) ||
+                      (!g->cov3D_precomp && (!out->dL_dscales || !out->dL_drotations))))
     return CFGS_ERR_INVALID_ARGUMENT;
-  if (!g->cov3D_precomp && (!out->dL_dscales || !out->dL_drotations || !g->scales || !g->rotations))
-    return CFGS_ERR_INVALID_ARGUMENT;
+  if (!g->cov3D_precomp && (!g->scales || !g->rotations)) return CFGS_ERR_INVALID_ARGUMENT;
+  if (means_only && g->shs && s->sh_degree != 0) return CFGS_ERR_INVALID_ARGUMENT;
   if ((g->shs == nullptr) == (g->colors_precomp == nullptr)) return CFGS_ERR_INVALID_ARGUMENT;
   if (g->shs && !s->campos) return CFGS_ERR_INVALID_ARGUMENT;
   if (capacity < 0 || capacity > 0x7fffffffll) return CFGS_ERR_INVALID_ARGUMENT;
@@ -579,9 +595,26 @@ extern "C" int cfgs_preprocess_backward(const CfgsSettings* s, const CfgsGaussia
   pa.flags = &iv.counts->flags;
   pa.sh_bulk = g->shs != nullptr && g->sh_coeffs == CFGS_SH_BULK_COEFFS && (((uintptr_t)g->shs) & 15) == 0 &&
                (out->dL_dsh == nullptr || (((uintptr_t)out->dL_dsh) & 15) == 0);
+  pa.means_only = means_only;
   launch_preprocess_bwd(pa, div_up(g->num_gaussians, 256), st);
   CFGS_CHECK_LAUNCH(s->debug, st);
   return CFGS_OK;
+}
+
+extern "C" int cfgs_preprocess_backward(const CfgsSettings* s, const CfgsGaussians* g, const int32_t* radii,
+                                        const void* geom, const void* image, int64_t capacity, const void* scratch,
+                                        const CfgsGradients* out, void* stream) {
+  return preprocess_backward(s, g, radii, geom, image, capacity, scratch, out, false, stream);
+}
+
+extern "C" int cfgs_preprocess_backward_means(const CfgsSettings* s, const CfgsGaussians* g, const int32_t* radii,
+                                              const void* geom, const void* image, int64_t capacity,
+                                              const void* scratch, float* dL_dmeans2D, float* dL_dmeans3D,
+                                              void* stream) {
+  CfgsGradients out{};
+  out.dL_dmeans2D = dL_dmeans2D;
+  out.dL_dmeans3D = dL_dmeans3D;
+  return preprocess_backward(s, g, radii, geom, image, capacity, scratch, &out, true, stream);
 }
 
 extern "C" int cfgs_backward(const CfgsSettings* s, const CfgsGaussians* g, const int32_t* radii, const void* geom,

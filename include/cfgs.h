@@ -245,6 +245,17 @@ int cfgs_preprocess_backward(const CfgsSettings* settings, const CfgsGaussians* 
                              const int32_t* radii, const void* geom, const void* image, int64_t capacity,
                              const void* scratch, const CfgsGradients* grads, void* stream);
 
+/* The two halves for a caller that wants the gradients of the 2D and 3D means alone (a pose
+ * step on fixed Gaussians), without depth gradients: the sums of the other gradients are
+ * left out. The colours must not depend on the viewing direction: colors_precomp, or SH of
+ * degree 0 (CFGS_ERR_INVALID_ARGUMENT otherwise). Both gradients equal the full form's. */
+int cfgs_render_backward_means(const CfgsSettings* settings, int32_t num_gaussians, const void* geom,
+                               const void* image, const void* binning, int64_t capacity, void* scratch,
+                               const float* dL_dcolor, const float* dL_dalpha, void* stream);
+int cfgs_preprocess_backward_means(const CfgsSettings* settings, const CfgsGaussians* gaussians,
+                                   const int32_t* radii, const void* geom, const void* image, int64_t capacity,
+                                   const void* scratch, float* dL_dmeans2D, float* dL_dmeans3D, void* stream);
+
 /* ---- allocation-free backward ----------------------------------------------------
  * No counterpart in the reference: an addition of this library.
  *
