@@ -317,19 +317,18 @@ def mark_visible(positions: torch.Tensor, viewmatrix: torch.Tensor, projmatrix: 
 
 
 def kernel_launches(width: int, height: int) -> dict:
-    """Kernels the forward and backward launch for one image (N > 0): preprocess and
-    the K sum; binning = depth sort (4 radix passes of count/scan/scatter), rank sums and
-    prefix, chunk starts, tile sort (count/scan/scatter per pass of at most 8 tile-index
-    bits; the first count forms the tile keys) and tile ranges; compositing; render
-    backward; preprocess backward. (Lists above 131,072 entries: shorter ones are sorted
-    without the scans. Memory clears the library enqueues with cudaMemsetAsync are not
-    counted.)"""
+    """Kernels the forward and backward launch for one image (N > 0): preprocess;
+    binning = depth sort (4 radix passes of count/scan/scatter), rank sums and prefix,
+    chunk starts, tile sort (count/scan/scatter per pass of at most 8 tile-index bits; the
+    first count forms the tile keys) and tile ranges; compositing; render backward;
+    preprocess backward. (Lists above 131,072 entries: shorter ones are sorted without the
+    scans. Memory clears the library enqueues with cudaMemsetAsync are not counted.)"""
     tiles = ((width + 15) // 16) * ((height + 15) // 16)
     bits = 1
     while bits < 31 and (1 << bits) < tiles:
         bits += 1
     tile_passes = (bits + 7) // 8
-    out = {"preprocess": 2, "bin": 4 * 3 + 3 + 3 * tile_passes + 1, "composite": 1, "render_bwd": 1,
+    out = {"preprocess": 1, "bin": 4 * 3 + 3 + 3 * tile_passes + 1, "composite": 1, "render_bwd": 1,
            "preprocess_bwd": 1}
     out["total"] = sum(out.values())
     return out

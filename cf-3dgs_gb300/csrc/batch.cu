@@ -129,10 +129,7 @@ extern "C" int cfgs_batch_iteration(const CfgsBatchArgs* a, void* stream) {
   if (!resolve_schedule(a->schedule, a->num_tiles, a->gauss_slots, a->capacity, &sched)) return CFGS_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   BatchViews v = views(a);
-  // the counts and the one-launch binning's barrier state (the header's first 256 bytes)
-  if (cudaMemsetAsync(v.iv.counts, 0, 256, st) != cudaSuccess) return CFGS_ERR_LAUNCH;
-  if (cudaMemsetAsync(v.iv.tile_count, 0, sizeof(uint32_t) * (size_t)a->num_tiles, st) != cudaSuccess)
-    return CFGS_ERR_LAUNCH;
+  if (!clear_counts(v.iv, a->num_tiles, st)) return CFGS_ERR_LAUNCH;
 
   CfgsGaussians g{};
   g.num_gaussians = (int32_t)a->gauss_slots;
@@ -150,7 +147,6 @@ extern "C" int cfgs_batch_iteration(const CfgsBatchArgs* a, void* stream) {
   pa.radii = a->radii;
   pa.total_slots = a->gauss_slots;
   launch_preprocess(pa, a->num_blocks, st);
-  launch_scan(v.gv.block_sums, a->num_blocks, v.iv.counts, st);
 
   BinArgs<SceneTable> ba;
   ba.scenes = v.table;

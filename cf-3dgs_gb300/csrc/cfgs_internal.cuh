@@ -67,7 +67,7 @@ struct GeomLayout {
     touched = o;      o = align256(o + sizeof(uint32_t) * (size_t)n);
     offset = o;       o = align256(o + sizeof(uint32_t) * (size_t)n);
     clamped = o;      o = align256(o + (size_t)n);
-    block_sums = o;   o = align256(o + sizeof(uint32_t) * (size_t)(num_blocks + 1));
+    block_sums = o;   o = align256(o + sizeof(uint32_t) * (size_t)(num_blocks + 1));  // unused: keeps the offsets
     depth_key = o;    o = align256(o + sizeof(uint32_t) * 2 * sn);
     depth_val = o;    o = align256(o + sizeof(uint32_t) * 2 * sn);
     rank_sums = o;    o = align256(o + sizeof(uint32_t) * (size_t)(num_blocks + 1));
@@ -85,7 +85,6 @@ struct GeomView {
   uint32_t* touched;   // tiles touched (0 = culled)
   uint32_t* offset;    // first instance index of the Gaussian (instances are numbered in depth order)
   uint8_t* clamped;    // bit c set: SH colour channel c was clamped at 0
-  uint32_t* block_sums;
   uint32_t* depth_key[2];  // depth sort ping-pong keys; depth_key[0] ends as the instance prefix by depth rank
   uint32_t* depth_val[2];  // depth sort ping-pong Gaussian ids; depth_val[1] = Gaussians in depth order
   uint32_t* rank_sums;     // instances per 1024 depth-ordered Gaussians
@@ -103,7 +102,6 @@ struct GeomView {
     touched = reinterpret_cast<uint32_t*>(b + L.touched);
     offset = reinterpret_cast<uint32_t*>(b + L.offset);
     clamped = reinterpret_cast<uint8_t*>(b + L.clamped);
-    block_sums = reinterpret_cast<uint32_t*>(b + L.block_sums);
     depth_key[0] = reinterpret_cast<uint32_t*>(b + L.depth_key);
     depth_key[1] = depth_key[0] + sn;
     depth_val[0] = reinterpret_cast<uint32_t*>(b + L.depth_val);
@@ -327,6 +325,24 @@ struct GridBarrier {
   unsigned int arrived, generation;
 };
 constexpr size_t kGridBarrierOffset = 128;  // bytes into the image workspace
+
+// The instance count while the preprocess blocks add to it, in the same header.
+struct CountSum {
+  unsigned long long total;
+  unsigned int done;  // blocks that have added theirs
+};
+constexpr size_t kCountSumOffset = 64;
+static_assert(sizeof(CfgsCounts) <= kCountSumOffset && kCountSumOffset + sizeof(CountSum) <= kGridBarrierOffset,
+              "the sum lies between the counts and the barrier");
+__host__ __device__ inline CountSum* count_sum(CfgsCounts* counts) {
+  return reinterpret_cast<CountSum*>(reinterpret_cast<char*>(counts) + kCountSumOffset);
+}
+// Clears the header (counts, sum, barrier) and the tile counts, which follow it.
+inline bool clear_counts(const ImageView& v, int64_t num_tiles, cudaStream_t st) {
+  const size_t bytes = (size_t)(reinterpret_cast<char*>(v.tile_count) - reinterpret_cast<char*>(v.counts)) +
+                       sizeof(uint32_t) * (size_t)num_tiles;
+  return cudaMemsetAsync(v.counts, 0, bytes, st) == cudaSuccess;
+}
 static_assert(sizeof(CfgsCounts) <= kGridBarrierOffset && kGridBarrierOffset + sizeof(GridBarrier) <= 256,
               "the barrier follows the counts inside the 256-byte header");
 constexpr uint32_t kGridBarrierMaxPolls = 1u << 22;

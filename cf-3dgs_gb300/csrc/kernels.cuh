@@ -15,6 +15,8 @@ struct PreArgs {
   CfgsCounts* counts;
   int32_t* radii;
   int64_t total_slots;  // Gaussian slots covered by the launch (padded in batches)
+  uint32_t* host = nullptr;  // page-locked slot for the counts, or NULL
+  uint32_t ticket = 0;
 };
 
 // Binning: depth sort, tile keys in depth order, tile sort, tile ranges.
@@ -115,7 +117,6 @@ struct PreBwdArgs {
 
 template <class Scenes>
 void launch_preprocess(const PreArgs<Scenes>& a, int blocks, cudaStream_t st);
-void launch_scan(uint32_t* block_sums, int num_blocks, CfgsCounts* counts, cudaStream_t st);
 template <class Scenes>
 int launch_binning(const BinArgs<Scenes>& a, cudaStream_t st);
 template <class Scenes>

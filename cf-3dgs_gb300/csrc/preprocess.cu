@@ -204,6 +204,22 @@ __device__ __forceinline__ uint32_t block_reduce_sum_u32(uint32_t v, uint32_t* s
   return t;  // valid in thread 0
 }
 
+// Writes the instance count K and the flags (all raised by now); with `host` (page-locked
+// host memory) also there, followed by the ticket the host waits for.
+__device__ __forceinline__ void publish_counts(CfgsCounts* counts, unsigned long long K, volatile uint32_t* host,
+                                               uint32_t ticket) {
+  const uint32_t rendered = K > 0xffffffffull ? 0xffffffffu : (uint32_t)K;
+  const uint32_t flags = *(volatile uint32_t*)&counts->flags | (K > 0x7fffffffull ? CFGS_FLAG_CAPACITY_OVERFLOW : 0u);
+  counts->num_rendered = rendered;
+  counts->flags = flags;
+  if (host) {
+    host[0] = rendered;
+    host[1] = flags;
+    __threadfence_system();
+    host[2] = ticket;
+  }
+}
+
 template <class Scenes>
 __global__ void __launch_bounds__(kPreprocessBlock) k_preprocess(PreArgs<Scenes> a) {
   __shared__ uint32_t sh_warp[kPreprocessBlock / 32];
@@ -293,8 +309,18 @@ __global__ void __launch_bounds__(kPreprocessBlock) k_preprocess(PreArgs<Scenes>
     a.geom.touched[idx] = touched;
     if (!valid) a.radii[idx] = 0;
   }
-  uint32_t bs = block_reduce_sum_u32(touched, sh_warp);
-  if (threadIdx.x == 0) a.geom.block_sums[blockIdx.x] = bs;
+  const uint32_t bs = block_reduce_sum_u32(touched, sh_warp);
+  if (threadIdx.x == 0) {
+    // The last block to finish publishes the sum, which the host waits for to size the
+    // instance list (16,384 Gaussians: 7.0 us and a launch of 5.6 for the sum -> 11.3 us).
+    CountSum* cs = count_sum(a.counts);
+    atomicAdd(&cs->total, (unsigned long long)bs);
+    __threadfence();
+    if (atomicAdd(&cs->done, 1u) == gridDim.x - 1) {
+      __threadfence();
+      publish_counts(a.counts, *(volatile unsigned long long*)&cs->total, a.host, a.ticket);
+    }
+  }
 }
 
 template <class Scenes>
@@ -304,31 +330,9 @@ void launch_preprocess(const PreArgs<Scenes>& a, int blocks, cudaStream_t st) {
 template void launch_preprocess<SingleScene>(const PreArgs<SingleScene>&, int, cudaStream_t);
 template void launch_preprocess<SceneTable>(const PreArgs<SceneTable>&, int, cudaStream_t);
 
-// Instance count K = sum of the per-block touched sums (one block of 1024 threads). With
-// `host` (page-locked host memory) the counts also go there, followed by the ticket the
-// host waits for.
-__global__ void __launch_bounds__(1024) k_scan(const uint32_t* block_sums, int num_blocks, CfgsCounts* counts,
-                                               volatile uint32_t* host, uint32_t ticket) {
-  __shared__ unsigned long long sh[32];
-  unsigned long long v = 0;
-  for (int i = threadIdx.x; i < num_blocks; i += blockDim.x) v += block_sums[i];
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned long long K = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) K += sh[w];
-    const uint32_t rendered = K > 0xffffffffull ? 0xffffffffu : (uint32_t)K;
-    counts->num_rendered = rendered;
-    const uint32_t flags = counts->flags | (K > 0x7fffffffull ? CFGS_FLAG_CAPACITY_OVERFLOW : 0u);
-    counts->flags = flags;  // the preprocess, which raises the other flag, is over
-    if (host) {
-      host[0] = rendered;
-      host[1] = flags;
-      __threadfence_system();
-      host[2] = ticket;
-    }
-  }
+// The counts of a forward without Gaussians.
+__global__ void k_publish_empty(CfgsCounts* counts, volatile uint32_t* host, uint32_t ticket) {
+  publish_counts(counts, 0, host, ticket);
 }
 
 __global__ void __launch_bounds__(256) k_mark_visible(int n, const float* means, const float* V,
@@ -341,10 +345,6 @@ __global__ void __launch_bounds__(256) k_mark_visible(int n, const float* means,
   float3 p = make_float3(means[3 * i], means[3 * i + 1], means[3 * i + 2]);
   float3 t = xform43(m, p);
   vis[i] = t.z <= CFGS_NEAR_Z ? 0 : 1;
-}
-
-void launch_scan(uint32_t* block_sums, int num_blocks, CfgsCounts* counts, cudaStream_t st) {
-  k_scan<<<1, 1024, 0, st>>>(block_sums, num_blocks, counts, nullptr, 0u);
 }
 
 }  // namespace cfgs
@@ -396,9 +396,7 @@ static int preprocess_forward(const CfgsSettings* s, const CfgsGaussians* g, voi
   ImageView iv(image, s->image_width, s->image_height);
   GeomView gv(geom, g->num_gaussians);
   GeomLayout GL(g->num_gaussians);
-  if (cudaMemsetAsync(iv.counts, 0, sizeof(CfgsCounts), st) != cudaSuccess) return CFGS_ERR_LAUNCH;
-  if (cudaMemsetAsync(iv.tile_count, 0, sizeof(uint32_t) * IL.num_tiles, st) != cudaSuccess)
-    return CFGS_ERR_LAUNCH;
+  if (!clear_counts(iv, IL.num_tiles, st)) return CFGS_ERR_LAUNCH;
   if (g->num_gaussians > 0) {
     PreArgs<SingleScene> a;
     a.scenes.d = single_scene_desc(s, g->num_gaussians, g->sh_coeffs);
@@ -407,10 +405,12 @@ static int preprocess_forward(const CfgsSettings* s, const CfgsGaussians* g, voi
     a.counts = iv.counts;
     a.radii = radii;
     a.total_slots = g->num_gaussians;
+    a.host = host_slot;
+    a.ticket = ticket;
     k_preprocess<SingleScene><<<GL.num_blocks, kPreprocessBlock, 0, st>>>(a);
-    CFGS_CHECK_LAUNCH(s->debug, st);
+  } else {
+    k_publish_empty<<<1, 1, 0, st>>>(iv.counts, host_slot, ticket);
   }
-  k_scan<<<1, 1024, 0, st>>>(gv.block_sums, GL.num_blocks, iv.counts, host_slot, ticket);
   CFGS_CHECK_LAUNCH(s->debug, st);
   return CFGS_OK;
 }
