@@ -380,14 +380,20 @@ __device__ __forceinline__ void best3_insert(float (&b)[3], float d) {
 
 // Bound by the distance checks' issue. One thread per query with its own divergent
 // traversal waited on one dependent load after another (161,225 points of a 640x360 frame:
-// 1671 us); the shared traversal reads each box once per warp: 135 us (issue 76% busy).
-constexpr int kKnnWarps = 8;
+// 1671 us); the shared traversal reads each box once per warp: 135 us. Most warps were then
+// done after 60; a few whose 32 points span a jump of the curve test hundreds of boxes (892
+// of 5,039) one after another. So box tests go four at a time from shared memory, the next
+// super-box is loaded ahead, and a box's distances are formed eight at a time before any is
+// compared: 105 us. (Tests of parts of the wide box instead: 137; the scan unrolled into each
+// of the four tests: 152, instruction fetch.)
+constexpr int kKnnWarps = 8, kKnnBatch = 8, kKnnTests = 4;
 
 __global__ void __launch_bounds__(32 * kKnnWarps) k_knn3(int64_t n, const float4* __restrict__ pts,
                                                          const float4* __restrict__ box,
                                                          const float4* __restrict__ sup, float* __restrict__ out) {
   static_assert(kKnnBox == 32 && kKnnSuper == 32, "a lane per query, box and super-box");
   __shared__ float4 s_pts[kKnnWarps][kKnnBox];
+  __shared__ float4 s_box[kKnnWarps][kKnnSuper][2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t nbox = (n + kKnnBox - 1) / kKnnBox;
   const int64_t nsup = (nbox + kKnnSuper - 1) / kKnnSuper;
@@ -406,54 +412,88 @@ __global__ void __launch_bounds__(32 * kKnnWarps) k_knn3(int64_t n, const float4
     s_pts[warp][lane] = k < n ? pts[k] : make_float4(INFINITY, 0.f, 0.f, 0.f);
     __syncwarp();
   };
-  stage(own);
-  for (int j = 0; j < kKnnBox; ++j) {
-    const float4 p = s_pts[warp][j];
-    if (j != lane) best3_insert(b, dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z));
-  }
-  auto worst = [&]() {  // the warp's largest third-best, with the margin
-    return __uint_as_float(__reduce_max_sync(0xffffffffu, active ? __float_as_uint(b[2]) : 0u)) * kKnnMargin;
-  };
-  auto visit = [&](int64_t sb, float bound) {  // the boxes of super-box sb
-    const int64_t bx = sb * kKnnSuper + lane;
-    float4 lo = own_lo, hi = own_hi;
-    bool may = bx < nbox && bx != own;
-    if (may) {
-      lo = box[2 * bx];
-      hi = box[2 * bx + 1];
-      may = !(box_dist2(own_lo, own_hi, lo, hi) > bound);
-    }
-    unsigned todo = __ballot_sync(0xffffffffu, may);
-    while (todo) {
-      const int l = __ffs(todo) - 1;
-      todo &= todo - 1;
-      float4 clo, chi;
-      clo.x = __shfl_sync(0xffffffffu, lo.x, l);
-      clo.y = __shfl_sync(0xffffffffu, lo.y, l);
-      clo.z = __shfl_sync(0xffffffffu, lo.z, l);
-      chi.x = __shfl_sync(0xffffffffu, hi.x, l);
-      chi.y = __shfl_sync(0xffffffffu, hi.y, l);
-      chi.z = __shfl_sync(0xffffffffu, hi.z, l);
-      if (!__any_sync(0xffffffffu, !(box_dist2(q, q, clo, chi) > b[2] * kKnnMargin))) continue;
-      stage(sb * kKnnSuper + l);
-#pragma unroll 8
-      for (int j = 0; j < kKnnBox; ++j) {
-        const float4 p = s_pts[warp][j];
-        best3_insert(b, dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z));
+  // the staged points, but the one at `skip`, kKnnBatch distances at a time: most batches of
+  // another box improve no lane's three
+  auto scan = [&](int skip) {
+#pragma unroll
+    for (int j = 0; j < kKnnBox; j += kKnnBatch) {
+      float d[kKnnBatch];
+#pragma unroll
+      for (int k = 0; k < kKnnBatch; ++k) {
+        const float4 p = s_pts[warp][j + k];
+        d[k] = dist2_ref(q.x, q.y, q.z, p.x, p.y, p.z);
+        if (j + k == skip) d[k] = INFINITY;
+      }
+      float least = d[0];
+#pragma unroll
+      for (int k = 1; k < kKnnBatch; ++k) least = fminf(least, d[k]);
+      if (least < b[2]) {
+#pragma unroll
+        for (int k = 0; k < kKnnBatch; ++k) best3_insert(b, d[k]);
       }
     }
   };
-  const int64_t own_sup = own / kKnnSuper;
-  visit(own_sup, worst());
-  float bound = worst();
-  for (int64_t s0 = 0; s0 < nsup; s0 += 32) {
-    const int64_t sb = s0 + lane;
-    const bool may = sb < nsup && sb != own_sup && !(box_dist2(own_lo, own_hi, sup[2 * sb], sup[2 * sb + 1]) > bound);
+  stage(own);
+  scan(lane);
+  auto worst = [&]() {  // the warp's largest third-best, with the margin
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, active ? __float_as_uint(b[2]) : 0u)) * kKnnMargin;
+  };
+  auto load_box = [&](int64_t sb, float4& lo, float4& hi) {  // this lane's box of super-box sb
+    const int64_t bx = sb * kKnnSuper + lane;
+    if (bx < nbox) {
+      lo = box[2 * bx];
+      hi = box[2 * bx + 1];
+    }
+  };
+  auto visit = [&](int64_t sb, const float4& lo, const float4& hi, float bound) {  // the boxes of super-box sb
+    const int64_t bx = sb * kKnnSuper + lane;
+    const bool may = bx < nbox && bx != own && !(box_dist2(own_lo, own_hi, lo, hi) > bound);
     unsigned todo = __ballot_sync(0xffffffffu, may);
+    if (!todo) return;
+    __syncwarp();
+    s_box[warp][lane][0] = lo;
+    s_box[warp][lane][1] = hi;
+    __syncwarp();
+    while (todo) {
+      unsigned need = 0;
+#pragma unroll
+      for (int k = 0; k < kKnnTests; ++k) {
+        const unsigned bit = todo & (0u - todo);
+        const int l = max(__ffs(todo) - 1, 0);
+        todo ^= bit;
+        if (__any_sync(0xffffffffu, !(box_dist2(q, q, s_box[warp][l][0], s_box[warp][l][1]) > b[2] * kKnnMargin)))
+          need |= bit;
+      }
+      while (need) {
+        const int l = __ffs(need) - 1;
+        need &= need - 1;
+        stage(sb * kKnnSuper + l);
+        scan(-1);
+      }
+    }
+  };
+  // its own super-box first, then those within the bound. The next one's boxes are on their
+  // way while one is visited.
+  const int64_t own_sup = own / kKnnSuper;
+  float bound = worst();
+  for (int64_t s0 = -32; s0 < nsup; s0 += 32) {
+    int64_t base = own_sup;
+    unsigned todo = 1u;
+    if (s0 >= 0) {
+      base = s0;
+      const int64_t sb = s0 + lane;
+      todo = __ballot_sync(0xffffffffu, sb < nsup && sb != own_sup &&
+                                            !(box_dist2(own_lo, own_hi, sup[2 * sb], sup[2 * sb + 1]) > bound));
+    }
+    float4 lo, hi, next_lo = own_lo, next_hi = own_hi;
+    if (todo) load_box(base + __ffs(todo) - 1, next_lo, next_hi);
     while (todo) {
       const int l = __ffs(todo) - 1;
       todo &= todo - 1;
-      visit(s0 + l, bound);
+      lo = next_lo;
+      hi = next_hi;
+      if (todo) load_box(base + __ffs(todo) - 1, next_lo, next_hi);
+      visit(base + l, lo, hi, bound);
       bound = worst();
     }
   }
