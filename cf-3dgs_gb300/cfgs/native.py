@@ -132,6 +132,8 @@ EXPORTS = {
                                        _vp]),
     "cfgs_preprocess_backward": (C.c_int, [C.POINTER(Settings), C.POINTER(Gaussians), _vp, _vp, _vp, C.c_int64, _vp,
                                            C.POINTER(Gradients), _vp]),
+    "cfgs_preprocess_backward_inputs": (C.c_int, [C.POINTER(Settings), C.POINTER(Gaussians), _vp, _vp, _vp, C.c_int64,
+                                                  _vp, C.POINTER(Gradients), _vp]),
     "cfgs_render_backward_means": (C.c_int, [C.POINTER(Settings), C.c_int32, _vp, _vp, _vp, C.c_int64, _vp, _vp, _vp,
                                              _vp]),
     "cfgs_preprocess_backward_means": (C.c_int, [C.POINTER(Settings), C.POINTER(Gaussians), _vp, _vp, _vp, C.c_int64,

@@ -231,9 +231,9 @@ def backward(rs, state: ForwardState, means3D, opacities, shs, colors_precomp, s
                                                   grad_color.data_ptr(), _ptr(grad_depth), _ptr(grad_alpha), st),
                          "cfgs_render_backward")
         with _Timed(timers, "preprocess_bwd"):
-            native.check(lib.cfgs_preprocess_backward(C.byref(s), C.byref(g), state.radii.data_ptr(),
-                                                      state.geom.data_ptr(), state.image.data_ptr(), K,
-                                                      scratch.data_ptr(), C.byref(gr), st),
+            per_gaussian = lib.cfgs_preprocess_backward_inputs if state.inputs_only else lib.cfgs_preprocess_backward
+            native.check(per_gaussian(C.byref(s), C.byref(g), state.radii.data_ptr(), state.geom.data_ptr(),
+                                      state.image.data_ptr(), K, scratch.data_ptr(), C.byref(gr), st),
                          "cfgs_preprocess_backward")
     return d_m2, d_col, d_op, d_m3, d_cov, d_sh, d_sc, d_rot
 

@@ -561,16 +561,22 @@ extern "C" int cfgs_render_backward_means(const CfgsSettings* s, int32_t num_gau
                          stream);
 }
 
+// Which gradient arrays a caller wants: all eight, those of its inputs, the means'.
+enum Wanted { kAllArrays, kInputArrays, kMeansArrays };
+
 static int preprocess_backward(const CfgsSettings* s, const CfgsGaussians* g, const int32_t* radii, const void* geom,
                                const void* image, int64_t capacity, const void* scratch, const CfgsGradients* out,
-                               bool means_only, void* stream) {
+                               Wanted wanted, void* stream) {
+  const bool means_only = wanted == kMeansArrays;
   if (!s || !g || !geom || !image || !scratch || !out || !s->viewmatrix || !s->projmatrix)
     return CFGS_ERR_INVALID_ARGUMENT;
   if (g->num_gaussians == 0) return CFGS_OK;
   if (g->num_gaussians < 0 || !radii || !g->means3D || !g->opacities) return CFGS_ERR_INVALID_ARGUMENT;
   if (!out->dL_dmeans2D || !out->dL_dmeans3D) return CFGS_ERR_INVALID_ARGUMENT;
-  if (!means_only && (!out->dL_dopacity || (!out->dL_dcolors && !g->shs) || (!out->dL_dcov3D && g->cov3D_precomp) ||
-                      (!g->cov3D_precomp && (!out->dL_dscales || !out->dL_drotations))))
+  if (!means_only && (!out->dL_dopacity || (!g->cov3D_precomp && (!out->dL_dscales || !out->dL_drotations))))
+    return CFGS_ERR_INVALID_ARGUMENT;
+  if (!means_only && ((!out->dL_dcolors && (wanted == kAllArrays || !g->shs)) ||
+                      (!out->dL_dcov3D && (wanted == kAllArrays || g->cov3D_precomp))))
     return CFGS_ERR_INVALID_ARGUMENT;
   if (!g->cov3D_precomp && (!g->scales || !g->rotations)) return CFGS_ERR_INVALID_ARGUMENT;
   if (means_only && g->shs && s->sh_degree != 0) return CFGS_ERR_INVALID_ARGUMENT;
@@ -604,7 +610,13 @@ static int preprocess_backward(const CfgsSettings* s, const CfgsGaussians* g, co
 extern "C" int cfgs_preprocess_backward(const CfgsSettings* s, const CfgsGaussians* g, const int32_t* radii,
                                         const void* geom, const void* image, int64_t capacity, const void* scratch,
                                         const CfgsGradients* out, void* stream) {
-  return preprocess_backward(s, g, radii, geom, image, capacity, scratch, out, false, stream);
+  return preprocess_backward(s, g, radii, geom, image, capacity, scratch, out, kAllArrays, stream);
+}
+
+extern "C" int cfgs_preprocess_backward_inputs(const CfgsSettings* s, const CfgsGaussians* g, const int32_t* radii,
+                                               const void* geom, const void* image, int64_t capacity,
+                                               const void* scratch, const CfgsGradients* out, void* stream) {
+  return preprocess_backward(s, g, radii, geom, image, capacity, scratch, out, kInputArrays, stream);
 }
 
 extern "C" int cfgs_preprocess_backward_means(const CfgsSettings* s, const CfgsGaussians* g, const int32_t* radii,
@@ -614,7 +626,7 @@ extern "C" int cfgs_preprocess_backward_means(const CfgsSettings* s, const CfgsG
   CfgsGradients out{};
   out.dL_dmeans2D = dL_dmeans2D;
   out.dL_dmeans3D = dL_dmeans3D;
-  return preprocess_backward(s, g, radii, geom, image, capacity, scratch, &out, true, stream);
+  return preprocess_backward(s, g, radii, geom, image, capacity, scratch, &out, kMeansArrays, stream);
 }
 
 extern "C" int cfgs_backward(const CfgsSettings* s, const CfgsGaussians* g, const int32_t* radii, const void* geom,

@@ -117,9 +117,7 @@ typedef struct CfgsGaussians {
 } CfgsGaussians;
 
 /* Gradient outputs of the backward pass (the 8 tensors upstream returns, in its
- * order). Every non-null array is fully overwritten (zeros for culled Gaussians).
- * dL_dcolors may be NULL with SH colours and dL_dcov3D with scales and rotations (neither
- * is then an input's gradient). */
+ * order). Every non-null array is fully overwritten (zeros for culled Gaussians). */
 typedef struct CfgsGradients {
   float* dL_dmeans2D;   /* [N,3] d/d(NDC x, NDC y), third column 0             */
   float* dL_dcolors;    /* [N,3] d/d(per-Gaussian RGB)                        */
@@ -244,6 +242,12 @@ int cfgs_render_backward(const CfgsSettings* settings, int32_t num_gaussians, co
 int cfgs_preprocess_backward(const CfgsSettings* settings, const CfgsGaussians* gaussians,
                              const int32_t* radii, const void* geom, const void* image, int64_t capacity,
                              const void* scratch, const CfgsGradients* grads, void* stream);
+
+/* The second half for a caller that wants the gradients of its inputs alone: dL_dcolors may
+ * be NULL with SH colours, and dL_dcov3D with scales and rotations. */
+int cfgs_preprocess_backward_inputs(const CfgsSettings* settings, const CfgsGaussians* gaussians,
+                                    const int32_t* radii, const void* geom, const void* image, int64_t capacity,
+                                    const void* scratch, const CfgsGradients* grads, void* stream);
 
 /* The two halves for a caller that wants the gradients of the 2D and 3D means alone (a pose
  * step on fixed Gaussians), without depth gradients: the sums of the other gradients are
