@@ -174,7 +174,7 @@ def render_bwd_design_bytes(K: int, kept: int) -> int:
 # fmul,ffma2,fadd2,fmul2}_pred_on.sum: FFMA 2, FADD/FMUL 1, FFMA2 4, FADD2/FMUL2 2 flops)
 # on the render kernels of a 250,000-Gaussian scene with the benchmark's distributions at
 # 1920x1080 (E = 634M): forward 5.24e9 and backward 8.46e9 flops per launch.
-FLOPS_PER_EVAL = {"composite": 5.24e9 / 633965142, "render_bwd": 8.46e9 / 633965142}
+FLOPS_PER_EVAL = {"composite": 5.56e9 / 633965142, "render_bwd": 9.80e9 / 633965142}
 
 
 def alu_roofline(E: int, phase_ms: dict, pb: dict, peaks: dict) -> dict:
