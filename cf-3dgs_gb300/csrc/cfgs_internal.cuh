@@ -332,10 +332,11 @@ struct CountSum {
   unsigned int done;  // blocks that have added theirs
 };
 constexpr size_t kCountSumOffset = 64;
-static_assert(sizeof(CfgsCounts) <= kCountSumOffset && kCountSumOffset + sizeof(CountSum) <= kGridBarrierOffset,
+static_assert(sizeof(CfgsCounts) <= kCountSumOffset && kCountSumOffset + 8 + sizeof(CountSum) <= kGridBarrierOffset,
               "the sum lies between the counts and the barrier");
+// On an 8-byte boundary also where the workspace, whose other words are of 4 bytes, is not.
 __host__ __device__ inline CountSum* count_sum(CfgsCounts* counts) {
-  return reinterpret_cast<CountSum*>(reinterpret_cast<char*>(counts) + kCountSumOffset);
+  return reinterpret_cast<CountSum*>((reinterpret_cast<uintptr_t>(counts) + kCountSumOffset + 7) & ~(uintptr_t)7);
 }
 // Clears the header (counts, sum, barrier) and the tile counts, which follow it.
 inline bool clear_counts(const ImageView& v, int64_t num_tiles, cudaStream_t st) {

@@ -90,3 +90,27 @@ def test_pageable_slot_is_refused():
     assert lib.cfgs_wait_counts(slot.data_ptr(), ticket, C.byref(c), st) == 0
     # a ticket nobody will write: the wait ends with the stream, as a launch error
     assert lib.cfgs_wait_counts(slot.data_ptr(), ticket.value + 7, C.byref(c), st) == 3
+
+
+@pytest.mark.parametrize("shift", [0, 4, 8, 12])
+def test_counts_in_a_workspace_on_a_4_byte_boundary(shift):
+    """The preprocess's 64-bit sum finds an aligned place in the image workspace's header."""
+    import ctypes as C
+    import diff_gaussian_rasterization as dgr
+    from cfgs import native, raster, scenes
+    from helpers import settings_for
+    sc = scenes.scene_small(n=700, width=64, height=48, seed=3)
+    s = sc.to("cuda")
+    lib, keep = native.load(), []
+    cs = raster.make_settings(settings_for(dgr, sc), keep)
+    g = raster.make_gaussians(s.means3D, s.opacities, s.shs, None, s.scales, s.rotations, None)
+    geom = torch.empty(lib.cfgs_geom_bytes(700), dtype=torch.uint8, device="cuda")
+    room = torch.empty(lib.cfgs_image_bytes(64, 48) + 16, dtype=torch.uint8, device="cuda")
+    image, radii = room[shift:], torch.empty(700, dtype=torch.int32, device="cuda")
+    stream = raster.stream_handle(s.means3D.device)
+    native.check(lib.cfgs_preprocess_forward(C.byref(cs), C.byref(g), geom.data_ptr(), image.data_ptr(),
+                                             radii.data_ptr(), stream), "cfgs_preprocess_forward")
+    counts = native.Counts()
+    native.check(lib.cfgs_read_counts(image.data_ptr(), C.byref(counts), stream), "cfgs_read_counts")
+    want = raster.forward(settings_for(dgr, sc), s.means3D, s.opacities, s.shs, None, s.scales, s.rotations, None)[4]
+    assert counts.num_rendered == want.num_rendered > 0 and counts.flags == 0
