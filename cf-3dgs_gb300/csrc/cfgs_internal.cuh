@@ -338,14 +338,21 @@ static_assert(sizeof(CfgsCounts) <= kCountSumOffset && kCountSumOffset + 8 + siz
 __host__ __device__ inline CountSum* count_sum(CfgsCounts* counts) {
   return reinterpret_cast<CountSum*>((reinterpret_cast<uintptr_t>(counts) + kCountSumOffset + 7) & ~(uintptr_t)7);
 }
-// Clears the header (counts, sum, barrier) and the tile counts, which follow it.
+// Set, in the same header but not among the flags a caller reads, when a visible Gaussian's
+// colour or depth is not finite: the render kernels then take the form that selects where
+// the usual one adds a zero weight's product.
+constexpr size_t kNonfiniteOffset = 192;
+__host__ __device__ inline uint32_t* nonfinite_word(const CfgsCounts* counts) {
+  return reinterpret_cast<uint32_t*>(reinterpret_cast<uintptr_t>(counts) + kNonfiniteOffset);
+}
+// Clears the header (counts, sum, barrier, word) and the tile counts, which follow it.
 inline bool clear_counts(const ImageView& v, int64_t num_tiles, cudaStream_t st) {
   const size_t bytes = (size_t)(reinterpret_cast<char*>(v.tile_count) - reinterpret_cast<char*>(v.counts)) +
                        sizeof(uint32_t) * (size_t)num_tiles;
   return cudaMemsetAsync(v.counts, 0, bytes, st) == cudaSuccess;
 }
-static_assert(sizeof(CfgsCounts) <= kGridBarrierOffset && kGridBarrierOffset + sizeof(GridBarrier) <= 256,
-              "the barrier follows the counts inside the 256-byte header");
+static_assert(kGridBarrierOffset + sizeof(GridBarrier) <= kNonfiniteOffset && kNonfiniteOffset + 4 <= 256,
+              "the barrier and the word follow the counts inside the 256-byte header");
 constexpr uint32_t kGridBarrierMaxPolls = 1u << 22;
 
 __device__ __forceinline__ bool grid_barrier(GridBarrier* b, uint32_t* flags) {

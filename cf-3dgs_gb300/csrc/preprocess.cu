@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(kPreprocessBlock, Scenes::kBatched ? 6 : 5) k_
                             sd.sh_coeffs == kMaxShCoeffs && (((uintptr_t)shp) & 15) == 0);
           }
           if (!(isfinite(rgb.x) && isfinite(rgb.y) && isfinite(rgb.z) && isfinite(t.z)))
-            atomicOr(&a.counts->flags, CFGS_FLAG_NONFINITE_COLOUR);
+            *nonfinite_word(a.counts) = 1u;
           a.geom.xy[idx] = pimg;
           a.geom.conic_op[idx] = make_float4(conic.x, conic.y, conic.z, opacity);
           a.geom.rgbd[idx] = make_float4(rgb.x, rgb.y, rgb.z, t.z);

@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS == 4 ? 9 : 6) k_render_fwd(R
   static_assert(BATCH % 32 == 0 && (WARPS == 4 || WARPS == 8), "whole ballot words; 8x8 or 8x4 warp boxes");
   __shared__ FwdShared<BATCH> sh;
   if ((int64_t)a.counts->num_rendered > a.cap) return;
-  if (WARPS == 4 && (a.counts->flags & CFGS_FLAG_NONFINITE_COLOUR)) composite_tile<Scenes, BATCH, WARPS, true>(a, sh);
+  if (WARPS == 4 && *nonfinite_word(a.counts)) composite_tile<Scenes, BATCH, WARPS, true>(a, sh);
   else composite_tile<Scenes, BATCH, WARPS, false>(a, sh);
 }
 

@@ -50,8 +50,6 @@ typedef enum CfgsStatus {
                                          /* that call's outputs are invalid               */
 #define CFGS_FLAG_BARRIER_TIMEOUT 0x8u   /* a bounded grid-wide wait of the one-launch    */
                                          /* binning ran out; outputs are invalid          */
-#define CFGS_FLAG_NONFINITE_COLOUR 0x10u /* a visible Gaussian's colour or depth is not   */
-                                         /* finite (information, not an error)            */
 
 /* Tile size of the screen-space binning (pixels). */
 #define CFGS_TILE_X 16
