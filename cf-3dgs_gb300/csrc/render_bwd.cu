@@ -9,6 +9,7 @@
 // preprocess backward sums its records in a fixed order: no atomics, bit-identical
 // results run to run.
 #include <mutex>
+#include <type_traits>
 
 #include "cfgs_internal.cuh"
 #include "kernels.cuh"
@@ -61,6 +62,10 @@ __device__ __forceinline__ void load_pixel(PixelBwd& p, const RenderBwdArgs<Scen
   p.dA_bg = dA - (__ldg(sd.bg + 0) * p.dC0 + __ldg(sd.bg + 1) * p.dC1 + __ldg(sd.bg + 2) * p.dC2);
 }
 
+__device__ __forceinline__ bool all_finite(const PixelBwd& p) {
+  return isfinite(p.dC0) && isfinite(p.dC1) && isfinite(p.dC2) && isfinite(p.dD) && isfinite(p.dA_bg);
+}
+
 // Back-to-front state of a lane's two pixels (.x: column c, .y: column c + 4): upstream
 // gradients, the transmittance being unwound, and the colour/depth accumulated behind the
 // current instance (updated right after each contributing instance, which gives the
@@ -101,8 +106,10 @@ __device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z,
 // Unwinds one instance at list position c for both pixels: g = G dL/dalpha (G the
 // Gaussian's value at the pixel) and w = alpha T, zero where the instance did not
 // contribute. A pixel the instance did not reach in the forward pass keeps its state: its
-// alpha and G count as 0. Returns whether the instance contributed to either pixel.
-template <bool DEPTH>
+// alpha and G count as 0. Returns whether the instance contributed to either pixel. ODD (a
+// tile whose image gradients, or a view whose colours or depths, are not all finite) selects
+// where a zero would multiply such a value.
+template <bool DEPTH, bool ODD>
 __device__ __forceinline__ bool unwind_pair(PairBwd& P, int c, float2 px, float2 py, const StagedInstance& s, float thr,
                                             float2& g, float2& w) {
   const bool in0 = c < (int)P.last0, in1 = c < (int)P.last1;
@@ -130,17 +137,23 @@ __device__ __forceinline__ bool unwind_pair(PairBwd& P, int c, float2 px, float2
   float2 dLda = mul2(e0, P.dC0);
   dLda = fma2(e1, P.dC1, dLda);
   dLda = fma2(e2, P.dC2, dLda);
-  P.acc0 = fma2(am, e0, P.acc0);
-  P.acc1 = fma2(am, e1, P.acc1);
-  P.acc2 = fma2(am, e2, P.acc2);
+  auto behind = [&](float2& acc, const float2& e) {
+    const float2 sum = fma2(am, e, acc);
+    acc = ODD ? make_float2(a0 ? sum.x : acc.x, a1 ? sum.y : acc.y) : sum;
+  };
+  behind(P.acc0, e0);
+  behind(P.acc1, e1);
+  behind(P.acc2, e2);
   if (DEPTH) {
     const float2 ed = sub2(hi2(s.bd), P.accd);
     dLda = fma2(ed, P.dD, dLda);
-    P.accd = fma2(am, ed, P.accd);
+    behind(P.accd, ed);
   }
   dLda = mul2(dLda, P.T);
   dLda = fma2(mul2(P.T_final, inv), P.dA_bg, dLda);
-  g = mul2(make_float2(a0 ? G.x : 0.0f, a1 ? G.y : 0.0f), dLda);  // d/d opacity
+  // d/d opacity
+  if (ODD) g = make_float2(a0 ? __fmul_rn(G.x, dLda.x) : 0.0f, a1 ? __fmul_rn(G.y, dLda.y) : 0.0f);
+  else g = mul2(make_float2(a0 ? G.x : 0.0f, a1 ? G.y : 0.0f), dLda);
   return true;
 }
 
@@ -194,14 +207,17 @@ __device__ __forceinline__ int pair_offset(int q, int y) {
 // instance over all 32 lanes by shuffles took about 70. The order of every sum is the one
 // of that reduction — rows y and y + 4, then y and y + 2, y and y + 1, then columns 4, 2
 // and 1 apart — so the records keep its bits. Odd slots take the odd rows first (an
-// exchange of the operands of one addition), so that loads meet no common bank.
-template <bool DEPTH, int BATCH, bool GEOM>
+// exchange of the operands of one addition), so that loads meet no common bank. ODD: as in
+// unwind_pair.
+template <bool ODD, bool DEPTH, int BATCH, bool GEOM>
 __device__ __forceinline__ void sum_slots(BwdShared<DEPTH, BATCH, GEOM>& sh, int warp, int lane, int n, int j, int bx0,
                                           int by0) {
   using Sh = BwdShared<DEPTH, BATCH, GEOM>;
   constexpr int kTerms = Sh::kTerms, kPlanes = Sh::kPlanes;
   const int slot = lane >> 2, q = lane & 3, odd_first = slot & 1;
   __syncwarp();
+  // an image gradient where the instance has a weight, else 0
+  auto where = [](float2 d, float2 w) { return ODD ? make_float2(w.x != 0.f ? d.x : 0.f, w.y != 0.f ? d.y : 0.f) : d; };
   float v[10];
 #pragma unroll
   for (int k = 0; k < 10; ++k) v[k] = 0.0f;
@@ -216,8 +232,8 @@ __device__ __forceinline__ void sum_slots(BwdShared<DEPTH, BATCH, GEOM>& sh, int
       for (int k = 0; k < kPlanes; ++k) {
         const float4 da = *reinterpret_cast<const float4*>(sh.image_grad[warp][k] + o);
         const float4 db = *reinterpret_cast<const float4*>(sh.image_grad[warp][k] + o + 32);
-        const float2 u = add2(fma2(hi2(da), hi2(wa), mul2(lo2(da), lo2(wa))),
-                              fma2(lo2(db), lo2(wb), mul2(hi2(db), hi2(wb))));
+        const float2 u = add2(fma2(where(hi2(da), hi2(wa)), hi2(wa), mul2(where(lo2(da), lo2(wa)), lo2(wa))),
+                              fma2(where(lo2(db), lo2(wb)), lo2(wb), mul2(where(hi2(db), hi2(wb)), hi2(wb))));
         c[k] = i ? add2(c[k], u) : u;
       }
     }
@@ -291,7 +307,10 @@ __device__ __forceinline__ void sum_slots(BwdShared<DEPTH, BATCH, GEOM>& sh, int
 // warp and instance, alpha_threshold per pixel). A lane leaves its two pixels' g and w of a
 // contributing instance in the warp's next slot; every eight instances the warp sums its
 // slots (sum_slots). The cross-warp sum of an instance adds only the warps it contributed
-// in (the others' terms are exact zeros). BATCH instances are staged per round; the
+// in (the others' terms are exact zeros). A tile whose image gradients are not all finite, or
+// a view with a colour or depth that is not, takes the ODD form, since the sums run over all
+// pixels of a box and 0 times such a value is no zero: it stays with the Gaussians that
+// contribute to its pixel. BATCH instances are staged per round; the
 // records do not depend on it (each instance's sums are formed the same way whatever batch
 // it is staged in), so the batch is a schedule choice. GEOM forms only the moments (the
 // terms of dL/dmean2D and dL/dconic), the same bits. Bound by instruction issue, and where
@@ -332,7 +351,8 @@ __global__ void __launch_bounds__(kBwdThreads, BLOCKS) k_render_bwd(RenderBwdArg
     if (DEPTH) *reinterpret_cast<float2*>(sh.image_grad[warp][3] + slot_at) = pp.dD;
   }
   if (threadIdx.x == 0) sh.max_last = 0;
-  __syncthreads();
+  // a tile with an image gradient, or a view with a colour or depth, that is not finite
+  const bool odd = __syncthreads_or(!(all_finite(p0) && all_finite(p1))) || *nonfinite_word(a.counts);
   const uint32_t my_last = max(p0.last, p1.last);
   if (my_last) atomicMax(&sh.max_last, my_last);
   // instances at or past the warp's largest contributor count reach none of its pixels
@@ -362,95 +382,100 @@ __global__ void __launch_bounds__(kBwdThreads, BLOCKS) k_render_bwd(RenderBwdArg
   // Batch b - 1 is copied asynchronously (its Gaussian ids were loaded a batch earlier)
   // while batch b is unwound; two block barriers per batch (staged, then partial sums
   // complete).
-  for (int b = nb - 1; b >= 0; --b) {
-    const int base = b * BATCH;
-    const int cnt = count_of(b);
-    cp_async_wait_all();
-    if (t < cnt) {  // raw values -> render form, own slot
-      const float2 m = sh.raw_xy[t];
-      const float4 co = sh.raw_co[t], c = sh.raw_rgbd[t];
-      StagedInstance& s = sh.inst[t];
-      const float ca = -0.5f * co.x, cb = -co.y, cc = -0.5f * co.z;
-      s.xy = make_float4(m.x, m.x, m.y, m.y);
-      s.ab = make_float4(ca, ca, cb, cb);
-      s.co = make_float4(cc, cc, co.w, co.w);
-      s.rg = make_float4(c.x, c.x, c.y, c.y);
-      s.bd = make_float4(c.z, c.z, c.w, c.w);
-      sh.thr[t] = alpha_threshold(co.w);
-      sh.pidx[t] = sh.raw_pidx[t];
-      *reinterpret_cast<uint32_t*>(sh.reached[t]) = 0u;
-    }
-    __syncthreads();  // batch b staged; batch b + 1 finished
-    if (b > 0) {
-      issue(b - 1);  // into this thread's own raw slot, read above
-      if (b > 1) load_id(b - 2);
-    }
-    uint32_t keep[BATCH / 32];
-#pragma unroll
-    for (int r = 0; r < BATCH / 32; ++r) {
-      const int j = r * 32 + lane;
-      bool kp = false;
-      if (j < cnt && base + j < warp_last) {
-        const StagedInstance& s = sh.inst[j];
-        const float4 xy = s.xy, ab = s.ab;
-        kp = box_may_contribute(make_float2(xy.x, xy.z), ab.x, ab.z, s.co.x, sh.thr[j], bxf0, bxf1, byf0, byf1);
+  auto unwind = [&](auto odd_form) {
+    constexpr bool ODD = decltype(odd_form)::value;
+    for (int b = nb - 1; b >= 0; --b) {
+      const int base = b * BATCH;
+      const int cnt = count_of(b);
+      cp_async_wait_all();
+      if (t < cnt) {  // raw values -> render form, own slot
+        const float2 m = sh.raw_xy[t];
+        const float4 co = sh.raw_co[t], c = sh.raw_rgbd[t];
+        StagedInstance& s = sh.inst[t];
+        const float ca = -0.5f * co.x, cb = -co.y, cc = -0.5f * co.z;
+        s.xy = make_float4(m.x, m.x, m.y, m.y);
+        s.ab = make_float4(ca, ca, cb, cb);
+        s.co = make_float4(cc, cc, co.w, co.w);
+        s.rg = make_float4(c.x, c.x, c.y, c.y);
+        s.bd = make_float4(c.z, c.z, c.w, c.w);
+        sh.thr[t] = alpha_threshold(co.w);
+        sh.pidx[t] = sh.raw_pidx[t];
+        *reinterpret_cast<uint32_t*>(sh.reached[t]) = 0u;
       }
-      keep[r] = __ballot_sync(0xffffffffu, kp);
-    }
-    // Back to front over the kept instances; the warp sums its slots whenever eight are
-    // pending and after the last instance.
-    int r = BATCH / 32 - 1;
-    uint32_t mk = keep[r];
-    for (bool more = true; more;) {
-      int used = 0;    // slots pending
-      int j_slot = 0;  // the instance in this lane's slot
-      while (used < kSlots) {
-        if (mk == 0) {
-          if (r == 0) {
-            more = false;
-            break;
+      __syncthreads();  // batch b staged; batch b + 1 finished
+      if (b > 0) {
+        issue(b - 1);  // into this thread's own raw slot, read above
+        if (b > 1) load_id(b - 2);
+      }
+      uint32_t keep[BATCH / 32];
+  #pragma unroll
+      for (int r = 0; r < BATCH / 32; ++r) {
+        const int j = r * 32 + lane;
+        bool kp = false;
+        if (j < cnt && base + j < warp_last) {
+          const StagedInstance& s = sh.inst[j];
+          const float4 xy = s.xy, ab = s.ab;
+          kp = box_may_contribute(make_float2(xy.x, xy.z), ab.x, ab.z, s.co.x, sh.thr[j], bxf0, bxf1, byf0, byf1);
+        }
+        keep[r] = __ballot_sync(0xffffffffu, kp);
+      }
+      // Back to front over the kept instances; the warp sums its slots whenever eight are
+      // pending and after the last instance.
+      int r = BATCH / 32 - 1;
+      uint32_t mk = keep[r];
+      for (bool more = true; more;) {
+        int used = 0;    // slots pending
+        int j_slot = 0;  // the instance in this lane's slot
+        while (used < kSlots) {
+          if (mk == 0) {
+            if (r == 0) {
+              more = false;
+              break;
+            }
+            --r;
+            mk = keep[0];
+  #pragma unroll
+            for (int k = 1; k < BATCH / 32; ++k)
+              if (k == r) mk = keep[k];
+            continue;
           }
-          --r;
-          mk = keep[0];
-#pragma unroll
-          for (int k = 1; k < BATCH / 32; ++k)
-            if (k == r) mk = keep[k];
-          continue;
+          const int bit = 31 - __clz(mk);
+          mk &= ~(1u << bit);
+          const int j = r * 32 + bit;
+          float2 g, w;
+          const bool contrib = unwind_pair<DEPTH, ODD>(pp, base + j, px, pyf, sh.inst[j], sh.thr[j], g, w);
+          if (!__any_sync(0xffffffffu, contrib)) continue;
+          *reinterpret_cast<float2*>(sh.g[warp][used] + slot_at) = g;
+          if constexpr (!GEOM) *reinterpret_cast<float2*>(sh.w[warp][used] + slot_at) = w;
+          if ((lane >> 2) == used) j_slot = j;
+          ++used;
         }
-        const int bit = 31 - __clz(mk);
-        mk &= ~(1u << bit);
-        const int j = r * 32 + bit;
-        float2 g, w;
-        const bool contrib = unwind_pair<DEPTH>(pp, base + j, px, pyf, sh.inst[j], sh.thr[j], g, w);
-        if (!__any_sync(0xffffffffu, contrib)) continue;
-        *reinterpret_cast<float2*>(sh.g[warp][used] + slot_at) = g;
-        if constexpr (!GEOM) *reinterpret_cast<float2*>(sh.w[warp][used] + slot_at) = w;
-        if ((lane >> 2) == used) j_slot = j;
-        ++used;
+        if (used) sum_slots<ODD>(sh, warp, lane, used, j_slot, bx0, by0);
       }
-      if (used) sum_slots(sh, warp, lane, used, j_slot, bx0, by0);
-    }
-    __syncthreads();  // every warp's partial sums of batch b are in
-    if (t < cnt) {
-      float sum[10];
-#pragma unroll
-      for (int q = 0; q < 10; ++q) sum[q] = 0.f;
-      const uint32_t reached = *reinterpret_cast<const uint32_t*>(sh.reached[t]);
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w)
-        if ((reached >> (8 * w)) & 0xffu) {
-#pragma unroll
-          for (int q = 0; q < Sh::kTerms; ++q) sum[q] += sh.part[w][t][q];
+      __syncthreads();  // every warp's partial sums of batch b are in
+      if (t < cnt) {
+        float sum[10];
+  #pragma unroll
+        for (int q = 0; q < 10; ++q) sum[q] = 0.f;
+        const uint32_t reached = *reinterpret_cast<const uint32_t*>(sh.reached[t]);
+  #pragma unroll
+        for (int w = 0; w < kWarps; ++w)
+          if ((reached >> (8 * w)) & 0xffu) {
+  #pragma unroll
+            for (int q = 0; q < Sh::kTerms; ++q) sum[q] += sh.part[w][t][q];
+          }
+        // An instance that reached no pixel has exact-zero gradients: no record, its byte stays 0.
+        if (reached) {
+          const uint32_t pidx = sh.pidx[t];
+          const float4 ab = sh.inst[t].ab, co = sh.inst[t].co;
+          finish_record(a.records + (size_t)kRecordFloat4 * pidx, sum, make_float4(ab.x, ab.z, co.x, co.z));
+          a.written[pidx] = 1;
         }
-      // An instance that reached no pixel has exact-zero gradients: no record, its byte stays 0.
-      if (reached) {
-        const uint32_t pidx = sh.pidx[t];
-        const float4 ab = sh.inst[t].ab, co = sh.inst[t].co;
-        finish_record(a.records + (size_t)kRecordFloat4 * pidx, sum, make_float4(ab.x, ab.z, co.x, co.z));
-        a.written[pidx] = 1;
       }
     }
-  }
+  };
+  if (odd) unwind(std::true_type{});
+  else unwind(std::false_type{});
   // Instances at or past the tile's last contributor reach no pixel: nothing to write.
 }
 
