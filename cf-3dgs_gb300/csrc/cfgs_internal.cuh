@@ -22,6 +22,13 @@ constexpr int kMaxShCoeffs = 16;  // SH degree 3
 // Workspace layouts. Every array starts on a 256-byte boundary.
 // ---------------------------------------------------------------------------
 __host__ __device__ inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
+// The first 16-byte boundary at or after p: where an array of wide words lies in a workspace
+// whose own boundary may be that of its 4-byte words. Its size allows for kAlignSlack.
+template <class T>
+inline T* aligned16(void* p) {
+  return reinterpret_cast<T*>((reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15);
+}
+constexpr size_t kAlignSlack = 15;
 
 // Raises a kernel's dynamic shared-memory limit to `bytes` on the current device, once
 // per device (a function attribute belongs to the device's context, so one flag per

@@ -338,7 +338,8 @@ __global__ void __launch_bounds__(256) k_densify_children(int64_t first_child, i
 }
 
 // Workspace of a plan: class bits, totals, sources and split ranks of up to 3 n rows, block
-// counts.
+// counts. The totals and block counts, of 16-byte words, begin at the next such boundary
+// (aligned16).
 struct DensifyLayout {
   size_t cls, tot, src, rank, bcount, total;
   explicit DensifyLayout(int64_t num) {
@@ -346,10 +347,10 @@ struct DensifyLayout {
     const size_t nb = (n + kDensBlock - 1) / kDensBlock;
     size_t o = 0;
     cls = o;    o = align256(o + sizeof(uint32_t) * n);
-    tot = o;    o = align256(o + sizeof(uint4));
+    tot = o;    o = align256(o + sizeof(uint4) + kAlignSlack);
     src = o;    o = align256(o + sizeof(uint32_t) * 3 * n);
     rank = o;   o = align256(o + sizeof(uint32_t) * 3 * n);
-    bcount = o; o = align256(o + sizeof(uint4) * nb);
+    bcount = o; o = align256(o + sizeof(uint4) * nb + kAlignSlack);
     total = o;
   }
 };
@@ -423,8 +424,8 @@ extern "C" int cfgs_densify_plan(int64_t num_gaussians, const float* grad_accum,
   const DensifyLayout L(n);
   char* w = static_cast<char*>(workspace);
   uint32_t* cls = reinterpret_cast<uint32_t*>(w + L.cls);
-  uint4* tot = reinterpret_cast<uint4*>(w + L.tot);
-  uint4* bcount = reinterpret_cast<uint4*>(w + L.bcount);
+  uint4* tot = aligned16<uint4>(w + L.tot);
+  uint4* bcount = aligned16<uint4>(w + L.bcount);
   const int nb = div_up(n, kDensBlock);
   DensifyParams d{max_grad, min_opacity, extent, percent_dense, prune_big};
   k_densify_classify<<<nb, kDensBlock, 0, st>>>(n, grad_accum, denom, scaling, opacity, d, cls, bcount);

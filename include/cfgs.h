@@ -133,7 +133,9 @@ typedef struct CfgsCounts {
   uint32_t flags;        /* CFGS_FLAG_* bits                                     */
 } CfgsCounts;
 
-/* ---- workspace sizing (host functions, no device work) ---------------------- */
+/* ---- workspace sizing (host functions, no device work) ----------------------
+ * A 16-byte boundary is enough for every workspace; the image and densification
+ * workspaces may lie on any 4-byte boundary. */
 
 /* Per-Gaussian workspace ("geomBuffer" upstream). */
 size_t cfgs_geom_bytes(int32_t num_gaussians);
