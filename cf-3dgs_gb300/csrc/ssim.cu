@@ -495,7 +495,8 @@ extern "C" size_t cfgs_ssim_scratch_bytes(int32_t channels, int32_t height, int3
   const SsimDims d = dims(channels, height, width);
   const size_t maps = sizeof(float) * 3 * (size_t)channels * height * width;
   const size_t parts = sizeof(double2) * (size_t)channels * d.tiles_x * d.tiles_y;
-  return align256(maps) + align256(parts) + align256(sizeof(double2) * (kSsimFoldBlocks + 1));
+  // the partial sums and what follows them begin at the next 16-byte boundary (aligned16)
+  return align256(maps) + align256(parts) + align256(sizeof(double2) * (kSsimFoldBlocks + 1) + kAlignSlack);
 }
 
 namespace {
@@ -509,7 +510,7 @@ int ssim_forward(int32_t channels, int32_t height, int32_t width, const float* i
   const SsimDims d = dims(channels, height, width);
   const size_t count = (size_t)channels * height * width;
   float* maps = static_cast<float*>(scratch);
-  double2* parts = reinterpret_cast<double2*>(static_cast<char*>(scratch) + align256(sizeof(float) * 3 * count));
+  double2* parts = aligned16<double2>(static_cast<char*>(scratch) + align256(sizeof(float) * 3 * count));
   const int tiles = d.tiles_x * d.tiles_y, pairs = tiles * channels;
   double2* sums = reinterpret_cast<double2*>(reinterpret_cast<char*>(parts) + align256(sizeof(double2) * (size_t)pairs));
   unsigned int* counter = reinterpret_cast<unsigned int*>(sums + kSsimFoldBlocks);

@@ -134,8 +134,8 @@ typedef struct CfgsCounts {
 } CfgsCounts;
 
 /* ---- workspace sizing (host functions, no device work) ----------------------
- * A 16-byte boundary is enough for every workspace; the image and densification
- * workspaces may lie on any 4-byte boundary. */
+ * A 16-byte boundary is enough for every workspace; the image, densification and SSIM
+* workspaces may lie on any 4-byte boundary. */
 
 /* Per-Gaussian workspace ("geomBuffer" upstream). */
 size_t cfgs_geom_bytes(int32_t num_gaussians);

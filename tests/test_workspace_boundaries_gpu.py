@@ -57,3 +57,34 @@ def test_densify(n, shift):
     assert (res["kept"], res["cloned"], res["split"], res["children_per_copy"]) == (keep, clone, split, child)
     for k, t in got.items():
         assert torch.equal(t, opt.params[k]), k
+
+
+@pytest.mark.parametrize("shift", [0, 4, 8, 12, 24])
+@pytest.mark.parametrize("shape", [(1, 5, 7), (3, 33, 36), (3, 64, 31), (3, 200, 264)])
+@pytest.mark.parametrize("lam", [None, 0.2])
+def test_ssim_and_photometric(shape, lam, shift):
+    from cfgs import native
+    from cfgs.raster import _ptr, stream_handle
+    lib, st = native.load(), stream_handle(torch.device(DEV))
+    g = torch.Generator().manual_seed(sum(shape))
+    x, y = ((torch.rand(shape, generator=g) * 1.2 - 0.1).to(DEV) for _ in range(2))
+    up = torch.full((), 0.7, device=DEV)
+
+    def run(ws):
+        out, dx = torch.empty((), device=DEV), torch.empty_like(x)
+        if lam is None:
+            native.check(lib.cfgs_ssim_forward(*shape, _ptr(x), _ptr(y), ws.data_ptr(), _ptr(out), st), "forward")
+            native.check(lib.cfgs_ssim_backward(*shape, _ptr(x), _ptr(y), ws.data_ptr(), _ptr(up), _ptr(dx), st), "backward")
+        else:
+            native.check(lib.cfgs_photometric_forward(*shape, _ptr(x), _ptr(y), lam, ws.data_ptr(), _ptr(out), st),
+                         "forward")
+            native.check(lib.cfgs_photometric_backward(*shape, _ptr(x), _ptr(y), lam, ws.data_ptr(), _ptr(up), _ptr(dx),
+                                                       st), "backward")
+        return out, dx
+
+    size = int(lib.cfgs_ssim_scratch_bytes(*shape))
+    ws, check = _carve(size, shift)
+    got = run(ws)
+    check()
+    want = run(torch.empty(size, dtype=torch.uint8, device=DEV))
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
