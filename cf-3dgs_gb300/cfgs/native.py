@@ -19,6 +19,7 @@ STATUS = {
     4: "CFGS_ERR_DEVICE_FLAG",
     5: "CFGS_ERR_TOO_LARGE",
 }
+ERR_INVALID_ARGUMENT = 1
 FLAG_FRUSTUM_VIOLATION = 0x1
 FLAG_CAPACITY_OVERFLOW = 0x2
 FLAG_COPY_TIMEOUT = 0x4

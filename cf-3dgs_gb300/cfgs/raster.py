@@ -113,14 +113,18 @@ class _Timed:
 
 
 _thread = threading.local()
-_ABANDONED: list = []  # slots of forwards that were interrupted before their count arrived
+_ABANDONED: list = []  # (slot, ticket) of forwards that were interrupted before their count arrived
+_abandoned_lock = threading.Lock()
 
 
 def _count_slot() -> torch.Tensor:
     """The calling thread's page-locked words for the instance count: a thread has one forward
-    waiting for its count at a time."""
+    waiting for its count at a time. (A thread that needs a new slot also gives back the
+    abandoned ones whose count has arrived since.)"""
     slot = getattr(_thread, "slot", None)
     if slot is None:
+        with _abandoned_lock:
+            _ABANDONED[:] = [(s, t) for s, t in _ABANDONED if int(s[2]) & 0xffffffff != t]
         slot = _thread.slot = torch.zeros(4, dtype=torch.int32, pin_memory=True)
     return slot
 
@@ -144,19 +148,23 @@ def forward(rs, means3D, opacities, shs, colors_precomp, scales, rotations, cov3
     depth = torch.empty((1, H, W), dtype=torch.float32, device=dev)
     alpha = torch.empty((1, H, W), dtype=torch.float32, device=dev)
     slot, ticket, counts = _count_slot(), C.c_uint32(), native.Counts()
+    refused = False
     try:
         with _Timed(timers, "preprocess"):
-            native.check(lib.cfgs_preprocess_counted(C.byref(s), C.byref(g), geom.data_ptr(), image.data_ptr(),
-                                                     radii.data_ptr() if N else None, slot.data_ptr(), C.byref(ticket),
-                                                     st), "cfgs_preprocess_counted")
+            status = lib.cfgs_preprocess_counted(C.byref(s), C.byref(g), geom.data_ptr(), image.data_ptr(),
+                                                 radii.data_ptr() if N else None, slot.data_ptr(), C.byref(ticket), st)
+            refused = status == native.ERR_INVALID_ARGUMENT
+            native.check(status, "cfgs_preprocess_counted")
         # The depth sort does not need K, so it is enqueued before the host waits for K, and
         # keeps the GPU busy meanwhile.
         with _Timed(timers, "depth_sort"):
             native.check(lib.cfgs_depth_order(N, geom.data_ptr(), st), "cfgs_depth_order")
         native.check(lib.cfgs_wait_counts(slot.data_ptr(), ticket, C.byref(counts), st), "cfgs_wait_counts")
     except BaseException:
-        _ABANDONED.append(slot)  # the kernel may still write to it
-        _thread.slot = None
+        if ticket.value and not refused:  # a kernel may still write to the slot
+            with _abandoned_lock:
+                _ABANDONED.append((slot, ticket.value))
+            _thread.slot = None
         raise
     if counts.flags & native.FLAG_FRUSTUM_VIOLATION:
         raise RuntimeError("prefiltered=True but a Gaussian lies at view z <= 0.2 (outside the frustum)")
