@@ -68,6 +68,12 @@ def dist_cuda2(points: torch.Tensor) -> torch.Tensor:
     return out
 
 
+def _differentiated(t: torch.Tensor) -> bool:
+    """Whether autograd follows t, backward or in forward mode (a tangent)."""
+    return (torch.is_grad_enabled() and t.requires_grad) or \
+        torch.autograd.forward_ad.unpack_dual(t).tangent is not None
+
+
 def gaussians_from_points(points: torch.Tensor, colors: torch.Tensor, sh_degree: int = 3,
                           view_dependent: bool = False) -> dict:
     """create_from_pcd (scene/gaussian_model_cf.py:175-210): colours as the DC term
@@ -79,6 +85,15 @@ def gaussians_from_points(points: torch.Tensor, colors: torch.Tensor, sh_degree:
     dc = ((col - 0.5) / C0 if view_dependent else col).to(p.device).expand(n, 3).contiguous()
     rest = (sh_degree + 1) ** 2 - 1
     f = dict(dtype=torch.float32, device=p.device)
+    if _differentiated(p) or _differentiated(dc):  # positions and features as differentiable copies
+        features = torch.zeros((n, 3, rest + 1), **f)
+        features[:, :, 0] = dc
+        scales = torch.log(torch.sqrt(torch.clamp_min(dist_cuda2(p), 0.0000001)))[..., None].repeat(1, 3)
+        rots = torch.zeros((n, 4), **f)
+        rots[:, 0] = 1
+        return {"xyz": p.clone(), "features_dc": features[:, :, 0:1].transpose(1, 2).contiguous(),
+                "features_rest": features[:, :, 1:].transpose(1, 2).contiguous(), "scaling": scales, "rotation": rots,
+                "opacity": torch.full((n, 1), math.log(0.1 / 0.9), **f)}
     out = {"xyz": torch.empty_like(p), "features_dc": torch.empty((n, 1, 3), **f),
            "features_rest": torch.empty((n, rest, 3), **f), "scaling": torch.empty((n, 3), **f),
            "rotation": torch.empty((n, 4), **f), "opacity": torch.empty((n, 1), **f)}
@@ -88,6 +103,4 @@ def gaussians_from_points(points: torch.Tensor, colors: torch.Tensor, sh_degree:
             n, 3 * rest, _ptr(p), _ptr(dc), _ptr(dist2), math.log(0.1 / 0.9), _ptr(out["xyz"]),
             _ptr(out["features_dc"]), _ptr(out["features_rest"]), _ptr(out["scaling"]), _ptr(out["rotation"]),
             _ptr(out["opacity"]), stream_handle(p.device)), "cfgs_init_gaussians")
-    if torch.is_grad_enabled() and (p.requires_grad or dc.requires_grad):
-        out["xyz"], out["features_dc"] = p.clone(), dc.reshape(n, 1, 3).clone()  # copies that gradients pass
     return out
