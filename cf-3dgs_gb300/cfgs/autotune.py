@@ -41,6 +41,7 @@ class Schedule:
 
 
 DEFAULT = Schedule()
+AUTO = Schedule(0, 0, 0)  # the library's own choice for each call's sizes (what no schedule means)
 FWD_CANDIDATES = [(128, 4), (64, 4), (256, 4), (128, 8), (256, 8)]  # (fwd_batch, fwd_warps), default first
 BWD_CANDIDATES = [64, 32, 128]
 
@@ -57,6 +58,16 @@ def c_schedule(s: Schedule | None = None) -> "native.RenderSchedule":
     return native.RenderSchedule(s.fwd_batch, s.fwd_warps, s.bwd_batch, s.bin_launch)
 
 
+def resolved(s: Schedule | None, num_tiles: int, num_gaussians: int, capacity: int) -> Schedule:
+    """The explicit schedule that a call under s (None or AUTO: the library chooses) uses over
+    num_tiles tiles with room for `capacity` instances of num_gaussians Gaussians."""
+    out = native.RenderSchedule()
+    native.check(native.load().cfgs_render_schedule_for(native.C.byref(c_schedule(s or AUTO)), int(num_tiles),
+                                                        int(num_gaussians), int(capacity), native.C.byref(out)),
+                 "cfgs_render_schedule_for")
+    return Schedule(out.fwd_batch, out.fwd_warps, out.bwd_batch, out.bin_launch)
+
+
 def set_schedule(s: Schedule) -> None:
     """Makes s the schedule of the calling thread's later rasteriser calls (checked by the
     library: an unsupported shape raises)."""
@@ -66,7 +77,8 @@ def set_schedule(s: Schedule) -> None:
 
 
 def get_schedule() -> Schedule:
-    """The calling thread's current schedule (DEFAULT until set)."""
+    """The calling thread's current schedule. DEFAULT until one is set, when calls run under
+    AUTO: resolved(None, ...) says what that is for given sizes."""
     return getattr(_thread, "schedule", None) or DEFAULT
 
 
@@ -177,14 +189,16 @@ class Autotuner:
         with using(sched):
             return time_cuda(run)
 
-    def tune(self, key: str, run: Callable[[], None], force: bool = False, margin: float = 0.02) -> Schedule:
+    def tune(self, key: str, run: Callable[[], None], force: bool = False, margin: float = 0.02,
+             incumbent: Schedule = DEFAULT, unbeaten: Schedule | None = None) -> Schedule:
         """The cached schedule for `key`, or the best candidate on run() (one unit of the
         workload, enqueued on the current stream), recorded in the cache. Coordinate
-        search: the forward shapes with the default backward batch, then the backward
-        batches with the best forward shape. A candidate displaces the incumbent (the
-        default first) only when it is faster by more than `margin`, and a choice other
-        than the default must win again in an interleaved confirmation, so timing noise
-        does not move the choice."""
+        search: the forward shapes with the incumbent's backward batch, then the backward
+        batches with the best forward shape. `incumbent` is the schedule the workload runs
+        under without tuning (resolved); a candidate displaces it only when it is faster by
+        more than `margin`, and must win again in an interleaved confirmation, so timing noise
+        does not move the choice. When nothing does, the choice is `unbeaten` (default: the
+        incumbent itself)."""
         if not force:
             hit = self.lookup(key)
             if hit is not None:
@@ -196,22 +210,26 @@ class Autotuner:
             timings[f"{s.fwd_batch}/{s.fwd_warps}/{s.bwd_batch}"] = round(ms, 5)
             return ms
 
-        fwd_t = {fw: trial(Schedule(fw[0], fw[1], DEFAULT.bwd_batch)) for fw in FWD_CANDIDATES}
-        best_fw = pick(FWD_CANDIDATES, fwd_t, margin)
-        bwd_t = {b: fwd_t[best_fw] if b == DEFAULT.bwd_batch else trial(Schedule(best_fw[0], best_fw[1], b))
-                 for b in BWD_CANDIDATES}
-        chosen = Schedule(best_fw[0], best_fw[1], pick(BWD_CANDIDATES, bwd_t, margin))
-        if chosen != DEFAULT:
+        own = (incumbent.fwd_batch, incumbent.fwd_warps)
+        fwd = [own] + [fw for fw in FWD_CANDIDATES if fw != own]
+        bwd = [incumbent.bwd_batch] + [b for b in BWD_CANDIDATES if b != incumbent.bwd_batch]
+        fwd_t = {fw: trial(Schedule(fw[0], fw[1], bwd[0])) for fw in fwd}
+        best_fw = pick(fwd, fwd_t, margin)
+        bwd_t = {b: fwd_t[best_fw] if b == bwd[0] else trial(Schedule(best_fw[0], best_fw[1], b)) for b in bwd}
+        chosen = Schedule(best_fw[0], best_fw[1], pick(bwd, bwd_t, margin))
+        if chosen != incumbent:
             # confirmation: both timed twice more, interleaved; the challenger must still win
             # by the margin on the sum
             a = b = 0.0
             for _ in range(2):
-                a += float(self.measure(run, DEFAULT))
+                a += float(self.measure(run, incumbent))
                 b += float(self.measure(run, chosen))
             timings["confirm_default"] = round(a / 2, 5)
             timings["confirm_chosen"] = round(b / 2, 5)
             if not b < a * (1.0 - margin):
-                chosen = DEFAULT
+                chosen = incumbent
+        if chosen == incumbent and unbeaten is not None:
+            chosen = unbeaten
         self.record(key, chosen, timings)
         return chosen
 
@@ -231,7 +249,7 @@ def tune_rasterizer(raster_settings, means3D, opacities, shs=None, colors_precom
                     apply: bool = True) -> Schedule:
     """Tunes the render schedule for one drop-in rasteriser workload (forward + backward
     with a unit image gradient) and, with apply=True, makes it the calling thread's
-    schedule."""
+    schedule. AUTO when no shape beats the library's own."""
     import torch
     from . import raster
     tuner = tuner or Autotuner()
@@ -247,7 +265,13 @@ def tune_rasterizer(raster_settings, means3D, opacities, shs=None, colors_precom
         raster.backward(raster_settings, st, means3D, opacities, shs, colors_precomp, scales, rotations,
                         cov3D_precomp, grad, None, None)
 
-    sched = tuner.tune(key, run)
+    sched = tuner.lookup(key)
+    if sched is None:
+        w, h, n = int(raster_settings.image_width), int(raster_settings.image_height), int(means3D.shape[0])
+        with using(AUTO):
+            K = raster.forward(raster_settings, means3D, opacities, shs, colors_precomp, scales, rotations,
+                               cov3D_precomp)[4].num_rendered
+        sched = tuner.tune(key, run, incumbent=resolved(AUTO, ((w + 15) // 16) * ((h + 15) // 16), n, K), unbeaten=AUTO)
     if apply:
         set_schedule(sched)
     return sched

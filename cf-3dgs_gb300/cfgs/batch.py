@@ -49,7 +49,7 @@ class BatchSolver:
 
     def __init__(self, problems: list[PoseProblem], lr: float = 1e-3, betas=(0.9, 0.999), eps: float = 1e-15,
                  capacity_factor: float = 1.25, graph_chunk: int = 25, use_graph: bool = True, autotune=None):
-        """autotune: None (keep the process-wide render schedule), True (tune with the
+        """autotune: None (keep the calling thread's render schedule), True (tune with the
         default cache) or an autotune.Autotuner; when set, the render schedule of this
         batch's shape is looked up or tuned on the batch itself before its iterations."""
         if not problems:
@@ -203,9 +203,18 @@ class BatchSolver:
 
             native.check(self.lib.cfgs_batch_init(C.byref(args), torch.cuda.current_stream(dev).cuda_stream),
                          "cfgs_batch_init")
-            sched = self.tuner.tune(key, run)
+            sched = self.tuner.tune(key, run, incumbent=self._resolved(autotune_mod.AUTO), unbeaten=autotune_mod.AUTO)
             self.load_state(*saved)
         self.schedule = sched
+
+    def _resolved(self, sched) -> "autotune_mod.Schedule":
+        return autotune_mod.resolved(sched, self.plan.num_tiles, self.plan.gauss_slots, self.capacity)
+
+    def schedule_in_use(self) -> "autotune_mod.Schedule":
+        """The explicit schedule of this batch's iterations: its own when tuned, else the calling
+        thread's, the library's choice for the batch's sizes filled in."""
+        c = autotune_mod.c_schedule(self.schedule)
+        return self._resolved(autotune_mod.Schedule(c.fwd_batch, c.fwd_warps, c.bwd_batch, c.bin_launch))
 
     def launch(self, iters: int) -> torch.cuda.Event:
         """Enqueues `iters` iterations of every solve from the current state (no reset)

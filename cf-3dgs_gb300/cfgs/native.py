@@ -169,6 +169,8 @@ EXPORTS = {
     "cfgs_photometric_backward": (C.c_int, [C.c_int32, C.c_int32, C.c_int32, _vp, _vp, C.c_double, _vp, _vp, _vp,
                                             _vp]),
     "cfgs_render_schedule_check": (C.c_int, [C.POINTER(RenderSchedule), C.POINTER(RenderSchedule)]),
+    "cfgs_render_schedule_for": (C.c_int, [C.POINTER(RenderSchedule), C.c_int64, C.c_int64, C.c_int64,
+                                           C.POINTER(RenderSchedule)]),
     "cfgs_diag_copy_timeout": (C.c_int, [C.c_uint32, _vp, _vp]),
     # include/cfgs_plain.h: the plain GPU path (published structure, comparison point)
     "cfgs_plain_work_bytes": (C.c_size_t, [C.c_int32, C.c_int64, C.c_int32, C.c_int32]),

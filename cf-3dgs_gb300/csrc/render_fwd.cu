@@ -294,6 +294,12 @@ bool resolve_schedule(const CfgsRenderSchedule& in, int64_t tiles, int64_t gauss
 
 using namespace cfgs;
 
+extern "C" int cfgs_render_schedule_for(const CfgsRenderSchedule* s, int64_t num_tiles, int64_t num_gaussians,
+                                        int64_t capacity, CfgsRenderSchedule* resolved) {
+  if (!s || !resolved || num_tiles < 0 || num_gaussians < 0 || capacity < 0) return CFGS_ERR_INVALID_ARGUMENT;
+  return resolve_schedule(*s, num_tiles, num_gaussians, capacity, resolved) ? CFGS_OK : CFGS_ERR_INVALID_ARGUMENT;
+}
+
 extern "C" int cfgs_render_schedule_check(const CfgsRenderSchedule* s, CfgsRenderSchedule* resolved) {
   if (!s) return CFGS_ERR_INVALID_ARGUMENT;
   CfgsRenderSchedule r;

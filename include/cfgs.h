@@ -69,16 +69,23 @@ typedef enum CfgsStatus {
  *              sort, emission, tile sort, tile ranges) as one launch per stage, 1 as one
  *              persistent cooperative launch with a bounded grid-wide wait between
  *              stages (same outputs)
- * All-zero fields mean the default: {128, 4, 64, 0}, or {256, 8, 64, 0} for a call over at
- * most 304 tiles or with room for fewer than four instances per Gaussian (the resolved
- * schedule reported below is the former); an unsupported combination makes the call return CFGS_ERR_INVALID_ARGUMENT. */
+ * All-zero first three fields mean the library's choice for the call's sizes: {256, 8, 64}
+ * for a call over at most 304 tiles or with room for fewer than four instances per
+ * Gaussian, else {128, 4, 64}. An unsupported combination makes the call return
+ * CFGS_ERR_INVALID_ARGUMENT. */
 typedef struct CfgsRenderSchedule {
   int32_t fwd_batch, fwd_warps, bwd_batch, bin_launch;
 } CfgsRenderSchedule;
 
-/* CFGS_OK when `schedule` is supported (zeros: the default), else
- * CFGS_ERR_INVALID_ARGUMENT; `resolved` (may be NULL) receives the schedule a call uses. */
+/* CFGS_OK when `schedule` is supported (zeros: the library's choice), else
+ * CFGS_ERR_INVALID_ARGUMENT; `resolved` (may be NULL) receives it with zeros replaced by the
+ * choice for a call of many tiles and large Gaussians. */
 int cfgs_render_schedule_check(const CfgsRenderSchedule* schedule, CfgsRenderSchedule* resolved);
+/* The same for given sizes: `resolved` receives the schedule a call uses over num_tiles tiles
+ * (of all images of a batch; 0: unknown) with room for `capacity` instances of num_gaussians
+ * Gaussians (a batch's slots). */
+int cfgs_render_schedule_for(const CfgsRenderSchedule* schedule, int64_t num_tiles, int64_t num_gaussians,
+                             int64_t capacity, CfgsRenderSchedule* resolved);
 
 /* GaussianRasterizationSettings (NamedTuple, 12 fields, order of
  * scene/gaussian_model_cf.py:811-824) plus the render schedule of the call. Tensor
