@@ -12,7 +12,8 @@ latency-bound and more, smaller warps can win.
 The tuner times the candidates on the caller's own workload with CUDA events and keeps
 the winner in a JSON cache keyed by the workload's shape — the Gaussian count rounded
 up to a power of two, the image size (or, for a batch of solves, the tile count rounded
-up to a power of two) and the SH width — so a shape is tuned once per cache.
+up to a power of two) and the SH width — so a shape is tuned once per cache and build of
+the library.
 
 The library keeps no schedule: each call carries one. On the host side the schedule
 calls use is the calling thread's current one (set_schedule / using), so threads that
@@ -29,6 +30,7 @@ from dataclasses import asdict, dataclass
 from pathlib import Path
 from typing import Callable
 
+from . import build as _build
 from . import native
 
 
@@ -162,9 +164,17 @@ class Autotuner:
             pass
         return "no-device"
 
+    @staticmethod
+    def _library() -> str:
+        try:
+            return _build.STAMP_PATH.read_text().strip()[:16]  # a hash of sources, flags and compiler
+        except OSError:
+            return "unstamped"
+
     def full_key(self, key: str) -> str:
-        """Cache entries are per GPU model: '<device name>|<workload key>'."""
-        return f"{self._device()}|{key}"
+        """Cache entries are per GPU model and build of the kernels they were timed with:
+        '<device name>|<library stamp>|<workload key>'."""
+        return f"{self._device()}|{self._library()}|{key}"
 
     def lookup(self, key: str) -> Schedule | None:
         e = self._cache.get(self.full_key(key))
