@@ -61,7 +61,7 @@ def _args():
     p.add_argument("--no-e2e", action="store_true")
     p.add_argument("--no-cpu", action="store_true")
     p.add_argument("--no-pose", action="store_true", help="skip the pose-solve half of the metric")
-    p.add_argument("--no-tune", action="store_true", help="keep the default render schedule (no autotuning)")
+    p.add_argument("--no-tune", action="store_true", help="keep the library's own render schedule (no autotuning)")
     p.add_argument("--no-plain", action="store_true", help="skip the plain GPU path's iteration")
     p.add_argument("--bin-launch", type=int, default=0, choices=[0, 1],
                    help="pose_iter/batch_iter: binning as one launch per stage (0) or one persistent launch (1)")
@@ -260,10 +260,8 @@ def run_ours(a) -> None:
 
     from cfgs import autotune
     from cfgs.loss import l1_loss_and_grad
-    if a.no_tune:
-        sched = autotune.DEFAULT
-        autotune.set_schedule(sched)
-    else:
+    sched = autotune.AUTO  # the library's own choice
+    if not a.no_tune:
         sched = autotune.tune_rasterizer(rs, s.means3D, s.opacities, s.shs, None, s.scales, s.rotations, None,
                                          tuner=autotune.Autotuner())
     loss_buf = torch.empty((), dtype=torch.float32, device=dev)
@@ -305,6 +303,7 @@ def run_ours(a) -> None:
     phase_ms = {k: sum(s_.elapsed_time(e_) for s_, e_ in v) / len(v) for k, v in timers.items()}
     D = (sc.sh_degree + 1) ** 2
     T = ((cam.width + 15) // 16) * ((cam.height + 15) // 16)
+    used = autotune.resolved(sched, T, sc.n, K)
     pb = phase_bytes(sc.n, K, HW, D, T)
     group_ms = {"preprocess": phase_ms["preprocess"], "binning": phase_ms["depth_sort"] + phase_ms["bin"],
                 "composite": phase_ms["composite"], "render_bwd": phase_ms["render_bwd"],
@@ -347,8 +346,8 @@ def run_ours(a) -> None:
             "warmup": a.warmup, "ms_per_step": round(ms_per_step, 4), "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": bench_config(sc, K, world),
-            "render_schedule": {"fwd_batch": sched.fwd_batch, "fwd_warps": sched.fwd_warps,
-                                "bwd_batch": sched.bwd_batch},
+            "render_schedule": {"fwd_batch": used.fwd_batch, "fwd_warps": used.fwd_warps,
+                                "bwd_batch": used.bwd_batch},
             "roofline": roofline, "phases": phases, "hbm_by_phase": hbm_groups,
             "iteration_hbm": {"algorithmic_bytes": iter_bytes,
                               "achieved_gbs": round(iter_bytes / (ms_per_step / 1000.0) / 1e9, 2),
@@ -651,8 +650,12 @@ def pose_single(dev, engine_reps: int = 5, plain_reps: int = 2) -> dict:
         res[mode] = {"solves_per_s": sps, "latency_s": lat, "xi": xi}
     tuner = autotune.Autotuner()
 
+    engine = None
+
     def engine_solve():
-        return batch.BatchSolver([prob], autotune=tuner).solve(300).xi[0]
+        nonlocal engine
+        engine = batch.BatchSolver([prob], autotune=tuner)
+        return engine.solve(300).xi[0]
 
     engine_solve()
     lat = []
@@ -678,7 +681,7 @@ def pose_single(dev, engine_reps: int = 5, plain_reps: int = 2) -> dict:
             "plain_vs_engine": {"rot_deg": eang, "trans": etr},
             "engine_vs_ground_truth": {"rot_deg": gerr[0], "trans": gerr[1]},
             "path": "solve engine (cfgs_batch_iteration in CUDA graphs), setup included",
-            "render_schedule": str(autotune.get_schedule())}
+            "render_schedule": str(engine.schedule_in_use())}
 
 
 def run_pose(a) -> None:
@@ -702,7 +705,7 @@ def run_pose_iter(a) -> None:
     prob = pose.make_problem(scenes.scene_pose(width=640, height=360, seed=2), dev)
     bs = batch.BatchSolver([prob])
     from cfgs import autotune
-    autotune.set_schedule(autotune.Schedule(bin_launch=a.bin_launch))
+    autotune.set_schedule(autotune.Schedule(0, 0, 0, a.bin_launch))
     args = bs.prepare()
     K0 = bs.capacity
     for _ in range(a.warmup):
@@ -731,7 +734,7 @@ def run_batch_iter(a) -> None:
     _, probs, _ = _pose_setup(dev, 64)
     bs = batch.BatchSolver(probs)
     from cfgs import autotune
-    autotune.set_schedule(autotune.Schedule(bin_launch=a.bin_launch))
+    autotune.set_schedule(autotune.Schedule(0, 0, 0, a.bin_launch))
     args = bs.prepare()
     for _ in range(a.warmup):
         bs.iterate(args)
@@ -781,7 +784,7 @@ def pose_batch(dev, probs, sample: int = 8) -> dict:
             "speedup_vs_plain": round(sps / plain_sps, 3),
             "batched_vs_fused_single_bit_identical": bool(np.array_equal(np.float32(xf), np.float32(r.xi[:sample]))),
             "batched_vs_plain_max": {"rot_deg": max(x[0] for x in agree), "trans": max(x[1] for x in agree)},
-            "graph_chunk": bs.graph_chunk, "render_schedule": str(bs.schedule)}
+            "graph_chunk": bs.graph_chunk, "render_schedule": str(bs.schedule_in_use())}
 
 
 def run_batch(a) -> None:
