@@ -74,7 +74,7 @@ struct GeomLayout {
     touched = o;      o = align256(o + sizeof(uint32_t) * (size_t)n);
     offset = o;       o = align256(o + sizeof(uint32_t) * (size_t)n);
     clamped = o;      o = align256(o + (size_t)n);
-    block_sums = o;   o = align256(o + sizeof(uint32_t) * (size_t)(num_blocks + 1));  // unused: keeps the offsets
+    block_sums = o;   // no room of its own: a place in the list of offsets that callers read by number
     depth_key = o;    o = align256(o + sizeof(uint32_t) * 2 * sn);
     depth_val = o;    o = align256(o + sizeof(uint32_t) * 2 * sn);
     rank_sums = o;    o = align256(o + sizeof(uint32_t) * (size_t)(num_blocks + 1));
@@ -95,7 +95,7 @@ struct GeomView {
   uint32_t* depth_key[2];  // depth sort ping-pong keys; depth_key[0] ends as the instance prefix by depth rank
   uint32_t* depth_val[2];  // depth sort ping-pong Gaussian ids; depth_val[1] = Gaussians in depth order
   uint32_t* rank_sums;     // instances per 1024 depth-ordered Gaussians
-  uint32_t* depth_counts;  // [256][chunks] per-pass digit counts, then first slots
+  uint32_t* depth_counts;  // per-pass digit counts: [256][chunks], then first slots; few chunks: [chunks][256]
   uint32_t* depth_totals;  // [passes][256] digit totals
   __host__ __device__ GeomView() {}
   __host__ __device__ GeomView(void* base, int32_t n) {
@@ -182,7 +182,7 @@ struct BinningView {
   uint2* pair[2];         // Gaussian id, instance index (position in depth order)
   uint32_t* sorted_gid;   // sorted position -> Gaussian id
   uint32_t* sorted_pidx;  // sorted position -> instance index
-  uint32_t* chunk_counts; // [256][chunks] per-pass digit counts, then first slots
+  uint32_t* chunk_counts; // as GeomView::depth_counts
   uint32_t* totals;       // [passes][256] digit totals
   uint32_t* starts;       // [chunks + 1] depth rank whose instances cover a chunk's first position
   __host__ __device__ BinningView() {}

@@ -1,5 +1,5 @@
 // Forward phase 1: per-Gaussian preprocess (EWA projection, SH colour, radius, tile
-// rectangle), per-tile instance counts and the two scans. Also markVisible.
+// rectangle) and the number of instances of all. Also markVisible.
 //
 // This translation unit is compiled with -fmad=false: every a*b+c below is two
 // IEEE-rounded operations unless written as fmaf(), so the CPU oracle reproduces the
@@ -14,26 +14,6 @@
 #include "kernels.cuh"
 
 namespace cfgs {
-
-struct CamConst {
-  float V[16];
-  float P[16];
-  float campos[3];
-};
-
-__device__ __forceinline__ void load_cam(const CfgsSettings& s, CamConst& c) {
-#pragma unroll
-  for (int i = 0; i < 16; ++i) c.V[i] = __ldg(s.viewmatrix + i);
-#pragma unroll
-  for (int i = 0; i < 16; ++i) c.P[i] = __ldg(s.projmatrix + i);
-  if (s.campos) {
-    c.campos[0] = __ldg(s.campos + 0);
-    c.campos[1] = __ldg(s.campos + 1);
-    c.campos[2] = __ldg(s.campos + 2);
-  } else {
-    c.campos[0] = c.campos[1] = c.campos[2] = 0.f;
-  }
-}
 
 // [p,1] @ M, columns 0..2 (row-vector convention of the stored matrices).
 __device__ __forceinline__ float3 xform43(const float* m, float3 p) {

@@ -500,8 +500,10 @@ void launch_render_bwd_batch(const RenderBwdArgs<Scenes>& a, int tiles, cudaStre
   if constexpr (GEOM) {
     if (tiles <= 8 * kBwdSms) launch_render_bwd_blocks<Scenes, DEPTH, BATCH, GEOM, 6>(a, tiles, st);
     else launch_render_bwd_blocks<Scenes, DEPTH, BATCH, GEOM, 7>(a, tiles, st);
+  } else if constexpr (DEPTH) {
+    launch_render_bwd_blocks<Scenes, DEPTH, BATCH, GEOM, 4>(a, tiles, st);
   } else {
-    if (DEPTH || tiles <= 4 * kBwdSms) launch_render_bwd_blocks<Scenes, DEPTH, BATCH, GEOM, 4>(a, tiles, st);
+    if (tiles <= 4 * kBwdSms) launch_render_bwd_blocks<Scenes, DEPTH, BATCH, GEOM, 4>(a, tiles, st);
     else launch_render_bwd_blocks<Scenes, DEPTH, BATCH, GEOM, 5>(a, tiles, st);
   }
 }

@@ -160,13 +160,14 @@ size_t cfgs_backward_scratch_bytes(int64_t capacity);
  * upstream exposes the same buffers as opaque uint8 tensors).
  * geom  (14): xy float2, conic_op float4 (a,b,c,opacity), rgbd float4 (r,g,b,depth),
  *             rect uint2 (x0|y0<<16, x1|y1<<16), touched u32, offset u32 (first instance
- *             index), clamped u8, block_sums u32, depth_key u32[2][N], depth_val u32[2][N]
- *             (depth_val[1] = Gaussian ids in (depth, id) order), rank_sums u32,
+ *             index), clamped u8, block_sums (nothing: no room of its own), depth_key u32[2][N]
+ *             ([0] = first instance of each depth rank, once the order is formed),
+ *             depth_val u32[2][N] ([1] = Gaussian ids in (depth, id) order), rank_sums u32,
  *             depth_counts u32, depth_totals u32, total bytes
  * image (6):  counts CfgsCounts, tile_count u32, tile_range u32[T+1], final_T f32,
  *             n_contrib u32, total bytes
- * binning (8): key u32[2][cap] (tile), gid u32[2][cap], pidx u32[2][cap],
- *             sorted_gid u32, sorted_pidx u32 (instance index), chunk_counts u32,
+ * binning (8): key u32[2][cap] (tile), gid and pidx: one buffer of cap (Gaussian,
+ *             instance index) pairs each, between the tile sort's passes, sorted_gid u32, sorted_pidx u32 (instance index), chunk_counts u32,
  *             totals u32, total bytes */
 void cfgs_geom_layout(int32_t num_gaussians, size_t offsets[14]);
 void cfgs_image_layout(int32_t image_width, int32_t image_height, size_t offsets[6]);
