@@ -167,8 +167,8 @@ size_t cfgs_backward_scratch_bytes(int64_t capacity);
  * image (6):  counts CfgsCounts, tile_count u32, tile_range u32[T+1], final_T f32,
  *             n_contrib u32, total bytes
  * binning (8): key u32[2][cap] (tile), gid and pidx: one buffer of cap (Gaussian,
- *             instance index) pairs each, between the tile sort's passes, sorted_gid u32, sorted_pidx u32 (instance index), chunk_counts u32,
- *             totals u32, total bytes */
+ *             instance index) pairs each, between the tile sort's passes, sorted_gid u32,
+ *             sorted_pidx u32 (instance index), chunk_counts u32, totals u32, total bytes */
 void cfgs_geom_layout(int32_t num_gaussians, size_t offsets[14]);
 void cfgs_image_layout(int32_t image_width, int32_t image_height, size_t offsets[6]);
 void cfgs_binning_layout(int64_t capacity, size_t offsets[8]);
