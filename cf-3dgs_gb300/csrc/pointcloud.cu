@@ -297,8 +297,8 @@ __device__ __forceinline__ uint32_t spread10(uint32_t x) {
 }
 
 __global__ void __launch_bounds__(256) k_morton(int64_t n, const float* __restrict__ xyz,
-                                                const uint32_t* __restrict__ bounds, int drop_bits,
-                                                uint32_t* __restrict__ code, uint32_t* __restrict__ idx) {
+                                                const uint32_t* __restrict__ bounds, uint32_t* __restrict__ code,
+                                                uint32_t* __restrict__ idx) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint32_t q[3];
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(256) k_morton(int64_t n, const float* __restri
     const float t = ext > 0.f ? (xyz[3 * i + a] - lo) / ext : 0.f;
     q[a] = (uint32_t)fminf(fmaxf(t * 1024.f, 0.f), 1023.f);
   }
-  code[i] = (spread10(q[0]) | (spread10(q[1]) << 1) | (spread10(q[2]) << 2)) >> drop_bits;
+  code[i] = spread10(q[0]) | (spread10(q[1]) << 1) | (spread10(q[2]) << 2);
   idx[i] = (uint32_t)i;
 }
 
@@ -581,12 +581,13 @@ extern "C" int cfgs_knn3_mean_dist2(int64_t num_points, const float* xyz, void* 
   float4* box = reinterpret_cast<float4*>(w + L.box);
   float4* sup = reinterpret_cast<float4*>(w + L.sup);
   if (!launch_bounds_pass(n, xyz, bounds, st)) return CFGS_ERR_LAUNCH;
-  // The order only groups neighbours; the search is exact in any. 8 bits an axis (three
-  // radix passes) still separate the points of up to 2^18; beyond that 10 bits (four).
-  const int drop = n <= (1 << 18) ? 6 : 0;
-  k_morton<<<div_up(n, 256), 256, 0, st>>>(n, xyz, bounds, drop, keys[0], vals[0]);
+  // 10 bits an axis, four radix passes. 8 bits would save one (160,000 points evenly spread or
+  // on a surface: 10 to 13 us of 186 to 361), but a few far points stretch the bounds, and
+  // the codes then no longer part the others (one in a thousand 30 times as far out: 3387 us
+  // against 556; 262,144 points 9424 against 1069).
+  k_morton<<<div_up(n, 256), 256, 0, st>>>(n, xyz, bounds, keys[0], vals[0]);
   int res = 0;
-  int s = sort_pairs(keys, vals, n, 30 - drop, reinterpret_cast<uint32_t*>(w + L.counts),
+  int s = sort_pairs(keys, vals, n, 30, reinterpret_cast<uint32_t*>(w + L.counts),
                      reinterpret_cast<uint32_t*>(w + L.totals), st, &res);
   if (s != CFGS_OK) return s;
   const int64_t nbox = (n + kKnnBox - 1) / kKnnBox;
