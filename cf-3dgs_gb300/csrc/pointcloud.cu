@@ -139,10 +139,10 @@ __global__ void __launch_bounds__(256) k_gather_u32(int64_t n, const uint32_t* _
 }
 
 // The voxels are the runs of equal keys in sorted order. A run's number is the count of
-// run heads before it: heads per block of 1024 positions, an exclusive prefix of those
+// run heads before it: heads per block of 512 positions, an exclusive prefix of those
 // (one block), then ballots inside the block. The scan by one block over all positions that
 // this replaces took 190 us for 230,400 points; count and prefix take 6.9 us.
-constexpr int kVoxelBlock = 1024;
+constexpr int kVoxelBlock = 512;
 
 __device__ __forceinline__ bool voxel_head(int64_t i, int64_t n, const uint32_t* __restrict__ lo,
                                            const uint32_t* __restrict__ hi) {
@@ -191,10 +191,13 @@ __global__ void __launch_bounds__(kVoxelBlock) k_voxel_prefix(int nblocks, uint3
 // averaged and rounded to float. Bound by the float64 pipe, which takes about 16 cycles of
 // its SM per warp instruction however few lanes take part, so only the runs of two or more
 // points go through it, packed into whole warps; a single point is its own average. The
-// block's 1024 positions are gathered to shared memory first; a run that goes on into the
-// next block reads the rest from memory. 230,400 points in 161,225 voxels: 62 us with a
-// thread at every run's head -> 28 us.
-__global__ void __launch_bounds__(kVoxelBlock) k_voxel_average(int64_t n, const uint32_t* __restrict__ lo,
+// block's 512 positions are gathered to shared memory first; a run that goes on into the
+// next block reads the rest from memory, one point ahead, which wants 40 registers and so
+// three blocks of 512 per SM (two of 1024 leave 32). 230,400 points in 161,225 voxels: 62 us
+// with a thread at every run's head -> 28 us. Long runs, whole calls: 20,000 points of which
+// two thirds share a voxel 5.7 -> 5.5 ms, 230,400 in 8 voxels 14.3 -> 11.6 ms (6.9 and 17.1 with
+// the rest of a run read key by key).
+__global__ void __launch_bounds__(kVoxelBlock, 3) k_voxel_average(int64_t n, const uint32_t* __restrict__ lo,
                                                                const uint32_t* __restrict__ hi,
                                                                const uint32_t* __restrict__ bprefix,
                                                                const uint32_t* __restrict__ order,
@@ -257,6 +260,7 @@ __global__ void __launch_bounds__(kVoxelBlock) k_voxel_average(int64_t n, const 
   const int start = (int)(s_run[threadIdx.x] & 0xffffu), end = (int)(s_run[threadIdx.x] >> 16);
   const size_t v = s_voxel[threadIdx.x];
   double s[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll 2
   for (int t = start; t < end; ++t) {
 #pragma unroll
     for (int a = 0; a < 3; ++a) s[a] += (double)s_val[a][t];
@@ -267,15 +271,37 @@ __global__ void __launch_bounds__(kVoxelBlock) k_voxel_average(int64_t n, const 
   }
   int64_t k = first + end;
   if (end == here) {
+    // its end by steps that double, then halve (the keys are sorted), so that the sums below
+    // know their count and load ahead
     const uint32_t klo = lo[first + start], khi = hi ? hi[first + start] : 0u;
-    for (; k < n && lo[k] == klo && (!hi || hi[k] == khi); ++k) {
-      const size_t j = order[k];
+    auto inside = [&](int64_t p) { return p < n && lo[p] == klo && (!hi || hi[p] == khi); };
+    int64_t last = k - 1, step = 1;
+    while (inside(last + step)) {
+      last += step;
+      step *= 2;
+    }
+    for (step /= 2; step > 0; step /= 2)
+      if (inside(last + step)) last += step;
+    // the next point's values and the one after's index are on their way while one is added
+    auto load = [&](uint32_t p, float (&v)[6]) {
 #pragma unroll
-      for (int a = 0; a < 3; ++a) s[a] += (double)xyz[3 * j + a];
-      if (rgb) {
-#pragma unroll
-        for (int a = 0; a < 3; ++a) s[3 + a] += (double)rgb[3 * j + a];
+      for (int a = 0; a < 3; ++a) {
+        v[a] = xyz[3 * (size_t)p + a];
+        v[3 + a] = rgb ? rgb[3 * (size_t)p + a] : 0.f;
       }
+    };
+    float ahead[6];
+    load(order[min(k, last)], ahead);
+    uint32_t next = order[min(k + 1, last)];
+#pragma unroll 1
+    for (; k <= last; ++k) {
+      float own[6];
+#pragma unroll
+      for (int a = 0; a < 6; ++a) own[a] = ahead[a];
+      load(next, ahead);
+      next = order[min(k + 2, last)];
+#pragma unroll
+      for (int a = 0; a < 6; ++a) s[a] += (double)own[a];
     }
   }
   const double count = (double)(k - (first + start)), inv = 1.0 / count;
