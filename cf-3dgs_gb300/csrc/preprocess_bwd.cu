@@ -17,6 +17,8 @@
 // 1,000,000 Gaussians, 12.4 million instances: 284 -> 230 us (record sums alone 154, the rest
 // alone 115; DRAM floor 103). Slower: three or four records at a time 240, 251 (registers),
 // the whole warp on one large Gaussian 246, 102 or 64 registers 243, 278.
+#include <type_traits>
+
 #include "cfgs_internal.cuh"
 #include "kernels.cuh"
 
@@ -47,6 +49,16 @@ __device__ __forceinline__ void group8_sum16(float (&v)[16], int lane) {
     const float keep = up ? v[k + 2] : v[k];
     v[k] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
   }
+}
+
+// Marks of eight slots, 8 apart from slot `slot` on (at instance i) below nt.
+template <class Args>
+__device__ __forceinline__ uint32_t marks_of(const Args& a, uint32_t i, uint32_t slot, uint32_t nt) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (slot + 8 * j < nt && __ldg(a.written + i + 8 * j)) m |= 1u << j;
+  return m;
 }
 
 enum BwdForm { kFullForm, kMeansForm, kPoseForm };
@@ -384,6 +396,12 @@ __device__ __forceinline__ void zero_gradients(const PreBwdArgs<Scenes>& a, int6
 }
 
 constexpr int kBwdThreads = 128;  // full form
+// A warp with a Gaussian of more tiles than this keeps four records and the next marks in
+// flight instead of two records and the next Gaussians' first ones, since that one
+// Gaussian's chain is what is left when the others are done: 300,000 Gaussians, eight of them
+// over all 8160 tiles, 538 -> 423 us, 100 such 1996 -> 1493. Not every warp: 1,000,000
+// Gaussians 245 us with the line here, 255 and 274 with it at 512 and 256.
+constexpr uint32_t kLongTiles = 1024;
 
 // One record's ten values; zeros when it was not written.
 struct Record {
@@ -421,7 +439,7 @@ template <class Scenes, BwdForm FORM>
 __global__ void __launch_bounds__(FORM == kPoseForm ? 256 : kBwdThreads, FORM == kPoseForm ? 4 : FORM == kMeansForm ? 8 : 6)
     k_preprocess_bwd(PreBwdArgs<Scenes> a) {
   constexpr bool POSE = FORM == kPoseForm;  // a.pose_partials is set exactly for this form
-  constexpr bool kPrefetch = FORM == kFullForm;
+  constexpr int kDeepRecords = 4;
   constexpr int kThreads = POSE ? 256 : kBwdThreads, kWarps = kThreads / 32;
   extern __shared__ __align__(128) float4 s_sh[];  // [kThreads][12] with sh_bulk
   __shared__ float s_acc[kThreads][11];
@@ -459,7 +477,8 @@ __global__ void __launch_bounds__(FORM == kPoseForm ? 256 : kBwdThreads, FORM ==
     off_l = a.geom.offset[idx];  // not set, and not used, for a Gaussian that touches no tile
     if (radius <= 0) nt_l = 0;
   }
-  {
+  auto sum_records = [&](auto deep_form) {
+    constexpr bool DEEP = decltype(deep_form)::value, kPrefetch = FORM == kFullForm && !DEEP;
     const int sub = lane & 7, grp = lane >> 3;
     // The written marks of this lane's first two instance slots (sub, sub + 8) of all
     // eight rounds first: sixteen independent byte loads in flight together, so each
@@ -494,10 +513,27 @@ __global__ void __launch_bounds__(FORM == kPoseForm ? 256 : kBwdThreads, FORM ==
       // slots r = sub, sub + 8, sub + 16, ... in order; unwritten slots are exact zeros
       add_record(v, n0);
       add_record(v, n1);
+      if constexpr (DEEP) {
+        uint32_t m = marks_of(a, off + sub + 16, sub + 16, nt);
+        for (uint32_t first = sub + 16; first < nt; first += 64) {
+          const uint32_t ahead = marks_of(a, off + first + 64, first + 64, nt);
+          while (m) {
+            Record t[kDeepRecords];
+#pragma unroll
+            for (int u = 0; u < kDeepRecords; ++u) {
+              t[u] = load_record(a.records, off + first + 8 * (__ffs(m) - 1), m != 0);
+              m &= m - 1;
+            }
+#pragma unroll
+            for (int u = 0; u < kDeepRecords; ++u) add_record(v, t[u]);
+          }
+          m = ahead;
+        }
+      }
       if (kPrefetch && q < 7) load_round(q + 1);
       // The rest 64 slots at a time: eight marks per lane in flight together, then the written
       // records two at a time.
-      for (uint32_t first = sub + 16; first < nt; first += 64) {
+      for (uint32_t first = sub + 16; !DEEP && first < nt; first += 64) {
         uint32_t m = 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -519,7 +555,9 @@ __global__ void __launch_bounds__(FORM == kPoseForm ? 256 : kBwdThreads, FORM ==
         s_acc[warp * 32 + src][2 * sub + 1] = v[1];
       }
     }
-  }
+  };
+  if (FORM != kPoseForm && __any_sync(0xffffffffu, nt_l > kLongTiles)) sum_records(std::true_type{});
+  else sum_records(std::false_type{});
   __syncwarp();
 
   // ---- phase 2: one thread per Gaussian ----------------------------------------------
