@@ -62,7 +62,8 @@ def c_schedule(s: Schedule | None = None) -> "native.RenderSchedule":
 
 def resolved(s: Schedule | None, num_tiles: int, num_gaussians: int, capacity: int) -> Schedule:
     """The explicit schedule that a call under s (None or AUTO: the library chooses) uses over
-    num_tiles tiles with room for `capacity` instances of num_gaussians Gaussians."""
+    num_tiles tiles with `capacity` instances of num_gaussians Gaussians that touch a tile (0:
+    not known)."""
     out = native.RenderSchedule()
     native.check(native.load().cfgs_render_schedule_for(native.C.byref(c_schedule(s or AUTO)), int(num_tiles),
                                                         int(num_gaussians), int(capacity), native.C.byref(out)),
@@ -277,11 +278,12 @@ def tune_rasterizer(raster_settings, means3D, opacities, shs=None, colors_precom
 
     sched = tuner.lookup(key)
     if sched is None:
-        w, h, n = int(raster_settings.image_width), int(raster_settings.image_height), int(means3D.shape[0])
+        w, h = int(raster_settings.image_width), int(raster_settings.image_height)
         with using(AUTO):
-            K = raster.forward(raster_settings, means3D, opacities, shs, colors_precomp, scales, rotations,
-                               cov3D_precomp)[4].num_rendered
-        sched = tuner.tune(key, run, incumbent=resolved(AUTO, ((w + 15) // 16) * ((h + 15) // 16), n, K), unbeaten=AUTO)
+            st = raster.forward(raster_settings, means3D, opacities, shs, colors_precomp, scales, rotations,
+                                cov3D_precomp)[4]
+        own = resolved(AUTO, ((w + 15) // 16) * ((h + 15) // 16), st.touching, st.num_rendered)
+        sched = tuner.tune(key, run, incumbent=own, unbeaten=AUTO)
     if apply:
         set_schedule(sched)
     return sched

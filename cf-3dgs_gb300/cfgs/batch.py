@@ -138,6 +138,7 @@ class BatchSolver:
         self.partials = torch.zeros(plan.num_blocks * 9, dtype=torch.float64, device=dev)
         self.xi = torch.zeros(self.S, 6, **f)
         self.adam = torch.zeros(self.S, 16, **f)
+        self.touching = 0  # Gaussians that touch a tile, once probed
         self._alloc_instances(0)
 
     def _alloc_instances(self, capacity: int):
@@ -161,8 +162,9 @@ class BatchSolver:
         a.pose_partials, a.xi, a.adam_state = self.partials.data_ptr(), self.xi.data_ptr(), self.adam.data_ptr()
         a.pose_states = self.pose_states.data_ptr()
         a.lr, a.beta1, a.beta2, a.eps = self.lr, float(self.betas[0]), float(self.betas[1]), self.eps
-        # this batch's tuned schedule, else the calling thread's current one
-        a.schedule = autotune_mod.c_schedule(self.schedule)
+        # this batch's tuned schedule, else the calling thread's current one, the library's choice
+        # for the batch's sizes filled in
+        a.schedule = autotune_mod.c_schedule(self.schedule_in_use())
         a.sh_degree_bound = 1 + max(int(sc.sh_degree) for sc in self.scenes)
         return a
 
@@ -208,7 +210,7 @@ class BatchSolver:
         self.schedule = sched
 
     def _resolved(self, sched) -> "autotune_mod.Schedule":
-        return autotune_mod.resolved(sched, self.plan.num_tiles, self.plan.gauss_slots, self.capacity)
+        return autotune_mod.resolved(sched, self.plan.num_tiles, self.touching, self.capacity)
 
     def schedule_in_use(self) -> "autotune_mod.Schedule":
         """The explicit schedule of this batch's iterations: its own when tuned, else the calling
@@ -283,6 +285,9 @@ class BatchSolver:
         native.check(self.lib.cfgs_batch_init(C.byref(args), st), "cfgs_batch_init")
         native.check(self.lib.cfgs_batch_iteration(C.byref(args), st), "cfgs_batch_iteration")
         K = int(self._counts().num_rendered)
+        touching = C.c_uint32()
+        native.check(self.lib.cfgs_read_touching(self.image.data_ptr(), C.byref(touching), st), "cfgs_read_touching")
+        self.touching = int(touching.value)
         return K
 
     def solve(self, iters: int = 300) -> BatchResult:

@@ -118,8 +118,10 @@ EXPORTS = {
     "cfgs_preprocess_counted": (C.c_int, [C.POINTER(Settings), C.POINTER(Gaussians), _vp, _vp, _vp, _vp,
                                           C.POINTER(C.c_uint32), _vp]),
     "cfgs_wait_counts": (C.c_int, [_vp, C.c_uint32, C.POINTER(Counts), _vp]),
+    "cfgs_wait_sizes": (C.c_int, [_vp, C.c_uint32, C.POINTER(Counts), C.POINTER(Settings), _vp]),
     "cfgs_preprocess_forward": (C.c_int, [C.POINTER(Settings), C.POINTER(Gaussians), _vp, _vp, _vp, _vp]),
     "cfgs_read_counts": (C.c_int, [_vp, C.POINTER(Counts), _vp]),
+    "cfgs_read_touching": (C.c_int, [_vp, C.POINTER(C.c_uint32), _vp]),
     "cfgs_render_forward": (C.c_int, [C.POINTER(Settings), C.POINTER(Gaussians), _vp, _vp, _vp, C.c_int64,
                                       _vp, _vp, _vp, _vp]),
     "cfgs_backward": (C.c_int, [C.POINTER(Settings), C.POINTER(Gaussians), _vp, _vp, _vp, _vp, C.c_int64, _vp,

@@ -91,6 +91,7 @@ class ForwardState:
     binning: torch.Tensor
     num_rendered: int
     radii: torch.Tensor
+    touching: int = 0  # Gaussians that touch a tile
     inputs_only: bool = False  # the backward forms the inputs' gradients only
 
 
@@ -159,7 +160,8 @@ def forward(rs, means3D, opacities, shs, colors_precomp, scales, rotations, cov3
         # keeps the GPU busy meanwhile.
         with _Timed(timers, "depth_sort"):
             native.check(lib.cfgs_depth_order(N, geom.data_ptr(), st), "cfgs_depth_order")
-        native.check(lib.cfgs_wait_counts(slot.data_ptr(), ticket, C.byref(counts), st), "cfgs_wait_counts")
+        # (and the library's choice of the compositing's shape, now that its sizes are known)
+        native.check(lib.cfgs_wait_sizes(slot.data_ptr(), ticket, C.byref(counts), C.byref(s), st), "cfgs_wait_sizes")
     except BaseException:
         if ticket.value and not refused:  # a kernel may still write to the slot
             with _abandoned_lock:
@@ -171,6 +173,7 @@ def forward(rs, means3D, opacities, shs, colors_precomp, scales, rotations, cov3
     if counts.flags & native.FLAG_CAPACITY_OVERFLOW:
         raise RuntimeError("more than 2^31 tile instances")
     K = int(counts.num_rendered)
+    touching = C.c_uint32.from_address(slot.data_ptr() + 12).value
     binning = torch.empty(lib.cfgs_binning_bytes(K), dtype=torch.uint8, device=dev)
     with _Timed(timers, "bin"):
         native.check(lib.cfgs_bin_instances(C.byref(s), C.byref(g), geom.data_ptr(), image.data_ptr(),
@@ -179,7 +182,7 @@ def forward(rs, means3D, opacities, shs, colors_precomp, scales, rotations, cov3
         native.check(lib.cfgs_composite_forward(C.byref(s), N, geom.data_ptr(), image.data_ptr(), binning.data_ptr(),
                                                 K, color.data_ptr(), depth.data_ptr(), alpha.data_ptr(), st),
                      "cfgs_composite_forward")
-    return color, radii, depth, alpha, ForwardState(geom, image, binning, K, radii)
+    return color, radii, depth, alpha, ForwardState(geom, image, binning, K, radii, touching)
 
 
 def backward(rs, state: ForwardState, means3D, opacities, shs, colors_precomp, scales, rotations,

@@ -126,7 +126,7 @@ extern "C" int cfgs_batch_init(const CfgsBatchArgs* a, void* stream) {
 extern "C" int cfgs_batch_iteration(const CfgsBatchArgs* a, void* stream) {
   if (!args_ok(a)) return CFGS_ERR_INVALID_ARGUMENT;
   CfgsRenderSchedule sched;
-  if (!resolve_schedule(a->schedule, a->num_tiles, a->gauss_slots, a->capacity, &sched)) return CFGS_ERR_INVALID_ARGUMENT;
+  if (!resolve_schedule(a->schedule, a->num_tiles, 0, 0, &sched)) return CFGS_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   BatchViews v = views(a);
   if (!clear_counts(v.iv, a->num_tiles, st)) return CFGS_ERR_LAUNCH;

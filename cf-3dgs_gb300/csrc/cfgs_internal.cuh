@@ -336,7 +336,8 @@ constexpr size_t kGridBarrierOffset = 128;  // bytes into the image workspace
 // The instance count while the preprocess blocks add to it, in the same header.
 struct CountSum {
   unsigned long long total;
-  unsigned int done;  // blocks that have added theirs
+  unsigned int done;      // blocks that have added theirs
+  unsigned int touching;  // Gaussians that touch a tile
 };
 constexpr size_t kCountSumOffset = 64;
 static_assert(sizeof(CfgsCounts) <= kCountSumOffset && kCountSumOffset + 8 + sizeof(CountSum) <= kGridBarrierOffset,

@@ -129,9 +129,9 @@ template <class Scenes>
 void launch_render_bwd(const RenderBwdArgs<Scenes>& a, int tiles, cudaStream_t st);
 template <class Scenes>
 void launch_preprocess_bwd(const PreBwdArgs<Scenes>& a, int blocks, cudaStream_t st);
-// The schedule a call over `tiles` tiles (0: unknown), with room for `capacity` instances of
-// `gaussians` Gaussians, uses: zeros become the default for those sizes; false when the
-// combination is not one the render kernels are instantiated for.
+// The schedule a call over `tiles` tiles (0: unknown), with `capacity` instances of `gaussians`
+// Gaussians that touch a tile (0: unknown), uses: zeros become the default for those sizes;
+// false when the combination is not one the render kernels are instantiated for.
 bool resolve_schedule(const CfgsRenderSchedule& in, int64_t tiles, int64_t gaussians, int64_t capacity,
                       CfgsRenderSchedule* out);
 

@@ -185,9 +185,10 @@ __device__ __forceinline__ uint32_t block_reduce_sum_u32(uint32_t v, uint32_t* s
 }
 
 // Writes the instance count K and the flags (all raised by now); with `host` (page-locked
-// host memory) also there, followed by the ticket the host waits for.
-__device__ __forceinline__ void publish_counts(CfgsCounts* counts, unsigned long long K, volatile uint32_t* host,
-                                               uint32_t ticket) {
+// host memory) also there, with the number of Gaussians that touch a tile, followed by the
+// ticket the host waits for.
+__device__ __forceinline__ void publish_counts(CfgsCounts* counts, unsigned long long K, uint32_t touching,
+                                               volatile uint32_t* host, uint32_t ticket) {
   const uint32_t rendered = K > 0xffffffffull ? 0xffffffffu : (uint32_t)K;
   const uint32_t flags = *(volatile uint32_t*)&counts->flags | (K > 0x7fffffffull ? CFGS_FLAG_CAPACITY_OVERFLOW : 0u);
   counts->num_rendered = rendered;
@@ -195,6 +196,7 @@ __device__ __forceinline__ void publish_counts(CfgsCounts* counts, unsigned long
   if (host) {
     host[0] = rendered;
     host[1] = flags;
+    host[3] = touching;
     __threadfence_system();
     host[2] = ticket;
   }
@@ -302,15 +304,18 @@ __global__ void __launch_bounds__(kPreprocessBlock, Scenes::kBatched ? 6 : 5) k_
     if (!valid) a.radii[idx] = 0;
   }
   const uint32_t bs = block_reduce_sum_u32(touched, sh_warp);
+  const int touching = __syncthreads_count(touched != 0);
   if (threadIdx.x == 0) {
     // The last block to finish publishes the sum, which the host waits for to size the
     // instance list (16,384 Gaussians: 7.0 us and a launch of 5.6 for the sum -> 11.3 us).
     CountSum* cs = count_sum(a.counts);
     atomicAdd(&cs->total, (unsigned long long)bs);
+    if (touching) atomicAdd(&cs->touching, (unsigned int)touching);
     __threadfence();
     if (atomicAdd(&cs->done, 1u) == gridDim.x - 1) {
       __threadfence();
-      publish_counts(a.counts, *(volatile unsigned long long*)&cs->total, a.host, a.ticket);
+      publish_counts(a.counts, *(volatile unsigned long long*)&cs->total, *(volatile unsigned int*)&cs->touching, a.host,
+                     a.ticket);
     }
   }
 }
@@ -324,7 +329,7 @@ template void launch_preprocess<SceneTable>(const PreArgs<SceneTable>&, int, cud
 
 // The counts of a forward without Gaussians.
 __global__ void k_publish_empty(CfgsCounts* counts, volatile uint32_t* host, uint32_t ticket) {
-  publish_counts(counts, 0, host, ticket);
+  publish_counts(counts, 0, 0u, host, ticket);
 }
 
 __global__ void __launch_bounds__(256) k_mark_visible(int n, const float* means, const float* V,
@@ -444,12 +449,35 @@ extern "C" int cfgs_wait_counts(const uint32_t* host_slot, uint32_t ticket, Cfgs
   }
 }
 
+extern "C" int cfgs_wait_sizes(const uint32_t* host_slot, uint32_t ticket, CfgsCounts* out, CfgsSettings* s,
+                               void* stream) {
+  if (!settings_ok(s)) return CFGS_ERR_INVALID_ARGUMENT;
+  const int status = cfgs_wait_counts(host_slot, ticket, out, stream);
+  if (status != CFGS_OK) return status;
+  CfgsRenderSchedule r;
+  if (!resolve_schedule(s->schedule, ImageLayout(s->image_width, s->image_height).num_tiles, host_slot[3],
+                        out->num_rendered, &r))
+    return CFGS_ERR_INVALID_ARGUMENT;
+  s->schedule = r;
+  return CFGS_OK;
+}
+
 extern "C" int cfgs_read_counts(const void* image, CfgsCounts* out, void* stream) {
   if (!image || !out) return CFGS_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   if (cudaMemcpyAsync(out, image, sizeof(CfgsCounts), cudaMemcpyDeviceToHost, st) != cudaSuccess)
     return CFGS_ERR_LAUNCH;
   if (cudaStreamSynchronize(st) != cudaSuccess) return CFGS_ERR_LAUNCH;
+  return CFGS_OK;
+}
+
+extern "C" int cfgs_read_touching(const void* image, uint32_t* out, void* stream) {
+  if (!image || !out) return CFGS_ERR_INVALID_ARGUMENT;
+  cudaStream_t st = (cudaStream_t)stream;
+  const CountSum* cs = count_sum(static_cast<CfgsCounts*>(const_cast<void*>(image)));
+  if (cudaMemcpyAsync(out, &cs->touching, sizeof(*out), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+      cudaStreamSynchronize(st) != cudaSuccess)
+    return CFGS_ERR_LAUNCH;
   return CFGS_OK;
 }
 

@@ -566,7 +566,7 @@ static int render_backward(const CfgsSettings* s, int32_t num_gaussians, const v
   ra.written = reinterpret_cast<uint8_t*>(static_cast<char*>(scratch) + SL.written);
   ra.cap = capacity;
   ra.counts = iv.counts;
-  if (!resolve_schedule(s->schedule, IL.num_tiles, num_gaussians, capacity, &ra.sched)) return CFGS_ERR_INVALID_ARGUMENT;
+  if (!resolve_schedule(s->schedule, IL.num_tiles, 0, 0, &ra.sched)) return CFGS_ERR_INVALID_ARGUMENT;
   ra.geom_only = means_only;
   if (capacity > 0 && cudaMemsetAsync(ra.written, 0, (size_t)capacity, st) != cudaSuccess) return CFGS_ERR_LAUNCH;
   launch_render_bwd(ra, IL.num_tiles, st);

@@ -264,10 +264,15 @@ template void launch_render_fwd<SceneTable>(const RenderArgs<SceneTable>&, int, 
 // The default shape. Eight warps of one pixel per lane issue more instructions per pixel
 // than four of two, but their 8x4 boxes keep fewer instances, and a warp's chain is
 // shorter. They win with at most two tiles per SM, where a tile's longest warp sets the
-// time (256 tiles: 58 against 74 us), and with small Gaussians, which reach fewer than four
-// tiles each (one 640x360 pose solve, 2.1 tiles each: 108 against 121 us; 16 solves: 1455
-// against 1535 us). With larger ones four win (1M at 1920x1080, 12.4 tiles each: 517 against
-// 649 us; 250,007 at 977x545, 4.5 each: 204 against 216 us).
+// time (256 tiles: 58 against 74 us; 304: 63 against 78), and go on winning for some way above
+// (1024 tiles with 5 instances per Gaussian 78 against 88; with 11 from 480 tiles on the
+// four). And they win with small Gaussians, which reach fewer than four tiles each (one
+// 640x360 pose solve, 2.1 tiles each: 108 against 121 us; 16 solves: 1455 against 1535 us; 1024
+// tiles, 3.2 each: 67 against 78, but at 1600 tiles 98 against 86). With larger ones four win
+// (1M at 1920x1080, 12.4 tiles each: 517 against 649 us; 250,007 at 977x545, 4.5 each: 204 against
+// 216 us). `gaussians` are those that touch a tile: 3M of which 95 % are culled have 0.6
+// instances each and 12 each of the others (207 us with four warps, 250 with eight). Calls that
+// know only how many were given pass 0 and take four.
 constexpr int64_t kFewTiles = 2 * 152;
 constexpr int64_t kSmallTouch = 4;
 
@@ -334,7 +339,7 @@ extern "C" int cfgs_composite_forward(const CfgsSettings* s, int32_t num_gaussia
   ra.out_alpha = out_alpha;
   ra.cap = capacity;
   ra.counts = iv.counts;
-  if (!resolve_schedule(s->schedule, IL.num_tiles, num_gaussians, capacity, &ra.sched)) return CFGS_ERR_INVALID_ARGUMENT;
+  if (!resolve_schedule(s->schedule, IL.num_tiles, 0, 0, &ra.sched)) return CFGS_ERR_INVALID_ARGUMENT;
   launch_render_fwd(ra, IL.num_tiles, st);
   CFGS_CHECK_LAUNCH(s->debug, st);
   return CFGS_OK;

@@ -70,8 +70,9 @@ typedef enum CfgsStatus {
  *              persistent cooperative launch with a bounded grid-wide wait between
  *              stages (same outputs)
  * All-zero first three fields mean the library's choice for the call's sizes: {256, 8, 64}
- * for a call over at most 304 tiles or with room for fewer than four instances per
- * Gaussian, else {128, 4, 64}. An unsupported combination makes the call return
+ * for a call over at most 304 tiles, else {128, 4, 64}. A caller that knows how many Gaussians
+ * touch a tile gets a better one from cfgs_render_schedule_for: {256, 8, 64} also for fewer
+ * than four instances each. An unsupported combination makes the call return
  * CFGS_ERR_INVALID_ARGUMENT. */
 typedef struct CfgsRenderSchedule {
   int32_t fwd_batch, fwd_warps, bwd_batch, bin_launch;
@@ -81,9 +82,9 @@ typedef struct CfgsRenderSchedule {
  * CFGS_ERR_INVALID_ARGUMENT; `resolved` (may be NULL) receives it with zeros replaced by the
  * choice for a call of many tiles and large Gaussians. */
 int cfgs_render_schedule_check(const CfgsRenderSchedule* schedule, CfgsRenderSchedule* resolved);
-/* The same for given sizes: `resolved` receives the schedule a call uses over num_tiles tiles
- * (of all images of a batch; 0: unknown) with room for `capacity` instances of num_gaussians
- * Gaussians (a batch's slots). */
+/* The same for given sizes: `resolved` receives the library's choice (or `schedule` itself
+ * where it is none) for a call over num_tiles tiles (of all images of a batch; 0: unknown)
+ * with `capacity` instances of num_gaussians Gaussians that touch a tile (0: unknown). */
 int cfgs_render_schedule_for(const CfgsRenderSchedule* schedule, int64_t num_tiles, int64_t num_gaussians,
                              int64_t capacity, CfgsRenderSchedule* resolved);
 
@@ -184,17 +185,23 @@ int cfgs_preprocess_forward(const CfgsSettings* settings, const CfgsGaussians* g
 /* Copies the CfgsCounts of an image workspace to host memory and synchronises
  * `stream`. (Upstream reads num_rendered back the same way.) */
 int cfgs_read_counts(const void* image, CfgsCounts* counts_host, void* stream);
+/* The number of Gaussians that touch a tile, of the same preprocess, the same way. */
+int cfgs_read_touching(const void* image, uint32_t* gaussians_host, void* stream);
 
 /* cfgs_preprocess_forward whose counts also reach the host on their own, without a copy or
  * an event: the count kernel writes them to `host_slot` (four page-locked uint32, zero at
- * first; one call at a time per slot, until cfgs_wait_counts has returned) and then the
- * ticket returned in *ticket (never zero, no two calls' the same for 2^32 calls).
+ * first; one call at a time per slot, until cfgs_wait_counts has returned, when the fourth
+ * holds what cfgs_read_touching returns) and then the ticket returned in *ticket (never
+ * zero, no two calls' the same for 2^32 calls).
  * cfgs_wait_counts returns them once they are there (it reads the slot; it does not
  * synchronise `stream`, so work enqueued in between keeps running), or CFGS_ERR_LAUNCH when
- * the stream has failed or finished without them. */
+ * the stream has failed or finished without them. cfgs_wait_sizes also replaces the zeros of
+ * settings->schedule by the library's choice for these sizes (cfgs_render_schedule_for). */
 int cfgs_preprocess_counted(const CfgsSettings* settings, const CfgsGaussians* gaussians, void* geom, void* image,
                             int32_t* radii, uint32_t* host_slot, uint32_t* ticket, void* stream);
 int cfgs_wait_counts(const uint32_t* host_slot, uint32_t ticket, CfgsCounts* counts_host, void* stream);
+int cfgs_wait_sizes(const uint32_t* host_slot, uint32_t ticket, CfgsCounts* counts_host, CfgsSettings* settings,
+                    void* stream);
 
 /* ---- rasteriser forward, phase 2 ---------------------------------------------
  * Replaces duplicateWithKeys / SortPairs / identifyTileRanges / render: sorts the
