@@ -25,7 +25,7 @@ struct StagedInstance {
   float4 co;   // (cc, cc, opacity, opacity)
 };
 
-// Front-to-back state of a lane's two pixels (.x: column c, .y: column c + 4) and one
+// Front-to-back state of a lane's two pixels (.x: row r, .y: row r + 4) and one
 // compositing step of both: the published loop body per pixel, with the exponential
 // skipped below the alpha threshold (exact, see alpha_threshold). The arithmetic runs on
 // packed pairs (bit-identical to the scalar operations); each pixel's decisions are its
@@ -105,16 +105,18 @@ __device__ __forceinline__ void composite_one(OneFwd& p, float px, float py, con
 }
 
 // Warp boxes and pixels of a lane: with 4 warps, warp w covers the 8x8 pixel box
-// (8 (w & 1), 8 (w >> 1)) and each lane two pixels of a row, columns c and c + 4; with 8
-// warps, warp w covers the 8x4 box (8 (w & 1), 4 (w >> 1)) and each lane one pixel.
+// (8 (w & 1), 8 (w >> 1)) and each lane two pixels of a column, rows r and r + 4, so that
+// the stores fill whole 32-byte sectors (with columns c and c + 4 they do not: 1000 Gaussians at
+// 1920x1080 31 us against 20, 300,000 at 3840x2160 378 against 365); with 8 warps, warp w
+// covers the 8x4 box (8 (w & 1), 4 (w >> 1)) and each lane one pixel.
 template <bool DEPTH, bool ODD>
 struct PairPixels {
   PairFwd p;
   float2 px, py;
   __device__ __forceinline__ PairPixels(int x, int y, bool in0, bool in1)
       : p{splat2(1.0f), splat2(0.0f), splat2(0.0f), splat2(0.0f), splat2(0.0f), 0u, 0u, !in0, !in1},
-        px(make_float2((float)x, (float)(x + 4))),
-        py(splat2((float)y)) {}
+        px(splat2((float)x)),
+        py(make_float2((float)y, (float)(y + 4))) {}
   __device__ __forceinline__ bool done() const { return p.done0 && p.done1; }
   __device__ __forceinline__ void step(const StagedInstance& s, float thr, const float4* rgbd, int j, uint32_t pos1) {
     composite_pair<DEPTH, ODD>(p, px, py, s, thr, rgbd, j, pos1);
@@ -157,12 +159,11 @@ __device__ __forceinline__ void composite_tile(const RenderArgs<Scenes>& a, FwdS
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int bx0 = (lt % sd.grid_x) * kTileX + (warp & 1) * 8;
   const int by0 = (lt / sd.grid_x) * kTileY + (warp >> 1) * kBoxRows;
-  const int px0 = bx0 + (WARPS == 4 ? lane & 3 : lane & 7);
-  const int py = by0 + (WARPS == 4 ? lane >> 2 : lane >> 3);
+  const int px = bx0 + (lane & 7), py0 = by0 + (lane >> 3);
   const float bxf0 = (float)bx0, bxf1 = (float)(bx0 + 7), byf0 = (float)by0, byf1 = (float)(by0 + kBoxRows - 1);
   const uint32_t lo = a.tile_range[tile];
   const int n = (int)(a.tile_range[tile + 1] - lo);
-  Pixels pixels(px0, py, px0 < sd.W && py < sd.H, px0 + 4 < sd.W && py < sd.H);
+  Pixels pixels(px, py0, px < sd.W && py0 < sd.H, px < sd.W && py0 + 4 < sd.H);
   for (int base = 0; base < n; base += BATCH) {
     if (__syncthreads_count(pixels.done()) == kThreads) break;
 #pragma unroll
@@ -208,7 +209,7 @@ __device__ __forceinline__ void composite_tile(const RenderArgs<Scenes>& a, FwdS
   float* col = a.out_color + 3 * (size_t)sd.pix_base;
 #pragma unroll
   for (int q = 0; q < kPixels; ++q) {
-    const int px = px0 + 4 * q;
+    const int py = py0 + 4 * q;
     if (px >= sd.W || py >= sd.H) continue;
     const OneFwd p = pixels.pixel(q);
     const size_t pix = (size_t)py * sd.W + px;
