@@ -326,6 +326,7 @@ __global__ void __launch_bounds__(kBwdThreads, BLOCKS) k_render_bwd(RenderBwdArg
   using Sh = BwdShared<DEPTH, BATCH, GEOM>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Sh& sh = *reinterpret_cast<Sh*>(smem_raw);
+  const bool odd_view = *nonfinite_word(a.counts) != 0;  // on its way with the count and the pixels
   if ((int64_t)a.counts->num_rendered > a.cap) return;
   const int tile = blockIdx.x;
   const SceneDesc& sd = a.scenes.for_tile(tile);
@@ -352,7 +353,7 @@ __global__ void __launch_bounds__(kBwdThreads, BLOCKS) k_render_bwd(RenderBwdArg
   }
   if (threadIdx.x == 0) sh.max_last = 0;
   // a tile with an image gradient, or a view with a colour or depth, that is not finite
-  const bool odd = __syncthreads_or(!(all_finite(p0) && all_finite(p1))) || *nonfinite_word(a.counts);
+  const bool odd = __syncthreads_or(odd_view || !(all_finite(p0) && all_finite(p1)));
   const uint32_t my_last = max(p0.last, p1.last);
   if (my_last) atomicMax(&sh.max_last, my_last);
   // instances at or past the warp's largest contributor count reach none of its pixels
