@@ -17,8 +17,6 @@
 // 1,000,000 Gaussians, 12.4 million instances: 284 -> 230 us (record sums alone 154, the rest
 // alone 115; DRAM floor 103). Slower: three or four records at a time 240, 251 (registers),
 // the whole warp on one large Gaussian 246, 102 or 64 registers 243, 278.
-#include <type_traits>
-
 #include "cfgs_internal.cuh"
 #include "kernels.cuh"
 
@@ -49,16 +47,6 @@ __device__ __forceinline__ void group8_sum16(float (&v)[16], int lane) {
     const float keep = up ? v[k + 2] : v[k];
     v[k] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
   }
-}
-
-// Marks of eight slots, 8 apart from slot `slot` on (at instance i) below nt.
-template <class Args>
-__device__ __forceinline__ uint32_t marks_of(const Args& a, uint32_t i, uint32_t slot, uint32_t nt) {
-  uint32_t m = 0;
-#pragma unroll
-  for (int j = 0; j < 8; ++j)
-    if (slot + 8 * j < nt && __ldg(a.written + i + 8 * j)) m |= 1u << j;
-  return m;
 }
 
 enum BwdForm { kFullForm, kMeansForm, kPoseForm };
@@ -396,11 +384,11 @@ __device__ __forceinline__ void zero_gradients(const PreBwdArgs<Scenes>& a, int6
 }
 
 constexpr int kBwdThreads = 128;  // full form
-// A warp with a Gaussian of more tiles than this keeps four records and the next marks in
-// flight instead of two records and the next Gaussians' first ones, since that one
-// Gaussian's chain is what is left when the others are done: 300,000 Gaussians, eight of them
-// over all 8160 tiles, 538 -> 423 us, 100 such 1996 -> 1493. Not every warp: 1,000,000
-// Gaussians 245 us with the line here, 255 and 274 with it at 512 and 256.
+// A Gaussian of more tiles is summed by its whole warp after the others: eight lanes read its
+// records in a chain that is left when all other warps are done (300,000 Gaussians, eight of
+// them over all 8160 tiles of 1920x1080: 321 -> 139 us, in one warp 530 -> 390; 100 such alone
+// 1990 -> 1470; without them 116 -> 104, 1,000,000 244 -> 247, 3,000,000 half of them culled
+// 599 -> 633). The line at 2048 or 4096 tiles changes none of the latter.
 constexpr uint32_t kLongTiles = 1024;
 
 // One record's ten values; zeros when it was not written.
@@ -419,6 +407,11 @@ __device__ __forceinline__ Record load_record(const float4* records, uint32_t i,
     r.r2 = *reinterpret_cast<const float2*>(rec + 2);
   }
   return r;
+}
+__device__ __forceinline__ Record shuffled(const Record& r, int src) {
+  auto get = [&](float x) { return __shfl_sync(0xffffffffu, x, src); };
+  return {make_float4(get(r.r0.x), get(r.r0.y), get(r.r0.z), get(r.r0.w)),
+          make_float4(get(r.r1.x), get(r.r1.y), get(r.r1.z), get(r.r1.w)), make_float2(get(r.r2.x), get(r.r2.y))};
 }
 __device__ __forceinline__ void add_record(float (&v)[16], const Record& r) {
   v[0] += r.r0.x; v[1] += r.r0.y; v[2] += r.r0.z; v[3] += r.r0.w;
@@ -439,7 +432,7 @@ template <class Scenes, BwdForm FORM>
 __global__ void __launch_bounds__(FORM == kPoseForm ? 256 : kBwdThreads, FORM == kPoseForm ? 4 : FORM == kMeansForm ? 8 : 6)
     k_preprocess_bwd(PreBwdArgs<Scenes> a) {
   constexpr bool POSE = FORM == kPoseForm;  // a.pose_partials is set exactly for this form
-  constexpr int kDeepRecords = 4;
+  constexpr bool kPrefetch = FORM == kFullForm;
   constexpr int kThreads = POSE ? 256 : kBwdThreads, kWarps = kThreads / 32;
   extern __shared__ __align__(128) float4 s_sh[];  // [kThreads][12] with sh_bulk
   __shared__ float s_acc[kThreads][11];
@@ -477,9 +470,9 @@ __global__ void __launch_bounds__(FORM == kPoseForm ? 256 : kBwdThreads, FORM ==
     off_l = a.geom.offset[idx];  // not set, and not used, for a Gaussian that touches no tile
     if (radius <= 0) nt_l = 0;
   }
-  auto sum_records = [&](auto deep_form) {
-    constexpr bool DEEP = decltype(deep_form)::value, kPrefetch = FORM == kFullForm && !DEEP;
+  {
     const int sub = lane & 7, grp = lane >> 3;
+    const uint32_t nt_short = POSE || nt_l <= kLongTiles ? nt_l : 0u;
     // The written marks of this lane's first two instance slots (sub, sub + 8) of all
     // eight rounds first: sixteen independent byte loads in flight together, so each
     // round below waits for its records only.
@@ -487,7 +480,7 @@ __global__ void __launch_bounds__(FORM == kPoseForm ? 256 : kBwdThreads, FORM ==
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int src = 4 * q + grp;
-      const uint32_t nt = __shfl_sync(0xffffffffu, nt_l, src);
+      const uint32_t nt = __shfl_sync(0xffffffffu, nt_short, src);
       const uint32_t off = __shfl_sync(0xffffffffu, off_l, src);
       if ((uint32_t)sub < nt && __ldg(a.written + off + sub)) marks |= 1u << (2 * q);
       if ((uint32_t)sub + 8 < nt && __ldg(a.written + off + sub + 8)) marks |= 2u << (2 * q);
@@ -504,7 +497,7 @@ __global__ void __launch_bounds__(FORM == kPoseForm ? 256 : kBwdThreads, FORM ==
 #pragma unroll 2
     for (int q = 0; q < 8; ++q) {
       const int src = 4 * q + grp;
-      const uint32_t nt = __shfl_sync(0xffffffffu, nt_l, src);
+      const uint32_t nt = __shfl_sync(0xffffffffu, nt_short, src);
       const uint32_t off = __shfl_sync(0xffffffffu, off_l, src);
       if (!kPrefetch) load_round(q);
       float v[16];
@@ -513,27 +506,10 @@ __global__ void __launch_bounds__(FORM == kPoseForm ? 256 : kBwdThreads, FORM ==
       // slots r = sub, sub + 8, sub + 16, ... in order; unwritten slots are exact zeros
       add_record(v, n0);
       add_record(v, n1);
-      if constexpr (DEEP) {
-        uint32_t m = marks_of(a, off + sub + 16, sub + 16, nt);
-        for (uint32_t first = sub + 16; first < nt; first += 64) {
-          const uint32_t ahead = marks_of(a, off + first + 64, first + 64, nt);
-          while (m) {
-            Record t[kDeepRecords];
-#pragma unroll
-            for (int u = 0; u < kDeepRecords; ++u) {
-              t[u] = load_record(a.records, off + first + 8 * (__ffs(m) - 1), m != 0);
-              m &= m - 1;
-            }
-#pragma unroll
-            for (int u = 0; u < kDeepRecords; ++u) add_record(v, t[u]);
-          }
-          m = ahead;
-        }
-      }
       if (kPrefetch && q < 7) load_round(q + 1);
       // The rest 64 slots at a time: eight marks per lane in flight together, then the written
       // records two at a time.
-      for (uint32_t first = sub + 16; !DEEP && first < nt; first += 64) {
+      for (uint32_t first = sub + 16; first < nt; first += 64) {
         uint32_t m = 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -555,9 +531,41 @@ __global__ void __launch_bounds__(FORM == kPoseForm ? 256 : kBwdThreads, FORM ==
         s_acc[warp * 32 + src][2 * sub + 1] = v[1];
       }
     }
-  };
-  if (FORM != kPoseForm && __any_sync(0xffffffffu, nt_l > kLongTiles)) sum_records(std::true_type{});
-  else sum_records(std::false_type{});
+    // The long ones, kAhead records per lane and the next marks in flight. Lane 8 j + sub loads
+    // what the lanes sub add as the j-th of 32 slots, so that the order is the same.
+    if (!POSE) {
+      constexpr int kAhead = FORM == kFullForm ? 3 : 4;
+      __syncwarp();
+      for (unsigned longs = __ballot_sync(0xffffffffu, nt_l > kLongTiles); longs; longs &= longs - 1) {
+        const int src = __ffs(longs) - 1;
+        const uint32_t nt = __shfl_sync(0xffffffffu, nt_l, src);
+        const uint32_t off = __shfl_sync(0xffffffffu, off_l, src);
+        auto mark = [&](uint32_t slot) { return slot < nt && __ldg(a.written + off + slot); };
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = 0.f;
+        bool m[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) m[u] = mark(lane + 32 * u);
+        for (uint32_t first = 0; first < nt; first += 32 * kAhead) {
+          Record t[kAhead];
+#pragma unroll
+          for (int u = 0; u < kAhead; ++u) t[u] = load_record(a.records, off + first + lane + 32 * u, m[u]);
+#pragma unroll
+          for (int u = 0; u < kAhead; ++u) m[u] = mark(first + lane + 32 * (kAhead + u));
+#pragma unroll
+          for (int u = 0; u < kAhead; ++u)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) add_record(v, shuffled(t[u], 8 * j + sub));
+        }
+        group8_sum16(v, lane);
+        if (lane < 5) {
+          s_acc[warp * 32 + src][2 * sub] = v[0];
+          s_acc[warp * 32 + src][2 * sub + 1] = v[1];
+        }
+      }
+    }
+  }
   __syncwarp();
 
   // ---- phase 2: one thread per Gaussian ----------------------------------------------

@@ -1,6 +1,6 @@
-"""Record sums of Gaussians that touch more tiles than the line from which a warp keeps more of
-them in flight: the same bits as the general form, which a Gaussian of a warp without such a
-neighbour takes, and the oracle's gradients within its float32 bound."""
+"""Record sums of Gaussians that touch more tiles than the line from which their whole warp sums
+them: the general form's order, slot by slot per eighth lane and then over the eight, to the
+bit; the oracle's gradients within its float32 bound; the others of the warp unchanged."""
 from __future__ import annotations
 
 import pytest
@@ -53,9 +53,9 @@ def test_long_gaussians_match_the_oracle(big):
 
 
 @pytest.mark.parametrize("means_only", [False, True])
-def test_the_form_does_not_change_the_sums(means_only):
-    """The same Gaussians with a huge, fully transparent one among them, which sends its warp to
-    the other form and adds nothing to any pixel."""
+def test_the_others_keep_their_sums(means_only):
+    """The same Gaussians with a huge, fully transparent one among them, which adds nothing to any
+    pixel."""
     base, sc = _scene([]), _scene([5])
     base.opacities[5] = sc.opacities[5] = 0.0
     want, few, _ = _backward(base, means_only)
@@ -65,3 +65,43 @@ def test_the_form_does_not_change_the_sums(means_only):
     for a, b in zip(got, want):
         if a is not None:
             assert torch.equal(a[keep], b[keep])
+
+
+@pytest.mark.parametrize("big", [[], [5], [5, 40, 69]])
+def test_order_of_the_sums(big):
+    """The opacity and colour gradients are sums of the records alone: formed here in numpy from
+    the records the render backward left."""
+    import ctypes as C
+
+    import diff_gaussian_rasterization as dgr
+    import numpy as np
+    from cfgs import native, raster
+    sc = _scene(big)
+    s = sc.to(DEV)
+    colors = torch.rand(sc.n, 3, generator=torch.Generator().manual_seed(2)).to(DEV)
+    args = (s.means3D, s.opacities, None, colors, s.scales, s.rotations, None)
+    rs = settings_for(dgr, sc)
+    state = raster.forward(rs, *args)[4]
+    gc = torch.randn(3, H, W, generator=torch.Generator().manual_seed(3)).to(DEV) * 1e-4
+    out = raster.backward(rs, state, *args, gc, None, None)
+    lib, keep, K = native.load(), [], state.num_rendered
+    scratch = torch.zeros(lib.cfgs_backward_scratch_bytes(K), dtype=torch.uint8, device=DEV)
+    native.check(lib.cfgs_render_backward(C.byref(raster.make_settings(rs, keep)), sc.n, state.geom.data_ptr(),
+                                          state.image.data_ptr(), state.binning.data_ptr(), K, scratch.data_ptr(),
+                                          gc.data_ptr(), None, None, raster.stream_handle(gc.device)),
+                 "cfgs_render_backward")
+    at = (48 * K + 255) // 256 * 256
+    rec = scratch[: 48 * K].view(torch.float32).reshape(K, 12).cpu().numpy()
+    written = scratch[at: at + K].cpu().numpy().astype(bool)
+    v = raster.inspect_state(state, W, H)
+    touched, offset = v["touched"].cpu().numpy(), v["offset"].cpu().numpy()
+    for g in range(sc.n):
+        r = np.where(written[offset[g]: offset[g] + touched[g], None], rec[offset[g]: offset[g] + touched[g], 5:9], 0)
+        lanes = np.zeros((8, 4), np.float32)
+        for i in range(0, len(r), 8):
+            lanes[: len(r[i:i + 8])] += r[i:i + 8].astype(np.float32)
+        a = lanes[:4] + lanes[4:]
+        b = a[:2] + a[2:]
+        want = b[0] + b[1]
+        got = np.concatenate([out[2][g].cpu().numpy(), out[1][g].cpu().numpy()])
+        np.testing.assert_array_equal(got, want, err_msg=str((g, touched[g])))
