@@ -308,7 +308,7 @@ def run_ours(a) -> None:
     phase_ms = {k: sum(s_.elapsed_time(e_) for s_, e_ in v) / len(v) for k, v in timers.items()}
     D = (sc.sh_degree + 1) ** 2
     T = ((cam.width + 15) // 16) * ((cam.height + 15) // 16)
-    used = autotune.resolved(sched, T, last_state[0].touching, K)
+    used = autotune.resolved(sched, T, raster.touching(last_state[0]), K)
     pb = phase_bytes(sc.n, K, HW, D, T)
     group_ms = {"preprocess": phase_ms["preprocess"], "binning": phase_ms["depth_sort"] + phase_ms["bin"],
                 "composite": phase_ms["composite"], "render_bwd": phase_ms["render_bwd"],

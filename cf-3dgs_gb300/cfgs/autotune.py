@@ -282,7 +282,7 @@ def tune_rasterizer(raster_settings, means3D, opacities, shs=None, colors_precom
         with using(AUTO):
             st = raster.forward(raster_settings, means3D, opacities, shs, colors_precomp, scales, rotations,
                                 cov3D_precomp)[4]
-        own = resolved(AUTO, ((w + 15) // 16) * ((h + 15) // 16), st.touching, st.num_rendered)
+        own = resolved(AUTO, ((w + 15) // 16) * ((h + 15) // 16), raster.touching(st), st.num_rendered)
         sched = tuner.tune(key, run, incumbent=own, unbeaten=AUTO)
     if apply:
         set_schedule(sched)

@@ -91,7 +91,6 @@ class ForwardState:
     binning: torch.Tensor
     num_rendered: int
     radii: torch.Tensor
-    touching: int = 0  # Gaussians that touch a tile
     inputs_only: bool = False  # the backward forms the inputs' gradients only
 
 
@@ -173,7 +172,6 @@ def forward(rs, means3D, opacities, shs, colors_precomp, scales, rotations, cov3
     if counts.flags & native.FLAG_CAPACITY_OVERFLOW:
         raise RuntimeError("more than 2^31 tile instances")
     K = int(counts.num_rendered)
-    touching = C.c_uint32.from_address(slot.data_ptr() + 12).value
     binning = torch.empty(lib.cfgs_binning_bytes(K), dtype=torch.uint8, device=dev)
     with _Timed(timers, "bin"):
         native.check(lib.cfgs_bin_instances(C.byref(s), C.byref(g), geom.data_ptr(), image.data_ptr(),
@@ -182,7 +180,15 @@ def forward(rs, means3D, opacities, shs, colors_precomp, scales, rotations, cov3
         native.check(lib.cfgs_composite_forward(C.byref(s), N, geom.data_ptr(), image.data_ptr(), binning.data_ptr(),
                                                 K, color.data_ptr(), depth.data_ptr(), alpha.data_ptr(), st),
                      "cfgs_composite_forward")
-    return color, radii, depth, alpha, ForwardState(geom, image, binning, K, radii, touching)
+    return color, radii, depth, alpha, ForwardState(geom, image, binning, K, radii)
+
+
+def touching(state: ForwardState) -> int:
+    """The number of Gaussians that touch a tile (synchronises the current stream)."""
+    n = C.c_uint32()
+    native.check(native.load().cfgs_read_touching(state.image.data_ptr(), C.byref(n), stream_handle(state.image.device)),
+                 "cfgs_read_touching")
+    return int(n.value)
 
 
 def backward(rs, state: ForwardState, means3D, opacities, shs, colors_precomp, scales, rotations,

@@ -2,8 +2,6 @@
 the instance count: culled ones are none of a view's small Gaussians."""
 from __future__ import annotations
 
-import ctypes as C
-
 import pytest
 import torch
 
@@ -40,16 +38,13 @@ def test_culled_gaussians_do_not_count(culled, scale, small, monkeypatch):
     args = (settings_for(dgr, sc), s.means3D, s.opacities, s.shs, None, s.scales, s.rotations, None)
     state = raster.forward(*args)[4]
     monkeypatch.undo()
-    touched = raster.inspect_state(state, 640, 480)["touched"]
-    assert state.touching == int((touched > 0).sum()) and (state.touching > 0) == (culled < 1.0)
+    touching = raster.touching(state)
+    assert touching == int((raster.inspect_state(state, 640, 480)["touched"] > 0).sum())
+    assert (touching > 0) == (culled < 1.0)
     if culled < 1.0:
-        assert (state.num_rendered < 4 * state.touching) == small
+        assert (state.num_rendered < 4 * touching) == small
         assert seen == [8 if small else 4]
-        assert seen == [autotune.resolved(None, 1200, state.touching, state.num_rendered).fwd_warps]
-    got = C.c_uint32()
-    native.check(lib.cfgs_read_touching(state.image.data_ptr(), C.byref(got), raster.stream_handle(s.means3D.device)),
-                 "cfgs_read_touching")
-    assert got.value == state.touching
+        assert seen == [autotune.resolved(None, 1200, touching, state.num_rendered).fwd_warps]
     with autotune.using(autotune.Schedule(64, 4, 32)):  # a chosen shape stays
         monkeypatch.setattr(native, "load", lambda: Spy())
         raster.forward(*args)
