@@ -324,8 +324,8 @@ class BatchSolver:
         """Captures graph_chunk iterations into one CUDA graph and replays it; returns
         the number of iterations run."""
         chunk = self.graph_chunk
-        # the first iteration runs outside the capture: the graph's memory must not be
-        # the first use of any buffer (warm-up)
+        # the capture needs a stream of its own; the buffers it names are in use already (the
+        # counting iteration)
         s = torch.cuda.Stream(self.dev)
         s.wait_stream(torch.cuda.current_stream(self.dev))
         g = torch.cuda.CUDAGraph()

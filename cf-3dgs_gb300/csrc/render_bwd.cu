@@ -495,7 +495,10 @@ void launch_render_bwd_blocks(const RenderBwdArgs<Scenes>& a, int tiles, cudaStr
 // registers win (fewer instructions per warp): 256 tiles 94 us at four blocks per SM, 99
 // at five; 920 pose tiles 175 us at six, 187 at seven. With many tiles the extra block
 // does: 8160 tiles 907 us at five, 987 at four; 20,960 pose tiles 2429 us at seven, 2551 at
-// six. The depth form, with more live sums, keeps four (2170 tiles: 313 us, 342 at five).
+// six. Around the lines (608 and 1216 tiles) neither matters much: 625 tiles with 5 instances
+// per Gaussian 119 us at four and at five, 800 tiles 121 and 119, 1024 tiles 136 and 129; pose
+// form 1024 tiles 119 and 121 us at six and seven, 1280 136 and 134, 1600 149 and 147. The
+// depth form, with more live sums, keeps four (2170 tiles: 313 us, 342 at five).
 template <class Scenes, bool DEPTH, int BATCH, bool GEOM>
 void launch_render_bwd_batch(const RenderBwdArgs<Scenes>& a, int tiles, cudaStream_t st) {
   if constexpr (GEOM) {
