@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kVoxelBlock) k_voxel_prefix(int nblocks, uint3
 // block's 512 positions are gathered to shared memory first; a run that goes on into the
 // next block reads the rest from memory, one point ahead, which wants 40 registers and so
 // three blocks of 512 per SM (two of 1024 leave 32). 230,400 points in 161,225 voxels: 62 us
-// with a thread at every run's head -> 28 us. Long runs, whole calls: 20,000 points of which
+// with a thread at every run's head -> 20 us. Long runs, whole calls: 20,000 points of which
 // two thirds share a voxel 5.7 -> 5.5 ms, 230,400 in 8 voxels 14.3 -> 11.6 ms (6.9 and 17.1 with
 // the rest of a run read key by key).
 __global__ void __launch_bounds__(kVoxelBlock, 3) k_voxel_average(int64_t n, const uint32_t* __restrict__ lo,
