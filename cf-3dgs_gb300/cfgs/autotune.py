@@ -36,6 +36,7 @@ from . import native
 
 @dataclass(frozen=True)
 class Schedule:
+    """The fields of CfgsRenderSchedule; zeros in the first three leave them to the library."""
     fwd_batch: int = 128
     fwd_warps: int = 4
     bwd_batch: int = 64
